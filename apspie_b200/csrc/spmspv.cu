@@ -62,7 +62,7 @@ template <typename T>
 __global__ void sv_expand(long long total, int nx, const int *__restrict__ off, const int *__restrict__ x_ind,
                           const unsigned *__restrict__ x_val, const int *__restrict__ row_ptr,
                           const int *__restrict__ col_ind, const unsigned *__restrict__ a_val,
-                          unsigned long long *key, unsigned *idx, unsigned *prod) {
+                          unsigned *key, unsigned *idx, unsigned *prod) {
     for (long long p = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; p < total;
          p += static_cast<long long>(gridDim.x) * blockDim.x) {
         int lo = 0, hi = nx - 1;  // last j with off[j] <= p
@@ -80,18 +80,20 @@ __global__ void sv_expand(long long total, int nx, const int *__restrict__ off, 
     }
 }
 
-__global__ void sv_run_flags(long long n, const unsigned long long *__restrict__ key, int *flag) {
+__global__ void sv_run_flags(long long n, const unsigned *__restrict__ key, int *flag) {
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<long long>(gridDim.x) * blockDim.x)
         flag[i] = (i == 0 || key[i] != key[i - 1]) ? 1 : 0;
 }
 
 template <typename T>
-__global__ void sv_reduce(long long n, const unsigned long long *__restrict__ key, const unsigned *__restrict__ idx,
-                          const unsigned *__restrict__ prod, const int *__restrict__ run, int *y_ind, unsigned *y_val) {
+__global__ void sv_reduce(long long n, const unsigned *__restrict__ key, const unsigned *__restrict__ idx,
+                          const unsigned *__restrict__ prod, const int *__restrict__ run, const int *sort_err,
+                          int *y_ind, unsigned *y_val) {
+    if (ld_volatile_i32(sort_err) != 0) return;  // the keys are not in order: the host reports it
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const unsigned long long k = key[i];
+        const unsigned k = key[i];
         if (i > 0 && key[i - 1] == k) continue;  // not the first of its run
         unsigned acc = 0u;                       // +0.0f and int 0 share the bit pattern
         for (long long t = i; t < n && key[t] == k; ++t) acc = sv_add<T>(acc, __ldg(prod + idx[t]));
@@ -150,8 +152,9 @@ extern "C" apspie_status apspie_spmspv(apspie_ctx *ctx, const apspie_csr *A, con
     const long long total = total_i;
     if (total == 0) return APSPIE_OK;
     // the products, sorted by column (the head buffers move to the front of a larger arena)
-    const size_t need = head + sort_need(total) +
-                        Carver::need({static_cast<size_t>(total) * 4, static_cast<size_t>(total + 1) * 4});
+    const size_t need = head + sort_need<unsigned>(total) +
+                        Carver::need({static_cast<size_t>(total) * 4, static_cast<size_t>(total + 1) * 4,
+                                      scan_scratch_bytes(total) + 64});
     std::vector<int> h_off;
     if (need > ctx->scratch_bytes) {
         // growing the arena drops its contents: keep the offsets on the host meanwhile
@@ -168,10 +171,10 @@ extern "C" apspie_status apspie_spmspv(apspie_ctx *ctx, const apspie_csr *A, con
     if (!h_off.empty() &&
         (e = cudaMemcpyAsync(off, h_off.data(), h_off.size() * 4, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
         return cuda_error(ctx, e, "apspie_spmspv offsets");
-    SortBufs s = carve_sort(c, total);
+    SortBufs<unsigned> s = carve_sort<unsigned>(c, total);
     unsigned *prod = c.take<unsigned>(total);
     int *run = c.take<int>(total + 1);
-    if ((e = cudaMemsetAsync(s.ovf, 0, 64, ctx->stream)) != cudaSuccess) return cuda_error(ctx, e, "apspie_spmspv reset");
+    void *run_tmp = c.take<char>(scan_scratch_bytes(total) + 64);
     const int g = sv_grid(ctx, total);
     const bool f32 = A->val_type == APSPIE_VAL_F32;
     const unsigned *xv = static_cast<const unsigned *>(d_x_val);
@@ -183,22 +186,25 @@ extern "C" apspie_status apspie_spmspv(apspie_ctx *ctx, const apspie_csr *A, con
         sv_expand<int><<<g, 256, 0, ctx->stream>>>(total, x_nnz, off, d_x_ind, xv, A->row_ptr, A->col_ind, av,
                                                     s.k[0], s.v[0], prod);
     int which = 0;
-    if ((st = radix_sort(ctx, s, total, bit_length(A->n), &which)) != APSPIE_OK) return st;
+    if ((st = radix_sort(ctx, s, rs_plan(0, bit_length(A->n)), s.k[0], s.v[0], total, 1, &which)) != APSPIE_OK)
+        return st;
     // run numbers: exclusive scan of run-start flags (held in the sort's spare value buffer)
     int *rflag = reinterpret_cast<int *>(s.v[which ^ 1]);
     sv_run_flags<<<g, 256, 0, ctx->stream>>>(total, s.k[which], rflag);
-    if ((st = device_exclusive_scan(ctx, rflag, total, run, s.scan_tmp, s.ovf)) != APSPIE_OK) return st;
+    if ((st = device_exclusive_scan(ctx, rflag, total, run, run_tmp, flags + 4)) != APSPIE_OK) return st;
     if (f32)
-        sv_reduce<float><<<g, 256, 0, ctx->stream>>>(total, s.k[which], s.v[which], prod, run, d_y_ind,
+        sv_reduce<float><<<g, 256, 0, ctx->stream>>>(total, s.k[which], s.v[which], prod, run, s.err, d_y_ind,
                                                       static_cast<unsigned *>(d_y_val));
     else
-        sv_reduce<int><<<g, 256, 0, ctx->stream>>>(total, s.k[which], s.v[which], prod, run, d_y_ind,
+        sv_reduce<int><<<g, 256, 0, ctx->stream>>>(total, s.k[which], s.v[which], prod, run, s.err, d_y_ind,
                                                     static_cast<unsigned *>(d_y_val));
-    int ny = 0;
+    int ny = 0, sort_err = 0;
     if ((e = cudaGetLastError()) != cudaSuccess ||
         (e = cudaMemcpyAsync(&ny, run + total, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(&sort_err, s.err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
         return cuda_error(ctx, e, "apspie_spmspv");
+    if (sort_err) return set_error(ctx, static_cast<apspie_status>(sort_err), "apspie_spmspv: sort");
     *y_nnz = ny;
     return APSPIE_OK;
 }

@@ -119,3 +119,50 @@ def test_transpose_matches_scipy(ctx, shape):
     np.testing.assert_array_equal(rp2, A.indptr)
     np.testing.assert_array_equal(ci2, A.indices)
     np.testing.assert_array_equal(v2, A.data)
+
+
+@pytest.mark.parametrize("ne", [1, 6143, 6144, 6145, 8191, 8192, 8193, 49153])
+def test_build_at_the_edges_of_sort_and_compaction_tiles(ctx, ne):
+    """Edge counts around the sort's tiles (6,144 pairs) and the compaction's (8,192); half of
+    the edges repeat others, a few are self-loops, and the last vertices have no edges."""
+    rng = np.random.default_rng(ne)
+    m = 70001  # 17 bits an id: two passes of 8 and more of fewer bits
+    src = rng.integers(0, m // 2, ne).astype(np.int32)
+    dst = rng.integers(0, m // 2, ne).astype(np.int32)
+    src[ne // 2:], dst[ne // 2:] = src[: ne - ne // 2], dst[: ne - ne // 2]
+    dst[::17] = src[::17]
+    val = rng.integers(1, 256, ne).astype(np.int32)
+    for flags in (SYM | DROP | DEDUP, SYM | DROP, DROP, 0):
+        got = ctx.build_csr(m, _dev(src), _dev(dst), _dev(val), flags).to_numpy()
+        for a, b in zip(got, _ref_build(m, src, dst, val, flags)):
+            np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("valued", [True, False])
+@pytest.mark.parametrize("lengths", ["one long row", "short rows", "tile ends"])
+def test_transpose_of_uneven_rows(ctx, valued, lengths):
+    """Rows longer than the 4,096-entry tiles in which entries find their rows, runs of empty
+    rows before, between and after them, rows that end at a tile's end; columns in any order
+    and repeated, so that the order of equal columns shows (it is the entries' order)."""
+    n = 333
+    deg = np.zeros(3000, dtype=np.int64)
+    if lengths == "one long row":
+        deg[[700, 701, 2500]] = [9000, 3, 1]
+    elif lengths == "short rows":
+        deg[100:2900] = np.arange(2800) % 7
+    else:
+        deg[[5, 600, 601, 602]] = [4095, 1, 4096, 4096]
+    rp = np.concatenate(([0], np.cumsum(deg))).astype(np.int32)
+    rng = np.random.default_rng(int(deg.sum()))
+    ci = rng.integers(0, n, rp[-1]).astype(np.int32)
+    val = rng.integers(-99, 99, rp[-1]).astype(np.int32) if valued else None
+    T = ctx.transpose(ap.DeviceGraph(ap.HostGraph(3000, n, rp, ci, val)))
+    trp, tci, tval = T.to_numpy()
+    order = np.argsort(ci, kind="stable")
+    rows = np.repeat(np.arange(3000), deg)
+    np.testing.assert_array_equal(trp, np.concatenate(([0], np.cumsum(np.bincount(ci, minlength=n)))))
+    np.testing.assert_array_equal(tci, rows[order])
+    if valued:
+        np.testing.assert_array_equal(tval, val[order])
+    else:
+        assert tval is None
