@@ -333,6 +333,50 @@ apspie_status alloc_owned(apspie_ctx *ctx, int m, int n, long long nnz, int val_
 }
 
 }  // namespace
+
+// A pattern's entries sorted by column, the row as the payload (8 bytes each through a pass);
+// row starts in out_rp. The last pass writes the rows to out_col.
+static apspie_status sort_pattern(apspie_ctx *ctx, const apspie_csr *A, SortBufs<unsigned> &s, unsigned *row_of,
+                                  int *out_rp, int *out_col, const unsigned **keys) {
+    const long long nnz = A->nnz;
+    const int n = A->n, g = grid_for(ctx, nnz);
+    const RsPlan pl = rs_plan(0, bit_length(n));
+    s.v[last_pair(pl.passes)] = reinterpret_cast<unsigned *>(out_col);
+    cudaError_t e = launch_expand_rows<false>(ctx, A, row_of, nullptr);
+    if (e != cudaSuccess) return cuda_error(ctx, e, "transpose rows");
+    int which = 0;
+    apspie_status st =
+        radix_sort(ctx, s, pl, reinterpret_cast<const unsigned *>(A->col_ind), row_of, nnz, 0, &which);
+    if (st != APSPIE_OK) return st;
+    if (nnz > 0) run_starts<unsigned><<<g, 256, 0, ctx->stream>>>(nnz, s.k[which], 0, ~0u, out_rp, s.err);
+    fill_tail<unsigned><<<grid_for(ctx, n + 1LL), 256, 0, ctx->stream>>>(nnz, s.k[which], 0, ~0u, n, out_rp, s.err);
+    *keys = s.k[which];
+    e = cudaGetLastError();
+    return e == cudaSuccess ? APSPIE_OK : cuda_error(ctx, e, "transpose");
+}
+
+size_t transpose_pattern_need(int n, long long nnz) {
+    const size_t c = static_cast<size_t>(nnz) + 1;
+    return sort_need<unsigned>(nnz) + Carver::need({c * 4, c * 4, (static_cast<size_t>(n) + 1) * 4});
+}
+
+apspie_status transpose_pattern(apspie_ctx *ctx, const apspie_csr *A, void *scratch, PatternCoo *out) {
+    Carver c(scratch);
+    SortBufs<unsigned> s = carve_sort<unsigned>(c, A->nnz);
+    unsigned *row_of = c.take<unsigned>(static_cast<size_t>(A->nnz) + 1);
+    int *col = c.take<int>(static_cast<size_t>(A->nnz) + 1);
+    int *rp = c.take<int>(static_cast<size_t>(A->n) + 1);
+    const unsigned *keys = nullptr;
+    apspie_status st = sort_pattern(ctx, A, s, row_of, rp, col, &keys);
+    *out = PatternCoo{rp, keys, col, s.err};
+    return st;
+}
+
+apspie_status expand_entry_rows(apspie_ctx *ctx, const apspie_csr *A, unsigned *row_of) {
+    cudaError_t e = launch_expand_rows<false>(ctx, A, row_of, nullptr);
+    return e == cudaSuccess ? APSPIE_OK : cuda_error(ctx, e, "entry rows");
+}
+
 }  // namespace apspie
 
 using namespace apspie;
@@ -443,10 +487,9 @@ apspie_status apspie_csr_build(apspie_ctx *ctx, int32_t m, int64_t nedges, const
     return APSPIE_OK;
 }
 
-// A pattern's entries sorted by (column, row) need 8 bytes each through a pass, with the row
-// as the payload; entries with values 12, keyed by (column, row) with the value as the
-// payload (an index as the payload, as before, costs two random reads per entry at the end).
-// The last pass writes the payload straight into the output.
+// Entries with values are sorted as (column, row) keys with the value as the payload, 12
+// bytes each through a pass (an index as the payload, as before, costs two random reads per
+// entry at the end); the last pass writes the payload straight into the output.
 apspie_status apspie_csr_transpose(apspie_ctx *ctx, const apspie_csr *A, apspie_csr_owned *out) {
     if (!ctx || !out) return APSPIE_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
@@ -490,17 +533,9 @@ apspie_status apspie_csr_transpose(apspie_ctx *ctx, const apspie_csr *A, apspie_
     } else {
         SortBufs<unsigned> s = carve_sort<unsigned>(c, nnz);
         unsigned *row_of = c.take<unsigned>(nnz + 1);
-        const RsPlan pl = rs_plan(0, bit_length(n));
-        s.v[last_pair(pl.passes)] = reinterpret_cast<unsigned *>(out->col_ind);
+        const unsigned *keys = nullptr;
         err = s.err;
-        e = launch_expand_rows<false>(ctx, A, row_of, nullptr);
-        if (e == cudaSuccess)
-            st = radix_sort(ctx, s, pl, reinterpret_cast<const unsigned *>(A->col_ind), row_of, nnz, 0, &which);
-        if (e == cudaSuccess && st == APSPIE_OK) {
-            if (nnz > 0)
-                run_starts<unsigned><<<g, 256, 0, ctx->stream>>>(nnz, s.k[which], 0, ~0u, out->row_ptr, err);
-            fill_tail<unsigned><<<gn, 256, 0, ctx->stream>>>(nnz, s.k[which], 0, ~0u, n, out->row_ptr, err);
-        }
+        st = sort_pattern(ctx, A, s, row_of, out->row_ptr, out->col_ind, &keys);
     }
     int sort_err = 0;
     if (st == APSPIE_OK &&

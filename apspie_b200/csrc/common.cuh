@@ -184,6 +184,21 @@ int sssp_group_count(const apspie_ctx *ctx, int nq);
 apspie_status sssp_batch_grouped(apspie_ctx *ctx, const apspie_csr *A, const int32_t *d_sources, int32_t nq,
                                  int32_t *d_dists, apspie_run_stats *stats);
 
+// A pattern's entries by row: row[e] and col[e] of entry e, ascending in row, and rp the
+// entries of each row. With *err != 0 on the device (a sort that gave up) the arrays hold
+// nothing of use.
+struct PatternCoo {
+    const int *rp;
+    const unsigned *row;
+    const int *col;
+    const int *err;  // may be null
+};
+// A's transposed pattern, in scratch of transpose_pattern_need(n, nnz) bytes (build.cu).
+size_t transpose_pattern_need(int n, long long nnz);
+apspie_status transpose_pattern(apspie_ctx *ctx, const apspie_csr *A, void *scratch, PatternCoo *out);
+// row_of[e] = the row of A's entry e.
+apspie_status expand_entry_rows(apspie_ctx *ctx, const apspie_csr *A, unsigned *row_of);
+
 // Device-wide exclusive scan (scan.cu): out[0..n) = prefix of in, out[n] = total.
 size_t scan_scratch_bytes(long long n);
 apspie_status device_exclusive_scan(apspie_ctx *ctx, const int *in, long long n, int *out, void *tmp,

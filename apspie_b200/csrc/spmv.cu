@@ -7,8 +7,8 @@
 //     the mean row length: 4, 8, 16 or 32), lane-strided partial sums reduced by shuffles
 //     (fixed order, so repeated calls give identical bits);
 //   * apspie_pagerank: power iteration r' = (1 - d) / n + d * (A^T (r / outdeg) + dangling
-//     mass / n) on the transposed graph (pull: no atomics), stopping when the L1 change is
-//     below tol or after max_iter iterations.
+//     mass / n) on the transposed graph (pull: no atomics on the ranks), stopping when the L1
+//     change is below tol or after max_iter iterations.
 #include <algorithm>
 #include <cstring>
 
@@ -58,33 +58,214 @@ apspie_status launch_spmv(apspie_ctx *ctx, const apspie_csr *A, const float *x, 
     return e == cudaSuccess ? APSPIE_OK : cuda_error(ctx, e, "spmv launch");
 }
 
-// x[u] = r[u] / outdeg(u); dangling mass (outdeg 0) summed into acc[0] (double)
-__global__ void pr_scale(int n, const int *__restrict__ rp, const float *__restrict__ r, float *x, double *acc) {
-    double dang = 0.0;
-    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
-        const int d = __ldg(rp + u + 1) - __ldg(rp + u);
-        x[u] = d > 0 ? r[u] / static_cast<float>(d) : 0.0f;
-        if (d == 0) dang += r[u];
-    }
-    for (int o = 16; o; o >>= 1) dang += __shfl_down_sync(0xffffffffu, dang, o);
-    if ((threadIdx.x & 31) == 0 && dang != 0.0) atomicAdd(acc, dang);
+// ---- PageRank -----------------------------------------------------------------------
+// An iteration is two launches: pr_gather sums x over every row's in-edges, pr_update turns
+// the sums into new ranks, their L1 change, the next x and the next dangling mass. Whether
+// to stop is decided on the device; the host looks every kPrBatch iterations (launches
+// enqueued past the end return at once).
+//
+// pr_gather cuts the entries, not the rows, into equal chunks: a thread takes 8 consecutive
+// entries (two 128-bit loads), sums the pieces of rows in them, and a segmented scan joins
+// pieces across threads. A chunk writes the sums of the rows that begin in it; what it holds
+// of a row that began earlier goes to carry[], which pr_update adds in chunk order, so
+// repeated calls give the same bits. Bound: 4 bytes an entry from HBM plus one gather from
+// L2. Measured, R-MAT of 700,001 vertices and 10.7M entries, per iteration: 16 lanes per
+// row 228 us (the row of 55,000 entries is the last to finish) + 34 us for the two vector
+// kernels, whose warps all added doubles to one word; now see pr_update.
+constexpr int kPrBlock = 256;
+constexpr int kPrItems = 8;
+constexpr int kPrChunk = kPrBlock * kPrItems;
+constexpr int kPrVec = 1024;  // threads a block in the vector kernels: two blocks an SM, one atomic each
+constexpr int kPrBatch = 4;
+
+struct PrState {
+    double dang[2];  // rank mass of the vertices without out-edges, by iteration parity
+    double diff[2];  // L1 change, by iteration parity
+    int done;        // iterations after which the change was below tol (0: not yet)
+    int pad;
+};
+
+__device__ __forceinline__ double block_sum(double v, double *tmp) {
+    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) tmp[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < static_cast<int>(blockDim.x) / 32; ++w) s += tmp[w];
+    __syncthreads();
+    return s;  // thread 0's
 }
 
-// r'[v] = (1 - d) / n + d * (y[v] + dangling / n); acc[1] += |r'[v] - r[v]|
-__global__ void pr_update(int n, float damping, const float *__restrict__ y, float *r, double *acc) {
-    const float base = static_cast<float>((1.0 - damping) / n + damping * acc[0] / n);
-    double diff = 0.0;
+// heads[b] bit j: entry 8 b + j is the first of its row
+__global__ void pr_heads(long long nnz, const unsigned *__restrict__ row, unsigned char *heads) {
+    const long long nb = (nnz + 7) / 8;
+    for (long long b = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; b < nb;
+         b += static_cast<long long>(gridDim.x) * blockDim.x) {
+        unsigned m = 0u;
+        unsigned prev = b > 0 ? __ldg(row + 8 * b - 1) : 0u;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const long long e = 8 * b + j;
+            if (e < nnz) {
+                const unsigned r = __ldg(row + e);
+                if (e == 0 || r != prev) m |= 1u << j;
+                prev = r;
+            }
+        }
+        heads[b] = static_cast<unsigned char>(m);
+    }
+}
+
+// r = 1 / n, x[u] = r[u] / outdeg(u), dang[0] = the mass of vertices without out-edges
+__global__ void __launch_bounds__(kPrVec) pr_init(int n, const int *__restrict__ out_rp, float *r, float *x,
+                                                    PrState *st) {
+    __shared__ double tmp[kPrVec / 32];
+    const float r0 = 1.0f / n;
+    double dang = 0.0;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const float nr = __fmaf_rn(damping, y[v], base);
+        const int d = __ldg(out_rp + v + 1) - __ldg(out_rp + v);
+        r[v] = r0;
+        x[v] = d > 0 ? r0 / static_cast<float>(d) : 0.0f;
+        if (d == 0) dang += r0;
+    }
+    dang = block_sum(dang, tmp);
+    if (threadIdx.x == 0 && dang != 0.0) atomicAdd(&st->dang[0], dang);
+}
+
+// VEC: col is 16-byte aligned
+template <bool VEC>
+__global__ void __launch_bounds__(kPrBlock) pr_gather(long long nnz, const int *__restrict__ col,
+                                                      const unsigned char *__restrict__ heads,
+                                                      const unsigned *__restrict__ row, const float *__restrict__ x,
+                                                      float *y, float *carry, PrState *st, int it, double tol,
+                                                      const int *err) {
+    __shared__ float s_val[kPrBlock / 32];
+    __shared__ int s_any[kPrBlock / 32];
+    if (err && ld_volatile_i32(err) != 0) return;
+    if (ld_volatile_i32(&st->done) != 0) return;
+    if (it > 0 && st->diff[(it - 1) & 1] < tol) {  // every block sees the same: the last launch wrote it
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->done = it;
+        return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // read by the last launch, added to by the next
+        st->dang[(it + 1) & 1] = 0.0;
+        st->diff[it & 1] = 0.0;
+    }
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const long long c0 = static_cast<long long>(blockIdx.x) * kPrChunk;
+    if (c0 >= nnz) return;
+    const long long e0 = c0 + tid * kPrItems;
+    int u[kPrItems];
+    if (VEC && e0 + kPrItems <= nnz) {
+        const int4 a = __ldg(reinterpret_cast<const int4 *>(col + e0));
+        const int4 b = __ldg(reinterpret_cast<const int4 *>(col + e0) + 1);
+        u[0] = a.x, u[1] = a.y, u[2] = a.z, u[3] = a.w;
+        u[4] = b.x, u[5] = b.y, u[6] = b.z, u[7] = b.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < kPrItems; ++j) u[j] = e0 + j < nnz ? __ldg(col + e0 + j) : -1;
+    }
+    const unsigned m = e0 < nnz ? __ldg(heads + (e0 >> 3)) : 0u;
+    float v[kPrItems];
+#pragma unroll
+    for (int j = 0; j < kPrItems; ++j) v[j] = u[j] >= 0 ? __ldg(x + u[j]) : 0.0f;
+    // pieces: before the thread's first head (`first`), whole rows, after its last head (`acc`)
+    float first = 0.0f, acc = 0.0f;
+    bool seen = false;
+#pragma unroll
+    for (int j = 0; j < kPrItems; ++j) {
+        if ((m >> j) & 1u) {
+            if (seen)
+                y[__ldg(row + e0 + j - 1)] = acc;
+            else
+                first = acc;
+            seen = true;
+            acc = 0.0f;
+        }
+        acc += v[j];
+    }
+    // inclusive segmented scan of (acc, seen) over the block's threads
+    float sv = acc;
+    int sf = seen;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float pv = __shfl_up_sync(0xffffffffu, sv, o);
+        const int pf = __shfl_up_sync(0xffffffffu, sf, o);
+        if (lane >= o) {
+            if (!sf) sv += pv;
+            sf |= pf;
+        }
+    }
+    if (lane == 31) {
+        s_val[warp] = sv;
+        s_any[warp] = sf;
+    }
+    float in = __shfl_up_sync(0xffffffffu, sv, 1);  // what the threads before hold of the open row
+    int any = __shfl_up_sync(0xffffffffu, sf, 1);   // and whether it began in this chunk
+    if (lane == 0) {
+        in = 0.0f;
+        any = 0;
+    }
+    __syncthreads();
+    float wv = 0.0f;
+    int wf = 0;
+    for (int w = 0; w < warp; ++w) {
+        wv = s_any[w] ? s_val[w] : wv + s_val[w];
+        wf |= s_any[w];
+    }
+    if (!any) in += wv;
+    any |= wf;
+    if (seen) {  // the row that is open before this thread ends at its first head
+        const float t = in + first;
+        if (any)
+            y[__ldg(row + e0 + (__ffs(m) - 1) - 1)] = t;
+        else
+            carry[blockIdx.x] = t;
+    }
+    if (tid == kPrBlock - 1) {  // the row that is open at the chunk's end
+        const long long last = (c0 + kPrChunk < nnz ? c0 + kPrChunk : nnz) - 1;
+        const float t = seen ? acc : in + acc;
+        if (seen || any)
+            y[__ldg(row + last)] = t;
+        else
+            carry[blockIdx.x] = t;
+    }
+}
+
+// r'[v] = (1 - d) / n + d * (sum over in-edges + dangling / n), the L1 change, and the next
+// iteration's x and dangling mass; 14 us for 700,001 vertices before (two kernels, 34 us, and
+// a wait for the host every iteration).
+__global__ void __launch_bounds__(kPrVec) pr_update(int n, float damping, const int *__restrict__ in_rp,
+                                                      const int *__restrict__ out_rp, const float *__restrict__ y,
+                                                      const float *__restrict__ carry, float *r, float *x,
+                                                      PrState *st, int it, const int *err) {
+    __shared__ double tmp[kPrVec / 32];
+    if (err && ld_volatile_i32(err) != 0) return;
+    if (ld_volatile_i32(&st->done) != 0) return;
+    const float base = static_cast<float>((1.0 - damping) / n + damping * st->dang[it & 1] / n);
+    double diff = 0.0, dang = 0.0;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const int a = __ldg(in_rp + v), b = __ldg(in_rp + v + 1);
+        float s = 0.0f;
+        if (b > a) {
+            s = y[v];
+            const int c1 = (b - 1) / kPrChunk;
+#pragma unroll 4
+            for (int c = a / kPrChunk + 1; c <= c1; ++c) s += __ldg(carry + c);
+        }
+        const float nr = __fmaf_rn(damping, s, base);
         diff += fabs(static_cast<double>(nr) - static_cast<double>(r[v]));
         r[v] = nr;
+        const int d = __ldg(out_rp + v + 1) - __ldg(out_rp + v);
+        x[v] = d > 0 ? nr / static_cast<float>(d) : 0.0f;
+        if (d == 0) dang += nr;
     }
-    for (int o = 16; o; o >>= 1) diff += __shfl_down_sync(0xffffffffu, diff, o);
-    if ((threadIdx.x & 31) == 0 && diff != 0.0) atomicAdd(acc + 1, diff);
-}
-
-__global__ void pr_init(int n, float *r) {
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) r[v] = 1.0f / n;
+    diff = block_sum(diff, tmp);
+    dang = block_sum(dang, tmp);
+    if (threadIdx.x == 0) {
+        if (diff != 0.0) atomicAdd(&st->diff[it & 1], diff);
+        if (dang != 0.0) atomicAdd(&st->dang[(it + 1) & 1], dang);
+    }
 }
 
 }  // namespace
@@ -121,46 +302,59 @@ apspie_status apspie_pagerank(apspie_ctx *ctx, const apspie_csr *A, float dampin
     if (ctx->validate && (st = validate_csr(ctx, A, true)) != APSPIE_OK) return st;
     const int n = A->m;
     // pull over in-edges: A^T, or A itself when the pattern is symmetric
-    apspie_csr_owned T;
-    std::memset(&T, 0, sizeof(T));
-    apspie_csr at = *A;
-    at.val_type = APSPIE_VAL_NONE;
-    at.val = nullptr;
-    if (!(A->flags & APSPIE_CSR_SYMMETRIC)) {
-        if ((st = apspie_csr_transpose(ctx, &at, &T)) != APSPIE_OK) return st;
-        at.row_ptr = T.row_ptr;
-        at.col_ind = T.col_ind;
-        at.nnz = T.nnz;
-    }
+    const long long nnz = A->nnz;
+    const bool sym = (A->flags & APSPIE_CSR_SYMMETRIC) != 0;
+    const size_t nn = static_cast<size_t>(n);
+    const size_t chunks = static_cast<size_t>(nnz / kPrChunk) + 1;
+    const size_t mat = sym ? (static_cast<size_t>(nnz) + 1) * 4 : transpose_pattern_need(A->n, nnz);
     void *base;
-    st = scratch_reserve(ctx, Carver::need({static_cast<size_t>(n) * 4, static_cast<size_t>(n) * 4, 64}), &base);
-    if (st != APSPIE_OK) {
-        apspie_csr_free(&T);
-        return st;
-    }
-    Carver c(base);
-    float *x = c.take<float>(n);
-    float *y = c.take<float>(n);
-    double *acc = c.take<double>(4);
-    const int blocks = std::max(1, std::min((n + 255) / 256, ctx->num_sms * 8));
-    pr_init<<<blocks, 256, 0, ctx->stream>>>(n, d_rank);
-    int it = 0;
-    double h_acc[2] = {0.0, 0.0};
-    cudaError_t e = cudaSuccess;
-    while (it < max_iter) {
-        if ((e = cudaMemsetAsync(acc, 0, 2 * sizeof(double), ctx->stream)) != cudaSuccess) break;
-        pr_scale<<<blocks, 256, 0, ctx->stream>>>(n, A->row_ptr, d_rank, x, acc);
-        if ((st = launch_spmv(ctx, &at, x, y, 1.0f, 0.0f)) != APSPIE_OK) break;
-        pr_update<<<blocks, 256, 0, ctx->stream>>>(n, damping, y, d_rank, acc);
-        ++it;
-        if ((e = cudaMemcpyAsync(h_acc, acc, sizeof(h_acc), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
-            break;
-        if (h_acc[1] < tol) break;
-    }
-    apspie_csr_free(&T);
+    st = scratch_reserve(ctx, Carver::need({mat, nn * 4, nn * 4, chunks * 4, static_cast<size_t>(nnz / 8) + 1,
+                                            sizeof(PrState)}),
+                         &base);
     if (st != APSPIE_OK) return st;
-    if (e != cudaSuccess) return cuda_error(ctx, e, "apspie_pagerank");
+    Carver c(base);
+    char *mat_base = c.take<char>(mat);
+    float *x = c.take<float>(nn);
+    float *y = c.take<float>(nn);
+    float *carry = c.take<float>(chunks);
+    unsigned char *heads = c.take<unsigned char>(static_cast<size_t>(nnz / 8) + 1);
+    PrState *state = c.take<PrState>(1);
+    cudaError_t e = cudaMemsetAsync(state, 0, sizeof(PrState), ctx->stream);
+    if (e != cudaSuccess) return cuda_error(ctx, e, "apspie_pagerank reset");
+    PatternCoo in{A->row_ptr, reinterpret_cast<const unsigned *>(mat_base), A->col_ind, nullptr};
+    st = sym ? expand_entry_rows(ctx, A, reinterpret_cast<unsigned *>(mat_base))
+             : transpose_pattern(ctx, A, mat_base, &in);
+    if (st != APSPIE_OK) return st;
+    const int vblocks = std::max(1, std::min((n + kPrVec - 1) / kPrVec, ctx->num_sms * 2));
+    const int gblocks = static_cast<int>((nnz + kPrChunk - 1) / kPrChunk);
+    if (nnz > 0)
+        pr_heads<<<static_cast<int>(std::min<long long>((nnz / 8 + 256) / 256, ctx->num_sms * 8LL)), 256, 0,
+                   ctx->stream>>>(nnz, in.row, heads);
+    pr_init<<<vblocks, kPrVec, 0, ctx->stream>>>(n, A->row_ptr, d_rank, x, state);
+    const bool vec = (reinterpret_cast<uintptr_t>(in.col) & 15u) == 0;
+    int it = 0;
+    PrState h;
+    for (;;) {
+        for (int k = 0; k < kPrBatch && it < max_iter; ++k, ++it) {
+            (vec ? pr_gather<true> : pr_gather<false>)<<<std::max(gblocks, 1), kPrBlock, 0, ctx->stream>>>(
+                nnz, in.col, heads, in.row, x, y, carry, state, it, tol, in.err);
+            pr_update<<<vblocks, kPrVec, 0, ctx->stream>>>(n, damping, in.rp, A->row_ptr, y, carry, d_rank, x,
+                                                             state, it, in.err);
+        }
+        int sort_err = 0;
+        if ((e = cudaGetLastError()) != cudaSuccess ||
+            (e = cudaMemcpyAsync(&h, state, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
+            (in.err &&
+             (e = cudaMemcpyAsync(&sort_err, in.err, 4, cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess) ||
+            (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
+            return cuda_error(ctx, e, "apspie_pagerank");
+        if (sort_err) return set_error(ctx, static_cast<apspie_status>(sort_err), "apspie_pagerank: transpose");
+        if (h.done != 0) {
+            it = h.done;
+            break;
+        }
+        if (it >= max_iter || h.diff[(it - 1) & 1] < tol) break;
+    }
     if (iterations) *iterations = it;
     return APSPIE_OK;
 }

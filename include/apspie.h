@@ -365,7 +365,7 @@ apspie_status apspie_spmv(apspie_ctx *ctx, const apspie_csr *A, const float *d_x
  * + (rank mass of vertices without out-edges) / n), until sum |r' - r| < tol or max_iter
  * iterations (*iterations reports how many ran). d_rank: float32[m], so a tol below what
  * float32 ranks resolve (about 1e-7 summed over the graph) runs all max_iter iterations.
- * Synchronises once per iteration. No reference counterpart (the reference ships
+ * Synchronises every few iterations. No reference counterpart (the reference ships
  * test_pr.mtx only). */
 apspie_status apspie_pagerank(apspie_ctx *ctx, const apspie_csr *A, float damping, double tol, int32_t max_iter,
                               float *d_rank, int32_t *iterations);

@@ -64,3 +64,33 @@ def test_pagerank_rmat(ctx, symmetric):
     r, it = ctx.pagerank(ap.DeviceGraph(g), 0.85, 1e-6, 100)
     ref, _ = oracle.pagerank(g.row_ptr, g.col_ind, 0.85, 1e-6, 100)
     np.testing.assert_allclose(r.cpu().numpy(), ref, rtol=2e-4, atol=1e-8)
+
+
+@pytest.mark.parametrize("n,hub", [(1, 0), (2, 3), (9000, 2047), (9000, 2048), (9000, 8999), (70001, 30000)])
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_pagerank_rows_across_entry_chunks(ctx, n, hub, symmetric):
+    """In-edge rows that end at, cross and cover whole 2,048-entry chunks, between runs of
+    vertices without in-edges and without out-edges. Bound: a float32 sum of d positive terms
+    is off by at most d * 2^-24 relative, and an iteration damps earlier errors by 0.85, so the
+    ranks are off by at most (2 + the longest partial sum) * 2^-24 / 0.15; sums inside a chunk
+    are at most 8 + 5 + 8 terms deep, a row's chunks at most 15."""
+    import torch
+
+    rng = np.random.default_rng(n + hub)
+    src = np.concatenate((rng.choice(n, min(hub, n), replace=False), rng.integers(0, n, n // 3)))
+    dst = np.concatenate((np.full(min(hub, n), n // 2), rng.integers(n // 4, max(n // 4 + 1, n // 2), n // 3)))
+    if symmetric:
+        src, dst = np.concatenate((src, dst)), np.concatenate((dst, src))
+    key = np.unique(src.astype(np.int64) * n + dst)
+    rp = np.concatenate(([0], np.cumsum(np.bincount(key // n, minlength=n)))).astype(np.int32)
+    ci = (key % n).astype(np.int32)
+    # an odd number of entries in front makes col_ind's address no multiple of 16
+    cols = torch.from_numpy(np.concatenate((np.zeros(3, dtype=np.int32), ci))).cuda()[3:]
+    g = ap.DeviceGraph.from_tensors(n, n, torch.from_numpy(rp).cuda(), cols, symmetric=symmetric)
+    for iters in (1, 7):  # 7: no multiple of the iterations enqueued at a time
+        r, it = ctx.pagerank(g, 0.85, 0.0, iters)
+        ref, _ = oracle.pagerank(rp, ci, 0.85, 0.0, iters)
+        assert it == iters
+        np.testing.assert_allclose(r.cpu().numpy(), ref, rtol=(2 + 21 + 15) * 2.0 ** -24 / 0.15, atol=0)
+        again, _ = ctx.pagerank(g, 0.85, 0.0, iters)
+        assert torch.allclose(r, again, rtol=2.0 ** -23, atol=0)  # the double sums' order may turn a last bit
