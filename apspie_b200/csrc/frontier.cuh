@@ -185,9 +185,13 @@ __device__ __forceinline__ void frontier_expand(int nf, int E, const int *__rest
         const int e1 = static_cast<int>(d1 - a1);
         const int jb = a0 > 0 ? a0 - 1 : 0;
         const int ne = a1 - jb;
+        // the tile's entries lie in chunk jb / C and, with chunks at least as long as a tile, the
+        // next one
+        const int jc = jb / C, jn = (jc + 1) * C;
         for (int k = lane; k < ne; k += 32) {
             const int j = jb + k;
-            ws.off[k] = sm.base[j / C] + __ldcg(loc_off + j);
+            const int c = C >= WT ? jc + (j >= jn ? 1 : 0) : j / C;
+            ws.off[k] = sm.base[c] + __ldcg(loc_off + j);
             ws.rs[k] = __ldcg(rs + j);
             load(j, k, ws);
         }

@@ -10,11 +10,19 @@
 // one 128-byte line, lab[(v * W + w) * 32 + q % 32]. Frontier entries are (vertex u, query
 // word w) pairs whose "changed" bits (the queries whose distance at u dropped in the
 // previous iteration) are non-zero; an entry's weight is deg(u), so the merge-path
-// expander balances the edges. Each warp then walks its lanes' edges one at a time with
-// the lanes standing for the word's 32 queries: lane q reads u's and v's labels of query q
-// (two coalesced line reads shared by the whole word), relaxes nd = dist[q][u] + w(u,v) if
-// q changed at u, and atomicMin's the label; a ballot collects the improved queries and the
-// edge's own lane ORs them into v's next changed word, enqueueing (v, w) on the first bit.
+// expander balances the edges. A warp keeps its tile's edges as 16-byte records in shared
+// memory and walks them four at a time, eight lanes to an edge, four queries to a lane: a lane
+// reads 16 bytes of u's and of v's label line, relaxes nd = dist[q][u] + w(u,v) where q
+// changed at u, and atomicMin's the label; the improved queries replace the changed ones in
+// the record, and at the end of the tile each lane ORs its own edges' into v's next changed
+// word, enqueueing (v, w) on the first bit.
+//
+// What bounds it: instruction issue (62 % of the slots used with one edge at a time) and the
+// latency of the label reads. 100 queries on R-MAT of 2^19 vertices (345M visits of a row's
+// entry for a word): one edge at a time, a lane per query, 18.9 ms; four edges a step with
+// their fields by shuffles 15.1 ms, target labels through L1 too 14.2 ms, fields as records
+// 12.9 ms (one step in flight instead of two: 14.6 ms; four blocks per SM instead of five:
+// 13.1 ms).
 // Every query reaches the same label-correcting fixed point as apspie_sssp computes alone
 // (exact shortest distances for non-negative integer weights). A last pass transposes the
 // labels into the query-major output out[q * m + v] (0xFFFFFFFF, -1 as int32, unreached).
@@ -27,21 +35,12 @@
 namespace apspie {
 namespace {
 
-#ifndef APSPIE_SB_MINB
-#define APSPIE_SB_MINB 5
-#endif
-#ifndef APSPIE_SB_UNROLL
-#define APSPIE_SB_UNROLL 4
-#endif
-#ifndef APSPIE_SB_VT
-#define APSPIE_SB_VT 2
-#endif
 constexpr int kSbBlock = 256;
-constexpr int kSbVT = APSPIE_SB_VT;
-constexpr int kSbUnroll = APSPIE_SB_UNROLL;  // edges whose label reads a warp issues together
+constexpr int kSbVT = 2;
+constexpr int kSbSteps = 2;  // steps of four edges whose label reads a warp issues together
 // every lane's edge is visited exactly once per pass: a second visit would not record the
 // queries it improves
-static_assert(32 % kSbUnroll == 0, "the unroll must divide the warp");
+static_assert(32 % (4 * kSbSteps) == 0, "the steps must divide the warp");
 using SbSmem = ExpandSmem<kSbBlock, kSbVT>;
 using SbWarp = SbSmem::Warp;
 using SbWQ = WarpQueue<SbSmem::QCAP>;
@@ -68,8 +67,9 @@ struct RowOfPacked {
     __device__ __forceinline__ int operator()(int e) const { return e / W; }
 };
 
-__global__ void __launch_bounds__(kSbBlock, APSPIE_SB_MINB) sssp_batch_kernel(SbArgs a) {
+__global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
     __shared__ SbSmem sm;
+    __shared__ uint4 s_rec[kSbBlock / 32][32 * kSbVT];
     timeline_mark(a.ctl, 0);
     const int G = gridDim.x;
     const int gtid = blockIdx.x * kSbBlock + threadIdx.x;
@@ -150,76 +150,95 @@ __global__ void __launch_bounds__(kSbBlock, APSPIE_SB_MINB) sssp_batch_kernel(Sb
                 ws.aux2[k] = static_cast<int>(__ldcg(cbits + j));
             },
             [&](const bool (&valid)[kSbVT], const int (&kk)[kSbVT], const int (&idx)[kSbVT], SbWarp &ws) {
-                // this lane's edges: target entry (v, w), weight, source entry and its changed bits
-                int tv[kSbVT], we[kSbVT], eu[kSbVT];
-                unsigned bits[kSbVT];
+                // the tile's edges as records: target entry (v, w), weight + 1, source entry and
+                // its changed bits, which the edge's improved queries replace
+                uint4 *rec = s_rec[wid];
+                int ned = 0, tv[kSbVT];
 #pragma unroll
                 for (int r = 0; r < kSbVT; ++r) {
-                    tv[r] = eu[r] = 0;
-                    we[r] = 0;
-                    bits[r] = 0u;
+                    uint4 e = make_uint4(0u, 0u, 0u, 0u);
+                    tv[r] = 0;
                     if (valid[r]) {
                         const int v = __ldg(col + idx[r]);
-                        we[r] = __ldg(wt + idx[r]);
-                        eu[r] = ws.aux[kk[r]];
+                        const int we = __ldg(wt + idx[r]);
                         tv[r] = v * W + ws.flag[kk[r]];
-                        bits[r] = static_cast<unsigned>(ws.aux2[kk[r]]);
-                        if (we[r] < 0) {  // reported once here; the edge is then left out
+                        e = make_uint4(static_cast<unsigned>(tv[r]), static_cast<unsigned>(we) + 1u,
+                                       static_cast<unsigned>(ws.aux[kk[r]]), static_cast<unsigned>(ws.aux2[kk[r]]));
+                        if (we < 0) {  // reported once here; the edge is then left out
                             raise_error(ctl, sticky, APSPIE_ERR_INVALID_ARG, kSiteSbNeg);
-                            bits[r] = 0u;
+                            e.w = 0u;
                         }
                     }
+                    rec[r * 32 + lane] = e;
+                    ned += __popc(__ballot_sync(0xffffffffu, valid[r]));
                 }
-                unsigned *lab_l = lab + lane;  // this lane's query in every label line
-#pragma unroll
-                for (int r = 0; r < kSbVT; ++r) {
-                    const unsigned vmask = __ballot_sync(0xffffffffu, bits[r] != 0u);
-                    if (vmask == 0u) continue;
-                    unsigned mine = 0u;  // improved queries of this lane's edge r
+                __syncwarp();
+                // four edges a step, eight lanes each, four queries (16 bytes of the label line) a lane
+                const int sub4 = 4 * (lane & 7), grp = lane >> 3;
+                bool over = false;
 #pragma unroll 1
-                    for (int l0 = 0; l0 < 32; l0 += kSbUnroll) {
-                        if (((vmask >> l0) & ((1u << kSbUnroll) - 1u)) == 0u) continue;
-                        unsigned du[kSbUnroll], dv[kSbUnroll];
-                        int ev[kSbUnroll], wl[kSbUnroll];
-                        bool act[kSbUnroll];
+                for (int l0 = 0; l0 < ned; l0 += 4 * kSbSteps) {
+                    uint4 du[kSbSteps], dv[kSbSteps];
+                    unsigned *lv[kSbSteps];
+                    unsigned act[kSbSteps], w1[kSbSteps];
 #pragma unroll
-                        for (int t = 0; t < kSbUnroll; ++t) {
-                            const int l = l0 + t;
-                            ev[t] = __shfl_sync(0xffffffffu, tv[r], l);
-                            wl[t] = __shfl_sync(0xffffffffu, we[r], l);
-                            const int u = __shfl_sync(0xffffffffu, eu[r], l);
-                            const unsigned b = __shfl_sync(0xffffffffu, bits[r], l);
-                            act[t] = (b >> lane) & 1u;
-                            // coherent reads: a label lowered since the entry was queued must be
-                            // seen (its change bit was consumed in phase A)
-                            du[t] = act[t] ? __ldcg(lab_l + static_cast<size_t>(u) * 32) : 0u;
-                            dv[t] = act[t] ? __ldcg(lab_l + static_cast<size_t>(ev[t]) * 32) : 0u;
+                    for (int t = 0; t < kSbSteps; ++t) {
+                        const uint4 e = rec[l0 + 4 * t + grp];
+                        act[t] = (e.w >> sub4) & 15u;
+                        w1[t] = e.y;
+                        lv[t] = lab + static_cast<size_t>(e.x) * 32 + sub4;
+                        if (act[t]) {
+                            // through L1 (a row's edges all read the same source line, and many edges
+                            // the lines of high-degree targets). u's labels: one lowered in this
+                            // iteration has its change bit set for the next, so any value since the
+                            // barrier will do. v's: a stale, larger value only costs an atomic and
+                            // one more expansion of v's query
+                            du[t] = *reinterpret_cast<const uint4 *>(lab + static_cast<size_t>(e.z) * 32 + sub4);
+                            dv[t] = *reinterpret_cast<const uint4 *>(lv[t]);
                         }
-                        // an improvement over the label just read is reported without waiting
-                        // for the atomic's old value: if another edge lowered the label further
-                        // meanwhile, v's query is only re-expanded once more (same values)
-                        bool imp[kSbUnroll];
+                    }
+                    // an improvement over the label just read is reported without waiting for the
+                    // atomic's old value: if another edge lowered the label further meanwhile, v's
+                    // query is only re-expanded once more (same values)
 #pragma unroll
-                        for (int t = 0; t < kSbUnroll; ++t) {
-                            imp[t] = false;
-                            // an active label is finite (< 2^31 - 1) and the weight is
-                            // non-negative, so the 32-bit sum cannot wrap
-                            const unsigned nd = du[t] + static_cast<unsigned>(wl[t]);
-                            if (act[t]) {
-                                if (nd >= 0x7fffffffu) {
-                                    raise_error(ctl, sticky, APSPIE_ERR_INVALID_ARG, kSiteSbOverflow);
-                                } else if (nd < dv[t]) {
-                                    atomicMin(lab_l + static_cast<size_t>(ev[t]) * 32, nd);
-                                    imp[t] = true;
-                                }
+                    for (int t = 0; t < kSbSteps; ++t) {
+                        unsigned imp = 0u;
+                        if (act[t]) {
+                            // s = candidate + 1. An active label is finite (< 2^31 - 1) and the weight
+                            // non-negative, so s does not wrap, and s > 2^31 - 1 is an overflow; an
+                            // inactive, unreached label wraps to the weight, below that
+                            unsigned s0 = du[t].x + w1[t], s1 = du[t].y + w1[t];
+                            unsigned s2 = du[t].z + w1[t], s3 = du[t].w + w1[t];
+                            if (static_cast<int>(s0 | s1 | s2 | s3) < 0) {
+                                const unsigned big = (s0 >> 31) | ((s1 >> 31) << 1) | ((s2 >> 31) << 2) | ((s3 >> 31) << 3);
+                                over |= (big & act[t]) != 0u;
+                                act[t] &= ~big;
+                            }
+                            imp = ((s0 <= dv[t].x ? 1u : 0u) | (s1 <= dv[t].y ? 2u : 0u) | (s2 <= dv[t].z ? 4u : 0u) |
+                                   (s3 <= dv[t].w ? 8u : 0u)) &
+                                  act[t];
+                            if (imp) {
+                                if (imp & 1u) atomicMin(lv[t], s0 - 1u);
+                                if (imp & 2u) atomicMin(lv[t] + 1, s1 - 1u);
+                                if (imp & 4u) atomicMin(lv[t] + 2, s2 - 1u);
+                                if (imp & 8u) atomicMin(lv[t] + 3, s3 - 1u);
                             }
                         }
-#pragma unroll
-                        for (int t = 0; t < kSbUnroll; ++t) {
-                            const unsigned nb = __ballot_sync(0xffffffffu, imp[t]);
-                            if (lane == l0 + t) mine = nb;
+                        unsigned m = 0u;
+                        if (__any_sync(0xffffffffu, imp != 0u)) {
+                            m = imp << sub4;
+                            m |= __shfl_xor_sync(0xffffffffu, m, 1);
+                            m |= __shfl_xor_sync(0xffffffffu, m, 2);
+                            m |= __shfl_xor_sync(0xffffffffu, m, 4);
                         }
+                        if (sub4 == 0) rec[l0 + 4 * t + grp].w = m;
                     }
+                }
+                if (over) raise_error(ctl, sticky, APSPIE_ERR_INVALID_ARG, kSiteSbOverflow);
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < kSbVT; ++r) {
+                    const unsigned mine = rec[r * 32 + lane].w;  // improved queries of this lane's edge r
                     bool fresh = false;
                     if (mine) fresh = atomicOr(cn + tv[r], mine) == 0u;
                     wq.push(fresh, tv[r]);

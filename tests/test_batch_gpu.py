@@ -223,3 +223,36 @@ def test_batch_source_out_of_range_reported(ctx, rmat14, kind, groups, bad):
     for q, s in enumerate([0, 5]):
         ref = oracle.bfs(g.row_ptr, g.col_ind, s) if kind == "bfs" else oracle.sssp(g.row_ptr, g.col_ind, g.val, s)
         np.testing.assert_array_equal(got[q], ref)
+
+
+@pytest.mark.parametrize("nq", [1, 4, 5, 31, 33])
+@pytest.mark.parametrize("case", ["zero weights", "largest distances", "one edge a vertex"])
+def test_sssp_batch_label_arithmetic_limits(ctx, case, nq):
+    """Weights of 0 beside unreached labels (candidate + 1 must not take an unreached label for
+    an overflow), distances up to the largest one, 2^31 - 2, and rows shorter than a step of
+    four edges; queries that fill part of a lane's four, a lane, and a word and a bit."""
+    import torch
+
+    rng = np.random.default_rng(nq)
+    m = 257
+    if case == "largest distances":  # a path whose far end is 2^31 - 2 away from vertex 0
+        src, dst = np.arange(m - 1), np.arange(1, m)
+        w = np.full(m - 1, (2 ** 31 - 2) // (m - 1), dtype=np.int64)
+        w[-1] += (2 ** 31 - 2) - w.sum()
+    elif case == "one edge a vertex":
+        src, dst = np.arange(m), rng.permutation(m)
+        w = rng.integers(0, 256, m)
+    else:
+        src, dst = rng.integers(0, m, 900), rng.integers(0, m, 900)
+        w = rng.choice([0, 0, 0, 1, 2 ** 22], 900)
+    order = np.lexsort((dst, src))
+    rp = np.concatenate(([0], np.cumsum(np.bincount(src, minlength=m)))).astype(np.int32)
+    g = ap.HostGraph(m, m, rp, dst[order].astype(np.int32), w[order].astype(np.int32))
+    dg = ap.DeviceGraph(g)
+    sources = np.concatenate(([0], rng.integers(0, m, nq)))[:nq].astype(np.int32)
+    out = ctx.sssp_batch(dg, torch.from_numpy(sources).cuda()).cpu().numpy()
+    ctx.synchronize()  # raises if the device reported an overflow
+    for q, s in enumerate(sources):
+        np.testing.assert_array_equal(out[q], oracle.sssp(g.row_ptr, g.col_ind, g.val, int(s)))
+    if case == "largest distances":
+        assert out[0, -1] == 2 ** 31 - 2
