@@ -125,6 +125,26 @@ def test_spgemm_er_full_size_properties(ctx):
     _check(ctx, e, e, exact_f32=True)
 
 
+@pytest.mark.parametrize("vt", [ap.VAL_F32, ap.VAL_I32])
+@pytest.mark.parametrize("n", [1, 31, 33, 1000, 32768, 32769, 49152, 49153])
+def test_spgemm_rows_of_many_products(ctx, n, vt):
+    """Rows past the shared-table tier over few columns (dense accumulators: up to 49,152
+    columns, one and two bitmap words a thread) and over one more (global tables); rows of the
+    three size classes, repeated columns, rows of B from empty to longer than a warp's step."""
+    rng = np.random.default_rng(n)
+    k, m = 2500, 40
+    lb = np.minimum(rng.choice([0, 1, 3, 31, 40, 130, 300], k), n)
+    rpb = np.concatenate(([0], np.cumsum(lb))).astype(np.int32)
+    cib = np.concatenate([np.sort(rng.choice(n, int(x), replace=False)) for x in lb]).astype(np.int32)
+    la = np.concatenate(([2500, 2000, 0, 1500, 1200], rng.integers(0, 60, m - 5)))
+    rpa = np.concatenate(([0], np.cumsum(la))).astype(np.int32)
+    cia = np.concatenate([np.sort(rng.choice(k, int(x), replace=False)) for x in la]).astype(np.int32)
+    f32 = vt == ap.VAL_F32
+    va, vb = (rng.uniform(-1, 1, s).astype(np.float32) if f32 else rng.integers(-8, 9, s).astype(np.int32)
+              for s in (cia.shape[0], cib.shape[0]))
+    _check(ctx, ap.HostGraph(m, k, rpa, cia, va), ap.HostGraph(k, n, rpb, cib, vb), exact_f32=False)
+
+
 def test_spgemm_rejects_mismatch(ctx):
     e = ap.gen_er(64, 4, 5, ap.VAL_F32)
     f = ap.gen_er(64, 4, 5, ap.VAL_I32)
