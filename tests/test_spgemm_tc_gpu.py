@@ -191,3 +191,51 @@ def test_tc_dense_clique_uses_block_and_global_tiers(ctx):
     rp[1:] = np.cumsum([len(r) for r in rows])
     ci = np.concatenate(rows)
     assert ctx.tc(ap.DeviceGraph(ap.HostGraph(n, n, rp, ci))) == n * (n - 1) * (n - 2) // 6
+
+
+@pytest.mark.parametrize("m", [2, 31, 33, 257, 5000, 1638400, 1638401])
+def test_tc_bitmap_and_hash_paths(ctx, m):
+    """Vertices around a bitmap word, the most whose bitmap fits an SM and one more; a vertex
+    with more partners than the first class begins at, lists from empty to longer than a
+    warp's step, beside a random part."""
+    rng = np.random.default_rng(m)
+    core = min(m, 700)
+    ids = np.sort(rng.choice(m, core, replace=False))
+    u, v = rng.integers(0, core, (2, 12 * core))
+    u[: core // 2], v[: core // 2] = 0, rng.integers(0, core, core // 2)  # one vertex meets half of them
+    u, v = ids[u], ids[v]
+    key = np.unique(np.maximum(u, v)[u != v].astype(np.int64) * m + np.minimum(u, v)[u != v])
+    rp = np.concatenate(([0], np.cumsum(np.bincount(key // m, minlength=m)))).astype(np.int32)
+    Lh = ap.HostGraph(m, m, rp, (key % m).astype(np.int32))
+    assert ctx.tc(ap.DeviceGraph(Lh)) == oracle.tc(Lh.row_ptr, Lh.col_ind)
+
+
+@pytest.mark.parametrize("what", ["equal neighbours", "a diagonal entry", "an upper entry"])
+def test_tc_of_what_is_no_set_of_lower_entries(ctx, what):
+    """sum((L*L) .* L) as given: what the bitmap path cannot count (rows that repeat an entry,
+    entries on or above the diagonal) is counted as it was before there was one."""
+    rng = np.random.default_rng(7)
+    m = 400
+    d = np.tril(rng.random((m, m)) < 0.1, -1).astype(np.int64)
+    if what == "a diagonal entry":
+        d[200, 200] = 1
+    elif what == "an upper entry":
+        d[100, 300] = 1
+    rows, cols = np.nonzero(d)
+    if what == "equal neighbours":
+        again = rng.choice(rows.size, 50, replace=False)
+        rows, cols = np.concatenate((rows, rows[again])), np.concatenate((cols, cols[again]))
+        order = np.lexsort((cols, rows))
+        rows, cols = rows[order], cols[order]
+    rp = np.concatenate(([0], np.cumsum(np.bincount(rows, minlength=m)))).astype(np.int32)
+    got = ctx.tc(ap.DeviceGraph(ap.HostGraph(m, m, rp, cols.astype(np.int32))))
+    if what == "equal neighbours":
+        # oriented by (degree, id), then every wedge's end looked up in the first vertex's set
+        deg = np.bincount(rows, minlength=m) + np.bincount(cols, minlength=m)
+        fwd = (deg[rows] < deg[cols]) | ((deg[rows] == deg[cols]) & (rows < cols))
+        a, b = np.where(fwd, rows, cols), np.where(fwd, cols, rows)
+        D = np.zeros((m, m), dtype=np.int64)
+        np.add.at(D, (a, b), 1)
+        assert got == int(((D @ D) * (D > 0)).sum())
+    else:
+        assert got == int(((d @ d) * d).sum())
