@@ -248,15 +248,35 @@ __device__ __forceinline__ int ld_volatile_i32(const int *p) {
     return *reinterpret_cast<const volatile int *>(p);
 }
 
+// What thread 0 of a block keeps of the grid barrier between its barriers.
+struct BarState {
+    unsigned phase;  // bit 31 of ctl->bar before the next barrier
+    int marks;       // timeline entries written (block 0)
+};
+__device__ __forceinline__ BarState &bar_state() {
+    __shared__ BarState s;
+    return s;
+}
+
 // Block 0, thread 0: records (site, globaltimer) in the control block's timeline.
 __device__ __forceinline__ void timeline_mark(TravCtl *ctl, int site) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const int k = ctl->tl_count;
+        const int k = bar_state().marks;
         if (k < kTimeline) {
             ctl->tl_site[k] = site;
             ctl->tl_ns[k] = globaltimer_ns();
-            ctl->tl_count = k + 1;
+            ctl->tl_count = bar_state().marks = k + 1;
         }
+    }
+}
+
+// Start of every kernel that uses grid_barrier: before its first arrival a block sees the
+// phase that its first barrier starts from, whoever else has arrived.
+__device__ __forceinline__ void grid_begin(TravCtl *ctl) {
+    if (threadIdx.x == 0) {
+        bar_state().phase = *reinterpret_cast<const volatile unsigned *>(&ctl->bar) & 0x80000000u;
+        bar_state().marks = 0;
+        timeline_mark(ctl, 0);
     }
 }
 
@@ -284,8 +304,10 @@ __device__ __forceinline__ VGrid hw_grid() { return VGrid{static_cast<int>(block
 // counter. Thread 0 of every block adds 1 to ctl->bar, except block 0, which adds
 // 2^31 - (G - 1); the G additions sum to 2^31, so bit 31 flips exactly when the last block
 // arrives and the low bits return to where they were (no reset). A waiter polls the pair
-// (bar, err) with one 64-bit load until bit 31 differs from what it saw before arriving,
-// or until an error is posted. Every wait is bounded (the control block's wait_limit_ns,
+// (bar, err) with one 64-bit load until bit 31 differs from the phase it keeps, or until an
+// error is posted; it knows the phase from the barrier before (grid_begin for the first), so
+// the addition's result is not waited for and the last arriver is through after one trip to
+// L2 instead of two. Every wait is bounded (the control block's wait_limit_ns,
 // else kBarrierTimeoutNs); on timeout it
 // raises APSPIE_ERR_TIMEOUT. Returns false when any block has raised an error, so that all
 // blocks leave the persistent loop together instead of hanging.
@@ -295,17 +317,18 @@ __device__ __forceinline__ bool grid_barrier(TravCtl *ctl, int *sticky, int wher
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned inc = vg.id == 0 ? 0x80000000u - static_cast<unsigned>(vg.n - 1) : 1u;
+        const unsigned before = bar_state().phase;
         __threadfence();
-        const unsigned before = atomicAdd(&ctl->bar, inc);
+        atomicAdd(&ctl->bar, inc);
         unsigned long long pair;
         unsigned long long t0 = 0;
-        const unsigned long long limit = ctl->wait_limit_ns ? ctl->wait_limit_ns : kBarrierTimeoutNs;
         for (unsigned spin = 1;; ++spin) {
             pair = ld_acquire_u64(&ctl->bar);
             if (((static_cast<unsigned>(pair) ^ before) & 0x80000000u) != 0u) break;
             if ((pair >> 32) != 0ull) break;  // an error was raised: leave now
             if ((spin & 1023u) == 0u) {
                 const unsigned long long t = globaltimer_ns();
+                const unsigned long long limit = ctl->wait_limit_ns ? ctl->wait_limit_ns : kBarrierTimeoutNs;
                 if (t0 == 0) {
                     t0 = t;
                 } else if (t - t0 > limit) {
@@ -316,10 +339,11 @@ __device__ __forceinline__ bool grid_barrier(TravCtl *ctl, int *sticky, int wher
             }
         }
         __threadfence();
+        bar_state().phase = before ^ 0x80000000u;
         s_ok = (pair >> 32) == 0ull;
-        timeline_mark(ctl, where);
     }
     __syncthreads();
+    timeline_mark(ctl, where);
     return s_ok != 0;
 }
 

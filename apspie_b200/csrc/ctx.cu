@@ -145,6 +145,7 @@ apspie_status reset_ctl(apspie_ctx *ctx) {
 // A cooperative grid that passes `rounds` grid barriers; block `absent` (when >= 0) leaves
 // before its first arrival, so the others' first wait runs out.
 __global__ void barrier_check_kernel(TravCtl *ctl, int *sticky, int rounds, int absent) {
+    grid_begin(ctl);
     if (static_cast<int>(blockIdx.x) == absent) return;
     for (int r = 0; r < rounds; ++r)
         if (!grid_barrier(ctl, sticky, 900 + r)) return;

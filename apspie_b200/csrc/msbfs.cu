@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
     __shared__ unsigned s_alive[W];   // bits this block found in the next frontier (engine)
     __shared__ int *s_row[SERVE ? 32 * W : 1];  // engine: each slot's output row this level
     __shared__ int s_base[SERVE ? 32 * W : 1];  // engine: each slot's start level
-    timeline_mark(a.ctl, 0);
+    grid_begin(a.ctl);
     const int G = gridDim.x;
     const int gtid = blockIdx.x * kMsBlock + threadIdx.x;
     const int gstride = G * kMsBlock;

@@ -70,7 +70,7 @@ struct RowOfPacked {
 __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
     __shared__ SbSmem sm;
     __shared__ uint4 s_rec[kSbBlock / 32][32 * kSbVT];
-    timeline_mark(a.ctl, 0);
+    grid_begin(a.ctl);
     const int G = gridDim.x;
     const int gtid = blockIdx.x * kSbBlock + threadIdx.x;
     const int gstride = G * kSbBlock;

@@ -125,7 +125,7 @@ struct BfsArgs {
 // frontier holds fewer than m/beta vertices. Depth results do not depend on the choice.
 __global__ void __launch_bounds__(kBlock) bfs_kernel(BfsArgs a) {
     __shared__ BfsSmem sm;
-    timeline_mark(a.ctl, 0);
+    grid_begin(a.ctl);
     const int G = gridDim.x;
     const int gtid = blockIdx.x * kBlock + threadIdx.x;
     const int gstride = G * kBlock;
@@ -323,7 +323,6 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
     static_assert(kBlock == kBandBins, "one histogram bin per thread");
     __shared__ SsspShared sh;
     SsspSmem &sm = sh.ex;
-    timeline_mark(a.ctl, 0);
     const int G = vg.n;
     const int gtid = vg.id * kBlock + threadIdx.x;
     const int gstride = G * kBlock;
@@ -707,7 +706,10 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
     }
 }
 
-__global__ void __launch_bounds__(kBlock, APSPIE_SSSP_MINB) sssp_kernel(SsspArgs a) { sssp_body(a, hw_grid()); }
+__global__ void __launch_bounds__(kBlock, APSPIE_SSSP_MINB) sssp_kernel(SsspArgs a) {
+    grid_begin(a.ctl);
+    sssp_body(a, hw_grid());
+}
 
 // Many sources in one launch: the grid splits into `groups` equal groups of blocks, each
 // with its own control block and scratch, and each group runs the single-source SSSP
@@ -747,6 +749,7 @@ __global__ void __launch_bounds__(kBlock, APSPIE_SSSP_MINB) sssp_group_kernel(Ss
     const int grp = static_cast<int>(blockIdx.x) / bpg;
     const VGrid vg{static_cast<int>(blockIdx.x) - grp * bpg, bpg};
     TravCtl *ctl = g.ctls + grp;
+    grid_begin(ctl);
     SsspArgs a = g.base;
     a.ctl = ctl;
     a.buf = shift_buffers(g.base.buf, g.buf_stride * grp);
@@ -905,7 +908,7 @@ __device__ __forceinline__ void mis_list_heavy(const MisArgs &a, unsigned long l
 __global__ void __launch_bounds__(kBlock) mis_kernel(MisArgs a) {
     __shared__ int qbuf[kBlock / 32][3][BfsSmem::QCAP];
     __shared__ int s_stop;
-    timeline_mark(a.ctl, 0);
+    grid_begin(a.ctl);
     const int G = gridDim.x;
     const int gtid = blockIdx.x * kBlock + threadIdx.x;
     const int gstride = G * kBlock;
