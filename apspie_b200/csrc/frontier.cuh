@@ -271,4 +271,204 @@ __device__ __forceinline__ void frontier_expand(int nf, int E, const int *__rest
     for (long long tb = t_begin; tb < t_end; tb += BATCH) run_batch(tb, tb + BATCH < t_end ? tb + BATCH : t_end);
 }
 
+// ---- edge queues ----------------------------------------------------------------------
+// A frontier queue whose entries carry the running sum of their row lengths, so that the
+// kernel that reads it needs neither a scan nor a search. Whoever appends entries reserves
+// room for them and for their edges with one 64-bit atomic on (entries << 32 | edges), which
+// makes edge offsets ascend with entry indices; an entry records its offset, its row start
+// minus that offset, and, for every unit of 1 << shift edges that begins inside its row, its
+// index as that unit's owner. A reader takes a unit per warp: the owner, the entries from it
+// on, and the edges, all of them a fixed number of dependent reads.
+//
+// It replaces phase A, its grid barrier and the merge-path searches above where the entries'
+// row lengths are final when they are appended (BFS); rows of length zero are only counted.
+struct EdgeQueue {
+    int *off;                  // edge offset of each entry
+    int *delta;                // row start - off: edge t of the queue is CSR entry t + delta
+    int *owner;                // entry that holds the first edge of each unit
+    unsigned long long *size;  // entries << 32 | edges
+    int *empty;                // entries without edges (counted, not stored)
+};
+
+constexpr int kEqTile = 128;  // edges a warp handles at a time: four per lane
+constexpr int kEqCap = kEqTile + 32;  // vertices a warp stages before it appends them
+
+// Per block: what its warps append at the end of a phase.
+template <int BLOCK>
+struct EqBlock {
+    unsigned long long size[BLOCK / 32];  // per warp: entries << 32 | edges, then where they go
+    int empty;
+};
+
+__device__ __forceinline__ void eq_own(int *owner, int shift, int idx, int off, int deg, int first, int step) {
+    const int c1 = (off + deg - 1) >> shift;
+    for (int c = (off > 0 ? ((off - 1) >> shift) + 1 : 0) + first; c <= c1; c += step) owner[c] = idx;
+}
+
+// Appends the warp's `count` staged vertices. With blk (then every warp of the block calls it)
+// room is reserved for the whole block at once: reservations are made one after the other in
+// L2. Once a reservation ends past `enough` entries or edges, the reader of the queue is known
+// not to need its entries (the next level pulls): they are counted and not written, which
+// spares the owners of the highest-degree vertices' rows (a source's first neighbours are
+// those: one warp wrote their owners for 8 us of a 15 us level at scale 20).
+template <int BLOCK>
+__device__ __forceinline__ void eq_append(const int *buf, int count, EqBlock<BLOCK> *blk, const EdgeQueue &q,
+                                              const int *__restrict__ row_ptr, int shift, int enough_entries,
+                                              int enough_edges) {
+    constexpr int PER = kEqCap / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncwarp();
+    int r0[PER], deg[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = k * 32 + lane;
+        const int v = i < count ? buf[i] : -1;
+        r0[k] = v >= 0 ? __ldg(row_ptr + v) : 0;
+        deg[k] = v >= 0 ? __ldg(row_ptr + v + 1) : 0;
+    }
+    int n = 0, d = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        deg[k] -= r0[k];
+        n += deg[k] > 0;
+        d += deg[k];
+    }
+    int sn = n, sd = d;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int yn = __shfl_up_sync(0xffffffffu, sn, o), yd = __shfl_up_sync(0xffffffffu, sd, o);
+        if (lane >= o) {
+            sn += yn;
+            sd += yd;
+        }
+    }
+    unsigned long long base =
+        (static_cast<unsigned long long>(static_cast<unsigned>(sn)) << 32) | static_cast<unsigned>(sd);
+    if (blk) {
+        if (lane == 31) {
+            blk->size[warp] = base;
+            if (sn < count) atomicAdd(&blk->empty, count - sn);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned long long mine = lane < BLOCK / 32 ? blk->size[lane] : 0ull;
+            unsigned long long sum = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += y;
+            }
+            unsigned long long at = 0ull;
+            if (lane == 31) {
+                if (sum) at = atomicAdd(q.size, sum);
+                if (blk->empty) atomicAdd(q.empty, blk->empty);
+                blk->empty = 0;
+            }
+            at = __shfl_sync(0xffffffffu, at, 31);
+            if (lane < BLOCK / 32) blk->size[lane] = at + sum - mine;
+        }
+        __syncthreads();
+        base = blk->size[warp];
+    } else {
+        if (lane == 31) {
+            base = atomicAdd(q.size, base);
+            if (sn < count) atomicAdd(q.empty, count - sn);
+        }
+        base = __shfl_sync(0xffffffffu, base, 31);
+    }
+    int idx = static_cast<int>(base >> 32) + sn - n;
+    int off = static_cast<int>(base & 0xffffffffull) + sd - d;
+    const int all_n = __shfl_sync(0xffffffffu, idx + n, 31), all_d = __shfl_sync(0xffffffffu, off + d, 31);
+    if (count == 0 || all_n > enough_entries || all_d > enough_edges) return;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const bool some = deg[k] > 0;
+        if (some) {
+            q.off[idx] = off;
+            q.delta[idx] = r0[k] - off;
+        }
+        // a row of many units is shared out among the lanes
+        const bool wide = deg[k] >> shift >= 64;
+        if (some && !wide) eq_own(q.owner, shift, idx, off, deg[k], 0, 1);
+        for (unsigned m = __ballot_sync(0xffffffffu, wide); m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            eq_own(q.owner, shift, __shfl_sync(0xffffffffu, idx, l), __shfl_sync(0xffffffffu, off, l),
+                   __shfl_sync(0xffffffffu, deg[k], l), lane, 32);
+        }
+        idx += some;
+        off += deg[k];
+    }
+}
+
+// Smallest unit (a power of two, at least a tile) for which the units of up to nnz edges fit
+// `slots` owners.
+__host__ __device__ inline int edge_unit_shift(long long nnz, long long slots) {
+    int s = 7;
+    while ((nnz >> s) + 1 > slots) ++s;
+    return s;
+}
+
+// op(valid, entry, idx) on every edge of the queue, four per lane (CSR positions idx[], queue
+// entries entry[]), called by all lanes of the warp. A tile's entries are read 32 at a time;
+// where each begins goes into a 128-bit mask in registers, so an edge finds its entry by
+// counting bits. `slice`: kEqTile ints of shared memory, private to the warp.
+template <class Op>
+__device__ __forceinline__ void edge_expand(const EdgeQueue &q, int nf, int E, int shift, int *slice, int gwarp,
+                                            int nwarps, Op op) {
+    const int lane = threadIdx.x & 31;
+    const unsigned upto = lane == 31 ? 0xffffffffu : (2u << lane) - 1u;
+    const int units = E > 0 ? ((E - 1) >> shift) + 1 : 0;
+    for (int u = gwarp; u < units; u += nwarps) {
+        int k = __ldcg(q.owner + u);
+        // the next unit's owner, read beside it: when it is the same entry, the unit lies inside
+        // that entry's row
+        const bool one = u + 1 < units && __ldcg(q.owner + u + 1) == k;
+        const long long uend = (static_cast<long long>(u) + 1) << shift;
+        const int end = uend < E ? static_cast<int>(uend) : E;
+        for (int t0 = u << shift; t0 < end; t0 += kEqTile) {
+            const int t1 = min(t0 + kEqTile, end);
+            unsigned begin[4] = {0u, 0u, 0u, 0u};
+            int n = 0, next = 0x7fffffff;
+            if (one) {
+                if (lane == 0) slice[0] = __ldcg(q.delta + k);
+                begin[0] = 1u;
+                n = 1;
+            }
+            while (!one) {
+                const int j = k + n + lane;
+                const int o = j < nf ? __ldcg(q.off + j) : 0x7fffffff;
+                const int d = j < nf ? __ldcg(q.delta + j) : 0;
+                const bool in = o < t1;
+                const int s = o > t0 ? o - t0 : 0;
+                if (in) slice[n + lane] = d;
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    begin[r] |= __reduce_or_sync(0xffffffffu, in && (s >> 5) == r ? 1u << (s & 31) : 0u);
+                const int c = __popc(__ballot_sync(0xffffffffu, in));
+                n += c;
+                if (c < 32) {
+                    next = __shfl_sync(0xffffffffu, o, c);
+                    break;
+                }
+            }
+            __syncwarp();
+            bool valid[4];
+            int entry[4], idx[4];
+            int before = -1;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int t = t0 + r * 32 + lane;
+                const int i = before + __popc(begin[r] & upto);
+                before += __popc(begin[r]);
+                valid[r] = t < t1;
+                entry[r] = k + i;
+                idx[r] = valid[r] ? t + slice[i] : 0;
+            }
+            op(valid, entry, idx);
+            k += next == t1 ? n : n - 1;  // the entry that holds the next tile's first edge
+            __syncwarp();
+        }
+    }
+}
+
 }  // namespace apspie

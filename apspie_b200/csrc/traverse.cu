@@ -98,160 +98,219 @@ TravBuffers carve_trav(void *base, int m) {
     return b;
 }
 
+// BFS's view of the buffers: edge queues in q0-q3, rs and loc_off, visited bitmaps in bits0-1.
+struct BfsArgs;
+void set_bfs_buffers(BfsArgs &a, const TravBuffers &b, int m, int nnz);
+
 // ================================================================================
 // BFS
 // ================================================================================
+constexpr int kBfsBlock = 256;
+constexpr int kPullSteps = 4;  // steps of four neighbours a lane scans alone in a pull level
+
 struct BfsArgs {
     int m, nnz, src, depth_cap;
     const int *__restrict__ row_ptr;
     const int *__restrict__ col_ind;
     int *depth;
-    TravBuffers buf;  // bits0 = visited, bits1/bits2 = frontier bitmaps (ping-pong)
+    EdgeQueue q[2];     // by level parity (size and empty are slots of the control block)
+    unsigned *vis[2];   // visited bitmap; a pull level reads one and writes the other
+    int shift;          // edges per queue unit: 1 << shift
     TravCtl *ctl;
     int *sticky;
     float alpha, beta;
     int allow_pull;  // pattern declared symmetric
 };
 
-// Level-synchronous BFS. Level L discovers the vertices at hop distance L.
-//  push (top-down): merge-path expansion of the frontier queue; a neighbour is claimed by
-//      an atomicOr test-and-set on the visited bitmap (the dedup that replaces the
-//      reference's radix sort, src/spmspvBfs.cuh:195-197), its depth written, and it is
-//      appended to the next queue by a warp-aggregated ballot.
+// Level-synchronous BFS, one grid barrier per level. Level L discovers the vertices at hop
+// distance L.
+//  push (top-down): the frontier is an edge queue; a neighbour is claimed by an atomicOr
+//      test-and-set on the visited bitmap (the dedup that replaces the reference's radix
+//      sort, src/spmspvBfs.cuh:195-197), its depth written, and it is appended to the next
+//      queue.
 //  pull (bottom-up): one warp per 32-vertex bitmap word; each unvisited vertex scans its
-//      row until it meets a frontier vertex (frontier bitmap built in phase A).
+//      row until it meets a visited vertex. That vertex is in the frontier: had it been
+//      visited a level earlier, its neighbour here would be visited too. So the visited
+//      bitmap as it was at the level's start is all that a pull level reads (through L1; it
+//      writes the next bitmap into the other buffer), and no frontier bitmap is kept. A lane
+//      scans its row alone for kPullSteps steps of four neighbours; what is left of longer
+//      rows the warp scans together.
 // The direction follows Beamer's rule on the edges out of the frontier (m_f) against the
 // edges still unexplored (m_u): push->pull when m_f > m_u/alpha, pull->push when the
-// frontier holds fewer than m/beta vertices. Depth results do not depend on the choice.
-__global__ void __launch_bounds__(kBlock) bfs_kernel(BfsArgs a) {
-    __shared__ BfsSmem sm;
+// frontier holds fewer than m/beta vertices; and m_f > nnz/(8 alpha), so that the last small
+// frontiers, when hardly any edge is left unexplored, don't read every row that is left (a
+// pull level of 9 us in place of a push level of 6 us at scale 20). Depth results do not
+// depend on the choice.
+//
+// What bounds it: at scale 14 the chain of dependent L2 reads in a level (queue, entry,
+// column, visited word, claim, row length, reservation) and its barrier; at scale 20 the pull
+// levels' gathers. Kernel time at scale 14 / 20 with a phase that scanned the frontier's row
+// lengths, two barriers a level and frontier bitmaps: 43.9 / 113 us; now 31 / 63 us. Blocks
+// of 256 threads, three an SM: four an SM 36 / 65 us, 512 threads 38 / 65 us, 128 threads
+// 34 / 68 us (fewer blocks make the barrier cheaper, more warps the pull levels).
+__global__ void __launch_bounds__(kBfsBlock, 3) bfs_kernel(BfsArgs a) {
+    __shared__ int s_buf[kBfsBlock / 32][kEqCap];
+    __shared__ int s_slice[kBfsBlock / 32][kEqTile];
+    __shared__ EqBlock<kBfsBlock> s_blk;
     grid_begin(a.ctl);
-    const int G = gridDim.x;
-    const int gtid = blockIdx.x * kBlock + threadIdx.x;
-    const int gstride = G * kBlock;
+    if (threadIdx.x == 0) s_blk.empty = 0;
+    const int gtid = blockIdx.x * kBfsBlock + threadIdx.x;
+    const int gstride = gridDim.x * kBfsBlock;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned before = (1u << lane) - 1u;
+    // warps of one block are far apart in the order in which work is handed out
+    const int gwarp = wid * gridDim.x + blockIdx.x, nwarps = gstride >> 5;
     const int m = a.m;
     const int words = (m + 31) >> 5;
-    unsigned *vis = a.buf.bits0;
+    const int *col = a.col_ind;
+    int *depth = a.depth;
+    // three slots: a level reads one, fills the next and clears the third
+    unsigned long long *size = a.ctl->rcnt64;
+    int *empty = a.ctl->rcnt;
 
-    for (int i = gtid; i < m; i += gstride) a.depth[i] = (i == a.src) ? 0 : -1;
-    for (int w = gtid; w < words; w += gstride) {
-        vis[w] = (w == (a.src >> 5)) ? (1u << (a.src & 31)) : 0u;
-        a.buf.bits1[w] = 0u;
-        a.buf.bits2[w] = 0u;
-    }
+    const int sr0 = __ldg(a.row_ptr + a.src), sdeg = __ldg(a.row_ptr + a.src + 1) - sr0;
+    for (int i = gtid; i < m; i += gstride) depth[i] = (i == a.src) ? 0 : -1;
+    for (int w = gtid; w < words; w += gstride) a.vis[0][w] = (w == (a.src >> 5)) ? (1u << (a.src & 31)) : 0u;
+    for (int c = gtid; sdeg > 0 && c <= (sdeg - 1) >> a.shift; c += gstride) a.q[0].owner[c] = 0;
     if (gtid == 0) {
-        a.buf.q0[0] = a.src;
-        a.ctl->qlen[0] = 1;
-        a.ctl->qlen[1] = 0;
+        a.q[0].off[0] = 0;
+        a.q[0].delta[0] = sr0;
+        size[0] = sdeg > 0 ? (1ull << 32) | static_cast<unsigned>(sdeg) : 0ull;
+        empty[0] = sdeg > 0 ? 0 : 1;
     }
     if (!grid_barrier(a.ctl, a.sticky, kSiteBfs)) return;
 
-    int cur = 0;
     bool pull = false;
-    long long visited_edges = 0, reached = 0, expanded = 0;
-    int levels = 0, npush = 0, npull = 0;
+    long long visited_edges = 0, reached = 0;
+    int levels = 0, npush = 0, npull = 0, vc = 0;
+    const double limit = static_cast<double>(m) / a.beta;  // fewer frontier vertices than this: push
+    const double tail = 0.125 * static_cast<double>(a.nnz);
     for (int L = 1;; ++L) {
-        const int nf = ld_volatile_i32(&a.ctl->qlen[cur]);
+        const int s0 = (L - 1) % 3, s1 = L % 3, s2 = (L + 1) % 3;
+        const unsigned long long sz = __ldcg(size + s0);
+        const int nq = static_cast<int>(sz >> 32), E = static_cast<int>(sz & 0xffffffffull);
+        const int nf = nq + ld_volatile_i32(empty + s0);
         if (nf == 0) break;
         if (a.depth_cap > 0 && L >= a.depth_cap) break;
-        int *qc = cur ? a.buf.q1 : a.buf.q0;
-        int *qn = cur ? a.buf.q0 : a.buf.q1;
-        unsigned *fbc = cur ? a.buf.bits2 : a.buf.bits1;
-        unsigned *fbn = cur ? a.buf.bits1 : a.buf.bits2;
-        int *qlen_next = &a.ctl->qlen[cur ^ 1];
-
-        // phase A: frontier degrees + frontier bitmap
-        frontier_phase_a<kBlock>(qc, nf, a.row_ptr, a.buf.rs, a.buf.loc_off, a.buf.chunk_sum,
-                                 sm.scan_tmp, [&](int, int v, int deg) {
-                                     atomicOr(fbc + (v >> 5), 1u << (v & 31));
-                                     return deg;
-                                 });
-        if (gtid == 0) *qlen_next = 0;
-        if (!grid_barrier(a.ctl, a.sticky, kSiteBfs + 1)) return;
-
-        const int E = frontier_chunk_bases<kBlock>(a.buf.chunk_sum, sm.base, sm.scan_tmp);
         visited_edges += E;
         reached += nf;
-        expanded += E;
         const long long m_u = static_cast<long long>(a.nnz) - visited_edges;
         if (!pull) {
             if (a.allow_pull && a.alpha > 0.0f &&
-                static_cast<double>(E) > static_cast<double>(m_u) / a.alpha)
+                static_cast<double>(E) > fmax(static_cast<double>(m_u), tail) / a.alpha)
                 pull = true;
-        } else if (static_cast<double>(nf) < static_cast<double>(m) / a.beta) {
+        } else if (static_cast<double>(nf) < limit) {
             pull = false;
         }
         ++levels;
-
-        // phase B
-        const int wid = threadIdx.x >> 5;
-        WQ wq(sm.qbuf[wid][0], qn, qlen_next);
+        if (gtid == 0) {
+            size[s2] = 0ull;
+            empty[s2] = 0;
+        }
+        EdgeQueue qc = a.q[(L - 1) & 1], qn = a.q[L & 1];
+        qn.size = size + s1;
+        qn.empty = empty + s1;
+        unsigned *vis = a.vis[vc];
+        int *buf = s_buf[wid];
+        int staged = 0;
+        // how long a next queue may get before the next level is known to pull
+        int enough_n = 0x7fffffff, enough_e = 0x7fffffff;
+        if (pull) {
+            if (limit < 2e9) enough_n = static_cast<int>(limit) + 1;
+        } else if (a.allow_pull && a.alpha > 0.0f) {
+            const double al = static_cast<double>(a.alpha);
+            const double e = fmax(static_cast<double>(m_u) / (al + 1.0), tail / al) + 1.0;
+            if (e < 2e9) enough_e = static_cast<int>(e) + 1;
+        }
+        auto append = [&](EqBlock<kBfsBlock> *blk) {
+            eq_append<kBfsBlock>(buf, staged, blk, qn, a.row_ptr, a.shift, enough_n, enough_e);
+            __syncwarp();
+            staged = 0;
+        };
         if (!pull) {
             ++npush;
-            const int *col = a.col_ind;
-            int *depth = a.depth;
-            frontier_expand<kBlock, kVT, false>(
-                nf, E, a.buf.loc_off, a.buf.rs, sm, [](int, int, BfsSlice &) {},
-                [&](const bool (&valid)[kVT], const int (&kk)[kVT], const int (&idx)[kVT],
-                    BfsSlice &) {
-                    int v[kVT];
-                    unsigned word[kVT];
+            // while few vertices are visited, claiming at once saves a trip to L2 per level; later
+            // most neighbours are visited and a look spares the atomic
+            const bool look = reached * 16 > m;
+            edge_expand(qc, nq, E, a.shift, s_slice[wid], gwarp, nwarps,
+                        [&](const bool (&valid)[4], const int (&)[4], const int (&idx)[4]) {
+                            int v[4];
+                            unsigned word[4];
+                            bool fresh[4];
 #pragma unroll
-                    for (int r = 0; r < kVT; ++r) v[r] = valid[r] ? __ldg(col + idx[r]) : 0;
+                            for (int r = 0; r < 4; ++r) v[r] = valid[r] ? __ldg(col + idx[r]) : 0;
 #pragma unroll
-                    for (int r = 0; r < kVT; ++r) word[r] = valid[r] ? __ldcg(vis + (v[r] >> 5)) : ~0u;
-                    bool fresh[kVT];
+                            for (int r = 0; r < 4; ++r)
+                                word[r] = valid[r] ? (look ? __ldcg(vis + (v[r] >> 5)) : 0u) : ~0u;
 #pragma unroll
-                    for (int r = 0; r < kVT; ++r) {
-                        const unsigned bit = 1u << (v[r] & 31);
-                        fresh[r] = false;
-                        if (valid[r] && !(word[r] & bit)) fresh[r] = !(atomicOr(vis + (v[r] >> 5), bit) & bit);
-                    }
+                            for (int r = 0; r < 4; ++r) {
+                                const unsigned bit = 1u << (v[r] & 31);
+                                fresh[r] = false;
+                                if (!(word[r] & bit)) fresh[r] = !(atomicOr(vis + (v[r] >> 5), bit) & bit);
+                            }
+                            if (staged > kEqCap - kEqTile) append(nullptr);
 #pragma unroll
-                    for (int r = 0; r < kVT; ++r) {
-                        if (fresh[r]) depth[v[r]] = L;
-                        wq.push(fresh[r], v[r]);
-                    }
-                },
-                NoPost());
-            wq.flush();
+                            for (int r = 0; r < 4; ++r) {
+                                if (fresh[r]) depth[v[r]] = L;
+                                const unsigned mask = __ballot_sync(0xffffffffu, fresh[r]);
+                                if (fresh[r]) buf[staged + __popc(mask & before)] = v[r];
+                                staged += __popc(mask);
+                            }
+                        });
         } else {
             ++npull;
-            const int lane = threadIdx.x & 31;
-            const int nwarps = gstride >> 5;
-            for (int w = gtid >> 5; w < words; w += nwarps) {
-                const unsigned vw = __ldcg(vis + w);
+            unsigned *visn = a.vis[vc ^ 1];
+            for (int w = gwarp; w < words; w += nwarps) {
+                const unsigned vw = vis[w];
                 const int v = (w << 5) + lane;
                 bool found = false;
+                int e = 0, r1 = 0;
                 if (v < m && !(vw & (1u << lane))) {
-                    const int r0 = __ldg(a.row_ptr + v), r1 = __ldg(a.row_ptr + v + 1);
-                    for (int e = r0; e < r1; ++e) {
-                        const int u = __ldg(a.col_ind + e);
-                        if (__ldcg(fbc + (u >> 5)) & (1u << (u & 31))) {
-                            found = true;
-                            break;
-                        }
+                    e = __ldg(a.row_ptr + v);
+                    r1 = __ldg(a.row_ptr + v + 1);
+                }
+#pragma unroll 1
+                for (int step = 0; step < kPullSteps && __any_sync(0xffffffffu, e < r1); ++step) {
+                    if (e < r1) {
+                        int u[4];
+                        unsigned uw[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) u[k] = __ldg(col + min(e + k, r1 - 1));
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) uw[k] = vis[u[k] >> 5];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) found |= (uw[k] >> (u[k] & 31)) & 1u;
+                        e = found ? r1 : e + 4;
                     }
                 }
-                const unsigned fm = __ballot_sync(0xffffffffu, found);
-                if (fm) {
-                    if (lane == 0) vis[w] = vw | fm;  // this warp owns word w in pull
-                    if (found) a.depth[v] = L;
-                    wq.push(found, v);
+                for (unsigned rest = __ballot_sync(0xffffffffu, e < r1); rest; rest &= rest - 1) {
+                    const int l = __ffs(rest) - 1;
+                    const int l1 = __shfl_sync(0xffffffffu, r1, l);
+                    bool hit = false;
+                    for (int b = __shfl_sync(0xffffffffu, e, l); b < l1 && !hit; b += 64) {
+                        const int u0 = __ldg(col + min(b + lane, l1 - 1)), u1 = __ldg(col + min(b + 32 + lane, l1 - 1));
+                        const unsigned w0 = vis[u0 >> 5], w1 = vis[u1 >> 5];
+                        hit = __any_sync(0xffffffffu, ((w0 >> (u0 & 31)) | (w1 >> (u1 & 31))) & 1u);
+                    }
+                    if (lane == l) found = hit;
                 }
+                const unsigned fm = __ballot_sync(0xffffffffu, found);
+                if (lane == 0) visn[w] = vw | fm;
+                if (found) depth[v] = L;
+                if (staged > kEqCap - 32) append(nullptr);
+                if (found) buf[staged + __popc(fm & before)] = v;
+                staged += __popc(fm);
             }
-            wq.flush();
+            vc ^= 1;
         }
-        // the other frontier bitmap is idle this level: clear it for level L+1
-        for (int w = gtid; w < words; w += gstride) fbn[w] = 0u;
+        append(&s_blk);
         if (!grid_barrier(a.ctl, a.sticky, kSiteBfs + 2)) return;
-        cur ^= 1;
     }
     if (gtid == 0) {
         a.ctl->iterations = levels;
         a.ctl->push_iterations = npush;
         a.ctl->pull_iterations = npull;
-        a.ctl->edges_expanded = expanded;
+        a.ctl->edges_expanded = visited_edges;
         a.ctl->edges_component = visited_edges;
         a.ctl->vertices_reached = reached;
     }
@@ -1199,6 +1258,14 @@ __global__ void spmspv_bool_kernel(int m, const int *__restrict__ row_ptr,
     }
 }
 
+void set_bfs_buffers(BfsArgs &a, const TravBuffers &b, int m, int nnz) {
+    a.q[0] = EdgeQueue{b.q0, b.q2, b.rs, nullptr, nullptr};
+    a.q[1] = EdgeQueue{b.q1, b.q3, b.loc_off, nullptr, nullptr};
+    a.vis[0] = b.bits0;
+    a.vis[1] = b.bits1;
+    a.shift = edge_unit_shift(nnz, static_cast<long long>(m) + 1);
+}
+
 apspie_status prepare_square(apspie_ctx *ctx, const apspie_csr *A, const char *who) {
     apspie_status st = check_csr_view(ctx, A, who);
     if (st != APSPIE_OK) return st;
@@ -1226,7 +1293,7 @@ constexpr size_t kNaQueueBytes = align256((kNaMaxV + 1) * sizeof(int));
 constexpr size_t kNaWordsBytes = align256(((kNaMaxV + 31) / 32) * sizeof(unsigned));
 constexpr size_t kNaCtlBytes = align256(sizeof(TravCtl)) + 256;  // control block + sticky error word
 constexpr size_t kNaBytes =
-    kNaCtlBytes + 4 * kNaQueueBytes + align256(kMaxGrid * sizeof(int)) + 3 * kNaWordsBytes;
+    kNaCtlBytes + 6 * kNaQueueBytes + 2 * kNaWordsBytes;
 
 // Shared by every apspie_bfs_noalloc call in the process (one copy per device). It keeps
 // the last call's contents; the control block is cleared at the start of each call and the
@@ -1344,7 +1411,7 @@ apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, i
     a.row_ptr = A->row_ptr;
     a.col_ind = A->col_ind;
     a.depth = d_depth;
-    a.buf = carve_trav(base, A->m);
+    set_bfs_buffers(a, carve_trav(base, A->m), A->m, A->nnz);
     a.ctl = ctx->d_ctl;
     a.sticky = ctx->d_sticky_err;
     const apspie_tune_params tp = effective_params(ctx, APSPIE_TUNE_BFS, A);
@@ -1352,7 +1419,7 @@ apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, i
     a.beta = tp.bfs_beta;
     a.allow_pull = (A->flags & APSPIE_CSR_SYMMETRIC) ? 1 : 0;
     void *args[] = {&a};
-    st = launch_persistent(ctx, reinterpret_cast<const void *>(bfs_kernel), kBlock, args, A->nnz);
+    st = launch_persistent(ctx, reinterpret_cast<const void *>(bfs_kernel), kBfsBlock, args, A->nnz);
     if (st != APSPIE_OK) return st;
     return finish_call(ctx, stats, "apspie_bfs");
 }
@@ -1582,17 +1649,15 @@ apspie_status apspie_bfs_noalloc(const apspie_csr *A, int32_t source, int32_t de
     int *sticky = reinterpret_cast<int *>(p + align256(sizeof(TravCtl)));
     p += kNaCtlBytes;
     BfsArgs a;
-    a.buf.q0 = reinterpret_cast<int *>(p);
-    a.buf.q1 = reinterpret_cast<int *>(p + kNaQueueBytes);
-    a.buf.rs = reinterpret_cast<int *>(p + 2 * kNaQueueBytes);
-    a.buf.loc_off = reinterpret_cast<int *>(p + 3 * kNaQueueBytes);
-    p += 4 * kNaQueueBytes;
-    a.buf.chunk_sum = reinterpret_cast<int *>(p);
-    p += align256(kMaxGrid * sizeof(int));
-    a.buf.bits0 = reinterpret_cast<unsigned *>(p);
-    a.buf.bits1 = reinterpret_cast<unsigned *>(p + kNaWordsBytes);
-    a.buf.bits2 = reinterpret_cast<unsigned *>(p + 2 * kNaWordsBytes);
-    a.buf.q2 = a.buf.q3 = a.buf.aux = a.buf.aux2 = nullptr;  // not used by BFS
+    TravBuffers b{};
+    int **queues[] = {&b.q0, &b.q1, &b.q2, &b.q3, &b.rs, &b.loc_off};
+    for (int **q : queues) {
+        *q = reinterpret_cast<int *>(p);
+        p += kNaQueueBytes;
+    }
+    b.bits0 = reinterpret_cast<unsigned *>(p);
+    b.bits1 = reinterpret_cast<unsigned *>(p + kNaWordsBytes);
+    set_bfs_buffers(a, b, A->m, A->nnz);
     if (cudaMemsetAsync(ctl, 0, kNaCtlBytes, stream) != cudaSuccess) return APSPIE_ERR_CUDA;
     a.m = A->m;
     a.nnz = A->nnz;
@@ -1608,7 +1673,7 @@ apspie_status apspie_bfs_noalloc(const apspie_csr *A, int32_t source, int32_t de
     a.allow_pull = (A->flags & APSPIE_CSR_SYMMETRIC) ? 1 : 0;
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_kernel, kBlock, 0) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_kernel, kBfsBlock, 0) != cudaSuccess ||
         per_sm < 1)
         return APSPIE_ERR_CUDA;
     long long grid = (static_cast<long long>(A->nnz) + kWorkPerBlock - 1) / kWorkPerBlock;
@@ -1617,7 +1682,7 @@ apspie_status apspie_bfs_noalloc(const apspie_csr *A, int32_t source, int32_t de
     if (grid > kMaxGrid) grid = kMaxGrid;
     void *args[] = {&a};
     if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(bfs_kernel), dim3(static_cast<int>(grid)),
-                                    dim3(kBlock), args, 0, stream) != cudaSuccess) {
+                                    dim3(kBfsBlock), args, 0, stream) != cudaSuccess) {
         (void)cudaGetLastError();
         return APSPIE_ERR_CUDA;
     }

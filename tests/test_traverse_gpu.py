@@ -397,3 +397,54 @@ def test_mis_int32_layout(ctx, rmat14):
     out = torch.empty(g.m, dtype=torch.int32, device="cuda")
     ctx.mis_int32_into(dg, torch.from_numpy(pr.view(np.int32)).cuda(), out)
     np.testing.assert_array_equal(out.cpu().numpy(), oracle.mis_greedy(g.row_ptr, g.col_ind, pr).astype(np.int32))
+
+
+def _csr(m, src, dst, symmetric):
+    if symmetric:
+        src, dst = np.concatenate((src, dst)), np.concatenate((dst, src))
+    key = np.unique(src.astype(np.int64) * m + dst)
+    rp = np.concatenate(([0], np.cumsum(np.bincount(key // m, minlength=m)))).astype(np.int32)
+    return ap.HostGraph(m, m, rp, (key % m).astype(np.int32), None, symmetric)
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("shape", ["star 127", "star 128", "star 129", "star 20000", "path", "dense", "hubs in a row",
+                                   "comb", "one vertex", "no edges"])
+def test_bfs_edge_queue_shapes(ctx, shape, symmetric):
+    """Rows that fill, just miss and cross an edge queue's 128-edge units and a warp's staging
+    buffer; a row of many units shared among lanes; a frontier of one entry per level; units of
+    more than a tile (mean degree above 128); rows without entries in the frontier; rows that a
+    pull level's lanes hand over to their warp. Push only, pull wherever allowed, and both."""
+    rng = np.random.default_rng(11)
+    if shape.startswith("star"):
+        k = int(shape.split()[1])
+        m, src, dst = k + 40, np.zeros(k, dtype=np.int64), np.arange(1, k + 1)
+    elif shape == "path":
+        m = 150
+        src, dst = np.arange(m - 1), np.arange(1, m)
+    elif shape == "dense":
+        m = 300
+        src, dst = np.nonzero(~np.eye(m, dtype=bool))
+    elif shape == "hubs in a row":  # vertex 0 leads to 200 vertices of 900 to 1,100 edges each
+        m = 6000
+        deg = rng.integers(900, 1100, 200)
+        src = np.concatenate((np.zeros(200, dtype=np.int64), np.repeat(np.arange(1, 201), deg)))
+        dst = np.concatenate((np.arange(1, 201), rng.integers(0, m, deg.sum())))
+    elif shape == "comb":  # long rows whose only visited vertex comes last
+        m = 3000
+        src = np.concatenate((np.full(40, m - 1), np.repeat(np.arange(40), 70)))
+        dst = np.concatenate((np.arange(40), 40 + rng.integers(0, 2000, 2800)))
+    else:
+        m = 1 if shape == "one vertex" else 70
+        src = dst = np.zeros(0, dtype=np.int64)
+    g = _csr(m, src[src != dst], dst[src != dst], symmetric)
+    dg = ap.DeviceGraph(g)
+    sources = {0, m - 1, m // 2}
+    try:
+        for alpha, beta in ((14.0, 24.0), (0.0, 24.0), (1e9, 1e9), (1e9, 2.0)):
+            ctx.set_bfs_tuning(alpha, beta)
+            for s in sources:
+                np.testing.assert_array_equal(ctx.bfs(dg, s).cpu().numpy(), oracle.bfs(g.row_ptr, g.col_ind, s),
+                                              err_msg=f"alpha {alpha} beta {beta} source {s}")
+    finally:
+        ctx.set_bfs_tuning(14.0, 24.0)
