@@ -317,10 +317,10 @@ int grid_for(const apspie_ctx *ctx, long long n) {
 
 apspie_status alloc_owned(apspie_ctx *ctx, int m, int n, long long nnz, int val_type, apspie_csr_owned *out) {
     std::memset(out, 0, sizeof(*out));
-    cudaError_t e = cudaMalloc(&out->row_ptr, (static_cast<size_t>(m) + 1) * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&out->col_ind, static_cast<size_t>(std::max(nnz, 1LL)) * 4);
+    cudaError_t e = owned_alloc(reinterpret_cast<void **>(&out->row_ptr), (static_cast<size_t>(m) + 1) * 4);
+    if (e == cudaSuccess) e = owned_alloc(reinterpret_cast<void **>(&out->col_ind), static_cast<size_t>(std::max(nnz, 1LL)) * 4);
     if (e == cudaSuccess && val_type != APSPIE_VAL_NONE)
-        e = cudaMalloc(&out->val, static_cast<size_t>(std::max(nnz, 1LL)) * 4);
+        e = owned_alloc(reinterpret_cast<void **>(&out->val), static_cast<size_t>(std::max(nnz, 1LL)) * 4);
     if (e != cudaSuccess) {
         apspie_csr_free(out);
         return cuda_error(ctx, e, "csr allocation");

@@ -114,6 +114,7 @@ struct apspie_ctx {
     unsigned long long wait_limit_ns = 0;  // grid-barrier wait bound (0: kBarrierTimeoutNs)
     unsigned long long *h_limit = nullptr;  // pinned copy of it, the source of the per-call upload
     std::vector<apspie_tune_entry> tune_table;
+    bool counted = false;  // among the contexts that keep blocks of owned matrices alive
 };
 
 namespace apspie {
@@ -198,6 +199,14 @@ size_t transpose_pattern_need(int n, long long nnz);
 apspie_status transpose_pattern(apspie_ctx *ctx, const apspie_csr *A, void *scratch, PatternCoo *out);
 // row_of[e] = the row of A's entry e.
 apspie_status expand_entry_rows(apspie_ctx *ctx, const apspie_csr *A, unsigned *row_of);
+
+// Device memory of library-owned matrices (ctx.cu): cudaMalloc behind a small cache of blocks
+// that owned_free gave back.
+cudaError_t owned_alloc(void **p, size_t bytes);
+void owned_free(void *p);
+// The process-unique id of the CUDA context current on this thread, 0 when there is none or
+// the driver cannot say.
+unsigned long long current_ctx_id();
 
 // Device-wide exclusive scan (scan.cu): out[0..n) = prefix of in, out[n] = total.
 size_t scan_scratch_bytes(long long n);

@@ -911,26 +911,26 @@ apspie_status apspie_spgemm(apspie_ctx *ctx, const apspie_csr *A, const apspie_c
     SgPlan p;
     if ((st = sg_plan(ctx, A, B, p)) != APSPIE_OK) return st;
     int32_t *rp = nullptr;
-    cudaError_t e = cudaMalloc(&rp, (static_cast<size_t>(A->m) + 1) * sizeof(int32_t));
+    cudaError_t e = owned_alloc(reinterpret_cast<void **>(&rp), (static_cast<size_t>(A->m) + 1) * sizeof(int32_t));
     if (e != cudaSuccess) return cuda_error(ctx, e, "apspie_spgemm row_ptr");
     long long nnz = 0;
     if ((st = sg_symbolic(ctx, A, B, p, rp, &nnz)) != APSPIE_OK) {
-        cudaFree(rp);
+        owned_free(rp);
         return st;
     }
     int32_t *ci = nullptr;
     void *val = nullptr;
     const size_t n = static_cast<size_t>(nnz > 0 ? nnz : 1);
-    if ((e = cudaMalloc(&ci, n * sizeof(int32_t))) != cudaSuccess ||
-        (e = cudaMalloc(&val, n * 4)) != cudaSuccess) {
-        cudaFree(rp);
-        if (ci) cudaFree(ci);
+    if ((e = owned_alloc(reinterpret_cast<void **>(&ci), n * sizeof(int32_t))) != cudaSuccess ||
+        (e = owned_alloc(reinterpret_cast<void **>(&val), n * 4)) != cudaSuccess) {
+        owned_free(rp);
+        if (ci) owned_free(ci);
         return cuda_error(ctx, e, "apspie_spgemm C");
     }
     if ((st = sg_numeric(ctx, A, B, p, rp, ci, val)) != APSPIE_OK) {
-        cudaFree(rp);
-        cudaFree(ci);
-        cudaFree(val);
+        owned_free(rp);
+        owned_free(ci);
+        owned_free(val);
         return st;
     }
     C->m = A->m;
@@ -945,9 +945,9 @@ apspie_status apspie_spgemm(apspie_ctx *ctx, const apspie_csr *A, const apspie_c
 
 void apspie_csr_free(apspie_csr_owned *C) {
     if (!C) return;
-    if (C->row_ptr) cudaFree(C->row_ptr);
-    if (C->col_ind) cudaFree(C->col_ind);
-    if (C->val) cudaFree(C->val);
+    if (C->row_ptr) owned_free(C->row_ptr);
+    if (C->col_ind) owned_free(C->col_ind);
+    if (C->val) owned_free(C->val);
     std::memset(C, 0, sizeof(*C));
 }
 

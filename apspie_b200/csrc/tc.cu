@@ -770,29 +770,29 @@ apspie_status apspie_csr_strict_lower_device(apspie_ctx *ctx, const apspie_csr *
     int *ovf = c.take<int>(16);
     cudaError_t e = cudaMemsetAsync(ovf, 0, sizeof(int), ctx->stream);
     int32_t *lrp = nullptr;
-    if (e == cudaSuccess) e = cudaMalloc(&lrp, mi * sizeof(int32_t));
+    if (e == cudaSuccess) e = owned_alloc(reinterpret_cast<void **>(&lrp), mi * sizeof(int32_t));
     if (e != cudaSuccess) return cuda_error(ctx, e, "strict lower alloc");
     const int blocks = std::max(1, std::min<int>((m * 32LL + 255) / 256, ctx->num_sms * 16));
     lower_count<<<blocks, 256, 0, ctx->stream>>>(m, A->row_ptr, A->col_ind, cnt);
     if ((st = device_exclusive_scan(ctx, cnt, m, lrp, stmp, ovf)) != APSPIE_OK) {
-        cudaFree(lrp);
+        owned_free(lrp);
         return st;
     }
     int nnz = 0;
     if ((e = cudaMemcpyAsync(&nnz, lrp + m, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) {
-        cudaFree(lrp);
+        owned_free(lrp);
         return cuda_error(ctx, e, "strict lower sync");
     }
     int32_t *lci = nullptr;
-    if ((e = cudaMalloc(&lci, std::max(nnz, 1) * sizeof(int32_t))) != cudaSuccess) {
-        cudaFree(lrp);
+    if ((e = owned_alloc(reinterpret_cast<void **>(&lci), std::max(nnz, 1) * sizeof(int32_t))) != cudaSuccess) {
+        owned_free(lrp);
         return cuda_error(ctx, e, "strict lower alloc");
     }
     lower_copy<<<blocks, 256, 0, ctx->stream>>>(m, A->row_ptr, A->col_ind, lrp, lci);
     if ((e = cudaGetLastError()) != cudaSuccess) {
-        cudaFree(lrp);
-        cudaFree(lci);
+        owned_free(lrp);
+        owned_free(lci);
         return cuda_error(ctx, e, "strict lower launch");
     }
     L->m = L->n = m;

@@ -1312,30 +1312,6 @@ struct NaEntry {
 std::vector<NaEntry> g_na_cache;
 std::mutex g_na_mu;
 
-using CtxGetCurrentFn = int (*)(void **);              // cuCtxGetCurrent(CUcontext *)
-using CtxGetIdFn = int (*)(void *, unsigned long long *);  // cuCtxGetId(CUcontext, id *)
-
-// The id of the context current on this thread, or 0 when there is none or the driver
-// cannot say (then the address is looked up on every call, which is always right).
-unsigned long long current_ctx_id() {
-    static CtxGetCurrentFn get_current = nullptr;
-    static CtxGetIdFn get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault) == cudaSuccess)
-            get_current = reinterpret_cast<CtxGetCurrentFn>(f);
-        f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault) == cudaSuccess)
-            get_id = reinterpret_cast<CtxGetIdFn>(f);
-        (void)cudaGetLastError();
-    });
-    void *c = nullptr;
-    unsigned long long id = 0;
-    if (!get_current || !get_id || get_current(&c) != 0 || !c || get_id(c, &id) != 0) return 0;
-    return id;
-}
-
 // Device address of g_bfs_noalloc_scratch in the current context, looked up (with
 // cudaGetSymbolAddress, which also loads the library's device code into the context under
 // lazy module loading) on the first call in each context.

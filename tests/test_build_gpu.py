@@ -166,3 +166,59 @@ def test_transpose_of_uneven_rows(ctx, valued, lengths):
         np.testing.assert_array_equal(tval, val[order])
     else:
         assert tval is None
+
+
+def test_matrices_from_reused_memory_in_two_threads(ctx):
+    """Memory of freed matrices is handed out again, across threads and streams: two threads
+    with contexts and streams of their own build, check and free matrices of changing sizes."""
+    import threading
+
+    import torch
+
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(seed):
+        try:
+            rng = np.random.default_rng(seed)
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream), ap.Context(0, stream) as c:
+                for k in range(12):
+                    m = int(rng.integers(2, 3000))
+                    src, dst = rng.integers(0, m, (2, 4 * m)).astype(np.int32)
+                    val = rng.integers(0, 99, 4 * m).astype(np.int32)
+                    d = [torch.from_numpy(x).cuda() for x in (src, dst, val)]
+                    A = c.build_csr(m, *d, DROP)
+                    T = c.transpose(A)
+                    A.free()  # its memory may come back for the next transpose
+                    B = c.transpose(T)
+                    got, T = B.to_numpy(), T.free()
+                    for x, y in zip(got, _ref_build(m, src, dst, val, DROP)):
+                        np.testing.assert_array_equal(x, y)
+                    B.free()
+        except BaseException as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in (1, 2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+
+
+def test_memory_kept_from_freed_matrices_is_bounded(ctx):
+    import torch
+
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    n = 60_000_000  # 240 MB a matrix
+    src = torch.zeros(1, dtype=torch.int32, device="cuda")
+    made = [ctx.build_csr(n + 20_000_000 * k, src, src) for k in range(8)]
+    assert sum(4 * c.m for c in made) > 3 << 30
+    scratch = ctx.scratch_bytes()
+    for c in made:
+        c.free()
+    torch.cuda.synchronize()
+    # at most 1 GiB of blocks, the context's scratch, and what the driver rounds up
+    assert before - torch.cuda.mem_get_info()[0] <= (1 << 30) + scratch + (64 << 20)
