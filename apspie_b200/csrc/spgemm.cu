@@ -20,9 +20,9 @@
 //  4. numeric: register tiers sort the products and sum each column's run; hash tiers
 //     accumulate values in the table, then emit the row sorted by ranking entries against
 //     a 64K-column bitmap window (prefix popcounts).
-// Bins: 0 no products | 1-3 ub <= 32 / 64 / 128: one warp per row, the row's products
-// held in registers (1, 2 or 4 per lane) and sorted by (column, product index) with a
-// register bitonic network; duplicates are then adjacent and summed in product order |
+// Bins: 0 no products | 1-3 ub <= 32 / 64 / 128: 8 or 16 lanes per row, the row's products
+// held in registers (4 or 8 per lane) and sorted by (column, product index) with a bitonic
+// network; duplicates are then adjacent and summed in product order |
 // 4 ub <= 1024: one block, 2048-slot shared table | 5-7 larger: with at most 49,152 columns
 // one block and a dense accumulator in shared memory, else (bin 5) one block and a global
 // table of >= 2*min(ub, columns) slots (power of two). Tables stay at most half full.
@@ -165,184 +165,280 @@ __global__ void sg_binlists(int m, const unsigned char *__restrict__ row_bin, in
 __device__ __forceinline__ void st_stream(float *p, float v) { __stcs(p, v); }
 __device__ __forceinline__ void st_stream(int *p, int v) { __stcs(p, v); }
 
-// ---------------------------------------------------------------- register (warp) tier
-template <int PL, typename V>
-struct RegTierSmem {
-    static constexpr int N = 32 * PL;
-    int soff[N + 1];  // exclusive product offset of each A entry
-    int bs[N];        // B row start of each A entry
-    V av[N];          // A values
-    V pv[N];          // product values, by product index
-    unsigned skey[N]; // sorted keys (numeric: walked by the head of each run)
-    int tab[2 * N];   // symbolic: hash set of the row's columns
+// ---------------------------------------------------------------- register tier
+// A group of G lanes per row of at most N = G * K products, K of them in each lane's
+// registers: 8 lanes x 4, 8 x 8 or 16 x 8.
+template <int G, int K>
+struct RegTier {
+    static constexpr int N = G * K;
+    static constexpr int WORDS = N / 32;
+    static constexpr int QB = N == 32 ? 5 : N == 64 ? 6 : 7;
+    static constexpr int ROWS = 32 / G;  // rows a warp handles side by side
+    // shared-memory words of a row: columns, values (with a word of padding after every 8, so
+    // that lanes that write 8 consecutive ranks each use different banks), A entries (two words
+    // each); the groups of a warp are 8 (16) words apart modulo the banks. Symbolic: the same
+    // words are a table of 4 N columns.
+    static constexpr int PADDED = N + N / 8;
+    static constexpr int STRIDE = 2 * PADDED + 2 * N + (N == 32 ? 0 : N == 64 ? 8 : 16);
+    __device__ static __forceinline__ int padded(int rank) { return rank + (rank >> 3); }
 };
 
-// One warp per row of at most N = 32 * PL products. Product q (element r * 32 + lane) of
-// A entry t gets the key (column << QB) | q; after a bitonic sort of the keys in registers
-// the products of one output column are adjacent and in increasing q, i.e. increasing
-// position in A's row, so a run's head sums them in the oracle's order (bit-identical
-// FP32). The symbolic pass only counts distinct columns, with a 2N-slot shared-memory hash
-// set instead of the sort. Requires B->n <= 2^24 (see bin_of).
-template <int PL, bool NUMERIC, typename V>
-__global__ void __launch_bounds__(kSgBlock) sg_reg(const int *__restrict__ rows, int nrows, Mat A, Mat B,
-                                                   int *cnt, const int *__restrict__ crp, int *cci, V *cval) {
-    constexpr int N = 32 * PL;
-    constexpr int QB = PL == 1 ? 5 : (PL == 2 ? 6 : 7);
-    constexpr unsigned QMASK = (1u << QB) - 1u;
-    constexpr unsigned PAD = 0xffffffffu;
-    using S = RegTierSmem<PL, V>;
-    __shared__ S smem[kSgBlock / 32];
-    const int lane = threadIdx.x & 31;
-    S &sm = smem[threadIdx.x >> 5];
+// Ascending sort of the group's N keys, element index sub * K + r: bitonic merges whose first
+// step compares mirrored elements, so that every comparison puts the smaller key first and no
+// direction has to be chosen. Elements of one lane are compared in registers; of the 21
+// steps for N = 64, 15 are (one lane per key took a shuffle for each).
+template <int G, int K>
+__device__ __forceinline__ void group_sort(unsigned (&key)[K], int sub) {
+    constexpr unsigned FULL = 0xffffffffu;
+#pragma unroll
+    for (int k = 2; k <= G * K; k <<= 1) {
+        if (k <= K) {
+#pragma unroll
+            for (int r = 0; r < K; ++r) {
+                const int p = r ^ (k - 1);
+                if (p > r) {
+                    const unsigned a = min(key[r], key[p]), b = max(key[r], key[p]);
+                    key[r] = a;
+                    key[p] = b;
+                }
+            }
+        } else {
+            unsigned other[K];
+#pragma unroll
+            for (int r = 0; r < K; ++r) other[r] = __shfl_xor_sync(FULL, key[K - 1 - r], k / K - 1, G);
+            const bool lower = (sub & (k / K / 2)) == 0;
+#pragma unroll
+            for (int r = 0; r < K; ++r) key[r] = lower ? min(key[r], other[r]) : max(key[r], other[r]);
+        }
+#pragma unroll
+        for (int j = k >> 2; j > 0; j >>= 1) {
+            if (j >= K) {
+                const bool lower = (sub & (j / K)) == 0;
+#pragma unroll
+                for (int r = 0; r < K; ++r) {
+                    const unsigned o = __shfl_xor_sync(FULL, key[r], j / K, G);
+                    key[r] = lower ? min(key[r], o) : max(key[r], o);
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < K; ++r) {
+                    const int p = r ^ j;
+                    if (p > r) {
+                        const unsigned a = min(key[r], key[p]), b = max(key[r], key[p]);
+                        key[r] = a;
+                        key[p] = b;
+                    }
+                }
+            }
+        }
+    }
+}
+
+template <typename V>
+__device__ __forceinline__ int as_word(V v);
+template <>
+__device__ __forceinline__ int as_word<float>(float v) { return __float_as_int(v); }
+template <>
+__device__ __forceinline__ int as_word<int>(int v) { return v; }
+template <typename V>
+__device__ __forceinline__ V from_word(int w);
+template <>
+__device__ __forceinline__ float from_word<float>(int w) { return __int_as_float(w); }
+template <>
+__device__ __forceinline__ int from_word<int>(int w) { return w; }
+
+// Product q of a row belongs to the last entry of A's row (among those whose row of B is not
+// empty) that begins at or before q: where the entries begin is an N-bit mask in every lane's
+// registers, and counting its bits gives the entry. The product gets the key
+// (column << QB) | q. Numeric: after the sort the products of one output column are adjacent
+// and in increasing q, i.e. increasing position in A's row, so a run's head sums them in the
+// oracle's order (bit-identical FP32); the row is put together in shared memory and written
+// by the whole warp. Symbolic: only the distinct columns are counted, without sorting: every
+// lane stores its keys in a table (a slot per hash of the column) and reads them back; the
+// key that is found was counted by its owner, an equal column is a repeat, anything else goes
+// into the next round with another hash. Nothing has to be cleared, and no atomics are made.
+// Requires B->n <= 2^24 (see bin_of).
+//
+// What bounds it: the shared-memory and shuffle pipe (68 % of its wavefronts in the symbolic
+// pass), then issue. C = A * A of 2^20 uniform rows of 8 (64 products each, 67M in all): one
+// warp per row, one lane per two keys, numeric 592 us and symbolic 422 us (atomicCAS table);
+// now 391 us and 215 us (numeric 515 us with ranks 8 words apart for neighbouring lanes and
+// every run looked for in shared memory).
+template <int G, int K, bool NUMERIC, typename V>
+__global__ void __launch_bounds__(kSgBlock) sg_reg(const int *__restrict__ rows, int nrows, Mat A, Mat B, int *cnt,
+                                                   const int *__restrict__ crp, int *cci, V *cval) {
+    using T = RegTier<G, K>;
+    constexpr int N = T::N, QB = T::QB, ROWS = T::ROWS, WORDS = T::WORDS;
+    constexpr unsigned QMASK = (1u << QB) - 1u, PAD = 0xffffffffu, FULL = 0xffffffffu;
+    constexpr unsigned GMASK = (1u << G) - 1u;
+    __shared__ __align__(16) int smem[kSgBlock / 32 * ROWS * T::STRIDE];
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), grp = lane / G;
+    int *row_sm = smem + ((threadIdx.x >> 5) * ROWS + grp) * T::STRIDE;
+    int *skey = row_sm, *spv = row_sm + T::PADDED, *sent = row_sm + 2 * T::PADDED;  // sent: (B position - q, A value)
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const V *aval = static_cast<const V *>(A.val);
     const V *bval = static_cast<const V *>(B.val);
-    for (int w = warp; w < nrows; w += nwarps) {
-        const int i = rows[w];
-        const int rA = __ldg(A.rp + i);
-        const int degA = __ldg(A.rp + i + 1) - rA;  // <= N by binning
-        // A entries: B row start and length, A value
-        int len[PL];
+    for (int w = warp * ROWS; w < nrows; w += nwarps * ROWS) {
+        const bool on = w + grp < nrows;
+        const int i = on ? __ldg(rows + w + grp) : 0;
+        const int rA = on ? __ldg(A.rp + i) : 0;
+        const int degA = on ? __ldg(A.rp + i + 1) - rA : 0;  // <= N by binning
+        // A's entries: rows of B that are not empty, their products' offsets
+        unsigned begin[WORDS];
 #pragma unroll
-        for (int r = 0; r < PL; ++r) {
-            const int t = r * 32 + lane;
-            len[r] = 0;
+        for (int x = 0; x < WORDS; ++x) begin[x] = 0u;
+        int ub = 0, listed = 0;
+#pragma unroll
+        for (int r = 0; r < K; ++r) {
+            if (!__any_sync(FULL, r * G < degA)) break;
+            const int t = r * G + sub;
+            int b0 = 0, len = 0;
+            V av = V(0);
             if (t < degA) {
                 const int k = __ldg(A.ci + rA + t);
-                const int b0 = __ldg(B.rp + k);
-                len[r] = __ldg(B.rp + k + 1) - b0;
-                sm.bs[t] = b0;
-                if (NUMERIC) sm.av[t] = aval[rA + t];
+                b0 = __ldg(B.rp + k);
+                len = __ldg(B.rp + k + 1) - b0;
+                if (NUMERIC) av = __ldg(aval + rA + t);
             }
-        }
-        int carry = 0;
+            int incl = len;
 #pragma unroll
-        for (int r = 0; r < PL; ++r) {
-            int incl = len[r];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
+            for (int o = 1; o < G; o <<= 1) {
+                const int y = __shfl_up_sync(FULL, incl, o, G);
+                if (sub >= o) incl += y;
             }
-            const int t = r * 32 + lane;
-            if (t < degA) sm.soff[t] = carry + incl - len[r];
-            carry += __shfl_sync(0xffffffffu, incl, 31);
+            const unsigned some = (__ballot_sync(FULL, len > 0) >> (grp * G)) & GMASK;
+            if (len > 0) {
+                const int q0 = ub + incl - len;
+                const int at = listed + __popc(some & ((1u << sub) - 1u));
+                *reinterpret_cast<int2 *>(sent + 2 * at) = make_int2(b0 - q0, NUMERIC ? as_word<V>(av) : 0);
+#pragma unroll
+                for (int x = 0; x < WORDS; ++x)
+                    if ((q0 >> 5) == x) begin[x] |= 1u << (q0 & 31);
+            }
+            listed += __popc(some);
+            ub += __shfl_sync(FULL, incl, G - 1, G);
         }
-        const int ub = carry;  // <= N by binning
-        if (lane == 0) sm.soff[degA] = ub;
+#pragma unroll
+        for (int x = 0; x < WORDS; ++x)
+#pragma unroll
+            for (int o = 1; o < G; o <<= 1) begin[x] |= __shfl_xor_sync(FULL, begin[x], o, G);
         __syncwarp();
-        // gather the products and build the keys
-        unsigned key[PL];
+        // the products, G at a time (so that neighbouring lanes read neighbouring entries of B)
+        unsigned key[K];
+        int e[K], aw[K];
 #pragma unroll
-        for (int r = 0; r < PL; ++r) {
-            const int q = r * 32 + lane;
-            key[r] = PAD;
+        for (int r = 0; r < K; ++r) {
+            const int q = r * G + sub;
+            int own = -1;
+#pragma unroll
+            for (int x = 0; x < WORDS; ++x) {
+                if (x < (r * G) / 32) own += __popc(begin[x]);
+                if (x == (r * G) / 32) own += __popc(begin[x] & (FULL >> (31 - (q & 31))));
+            }
+            e[r] = -1;
+            aw[r] = 0;
             if (q < ub) {
-                int lo = 0, hi = degA;  // last t with soff[t] <= q
-                while (hi - lo > 1) {
-                    const int mid = (lo + hi) >> 1;
-                    if (sm.soff[mid] <= q)
-                        lo = mid;
-                    else
-                        hi = mid;
-                }
-                const int e = sm.bs[lo] + (q - sm.soff[lo]);
-                key[r] = (static_cast<unsigned>(__ldg(B.ci + e)) << QB) | static_cast<unsigned>(q);
-                if (NUMERIC) sm.pv[q] = vmul<V>(sm.av[lo], bval[e]);
+                const int2 en = *reinterpret_cast<const int2 *>(sent + 2 * own);
+                e[r] = en.x + q;
+                aw[r] = en.y;
             }
         }
+#pragma unroll
+        for (int r = 0; r < K; ++r)
+            key[r] = e[r] >= 0 ? (static_cast<unsigned>(__ldg(B.ci + e[r])) << QB) | static_cast<unsigned>(r * G + sub)
+                               : PAD;
         if (!NUMERIC) {
-            // count distinct columns: insert into the (half-full at most) set
-#pragma unroll
-            for (int r = 0; r < 2 * PL; ++r) sm.tab[r * 32 + lane] = -1;
-            __syncwarp();
+            __syncwarp();  // the entries were read: their words become part of the table
             int fresh = 0;
+            unsigned todo = 0u;
 #pragma unroll
-            for (int r = 0; r < PL; ++r) {
-                if (key[r] == PAD) continue;
-                const int col = static_cast<int>(key[r] >> QB);
-                unsigned slot = (static_cast<unsigned>(col) * 2654435761u) >> (32 - (QB + 1));
-                for (int probe = 0; probe < 2 * N; ++probe) {
-                    const int old = atomicCAS(&sm.tab[slot], -1, col);
-                    if (old == -1) {
-                        ++fresh;
-                        break;
-                    }
-                    if (old == col) break;
-                    slot = (slot + 1) & (2 * N - 1);
+            for (int r = 0; r < K; ++r) todo |= key[r] != PAD ? 1u << r : 0u;
+            for (unsigned mul = 2654435761u; __any_sync(FULL, todo != 0u); mul = mul * 0x9e3779b1u + 2u) {
+                constexpr int LOG = QB + 2;  // SLOTS = 4 N
+                unsigned slot[K];
+#pragma unroll
+                for (int r = 0; r < K; ++r) {
+                    slot[r] = ((key[r] >> QB) * mul) >> (32 - LOG);
+                    if ((todo >> r) & 1u) row_sm[slot[r]] = static_cast<int>(key[r]);
                 }
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < K; ++r) {
+                    if (!((todo >> r) & 1u)) continue;
+                    const unsigned got = static_cast<unsigned>(row_sm[slot[r]]);
+                    fresh += got == key[r];
+                    if ((got ^ key[r]) <= QMASK) todo &= ~(1u << r);
+                }
+                __syncwarp();
             }
 #pragma unroll
-            for (int o = 16; o; o >>= 1) fresh += __shfl_down_sync(0xffffffffu, fresh, o);
-            if (lane == 0) cnt[i] = fresh;
-            __syncwarp();
+            for (int o = 1; o < G; o <<= 1) fresh += __shfl_xor_sync(FULL, fresh, o, G);
+            if (on && sub == 0) cnt[i] = fresh;
             continue;
         }
-        // bitonic sort of the N keys, element index r * 32 + lane
 #pragma unroll
-        for (int k = 2; k <= N; k <<= 1) {
+        for (int r = 0; r < K; ++r)
+            if (e[r] >= 0) spv[r * G + sub] = as_word<V>(vmul<V>(from_word<V>(aw[r]), __ldg(bval + e[r])));
+        group_sort<G, K>(key, sub);
+        unsigned prev = __shfl_up_sync(FULL, key[K - 1], 1, G);
+        if (sub == 0) prev = ~key[0];  // another column, whatever key[0] is
+        unsigned heads = 0u, repeats = 0u;
 #pragma unroll
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                if (j >= 32) {
+        for (int r = 0; r < K; ++r) {
+            const unsigned before = r == 0 ? prev : key[r > 0 ? r - 1 : 0];
+            if (key[r] != PAD) ((before ^ key[r]) > QMASK ? heads : repeats) |= 1u << r;
+        }
+        __syncwarp();  // the products are there
+        // a run's head sums it; its column and sum go to the run's rank
+        V sum[K];
 #pragma unroll
-                    for (int r = 0; r < PL; ++r) {
-                        const int p = r ^ (j >> 5);
-                        if (p > r) {
-                            const bool up = (((r * 32) & k) == 0);
-                            const unsigned a = key[r], b = key[p];
-                            if ((a > b) == up) {
-                                key[r] = b;
-                                key[p] = a;
-                            }
-                        }
-                    }
-                } else {
+        for (int r = 0; r < K; ++r) sum[r] = ((heads >> r) & 1u) ? from_word<V>(spv[key[r] & QMASK]) : V(0);
+        if (__any_sync(FULL, repeats != 0u)) {  // some row of the warp has equal columns: runs are walked
 #pragma unroll
-                    for (int r = 0; r < PL; ++r) {
-                        const unsigned other = __shfl_xor_sync(0xffffffffu, key[r], j);
-                        const bool up = (((r * 32 + lane) & k) == 0);
-                        const bool lower = (lane & j) == 0;
-                        key[r] = (lower == up) ? min(key[r], other) : max(key[r], other);
-                    }
+            for (int r = 0; r < K; r += 4)
+                *reinterpret_cast<uint4 *>(skey + sub * K + r) = make_uint4(key[r], key[r + 1], key[r + 2], key[r + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < K; ++r) {
+                if (!((heads >> r) & 1u)) continue;
+                if (r + 1 < K && !((repeats >> (r + 1)) & 1u)) continue;
+                for (int f = sub * K + r + 1; f < ub; ++f) {
+                    const unsigned kf = static_cast<unsigned>(skey[f]);
+                    if ((kf ^ key[r]) > QMASK) break;
+                    sum[r] = vadd<V>(sum[r], from_word<V>(spv[kf & QMASK]));
                 }
             }
         }
-        // run heads: first element of each column
-        bool head[PL];
-        unsigned hmask[PL];
+        const int mine = __popc(heads);
+        int incl = mine;
 #pragma unroll
-        for (int r = 0; r < PL; ++r) {
-            unsigned prev = __shfl_up_sync(0xffffffffu, key[r], 1);
-            if (r > 0) {
-                const unsigned last = __shfl_sync(0xffffffffu, key[r - 1], 31);
-                if (lane == 0) prev = last;
-            }
-            head[r] = key[r] != PAD && ((r == 0 && lane == 0) || (prev >> QB) != (key[r] >> QB));
-            hmask[r] = __ballot_sync(0xffffffffu, head[r]);
+        for (int o = 1; o < G; o <<= 1) {
+            const int y = __shfl_up_sync(FULL, incl, o, G);
+            if (sub >= o) incl += y;
         }
+        const int total = __shfl_sync(FULL, incl, G - 1, G);
+        const int c0 = on ? __ldg(crp + i) : 0;
+        __syncwarp();  // keys and products were read: their words take the row
+        int at = incl - mine;
 #pragma unroll
-        for (int r = 0; r < PL; ++r) sm.skey[r * 32 + lane] = key[r];
+        for (int r = 0; r < K; ++r)
+            if ((heads >> r) & 1u) {
+                skey[T::padded(at)] = static_cast<int>(key[r] >> QB);
+                spv[T::padded(at)] = as_word<V>(sum[r]);
+                ++at;
+            }
         __syncwarp();
-        const int c0 = crp[i];
-        int before = 0;
+        // streaming stores: C is written once and never re-read here, so it should not push B
+        // (re-read by every row that names it) out of L2
 #pragma unroll
-        for (int r = 0; r < PL; ++r) {
-            if (head[r]) {
-                const int rank = before + __popc(hmask[r] & ((1u << lane) - 1u));
-                const unsigned col = key[r] >> QB;
-                V sum = sm.pv[key[r] & QMASK];
-                for (int f = r * 32 + lane + 1; f < ub; ++f) {
-                    const unsigned kf = sm.skey[f];
-                    if ((kf >> QB) != col) break;
-                    sum = vadd<V>(sum, sm.pv[kf & QMASK]);
-                }
-                // streaming stores: C is written once and never re-read here, so it should
-                // not push B (re-read by every row that names it) out of L2
-                __stcs(cci + c0 + rank, static_cast<int>(col));
-                st_stream(cval + c0 + rank, sum);
+        for (int g = 0; g < ROWS; ++g) {
+            const int n = __shfl_sync(FULL, total, g * G), c = __shfl_sync(FULL, c0, g * G);
+            const int *rs = row_sm + (g - grp) * T::STRIDE;
+            for (int q = lane; q < n; q += 32) {
+                __stcs(cci + c + q, rs[T::padded(q)]);
+                st_stream(cval + c + q, from_word<V>(rs[T::PADDED + T::padded(q)]));
             }
-            before += __popc(hmask[r]);
         }
         __syncwarp();
     }
@@ -735,18 +831,19 @@ apspie_status sg_run(apspie_ctx *ctx, const apspie_csr *A, const apspie_csr *B, 
     // per-bin lists are laid out with stride m (sg_rowinfo)
     auto rows = [&](int bin) { return p.bin_rows + static_cast<long long>(bin) * m; };
     const int reg_cap = ctx->num_sms * 16;
+    auto reg_grid = [&](int n, int rows_per_warp) {
+        const int per_block = rows_per_warp * kSgBlock / 32;
+        return std::min((n + per_block - 1) / per_block, reg_cap);
+    };
     int nb = p.h.bin_count[1];
     if (nb > 0)
-        sg_reg<1, NUMERIC, V><<<std::min((nb + 7) / 8, reg_cap), kSgBlock, 0, ctx->stream>>>(rows(1), nb, a, b,
-                                                                                             p.cnt, crp, cci, cval);
+        sg_reg<8, 4, NUMERIC, V><<<reg_grid(nb, 4), kSgBlock, 0, ctx->stream>>>(rows(1), nb, a, b, p.cnt, crp, cci, cval);
     nb = p.h.bin_count[2];
     if (nb > 0)
-        sg_reg<2, NUMERIC, V><<<std::min((nb + 7) / 8, reg_cap), kSgBlock, 0, ctx->stream>>>(rows(2), nb, a, b,
-                                                                                             p.cnt, crp, cci, cval);
+        sg_reg<8, 8, NUMERIC, V><<<reg_grid(nb, 4), kSgBlock, 0, ctx->stream>>>(rows(2), nb, a, b, p.cnt, crp, cci, cval);
     nb = p.h.bin_count[3];
     if (nb > 0)
-        sg_reg<4, NUMERIC, V><<<std::min((nb + 7) / 8, reg_cap), kSgBlock, 0, ctx->stream>>>(rows(3), nb, a, b,
-                                                                                             p.cnt, crp, cci, cval);
+        sg_reg<16, 8, NUMERIC, V><<<reg_grid(nb, 2), kSgBlock, 0, ctx->stream>>>(rows(3), nb, a, b, p.cnt, crp, cci, cval);
     nb = p.h.bin_count[kBinBlock];
     if (nb > 0) {
         const int g = std::min(nb, grid_cap);

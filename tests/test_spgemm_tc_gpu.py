@@ -126,6 +126,42 @@ def test_spgemm_er_full_size_properties(ctx):
 
 
 @pytest.mark.parametrize("vt", [ap.VAL_F32, ap.VAL_I32])
+@pytest.mark.parametrize("n", [1, 9, 200, 1 << 24])
+def test_spgemm_register_tier_edges(ctx, n, vt):
+    """Rows of as many products as a register tier takes, one fewer and one more, from few
+    columns (runs of equal columns that cross lanes, one run a row, a run up to the last
+    product) to the most columns that the keys hold; more entries than products, rows of B
+    that are empty, and numbers of rows that leave groups of a warp without one. Sums are in
+    the oracle's order up to 128 products, so FP32 is compared exactly."""
+    rng = np.random.default_rng(n)
+    k = 400
+    lb = rng.integers(0, 9, k)
+    lb[:60] = 0
+    lb[60:64] = 1
+    rpb = np.concatenate(([0], np.cumsum(lb))).astype(np.int32)
+    # columns of a row may repeat: both sides treat every entry as one product
+    cib = (np.sort(rng.integers(0, n, lb.sum())) if n < 1000 else rng.integers(0, n, lb.sum())).astype(np.int32)
+    if n == 1 << 24:
+        cib[:: 7] = n - 1
+    rows = []
+    for want in (1, 2, 31, 32, 33, 63, 64, 65, 127, 128) * 3 + (5,):
+        row, left = [], want
+        while left:
+            c = int(rng.integers(60, k))
+            if lb[c] and lb[c] <= left:
+                row.append(c)
+                left -= lb[c]
+        row += [int(x) for x in rng.integers(0, 60, rng.integers(0, 20))]  # empty rows of B
+        rows.append(rng.permutation(row))
+    rpa = np.concatenate(([0], np.cumsum([len(r) for r in rows]))).astype(np.int32)
+    cia = np.concatenate(rows).astype(np.int32)
+    f32 = vt == ap.VAL_F32
+    va, vb = (rng.uniform(-1, 1, s).astype(np.float32) if f32 else rng.integers(-8, 9, s).astype(np.int32)
+              for s in (cia.shape[0], cib.shape[0]))
+    _check(ctx, ap.HostGraph(len(rows), k, rpa, cia, va), ap.HostGraph(k, n, rpb, cib, vb))
+
+
+@pytest.mark.parametrize("vt", [ap.VAL_F32, ap.VAL_I32])
 @pytest.mark.parametrize("n", [1, 31, 33, 1000, 32768, 32769, 49152, 49153])
 def test_spgemm_rows_of_many_products(ctx, n, vt):
     """Rows past the shared-table tier over few columns (dense accumulators: up to 49,152
