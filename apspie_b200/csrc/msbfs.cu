@@ -9,11 +9,18 @@
 //       (u, v) the bits fr[u] & ~visited[v] are OR-ed into next[v] (one atomicOr per
 //       non-zero word) and v is put on a touched list; a finalize pass turns next[v] into
 //       the exact new bits, writes their depths and builds the next active list;
-//  pull (many frontier vertices): one thread per vertex ORs its neighbours' frontier
-//       words restricted to its still-unvisited queries and stops as soon as every such
-//       query is covered.
-// Depths go straight to the query-major output out[q * m + v] (warp-coalesced in pull).
+//  pull (many frontier vertices): a vertex's row is scanned by a lane, eight lanes or a warp,
+//       by its length (long rows in pieces), ORing the neighbours' frontier words restricted
+//       to its still-unvisited queries, and stopping as soon as every such query is covered.
+// Depths are kept as bit planes beside the visited bits and written to the query-major output
+// out[q * m + v] at the end, every entry once.
 // The per-query answers are exactly those of independent BFS runs.
+//
+// Measured (32 queries at scale 22 / 100 at scale 20 / 512 at scale 18): a lane per row of up
+// to 128, a block per longer row, depths stored as they were found 2.44 / 1.75 / 2.95 ms; rows
+// by length 1.57 / 1.08 / 1.32 ms; bit planes 1.40 / 0.93 / 1.13 ms. What bounds it now: at
+// scale 22 the two big pull levels (0.84 ms of dependent column and frontier-word reads, 40
+// warps on an SM), then the output (0.09 ms for 537 MB, at the HBM rate).
 //
 // Active lists rotate through three queues so that the frontier buffer written at level L
 // is zeroed (by the list of level L-2) in the same phase that resets the list length,
@@ -35,7 +42,17 @@ using MsWarp = MsSmem::Warp;
 using MsWQ = WarpQueue<MsSmem::QCAP>;
 
 enum : int { kSiteMs = 400, kSiteMsBadSource = 450 };
-constexpr int kHeavyDeg = 128;  // pull: rows longer than this are scanned by a whole block
+// Pull: rows of at most kLaneDeg neighbours are scanned by a lane (up to 128 queries), of at
+// most kHeavyDeg by eight lanes, of at most kPiece by a warp, longer ones in pieces of kPiece
+// by a warp each. A row scanned by one lane costs a cache-line lookup per neighbour for the
+// column alone, and the lookups (one per SM and cycle) are what a pull level is bound by; a
+// block per row of 129 neighbours spends most of its time in its barriers, and a row of
+// 400,000 kept one block busy while all others waited (half of all warps' time at scale 22).
+constexpr int kLaneDeg = 4;
+constexpr int kHeavyDeg = 128;
+constexpr int kPiece = 2048;
+// Room for this many pieces; the rows that don't fit are scanned whole by a warp each.
+inline int piece_room(int m) { return m / 8 + 64; }
 
 // ---- continuous batching (the server's BFS engine) ----
 // The engine is the same kernel with SERVE = true: instead of a fixed set of sources it
@@ -99,14 +116,19 @@ struct MsArgs {
     const int *__restrict__ row_ptr;
     const int *__restrict__ col_ind;
     const int *__restrict__ srcs;
-    int *out;             // nq x m, pre-filled with -1 (when rows is null)
-    int *const *rows;     // else: query q's depths go to rows[q][0..m), pre-filled with -1
+    int *out;             // nq x m (when rows is null)
+    int *const *rows;     // else: query q's depths go to rows[q][0..m)
     unsigned *vis;        // m x W
     unsigned *fr[2];      // m x W each
+    // Batch: depths as bit planes, bit k of (depth + 1 - base) of every (vertex, query) in
+    // planes + k * m * W, laid out as vis; 0: not found since base (see write_depths)
+    unsigned *planes;
     unsigned *touched;    // m bits
     int *q[3];            // active lists (rotating)
     int *tq;              // touched list
-    int *heavy;           // vertices with more than kHeavyDeg neighbours (pulled by a block)
+    int *heavy;           // vertices of more than kHeavyDeg neighbours that a warp scans whole
+    int2 *pieces;         // (vertex, first entry) of the pieces of longer rows
+    int max_pieces;
     int *rs, *loc_off, *chunk_sum;
     TravCtl *ctl;         // qlen[0..1] + aux[0] used as qlen[2], aux[1] as touched length
     int *sticky;
@@ -256,16 +278,27 @@ __device__ __forceinline__ int *depth_row(const MsArgs &a, int q) {
     return a.rows ? a.rows[q] : a.out + static_cast<long long>(q) * a.m;
 }
 
-// Writes depth L + 1 of vertex v for query slot q (in the engine: relative to the level the
-// query started at, and into the row its request gave; both are copied into shared memory
-// at the start of every level: s_row, s_base).
-template <bool SERVE>
-__device__ __forceinline__ void put_depth(const MsArgs &a, int q, int v, int L, int *const *s_row,
-                                          const int *s_base) {
-    if (SERVE)
-        s_row[q][v] = L + 1 - s_base[q];
-    else
-        depth_row(a, q)[v] = L + 1;
+// Engine: writes depth L + 1 of vertex v for query slot q, relative to the level the query
+// started at, into the row its request gave (both are copied into shared memory at the start
+// of every level: s_row, s_base).
+__device__ __forceinline__ void put_depth(int q, int v, int L, int *const *s_row, const int *s_base) {
+    s_row[q][v] = L + 1 - s_base[q];
+}
+
+// Batch: the depths of the queries `bits` of word x (= v * W + w) are `code` - 1 above the
+// planes' base. ATOMIC: other warps may be setting bits of the same word.
+constexpr int kPlanes = 4;
+template <bool ATOMIC>
+__device__ __forceinline__ void set_planes(const MsArgs &a, long long mw, long long x, unsigned bits, int code) {
+#pragma unroll
+    for (int k = 0; k < kPlanes; ++k)
+        if ((code >> k) & 1) {
+            unsigned *p = a.planes + k * mw + x;
+            if (ATOMIC)
+                atomicOr(p, bits);
+            else
+                *p |= bits;
+        }
 }
 
 // Bits of word w that belong to real queries (0..nq-1).
@@ -280,8 +313,143 @@ __device__ __forceinline__ int *qlen_ptr(TravCtl *ctl, int k) {
     return k < 2 ? &ctl->qlen[k] : reinterpret_cast<int *>(&ctl->aux[0]);
 }
 
+// How a neighbour's W frontier words are read in a pull level: by LQ lanes, VW words (at most
+// 16 bytes) each, so that they cost one cache-line lookup however many words there are.
+template <int W>
+struct PullShape {
+    static constexpr int LQ = W >= 8 ? W / 4 : 1;
+    static constexpr int VW = W / LQ;
+};
+
+template <int VW>
+__device__ __forceinline__ void load_words(unsigned (&x)[VW], const unsigned *p) {
+    if constexpr (VW == 1) {
+        x[0] = *p;
+    } else if constexpr (VW == 2) {
+        const uint2 t = *reinterpret_cast<const uint2 *>(p);
+        x[0] = t.x, x[1] = t.y;
+    } else {
+        const uint4 t = *reinterpret_cast<const uint4 *>(p);
+        x[0] = t.x, x[1] = t.y, x[2] = t.z, x[3] = t.w;
+    }
+}
+
+// A group of P lanes ORs the frontier words of v's neighbours [r0, r1), restricted to need,
+// until all of it is covered; every group of the warp runs along until the last is done.
+// Lane `sub` of the group holds words [VW * (sub % LQ), ...) of need and, at the end, of got.
+// The frontier words are read through L1: nobody writes them during the level.
+template <int W, int P>
+__device__ __forceinline__ void pull_row(const int *__restrict__ col, const unsigned *frc, int r0, int r1, int sub,
+                                         const unsigned (&need)[PullShape<W>::VW],
+                                         unsigned (&got)[PullShape<W>::VW]) {
+    constexpr int LQ = PullShape<W>::LQ, VW = PullShape<W>::VW, NB = P / LQ, U = 4;
+    const int slot = sub / LQ, quad = sub % LQ;
+    const unsigned gmask = P == 32 ? 0xffffffffu : ((1u << (P & 31)) - 1u) << ((threadIdx.x & 31) - sub);
+#pragma unroll
+    for (int k = 0; k < VW; ++k) got[k] = 0u;
+    bool more = r0 < r1;
+    for (int e = r0 + slot; __any_sync(0xffffffffu, more); e += U * NB) {
+        int u[U];
+        unsigned f[U][VW];
+#pragma unroll
+        for (int t = 0; t < U; ++t) u[t] = more && e + t * NB < r1 ? __ldg(col + e + t * NB) : -1;
+#pragma unroll
+        for (int t = 0; t < U; ++t) {
+#pragma unroll
+            for (int k = 0; k < VW; ++k) f[t][k] = 0u;
+            if (u[t] >= 0) load_words<VW>(f[t], frc + static_cast<long long>(u[t]) * W + quad * VW);
+        }
+        bool all = true;
+#pragma unroll
+        for (int k = 0; k < VW; ++k) {
+#pragma unroll
+            for (int t = 0; t < U; ++t) got[k] |= f[t][k] & need[k];
+#pragma unroll
+            for (int o = LQ; o < P; o <<= 1) got[k] |= __shfl_xor_sync(0xffffffffu, got[k], o);
+            all &= got[k] == need[k];
+        }
+        const unsigned covered = __ballot_sync(0xffffffffu, all);
+        // e - slot is the same for the group's lanes
+        more = more && (covered & gmask) != gmask && e - slot + U * NB < r1;
+    }
+}
+
+// Eight bits, one into the lowest bit of each nibble.
+__device__ __forceinline__ unsigned spread_nibbles(unsigned x) {
+    x = (x | (x << 12)) & 0x000f000fu;
+    x = (x | (x << 6)) & 0x03030303u;
+    return (x | (x << 3)) & 0x11111111u;
+}
+
+// Turns the planes into depths, a warp per 128 vertices: query-major rows written once, 512
+// bytes at a time (four consecutive vertices a lane) where rows begin at multiples of 16
+// bytes, else 128 at a time (vertices 32 apart). Depths that were stored
+// as they were found (each a 4-byte write into another row, or a part of one by a warp, over
+// rows that a memset had filled before) made three quarters of the traffic of a batch. With
+// `all`, entries without a code get -1; without, they are left alone (they were written
+// before). CLEAR: the planes start over.
+template <int W, bool CLEAR>
+__device__ void write_depths(const MsArgs &a, long long mw, int base, bool all) {
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * kMsBlock + threadIdx.x) >> 5, nwarps = gridDim.x * kMsBlock / 32;
+    const bool quads = (a.m & 3) == 0 && (a.rows || (reinterpret_cast<uintptr_t>(a.out) & 15u) == 0);
+    const int step = quads ? 1 : 32;  // between a lane's vertices
+    for (int v0 = warp * 128; v0 < a.m; v0 += nwarps * 128) {
+        const int v = v0 + (quads ? 4 * lane : lane);
+        const int nv = v < a.m ? min(4, (a.m - 1 - v) / step + 1) : 0;
+#pragma unroll 1
+        for (int w = 0; w < W; ++w) {
+            unsigned p[kPlanes][4];
+#pragma unroll
+            for (int k = 0; k < kPlanes; ++k) {
+                unsigned *at = a.planes + k * mw + static_cast<long long>(v) * W + w;
+                if (W == 1 && quads && nv == 4) {  // m is a multiple of 4: every plane is 16-byte aligned
+                    const uint4 t = *reinterpret_cast<const uint4 *>(at);
+                    p[k][0] = t.x, p[k][1] = t.y, p[k][2] = t.z, p[k][3] = t.w;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) p[k][i] = i < nv ? at[i * step * W] : 0u;
+                }
+                if (CLEAR) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (i < nv) at[i * step * W] = 0u;
+                }
+            }
+            const int nq = min(32, a.nq - w * 32);
+            for (int q0 = 0; q0 < nq; q0 += 8) {
+                unsigned codes[4];  // of eight queries
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    codes[i] = 0u;
+#pragma unroll
+                    for (int k = 0; k < kPlanes; ++k) codes[i] |= spread_nibbles((p[k][i] >> q0) & 255u) << k;
+                }
+                const int n8 = min(8, nq - q0);
+                for (int q = 0; q < n8; ++q) {
+                    int d[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int code = codes[i] & 15u;
+                        codes[i] >>= 4;
+                        d[i] = code ? base + code - 1 : -1;
+                    }
+                    int *out = depth_row(a, w * 32 + q0 + q) + v;
+                    if (all && quads && nv == 4 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+                        __stcs(reinterpret_cast<int4 *>(out), make_int4(d[0], d[1], d[2], d[3]));
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if (i < nv && (all || d[i] >= 0)) __stcs(out + i * step, d[i]);
+                    }
+                }
+            }
+        }
+    }
+}
+
 template <int W, bool SERVE>
-__global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs a) {
+__global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_kernel(MsArgs a) {
     __shared__ MsSmem sm;
     __shared__ unsigned s_qmask[W];   // query slots in flight this level
     __shared__ unsigned s_alive[W];   // bits this block found in the next frontier (engine)
@@ -301,15 +469,27 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
         a.vis[i] = 0u;
         a.fr[0][i] = 0u;
         a.fr[1][i] = 0u;
+        if (!SERVE) {
+#pragma unroll
+            for (int k = 0; k < kPlanes; ++k) a.planes[k * mw + i] = 0u;
+        }
     }
     for (int w = gtid; w < (m + 31) / 32; w += gstride) a.touched[w] = 0u;
     int *hlen = reinterpret_cast<int *>(&a.ctl->aux[2]);
+    int *glen = reinterpret_cast<int *>(&a.ctl->aux[3]);
     {
         MsWQ hq(sm.qbuf[wid][0], a.heavy, hlen);
         for (int base = blockIdx.x * kMsBlock; base < m; base += gstride) {
             const int v = base + threadIdx.x;
-            const bool h = v < m && (__ldg(a.row_ptr + v + 1) - __ldg(a.row_ptr + v)) > kHeavyDeg;
-            hq.push(h, v);
+            const int d = v < m ? __ldg(a.row_ptr + v + 1) - __ldg(a.row_ptr + v) : 0;
+            bool whole = d > kHeavyDeg;
+            if (d > kPiece) {
+                const int n = (d + kPiece - 1) / kPiece, at = atomicAdd(glen, n);
+                whole = at > a.max_pieces - n;
+                for (int k = at; k < at + n && k < a.max_pieces; ++k)
+                    a.pieces[k] = whole ? make_int2(-1, 0) : make_int2(v, (k - at) * kPiece);
+            }
+            hq.push(whole, v);
         }
         hq.flush();
     }
@@ -323,7 +503,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
         s_alive[threadIdx.x] = 0u;
     }
     if (!grid_barrier(a.ctl, a.sticky, kSiteMs)) return;
-    const int nheavy = ld_volatile_i32(hlen);
+    const int nheavy = ld_volatile_i32(hlen), npieces = min(ld_volatile_i32(glen), a.max_pieces);
     // level 0: the sources (the engine admits its queries level by level instead)
     if (!SERVE) {
         MsWQ wq(sm.qbuf[wid][0], a.q[0], qlen_ptr(a.ctl, 0));
@@ -340,7 +520,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
                     const unsigned bit = 1u << (qi & 31);
                     atomicOr(a.vis + static_cast<long long>(v) * W + (qi >> 5), bit);
                     atomicOr(a.fr[0] + static_cast<long long>(v) * W + (qi >> 5), bit);
-                    depth_row(a, qi)[v] = 0;
+                    set_planes<true>(a, mw, static_cast<long long>(v) * W + (qi >> 5), bit, 1);
                     const unsigned tb = 1u << (v & 31);
                     first = !(atomicOr(a.touched + (v >> 5), tb) & tb);
                 }
@@ -362,6 +542,8 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
     const double mean_deg = m ? static_cast<double>(a.nnz) / m : 0.0;
     int prev_n = 0;  // length of the level L-1 list (all blocks read it at that level)
     int levels = 0, npush = 0, npull = 0;
+    int plane_base = 0;    // batch: a code is depth + 1 - plane_base
+    bool written = false;  // batch: every entry of the output has been written
     for (int L = 0;; ++L) {
         const int cur = L % 3, nxt = (L + 1) % 3, prv = (L + 2) % 3;
         if (SERVE) {
@@ -415,6 +597,12 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
         if (!SERVE && nA == 0) break;
         if (!SERVE && a.depth_cap > 0 && L + 1 >= a.depth_cap) break;
         ++levels;
+        if (!SERVE && L + 2 - plane_base >= 1 << kPlanes) {  // the planes are full: their depths go out
+            write_depths<W, true>(a, mw, plane_base, !written);
+            written = true;
+            plane_base = L + 1;
+        }
+        const int code = L + 2 - plane_base;  // of depth L + 1
         const unsigned *frc = a.fr[L & 1];
         unsigned *frn = a.fr[(L + 1) & 1];
         // zero the level L-1 frontier words (buffer frn) and reset the next list
@@ -424,6 +612,11 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
                 const int v = __ldcg(qp + x / W);
                 frn[static_cast<long long>(v) * W + x % W] = 0u;
             }
+        }
+        // the marks by which pieces of a row list their vertex once
+        for (int h = gtid; h < npieces; h += gstride) {
+            const int2 pc = __ldcg(a.pieces + h);
+            if (pc.x >= 0 && pc.y == 0) atomicAnd(a.touched + (pc.x >> 5), ~(1u << (pc.x & 31)));
         }
         const bool push = static_cast<double>(nA) * mean_deg < a.push_frac * a.nnz;
         int E = 0;
@@ -496,12 +689,12 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
                         if (nb) {
                             vv[w] |= nb;
                             any = true;
-                            if (SERVE) atomicOr(&s_alive[w], nb);
-                            unsigned b = nb;
-                            while (b) {
-                                const int bit = __ffs(b) - 1;
-                                b &= b - 1;
-                                put_depth<SERVE>(a, w * 32 + bit, v, L, s_row, s_base);
+                            if (SERVE) {
+                                atomicOr(&s_alive[w], nb);
+                                for (unsigned b = nb; b; b &= b - 1)
+                                    put_depth(w * 32 + __ffs(b) - 1, v, L, s_row, s_base);
+                            } else {
+                                set_planes<false>(a, mw, static_cast<long long>(v) * W + w, nb, code);
                             }
                         }
                     }
@@ -512,148 +705,186 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
         } else {
             ++npull;
             MsWQ aw(sm.qbuf[wid][1], a.q[nxt], qlen_ptr(a.ctl, nxt));
-            const unsigned lanemask_all = 0xffffffffu;
+            constexpr int LQ = PullShape<W>::LQ, VW = PullShape<W>::VW;
+            constexpr unsigned FULL = 0xffffffffu;
+            unsigned *frw = a.fr[(L + 1) & 1];
+            // the expander's slice of this warp holds the results of rows scanned by groups
+            static_assert(sizeof(MsWarp) >= 32 * (W + 1) * 4 + 32 * 4, "a warp's results fit its slice");
+            unsigned *s_got = reinterpret_cast<unsigned *>(&sm.w[wid]);
+            int *s_list = reinterpret_cast<int *>(s_got + 32 * (W + 1));
             for (int base = blockIdx.x * kMsBlock; base < m; base += gstride) {
                 const int v = base + threadIdx.x;
-                unsigned need[W], got[W];
-                bool todo = false;
+                int r0 = 0, r1 = 0;
+                bool todo = false, grouped = false;
+                unsigned got[W];
+#pragma unroll
+                for (int w = 0; w < W; ++w) got[w] = 0u;
                 if (v < m) {
+                    unsigned need[W];
                     const unsigned *vv = a.vis + static_cast<long long>(v) * W;
 #pragma unroll
-                    for (int w = 0; w < W; ++w) {
-                        need[w] = ~__ldcg(vv + w) & s_qmask[w];
-                        got[w] = 0u;
-                        todo |= need[w] != 0u;
-                    }
-                } else {
+                    for (int x = 0; x < LQ; ++x) {
+                        unsigned t[VW];
+                        load_words<VW>(t, vv + x * VW);
 #pragma unroll
-                    for (int w = 0; w < W; ++w) need[w] = got[w] = 0u;
-                }
-                int r0 = 0, r1 = 0;
-                if (todo) {
-                    r0 = __ldg(a.row_ptr + v);
-                    r1 = __ldg(a.row_ptr + v + 1);
-                    if (r1 - r0 > kHeavyDeg) todo = false;  // handled by a block below
-                }
-                if (todo) {
-                    // four neighbours per step: all their frontier words are loaded before the
-                    // coverage test, so a thread keeps several loads in flight
-                    constexpr int U = W >= 8 ? 2 : 4;
-                    for (int e0 = r0; e0 < r1; e0 += U) {
-                        int u[U];
-#pragma unroll
-                        for (int k = 0; k < U; ++k) u[k] = e0 + k < r1 ? __ldg(a.col_ind + e0 + k) : -1;
-                        unsigned f[U][W];
-#pragma unroll
-                        for (int k = 0; k < U; ++k)
-#pragma unroll
-                            for (int w = 0; w < W; ++w)
-                                f[k][w] = u[k] >= 0 ? __ldcg(frc + static_cast<long long>(u[k]) * W + w) : 0u;
-                        bool done = true;
-#pragma unroll
-                        for (int w = 0; w < W; ++w) {
-#pragma unroll
-                            for (int k = 0; k < U; ++k) got[w] |= f[k][w] & need[w];
-                            done &= got[w] == need[w];
+                        for (int k = 0; k < VW; ++k) {
+                            need[x * VW + k] = ~t[k] & s_qmask[x * VW + k];
+                            todo |= need[x * VW + k] != 0u;
                         }
-                        if (done) break;
                     }
+                    if (todo) {
+                        r0 = __ldg(a.row_ptr + v);
+                        r1 = __ldg(a.row_ptr + v + 1);
+                    }
+                    const int d = r1 - r0;
+                    grouped = d > (W <= 4 ? kLaneDeg : 0) && d <= kHeavyDeg;
+                    if (W <= 4 && d > 0 && d <= kLaneDeg) {
+                        int u[kLaneDeg];
+#pragma unroll
+                        for (int k = 0; k < kLaneDeg; ++k) u[k] = __ldg(a.col_ind + min(r0 + k, r1 - 1));
+#pragma unroll
+                        for (int k = 0; k < kLaneDeg; ++k) {
+                            unsigned f[VW];
+                            load_words<VW>(f, frc + static_cast<long long>(u[k]) * W);
+#pragma unroll
+                            for (int w = 0; w < VW; ++w) got[w] |= f[w] & need[w];
+                        }
+                    }
+                }
+                const unsigned list = __ballot_sync(FULL, grouped);
+                if (list) {
+                    if (grouped) s_list[__popc(list & ((1u << lane) - 1u))] = lane;
+                    __syncwarp();
+                    const int n = __popc(list);
+                    for (int i = 0; i < n; i += 4) {
+                        const int sub = lane & 7, mine = i + (lane >> 3);
+                        const int l = mine < n ? s_list[mine] : 0;
+                        const int b0 = __shfl_sync(FULL, r0, l), b1 = __shfl_sync(FULL, r1, l);
+                        unsigned nd[VW], g[VW];
+                        load_words<VW>(nd, a.vis + static_cast<long long>(v - lane + l) * W + (sub % LQ) * VW);
+#pragma unroll
+                        for (int k = 0; k < VW; ++k) nd[k] = ~nd[k] & s_qmask[(sub % LQ) * VW + k];
+                        pull_row<W, 8>(a.col_ind, frc, b0, mine < n ? b1 : b0, sub, nd, g);
+                        if (mine < n && sub < LQ) {
+#pragma unroll
+                            for (int k = 0; k < VW; ++k) s_got[l * (W + 1) + sub * VW + k] = g[k];
+                        }
+                    }
+                    __syncwarp();
+                    if (grouped) {
+#pragma unroll
+                        for (int w = 0; w < W; ++w) got[w] = s_got[lane * (W + 1) + w];
+                    }
+                    __syncwarp();
                 }
                 bool any = false;
-                if (v < m) {
-#pragma unroll
-                    for (int w = 0; w < W; ++w) {
-                        if (got[w]) {
-                            any = true;
-                            a.fr[(L + 1) & 1][static_cast<long long>(v) * W + w] = got[w];
-                            a.vis[static_cast<long long>(v) * W + w] |= got[w];
-                        }
-                    }
-                }
-                // depths: one coalesced store per query that any lane of the warp found
 #pragma unroll
                 for (int w = 0; w < W; ++w) {
-                    unsigned anyb = __reduce_or_sync(lanemask_all, got[w]);
-                    while (anyb) {
-                        const int bit = __ffs(anyb) - 1;
-                        anyb &= anyb - 1;
-                        if ((got[w] >> bit) & 1u) put_depth<SERVE>(a, w * 32 + bit, v, L, s_row, s_base);
+                    if (got[w]) {
+                        any = true;
+                        frw[static_cast<long long>(v) * W + w] = got[w];
+                        a.vis[static_cast<long long>(v) * W + w] |= got[w];
+                        if (!SERVE) set_planes<false>(a, mw, static_cast<long long>(v) * W + w, got[w], code);
                     }
-                    if (SERVE) {
-                        const unsigned wa = __reduce_or_sync(lanemask_all, got[w]);
-                        if (lane == 0 && wa) atomicOr(&s_alive[w], wa);
+                }
+                // engine: depths at once, one coalesced store per query that any lane found
+                if (SERVE) {
+#pragma unroll
+                    for (int w = 0; w < W; ++w) {
+                        const unsigned found = __reduce_or_sync(FULL, got[w]);
+                        for (unsigned anyb = found; anyb; anyb &= anyb - 1) {
+                            const int bit = __ffs(anyb) - 1;
+                            if ((got[w] >> bit) & 1u) put_depth(w * 32 + bit, v, L, s_row, s_base);
+                        }
+                        if (lane == 0 && found) atomicOr(&s_alive[w], found);
                     }
                 }
                 aw.push(any, v);
             }
-            aw.flush();
-            // heavy rows: one block per row, OR-reducing 256 neighbours per step and stopping
-            // as soon as every still-unvisited query of the row is covered
-            __shared__ unsigned s_need[W], s_acc[W];
-            __shared__ int s_done;
-            for (int h = blockIdx.x; h < nheavy; h += G) {
+            // long rows, a warp each
+            for (int h = gtid >> 5; h < nheavy; h += gstride >> 5) {
                 const int v = __ldcg(a.heavy + h);
                 unsigned *vv = a.vis + static_cast<long long>(v) * W;
-                if (threadIdx.x < W) {
-                    s_need[threadIdx.x] = ~__ldcg(vv + threadIdx.x) & s_qmask[threadIdx.x];
-                    s_acc[threadIdx.x] = 0u;
+                const int quad = lane % LQ;
+                unsigned nd[VW], old[VW], g[VW];
+                load_words<VW>(old, vv + quad * VW);
+                bool some = false;
+#pragma unroll
+                for (int k = 0; k < VW; ++k) {
+                    nd[k] = ~old[k] & s_qmask[quad * VW + k];
+                    some |= nd[k] != 0u;
                 }
-                __syncthreads();
-                bool need_any = false;
+                if (!__any_sync(FULL, some)) continue;
+                pull_row<W, 32>(a.col_ind, frc, __ldg(a.row_ptr + v), __ldg(a.row_ptr + v + 1), lane, nd, g);
+                bool any = false;
 #pragma unroll
-                for (int w = 0; w < W; ++w) need_any |= s_need[w] != 0u;
-                if (need_any) {
-                    const int r0 = __ldg(a.row_ptr + v), r1 = __ldg(a.row_ptr + v + 1);
-                    for (int e0 = r0; e0 < r1; e0 += kMsBlock) {
-                        const int e = e0 + threadIdx.x;
-                        unsigned bits[W];
-                        if (e < r1) {
-                            const unsigned *fu = frc + static_cast<long long>(__ldg(a.col_ind + e)) * W;
-#pragma unroll
-                            for (int w = 0; w < W; ++w) bits[w] = __ldcg(fu + w) & s_need[w];
-                        } else {
-#pragma unroll
-                            for (int w = 0; w < W; ++w) bits[w] = 0u;
-                        }
-#pragma unroll
-                        for (int w = 0; w < W; ++w) {
-                            const unsigned r = __reduce_or_sync(0xffffffffu, bits[w]);
-                            if (lane == 0 && r) atomicOr(&s_acc[w], r);
-                        }
-                        __syncthreads();
-                        if (threadIdx.x == 0) {
-                            int done = 1;
-#pragma unroll
-                            for (int w = 0; w < W; ++w) done &= s_acc[w] == s_need[w];
-                            s_done = done;
-                        }
-                        __syncthreads();
-                        if (s_done) break;
-                    }
-                    if (threadIdx.x < W) {
-                        const unsigned got = s_acc[threadIdx.x];
-                        if (got) {
-                            a.fr[(L + 1) & 1][static_cast<long long>(v) * W + threadIdx.x] = got;
-                            vv[threadIdx.x] |= got;
-                            if (SERVE) atomicOr(&s_alive[threadIdx.x], got);
-                            unsigned b = got;
-                            while (b) {
-                                const int bit = __ffs(b) - 1;
-                                b &= b - 1;
-                                put_depth<SERVE>(a, threadIdx.x * 32 + bit, v, L, s_row, s_base);
-                            }
-                        }
-                    }
-                    __syncthreads();
-                    if (threadIdx.x == 0) {
-                        bool any = false;
-#pragma unroll
-                        for (int w = 0; w < W; ++w) any |= s_acc[w] != 0u;
-                        if (any) a.q[nxt][atomicAdd(qlen_ptr(a.ctl, nxt), 1)] = v;
+                for (int w = 0; w < W; ++w) {
+                    const unsigned got = __shfl_sync(FULL, g[w % VW], w / VW);
+                    if (got == 0u) continue;
+                    any = true;
+                    if (SERVE) {
+                        if ((got >> lane) & 1u) put_depth(w * 32 + lane, v, L, s_row, s_base);
+                        if (lane == 0) atomicOr(&s_alive[w], got);
+                    } else if (lane == 0) {
+                        set_planes<false>(a, mw, static_cast<long long>(v) * W + w, got, code);
                     }
                 }
-                __syncthreads();
+                if (lane < LQ) {
+#pragma unroll
+                    for (int k = 0; k < VW; ++k)
+                        if (g[k]) {
+                            frw[static_cast<long long>(v) * W + quad * VW + k] = g[k];
+                            vv[quad * VW + k] = old[k] | g[k];
+                        }
+                }
+                aw.push(any && lane == 0, v);
             }
+            // pieces of the longest rows: what a piece finds that no other has found it writes
+            for (int h = gtid >> 5; h < npieces; h += gstride >> 5) {
+                const int2 pc = __ldcg(a.pieces + h);
+                const int v = pc.x;
+                if (v < 0) continue;
+                unsigned *vv = a.vis + static_cast<long long>(v) * W;
+                const int quad = lane % LQ;
+                unsigned nd[VW], g[VW];
+                bool some = false;
+#pragma unroll
+                for (int k = 0; k < VW; ++k) {
+                    nd[k] = ~__ldcg(vv + quad * VW + k) & s_qmask[quad * VW + k];
+                    some |= nd[k] != 0u;
+                }
+                if (!__any_sync(FULL, some)) continue;
+                const int r0 = __ldg(a.row_ptr + v) + pc.y, r1 = min(r0 + kPiece, __ldg(a.row_ptr + v + 1));
+                pull_row<W, 32>(a.col_ind, frc, r0, r1, lane, nd, g);
+                bool fresh = false;
+#pragma unroll
+                for (int k = 0; k < VW; ++k) {
+                    if (lane < LQ && g[k]) {
+                        g[k] &= ~atomicOr(frw + static_cast<long long>(v) * W + quad * VW + k, g[k]);
+                        if (g[k]) atomicOr(vv + quad * VW + k, g[k]);
+                    }
+                    fresh |= lane < LQ && g[k] != 0u;
+                }
+                if (!__any_sync(FULL, fresh)) continue;
+#pragma unroll
+                for (int w = 0; w < W; ++w) {
+                    const unsigned got = __shfl_sync(FULL, g[w % VW], w / VW);
+                    if (got == 0u) continue;
+                    if (SERVE) {
+                        if ((got >> lane) & 1u) put_depth(w * 32 + lane, v, L, s_row, s_base);
+                        if (lane == 0) atomicOr(&s_alive[w], got);
+                    } else if (lane == 0) {
+                        set_planes<true>(a, mw, static_cast<long long>(v) * W + w, got, code);
+                    }
+                }
+                bool first = false;
+                if (lane == 0) {
+                    const unsigned tb = 1u << (v & 31);
+                    first = !(atomicOr(a.touched + (v >> 5), tb) & tb);
+                }
+                aw.push(first, v);
+            }
+            aw.flush();
         }
         if (SERVE) {
             // this block's share of the next frontier's query bits: the queries still alive
@@ -666,6 +897,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : 4) msbfs_kernel(MsArgs
         if (!grid_barrier(a.ctl, a.sticky, kSiteMs + 5)) return;
         prev_n = nA;
     }
+    if (!SERVE) write_depths<W, false>(a, mw, plane_base, !written);
     if (gtid == 0) {
         a.ctl->iterations = levels;
         a.ctl->push_iterations = npush;
@@ -683,12 +915,12 @@ const void *msbfs_serve_fn() {
     return reinterpret_cast<const void *>(msbfs_kernel<W, true>);
 }
 
-size_t batch_need(int m, int Wp) {
+size_t batch_need(int m, int Wp) {  // without the depth planes of the batch
     const size_t mi = static_cast<size_t>(m) + 1;
     const size_t mw = static_cast<size_t>(m) * Wp;
     const size_t words = (static_cast<size_t>(m) + 31) / 32;
     return Carver::need({mw * 4, mw * 4, mw * 4, words * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4,
-                         kMaxGrid * 4});
+                         kMaxGrid * 4, static_cast<size_t>(piece_room(m)) * sizeof(int2)});
 }
 
 int padded_words(int nq) {
@@ -698,7 +930,10 @@ int padded_words(int nq) {
 
 }  // namespace
 
-size_t bfs_batch_scratch_need(int m, int nq) { return batch_need(m, padded_words(nq < 512 ? nq : 512)); }
+size_t bfs_batch_scratch_need(int m, int nq) {
+    const int Wp = padded_words(nq < 512 ? nq : 512);
+    return batch_need(m, Wp) + Carver::need({static_cast<size_t>(m) * Wp * 4 * kPlanes});
+}
 
 }  // namespace apspie
 
@@ -730,7 +965,8 @@ apspie_status bfs_batch_impl(apspie_ctx *ctx, const apspie_csr *A, const int32_t
         const size_t mw = static_cast<size_t>(m) * Wp;
         const size_t words = (static_cast<size_t>(m) + 31) / 32;
         void *base;
-        st = scratch_reserve(ctx, batch_need(m, Wp) + (h_rows ? Carver::need({kMaxQ * sizeof(int *)}) : 0), &base);
+        st = scratch_reserve(ctx, bfs_batch_scratch_need(m, nq) + (h_rows ? Carver::need({kMaxQ * sizeof(int *)}) : 0),
+                             &base);
         if (st != APSPIE_OK) return st;
         Carver c(base);
         MsArgs a;
@@ -747,6 +983,9 @@ apspie_status bfs_batch_impl(apspie_ctx *ctx, const apspie_csr *A, const int32_t
         a.rs = c.take<int>(mi);
         a.loc_off = c.take<int>(mi);
         a.chunk_sum = c.take<int>(kMaxGrid);
+        a.pieces = c.take<int2>(piece_room(m));
+        a.max_pieces = piece_room(m);
+        a.planes = c.take<unsigned>(mw * kPlanes);
         a.m = m;
         a.nnz = A->nnz;
         a.nq = nq;
@@ -767,18 +1006,17 @@ apspie_status bfs_batch_impl(apspie_ctx *ctx, const apspie_csr *A, const int32_t
             // pageable source: the copy is staged before the call returns
             e = cudaMemcpyAsync(table, h_rows + q0, static_cast<size_t>(nq) * sizeof(int32_t *),
                                 cudaMemcpyHostToDevice, ctx->stream);
-            for (int q = 0; q < nq && e == cudaSuccess; ++q)
-                e = cudaMemsetAsync(h_rows[q0 + q], 0xff, static_cast<size_t>(m) * sizeof(int32_t), ctx->stream);
             a.rows = table;
-        } else {
-            e = cudaMemsetAsync(a.out, 0xff, static_cast<size_t>(nq) * m * sizeof(int32_t), ctx->stream);
+            if (e != cudaSuccess) return cuda_error(ctx, e, "apspie_bfs_batch reset");
         }
-        if (e != cudaSuccess) return cuda_error(ctx, e, "apspie_bfs_batch reset");
         if ((st = reset_ctl(ctx)) != APSPIE_OK) return st;
         const void *fn = Wp == 1 ? msbfs_fn<1>() : Wp == 2 ? msbfs_fn<2>() : Wp == 4 ? msbfs_fn<4>()
                          : Wp == 8 ? msbfs_fn<8>() : msbfs_fn<16>();
         void *args[] = {&a};
-        st = launch_persistent(ctx, fn, kMsBlock, args, 1LL << 40);
+        // up to 64 queries five blocks fit on an SM: worth their dearer barriers on large graphs
+        // only (32 queries at scale 22: 1,400 us against 1,457 us, at scale 20: 482 against 473)
+        const long long blocks = A->nnz >= (1 << 26) ? kMaxGrid : 4LL * ctx->num_sms;
+        st = launch_persistent(ctx, fn, kMsBlock, args, blocks * kWorkPerBlock);
         if (st != APSPIE_OK) return st;
         if (stats) {
             apspie_run_stats part;
@@ -900,6 +1138,8 @@ apspie_status bfs_engine_launch(apspie_ctx *ctx, const apspie_csr *A, int W, Bfs
     a.rs = c.take<int>(ml);
     a.loc_off = c.take<int>(ml);
     a.chunk_sum = c.take<int>(kMaxGrid);
+    a.pieces = c.take<int2>(piece_room(m));
+    a.max_pieces = piece_room(m);
     a.sv = c.take<ServeState>(1);
     a.mb = e->d_mb;
     a.rows = a.sv->rows;

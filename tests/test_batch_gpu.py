@@ -256,3 +256,42 @@ def test_sssp_batch_label_arithmetic_limits(ctx, case, nq):
         np.testing.assert_array_equal(out[q], oracle.sssp(g.row_ptr, g.col_ind, g.val, int(s)))
     if case == "largest distances":
         assert out[0, -1] == 2 ** 31 - 2
+
+
+@pytest.mark.parametrize("nq", [1, 33, 100, 129, 300])
+@pytest.mark.parametrize("m", [4096, 4097, 9001])
+def test_bfs_batch_row_classes_and_long_paths(ctx, nq, m):
+    """Rows of every way a pull level scans them (a lane, eight lanes, a warp, pieces of 2,048
+    by several warps), output rows that begin at any multiple of 4 bytes, and a path of 40
+    vertices, so that depths pass the 15 that the bit planes hold (twice)."""
+    import torch
+
+    rng = np.random.default_rng(m + nq)
+    n = m - 40
+    src, dst = [np.arange(n - 1, m - 1)], [np.arange(n, m)]  # the path hangs off vertex n - 1
+    for hub, deg in ((0, n - 2), (1, 2500), (2, 2049), (3, 2048), (4, 129), (5, 128), (6, 5), (7, 4)):
+        src.append(np.full(min(deg, n - 1), hub))
+        dst.append(rng.choice(n, min(deg, n - 1), replace=False))
+    src.append(rng.integers(0, n, 2 * n))
+    dst.append(rng.integers(0, n, 2 * n))
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    src, dst = np.concatenate((src, dst)), np.concatenate((dst, src))
+    key = np.unique((src * m + dst)[src != dst])
+    rp = np.concatenate(([0], np.cumsum(np.bincount(key // m, minlength=m)))).astype(np.int32)
+    g = ap.HostGraph(m, m, rp, (key % m).astype(np.int32), None, True)
+    dg = ap.DeviceGraph(g)
+    sources = np.concatenate(([m - 1, 0], rng.integers(0, m, nq)))[:nq].astype(np.int32)
+    buf = torch.full((nq * m + 1,), 77, dtype=torch.int32, device="cuda")
+    try:
+        for frac in (0.05, 0.0, 1e9):
+            ctx.set_batch_push_frac(frac)
+            for first in (0, 1):
+                out = buf[first:first + nq * m].view(nq, m)
+                ctx.bfs_batch_into(dg, torch.from_numpy(sources).cuda(), out)
+                got = out.cpu().numpy()
+                for q in {0, 1 % nq, nq // 2, nq - 1}:
+                    np.testing.assert_array_equal(got[q], oracle.bfs(g.row_ptr, g.col_ind, int(sources[q])))
+    finally:
+        ctx.set_batch_push_frac(0.05)
+    cap = ctx.bfs_batch(dg, torch.from_numpy(sources[:1]).cuda(), depth_cap=18).cpu().numpy()[0]
+    np.testing.assert_array_equal(cap, ctx.bfs(dg, int(sources[0]), depth_cap=18).cpu().numpy())
