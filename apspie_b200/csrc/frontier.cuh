@@ -290,7 +290,7 @@ struct EdgeQueue {
     int *empty;                // entries without edges (counted, not stored)
 };
 
-constexpr int kEqTile = 128;  // edges a warp handles at a time: four per lane
+constexpr int kEqTile = 128;  // edges of a BFS warp at a time: four per lane
 constexpr int kEqCap = kEqTile + 32;  // vertices a warp stages before it appends them
 
 // Per block: what its warps append at the end of a phase.
@@ -303,6 +303,24 @@ struct EqBlock {
 __device__ __forceinline__ void eq_own(int *owner, int shift, int idx, int off, int deg, int first, int step) {
     const int c1 = (off + deg - 1) >> shift;
     for (int c = (off > 0 ? ((off - 1) >> shift) + 1 : 0) + first; c <= c1; c += step) owner[c] = idx;
+}
+
+// Writes entry idx (row start r0, deg > 0 edges from offset off on; nothing if !some) and its
+// units' owners; all lanes of the warp call it. A row of many units is shared out among the
+// lanes.
+__device__ __forceinline__ void eq_write(int *q_off, int *q_delta, int *q_owner, int shift, bool some, int idx, int off,
+                                         int r0, int deg) {
+    if (some) {
+        q_off[idx] = off;
+        q_delta[idx] = r0 - off;
+    }
+    const bool wide = some && deg >> shift >= 64;
+    if (some && !wide) eq_own(q_owner, shift, idx, off, deg, 0, 1);
+    for (unsigned m = __ballot_sync(0xffffffffu, wide); m; m &= m - 1) {
+        const int l = __ffs(m) - 1;
+        eq_own(q_owner, shift, __shfl_sync(0xffffffffu, idx, l), __shfl_sync(0xffffffffu, off, l),
+               __shfl_sync(0xffffffffu, deg, l), threadIdx.x & 31, 32);
+    }
 }
 
 // Appends the warp's `count` staged vertices. With blk (then every warp of the block calls it)
@@ -383,18 +401,7 @@ __device__ __forceinline__ void eq_append(const int *buf, int count, EqBlock<BLO
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
         const bool some = deg[k] > 0;
-        if (some) {
-            q.off[idx] = off;
-            q.delta[idx] = r0[k] - off;
-        }
-        // a row of many units is shared out among the lanes
-        const bool wide = deg[k] >> shift >= 64;
-        if (some && !wide) eq_own(q.owner, shift, idx, off, deg[k], 0, 1);
-        for (unsigned m = __ballot_sync(0xffffffffu, wide); m; m &= m - 1) {
-            const int l = __ffs(m) - 1;
-            eq_own(q.owner, shift, __shfl_sync(0xffffffffu, idx, l), __shfl_sync(0xffffffffu, off, l),
-                   __shfl_sync(0xffffffffu, deg[k], l), lane, 32);
-        }
+        eq_write(q.off, q.delta, q.owner, shift, some, idx, off, r0[k], deg[k]);
         idx += some;
         off += deg[k];
     }
@@ -402,19 +409,23 @@ __device__ __forceinline__ void eq_append(const int *buf, int count, EqBlock<BLO
 
 // Smallest unit (a power of two, at least a tile) for which the units of up to nnz edges fit
 // `slots` owners.
-__host__ __device__ inline int edge_unit_shift(long long nnz, long long slots) {
+__host__ __device__ inline int edge_unit_shift(long long nnz, long long slots, int tile) {
     int s = 7;
+    while ((1 << s) < tile) ++s;
     while ((nnz >> s) + 1 > slots) ++s;
     return s;
 }
 
-// op(valid, entry, idx) on every edge of the queue, four per lane (CSR positions idx[], queue
-// entries entry[]), called by all lanes of the warp. A tile's entries are read 32 at a time;
-// where each begins goes into a 128-bit mask in registers, so an edge finds its entry by
-// counting bits. `slice`: kEqTile ints of shared memory, private to the warp.
-template <class Op>
-__device__ __forceinline__ void edge_expand(const EdgeQueue &q, int nf, int E, int shift, int *slice, int gwarp,
-                                            int nwarps, Op op) {
+// op(valid, pay, idx) on every edge of the queue, VT per lane (CSR positions idx[]; with PAY,
+// pay[] is the `payload` of each edge's entry), called by all lanes of the warp. A tile's
+// entries are read 32 at a time; where each begins goes into a mask of its edges in registers, so
+// an edge finds its entry by counting bits. `slice`: 32 * VT ints of shared memory (twice as
+// many with PAY), private to the warp; units are at least a tile. (Fetching the next tile's entries, columns and weights
+// while one is worked on made SSSP slower: 650 us against 619 us at scale 20.)
+template <int VT, bool PAY, class Op>
+__device__ __forceinline__ void edge_expand(const EdgeQueue &q, const int *payload, int nf, int E, int shift,
+                                            int *slice, int gwarp, int nwarps, Op op) {
+    constexpr int TILE = 32 * VT;
     const int lane = threadIdx.x & 31;
     const unsigned upto = lane == 31 ? 0xffffffffu : (2u << lane) - 1u;
     const int units = E > 0 ? ((E - 1) >> shift) + 1 : 0;
@@ -425,12 +436,15 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, int nf, int E, i
         const bool one = u + 1 < units && __ldcg(q.owner + u + 1) == k;
         const long long uend = (static_cast<long long>(u) + 1) << shift;
         const int end = uend < E ? static_cast<int>(uend) : E;
-        for (int t0 = u << shift; t0 < end; t0 += kEqTile) {
-            const int t1 = min(t0 + kEqTile, end);
-            unsigned begin[4] = {0u, 0u, 0u, 0u};
+        for (int t0 = u << shift; t0 < end; t0 += TILE) {
+            const int t1 = min(t0 + TILE, end);
+            unsigned begin[VT];
+#pragma unroll
+            for (int r = 0; r < VT; ++r) begin[r] = 0u;
             int n = 0, next = 0x7fffffff;
             if (one) {
                 if (lane == 0) slice[0] = __ldcg(q.delta + k);
+                if (PAY && lane == 1) slice[TILE] = __ldcg(payload + k);
                 begin[0] = 1u;
                 n = 1;
             }
@@ -438,11 +452,13 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, int nf, int E, i
                 const int j = k + n + lane;
                 const int o = j < nf ? __ldcg(q.off + j) : 0x7fffffff;
                 const int d = j < nf ? __ldcg(q.delta + j) : 0;
+                const int p = PAY && j < nf ? __ldcg(payload + j) : 0;
                 const bool in = o < t1;
                 const int s = o > t0 ? o - t0 : 0;
                 if (in) slice[n + lane] = d;
+                if (PAY && in) slice[TILE + n + lane] = p;
 #pragma unroll
-                for (int r = 0; r < 4; ++r)
+                for (int r = 0; r < VT; ++r)
                     begin[r] |= __reduce_or_sync(0xffffffffu, in && (s >> 5) == r ? 1u << (s & 31) : 0u);
                 const int c = __popc(__ballot_sync(0xffffffffu, in));
                 n += c;
@@ -452,19 +468,19 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, int nf, int E, i
                 }
             }
             __syncwarp();
-            bool valid[4];
-            int entry[4], idx[4];
+            bool valid[VT];
+            int pay[VT], idx[VT];
             int before = -1;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
+            for (int r = 0; r < VT; ++r) {
                 const int t = t0 + r * 32 + lane;
                 const int i = before + __popc(begin[r] & upto);
                 before += __popc(begin[r]);
                 valid[r] = t < t1;
-                entry[r] = k + i;
                 idx[r] = valid[r] ? t + slice[i] : 0;
+                pay[r] = PAY && valid[r] ? slice[TILE + i] : 0;
             }
-            op(valid, entry, idx);
+            op(valid, pay, idx);
             k += next == t1 ? n : n - 1;  // the entry that holds the next tile's first edge
             __syncwarp();
         }

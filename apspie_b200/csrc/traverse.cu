@@ -17,35 +17,11 @@ namespace apspie {
 
 namespace {
 
-// Build-time knobs of the SSSP kernel (defaults are the tuned values).
-#ifndef APSPIE_SSSP_VT
-#define APSPIE_SSSP_VT 4
-#endif
-#ifndef APSPIE_SSSP_MINB
-#define APSPIE_SSSP_MINB 4
-#endif
-#ifndef APSPIE_SSSP_RED
-#define APSPIE_SSSP_RED 1
-#endif
-#ifndef APSPIE_SSSP_PREREAD
-#define APSPIE_SSSP_PREREAD 1
-#endif
-
-
 constexpr int kBlock = 256;
-constexpr int kVT = 4;
-using BfsSmem = ExpandSmem<kBlock, kVT, false>;
-using BfsSlice = BfsSmem::Warp;
-constexpr int kSsspVT = APSPIE_SSSP_VT;
+constexpr int kSsspVT = 4;  // edges per lane of a tile
 constexpr int kSsspPA = 4;  // frontier entries per thread per phase-A step
-using SsspSmem = ExpandSmem<kBlock, kSsspVT, false>;
-using SsspSlice = SsspSmem::Warp;
-using WQ = WarpQueue<BfsSmem::QCAP>;
-
-struct NoPost {
-    template <class S>
-    __device__ void operator()(int, S &) const {}
-};
+constexpr int kQCap = 128;  // per-warp queue staging (see WarpQueue)
+using WQ = WarpQueue<kQCap>;
 
 constexpr int kInf = 0x7fffffff;
 
@@ -67,15 +43,14 @@ enum : int {
 };
 
 struct TravBuffers {
-    int *q0, *q1, *q2, *q3, *rs, *loc_off, *chunk_sum, *aux, *aux2;
-    unsigned *bits0, *bits1, *bits2;
+    int *q0, *q1, *q2, *q3, *rs, *loc_off, *aux, *aux2, *aux3;
+    unsigned *bits0, *bits1;
 };
 
 size_t trav_scratch_bytes(int m) {
     const size_t words = (static_cast<size_t>(m) + 31) / 32;
     const size_t mi = static_cast<size_t>(m) + 1;
-    return Carver::need({mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, kMaxGrid * 4, mi * 4,
-                         mi * 4, words * 4, words * 4, words * 4});
+    return Carver::need({mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, words * 4, words * 4});
 }
 
 TravBuffers carve_trav(void *base, int m) {
@@ -89,12 +64,11 @@ TravBuffers carve_trav(void *base, int m) {
     b.q3 = c.take<int>(mi);
     b.rs = c.take<int>(mi);
     b.loc_off = c.take<int>(mi);
-    b.chunk_sum = c.take<int>(kMaxGrid);
     b.aux = c.take<int>(mi);
     b.aux2 = c.take<int>(mi);
+    b.aux3 = c.take<int>(mi);
     b.bits0 = c.take<unsigned>(words);
     b.bits1 = c.take<unsigned>(words);
-    b.bits2 = c.take<unsigned>(words);
     return b;
 }
 
@@ -232,7 +206,7 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_kernel(BfsArgs a) {
             // while few vertices are visited, claiming at once saves a trip to L2 per level; later
             // most neighbours are visited and a look spares the atomic
             const bool look = reached * 16 > m;
-            edge_expand(qc, nq, E, a.shift, s_slice[wid], gwarp, nwarps,
+            edge_expand<4, false>(qc, nullptr, nq, E, a.shift, s_slice[wid], gwarp, nwarps,
                         [&](const bool (&valid)[4], const int (&)[4], const int (&idx)[4]) {
                             int v[4];
                             unsigned word[4];
@@ -321,7 +295,6 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_kernel(BfsArgs a) {
 // ================================================================================
 struct SsspArgs {
     int m, nnz, src, delta_hint;
-    int is_float;        // weights/distances are non-negative float32 held as their bit patterns
     int unreached_bits;  // written for unreached vertices (int -1, or a float's bits)
     long long band;      // edges per iteration of the distance band; <= 0: whole frontier
     const int *__restrict__ row_ptr;
@@ -329,9 +302,11 @@ struct SsspArgs {
     const int *__restrict__ w;
     int *dist;
     // bits0 = queued in the near frontier, bits1 = held in the far pile;
-    // q0/q1 near queues, q2/q3 far piles, aux = distance snapshot of each near entry,
+    // q0/q1 near queues (vertices), q2/q3 far piles; rs, loc_off, aux3 = the edge queue of the
+    // entries expanded this iteration (off, delta, owner), aux = their distances;
     // aux2 = distance each vertex was last expanded with
     TravBuffers buf;
+    int shift;  // edges per queue unit: 1 << shift
     TravCtl *ctl;
     int *sticky;
 };
@@ -355,12 +330,21 @@ __device__ __forceinline__ int band_bin(int d, int hb, int is_float, float inv_u
     return bin < kBandBins - 1 ? bin : kBandBins - 1;
 }
 
+// The band histogram takes one vertex in kSampleOf, by a hash, with kSampleOf times its
+// degree: it only decides how much work an iteration takes on.
+constexpr int kSampleOf = 4;
+__device__ __forceinline__ bool sampled(int v) { return (static_cast<unsigned>(v) * 2654435761u) >> 30 == 0u; }
+
 struct SsspShared {
-    SsspSmem ex;
-    unsigned long long hist[kBandBins];  // this block's share of the next band histogram
+    int slice[kBlock / 32][64 * kSsspVT];  // edge_expand's
+    int near[kBlock / 32][32 * kSsspVT + 32];  // vertices on their way to the next queue,
+    int far[kBlock / 32][kQCap];          // to the far pile
+    unsigned long long hist[kBandBins];   // this block's share of the next band histogram
     unsigned long long scan[33];
-    int hmin;                            // least distance this block queued
-    int dbase;                           // where this block's deferred entries go
+    int hmin;                             // least distance this block queued
+    int dbase;                            // where this block's deferred entries go
+    unsigned long long abase;             // and its expanded entries and their edges
+    int sent[kBlock / 32];                // per warp: vertices it queues at the end, then where
 };
 
 // Min-plus SpMSpV iterated to the fixed point with near/far buckets (delta-stepping in
@@ -378,11 +362,22 @@ struct SsspShared {
 // stops after the CPU BFS depth; here a relaxation is a plain read of dist[v] and, only
 // if it improves, an atomicMin, and the loop ends when both piles are empty. The result is
 // the exact fixed point for non-negative integer weights, independent of relaxation order.
+//
+// An iteration is two phases with a grid barrier each: phase A goes through the queue (what
+// is above the band it only reads the distance of) and puts what is expanded on an edge queue;
+// phase B relaxes that queue's edges, a warp per 128. What bounds it (scale 20, 12 iterations):
+// phase B at 90-140G relaxations/s with 40 warps on an SM each waiting for a chain of queue
+// entry, column, distance (27 % of the issue slots, 28 % of L2); phase A and the barriers
+// about 14 us an iteration. Measured: merge-path tiles found by searches with block barriers
+// between batches, and every entry read in full each iteration, 709 us; edge queues 619 us;
+// reading only the distance of deferred entries and queueing per block 571 us; five blocks
+// per SM 553 us. Two, six or eight edges per lane instead of four: 596 / 623 / 580 us.
+template <bool F>
 __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
     static_assert(kBlock == kBandBins, "one histogram bin per thread");
     __shared__ SsspShared sh;
-    SsspSmem &sm = sh.ex;
     const int G = vg.n;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gtid = vg.id * kBlock + threadIdx.x;
     const int gstride = G * kBlock;
     const int m = a.m;
@@ -393,7 +388,7 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
 
     // non-negative float32 values order like their int bit patterns, so one integer
     // atomicMin serves both weight types; +inf is the float "infinity"
-    const int INF = a.is_float ? 0x7f800000 : kInf;
+    const int INF = F ? 0x7f800000 : kInf;
     for (int i = gtid; i < m; i += gstride) {
         a.dist[i] = (i == a.src) ? 0 : INF;
         last[i] = -1;
@@ -409,7 +404,7 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
         double ws = 0.0;
         for (int k = gtid; k < nsamp; k += gstride) {
             const int wb = __ldg(a.w + static_cast<long long>(k) * a.nnz / nsamp);
-            ws += a.is_float ? static_cast<double>(__int_as_float(wb)) : static_cast<double>(wb);
+            ws += F ? static_cast<double>(__int_as_float(wb)) : static_cast<double>(wb);
         }
         for (int o = 16; o; o >>= 1) ws += __shfl_down_sync(0xffffffffu, ws, o);
         if ((threadIdx.x & 31) == 0 && ws != 0.0) atomicAdd(reinterpret_cast<double *>(&a.ctl->aux[0]), ws);
@@ -422,6 +417,7 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
         a.ctl->flen[1] = 0;
         a.ctl->sbase[0] = 0;  // the source's distance
         a.ctl->sbase[1] = INF;
+        a.ctl->rcnt64[0] = a.ctl->rcnt64[1] = 0ull;
     }
     sh.hist[threadIdx.x] = 0ull;
     if (threadIdx.x == 0) sh.hmin = INF;
@@ -431,17 +427,18 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
     const double sum_w = __longlong_as_double(__ldcg(&a.ctl->aux[0]));
     const double mean_w = nsamp ? sum_w / nsamp : 1.0;
     // float distances are binned in units of mean weight / 256
-    const float inv_unit = (a.is_float && mean_w > 0.0) ? static_cast<float>(256.0 / mean_w) : 1.0f;
+    const float inv_unit = (F && mean_w > 0.0) ? static_cast<float>(256.0 / mean_w) : 1.0f;
     double delta = a.delta_hint;
     if (delta <= 0 && banded) {
         delta = 1e300;  // the band orders the work: no far pile
     } else if (delta <= 0) {
         const double mean_deg = m ? static_cast<double>(a.nnz) / m : 1.0;
         delta = 32.0 * mean_w / (mean_deg > 1.0 ? mean_deg : 1.0);
-        if (!a.is_float) delta = floor(delta);
-        if (!(delta >= 1.0)) delta = a.is_float ? (delta > 0.0 ? delta : 1.0) : 1.0;
+        if (!F) delta = floor(delta);
+        if (!(delta >= 1.0)) delta = F ? (delta > 0.0 ? delta : 1.0) : 1.0;
     }
     double thresh = delta;
+    const bool piles = delta < 1e300;
     int hb = 0;  // base of the histogram in ctl->shist[cur] (the previous iteration's base)
     int cur = 0, fc = 0;
     long long expanded = 0;
@@ -465,8 +462,8 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
             thresh += delta;
             // every block must have read qlen[cur] (== 0) before any block appends to it
             if (!grid_barrier(a.ctl, a.sticky, kSiteSsspBarF0, vg)) return;
-            WQ wn(sm.qbuf[threadIdx.x >> 5][0], qc, &a.ctl->qlen[cur]);
-            WQ wf(sm.qbuf[threadIdx.x >> 5][1], fnext, &a.ctl->flen[fc ^ 1]);
+            WQ wn(sh.near[wid], qc, &a.ctl->qlen[cur]);
+            WQ wf(sh.far[wid], fnext, &a.ctl->flen[fc ^ 1]);
             for (int base = vg.id * kBlock; base < nfar; base += gstride) {
                 const int i = base + threadIdx.x;
                 bool to_near = false, stay = false;
@@ -474,7 +471,7 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
                 if (i < nfar) {
                     v = __ldcg(fcur + i);
                     const int d = __ldcg(dist + v);
-                    const double dv = a.is_float ? static_cast<double>(__int_as_float(d)) : static_cast<double>(d);
+                    const double dv = F ? static_cast<double>(__int_as_float(d)) : static_cast<double>(d);
                     if (dv < thresh) {
                         atomicAnd(infar + (v >> 5), ~(1u << (v & 31)));
                         const unsigned bit = 1u << (v & 31);
@@ -511,19 +508,17 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
         }
         const int hb_prev = hb;
         hb = base_i;
-        const int is_float_a = a.is_float;
-
-        // phase A: dequeue (clear queued bit), snapshot distance, skip unchanged vertices;
+        // phase A: dequeue (clear queued bit), skip vertices whose distance is the one they were
+        // expanded with, put the others on the iteration's edge queue with their distance;
         // vertices above the band stay queued (re-appended to the next queue, bit kept)
+        unsigned long long *asize = a.ctl->rcnt64 + (iters & 1);
         {
-            // kSsspPA entries per thread per step, their loads issued together; the chunk
-            // layout (chunk c = entries [c*C, (c+1)*C)) is the one frontier_expand reads
+            // kSsspPA entries per thread per step, their loads issued together
             constexpr int PA = kSsspPA;
             const int C = (nf + G - 1) / G;
             const int c0 = min(vg.id * C, nf);
             const int c1 = min(c0 + C, nf);
             const int *rpa = a.row_ptr;
-            int carry = 0;
             for (int base = c0; base < c1; base += kBlock * PA) {
                 const int i0 = base + static_cast<int>(threadIdx.x) * PA;
                 int v[PA], r0[PA], r1[PA], d[PA], lst[PA], out[PA];
@@ -534,192 +529,198 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
                     v[k] = valid[k] ? __ldcg(qc + i0 + k) : 0;
                 }
 #pragma unroll
-                for (int k = 0; k < PA; ++k) {
-                    r0[k] = valid[k] ? __ldg(rpa + v[k]) : 0;
-                    r1[k] = valid[k] ? __ldg(rpa + v[k] + 1) : 0;
-                    d[k] = valid[k] ? __ldcg(dist + v[k]) : 0;
-                }
+                for (int k = 0; k < PA; ++k) d[k] = valid[k] ? __ldcg(dist + v[k]) : 0;
+                // most of a long queue is deferred: only what is expanded, and the sample of the
+                // deferred that the histogram takes, needs more than its distance
 #pragma unroll
                 for (int k = 0; k < PA; ++k) {
                     defer[k] = valid[k] && cut < kBandBins && d[k] != base_i &&
-                               band_bin(d[k], hb_prev, is_float_a, inv_unit) > cut;
-                    lst[k] = (valid[k] && !defer[k]) ? __ldcg(last + v[k]) : 0;
+                               band_bin(d[k], hb_prev, F, inv_unit) > cut;
+                    const bool row = valid[k] && (!defer[k] || sampled(v[k]));
+                    r0[k] = row ? __ldg(rpa + v[k]) : 0;
+                    r1[k] = row ? __ldg(rpa + v[k] + 1) : 0;
+                    lst[k] = valid[k] && !defer[k] ? __ldcg(last + v[k]) : 0;
                 }
-                int sum = 0;
+                int sum = 0, nact = 0, ndef = 0;
 #pragma unroll
                 for (int k = 0; k < PA; ++k) {
                     out[k] = 0;
-                    if (valid[k]) {
-                        snap[i0 + k] = d[k];
-                        a.buf.rs[i0 + k] = r0[k];
-                        if (!defer[k]) {
-                            atomicAnd(inq + (v[k] >> 5), ~(1u << (v[k] & 31)));
-                            if (lst[k] != d[k]) {
-                                last[v[k]] = d[k];
-                                out[k] = r1[k] - r0[k];
-                            }
+                    if (valid[k] && !defer[k]) {
+                        atomicAnd(inq + (v[k] >> 5), ~(1u << (v[k] & 31)));
+                        if (lst[k] != d[k]) {
+                            last[v[k]] = d[k];
+                            out[k] = r1[k] - r0[k];
                         }
                     }
                     sum += out[k];
+                    nact += out[k] > 0;
                 }
-                int ndef = 0;
 #pragma unroll
                 for (int k = 0; k < PA; ++k) {
-                    // deferred entries of a warp mostly share one bin: one atomic then
-                    const int bin = defer[k] ? band_bin(d[k], base_i, is_float_a, inv_unit) : -1;
-                    const int bin0 = __shfl_sync(0xffffffffu, bin, 0);
-                    if (__all_sync(0xffffffffu, bin == bin0)) {
-                        const unsigned tot =
-                            __reduce_add_sync(0xffffffffu, static_cast<unsigned>(min(r1[k] - r0[k], 1 << 26)));
-                        if (bin0 >= 0 && (threadIdx.x & 31) == 0)
-                            atomicAdd(&sh.hist[bin0], static_cast<unsigned long long>(tot));
-                    } else if (defer[k]) {
-                        atomicAdd(&sh.hist[bin], static_cast<unsigned long long>(r1[k] - r0[k]));
-                    }
+                    if (defer[k] && r1[k] > r0[k])
+                        atomicAdd(&sh.hist[band_bin(d[k], base_i, F, inv_unit)],
+                                  static_cast<unsigned long long>(kSampleOf) * static_cast<unsigned>(r1[k] - r0[k]));
                     const int mn = __reduce_min_sync(0xffffffffu, defer[k] ? d[k] : 0x7fffffff);
-                    if (mn != 0x7fffffff && (threadIdx.x & 31) == 0) atomicMin(&sh.hmin, mn);
+                    if (mn != 0x7fffffff && lane == 0) atomicMin(&sh.hmin, mn);
                     ndef += defer[k] ? 1 : 0;
                 }
-                // one scan carries both the edge count (high half) and the deferred count
-                // (low half, at most kBlock * PA per step, so it never carries over)
-                const unsigned long long packed =
-                    (static_cast<unsigned long long>(sum) << 32) | static_cast<unsigned>(ndef);
+                // one scan carries the edges, the expanded entries and the deferred ones (the
+                // counts at most kBlock * PA = 1024 per step, so neither carries over)
+                static_assert(kBlock * PA <= 1024, "counts fit 11 bits");
+                const unsigned long long packed = (static_cast<unsigned long long>(sum) << 22) |
+                                                  (static_cast<unsigned>(nact) << 11) | static_cast<unsigned>(ndef);
                 const unsigned long long incl = block_inclusive_scan_u64<kBlock>(packed, sh.scan);
                 const unsigned long long excl = incl - packed;
-                const unsigned long long total = sh.scan[32];
-                if (threadIdx.x == 0 && static_cast<unsigned>(total) != 0u)
-                    sh.dbase = atomicAdd(qlen_next, static_cast<int>(static_cast<unsigned>(total)));
+                if (threadIdx.x == 0) {
+                    const unsigned long long total = sh.scan[32];
+                    const unsigned td = static_cast<unsigned>(total) & 2047u, ta = static_cast<unsigned>(total >> 11) & 2047u;
+                    if (td) sh.dbase = atomicAdd(qlen_next, static_cast<int>(td));
+                    if (ta) sh.abase = atomicAdd(asize, (static_cast<unsigned long long>(ta) << 32) | (total >> 22));
+                }
                 __syncthreads();
-                int run = carry + static_cast<int>(excl >> 32);
-                int dpos = sh.dbase + static_cast<int>(static_cast<unsigned>(excl));
+                const unsigned long long ab = sh.abase;
+                int idx = static_cast<int>(ab >> 32) + static_cast<int>(static_cast<unsigned>(excl >> 11) & 2047u);
+                int off = static_cast<int>(ab & 0xffffffffull) + static_cast<int>(excl >> 22);
+                int dpos = sh.dbase + static_cast<int>(static_cast<unsigned>(excl) & 2047u);
 #pragma unroll
                 for (int k = 0; k < PA; ++k) {
-                    if (valid[k]) a.buf.loc_off[i0 + k] = run;
-                    run += out[k];
+                    const bool some = out[k] > 0;
+                    eq_write(a.buf.rs, a.buf.loc_off, a.buf.aux3, a.shift, some, idx, off, r0[k], out[k]);
+                    if (some) snap[idx] = d[k];
+                    idx += some;
+                    off += out[k];
                     if (defer[k]) qn[dpos++] = v[k];
                 }
-                carry += static_cast<int>(total >> 32);
-                __syncthreads();  // sh.scan and sh.dbase are reused by the next step
+                __syncthreads();  // sh.scan and the bases are reused by the next step
             }
-            if (threadIdx.x == 0) a.buf.chunk_sum[vg.id] = carry;
         }
         if (!grid_barrier(a.ctl, a.sticky, kSiteSsspBarA, vg)) return;
-        // every block has read this queue's length, base and histogram: reset them for the
-        // iteration that fills this queue next
+        // every block has read this queue's length, base and histogram, and the last iteration's
+        // edge queue: reset them for the iteration that fills them next
         if (gtid < kBandBins) a.ctl->shist[cur][gtid] = 0ull;
         if (gtid == 0) {
             a.ctl->qlen[cur] = 0;
             a.ctl->sbase[cur] = INF;
+            a.ctl->rcnt64[(iters & 1) ^ 1] = 0ull;
         }
-
-        const int E = frontier_chunk_bases<kBlock>(a.buf.chunk_sum, sm.base, sm.scan_tmp, vg);
+        const unsigned long long asz = __ldcg(asize);
+        const int nact = static_cast<int>(asz >> 32), E = static_cast<int>(asz & 0xffffffffull);
         expanded += E;
         ++iters;
         const int *col = a.col_ind;
         const int *wt = a.w;
         const int *rp = a.row_ptr;
-        TravCtl *ctl = a.ctl;
-        int *sticky = a.sticky;
-        int *flen = &a.ctl->flen[fc];
-        const double T = thresh;
-        const int is_float = a.is_float;
-        WQ wn(sm.qbuf[threadIdx.x >> 5][0], qn, qlen_next);
-        WQ wf(sm.qbuf[threadIdx.x >> 5][1], fcur, flen);
-        auto relax = [&](const bool (&valid)[kSsspVT], const int (&kk)[kSsspVT], const int (&idx)[kSsspVT],
-                         auto &ws) {
-                constexpr int kVT = kSsspVT;
-                int v[kVT], we[kVT], cd[kVT], nd[kVT];
-                bool imp[kVT];
+        // nd < Tkey exactly when the distance nd (bits, if float) is below thresh
+        const int Tkey = F ? __float_as_int(__double2float_ru(thresh))
+                           : thresh < 2147483647.0 ? static_cast<int>(ceil(thresh)) : kInf;
+        int *near = sh.near[wid];
+        int staged = 0;
+        const unsigned before = (1u << lane) - 1u;
+        auto send = [&]() {  // staged vertices -> next queue
+            __syncwarp();
+            int at = 0;
+            if (lane == 0) at = atomicAdd(qlen_next, staged);
+            at = __shfl_sync(0xffffffffu, at, 0);
+            for (int i = lane; i < staged; i += 32) qn[at + i] = near[i];
+            __syncwarp();
+            staged = 0;
+        };
+        WQ wf(sh.far[wid], fcur, &a.ctl->flen[fc]);
+        bool bad = false, over = false;
+        EdgeQueue qa{a.buf.rs, a.buf.loc_off, a.buf.aux3, nullptr, nullptr};
+        edge_expand<kSsspVT, true>(
+            qa, snap, nact, E, a.shift, sh.slice[wid], wid * G + vg.id, G * (kBlock / 32),
+            [&](const bool (&valid)[kSsspVT], const int (&du)[kSsspVT], const int (&idx)[kSsspVT]) {
+                int v[kSsspVT], we[kSsspVT], cd[kSsspVT], nd[kSsspVT];
+                bool got[kSsspVT], queue[kSsspVT];
 #pragma unroll
-                for (int r = 0; r < kVT; ++r) {
+                for (int r = 0; r < kSsspVT; ++r) {
                     v[r] = valid[r] ? __ldg(col + idx[r]) : 0;
                     we[r] = valid[r] ? __ldg(wt + idx[r]) : 0;
                 }
-                // plain (L1-cacheable) reads: a stale, larger value only costs an extra atomic
+                // coherent reads; a slot without an edge relaxes 0 + 0 against 0
 #pragma unroll
-                for (int r = 0; r < kVT; ++r)
-                    cd[r] = (valid[r] && APSPIE_SSSP_PREREAD) ? (APSPIE_SSSP_RED ? __ldcg(dist + v[r]) : dist[v[r]]) : INF;
+                for (int r = 0; r < kSsspVT; ++r) cd[r] = valid[r] ? __ldcg(dist + v[r]) : 0;
 #pragma unroll
-                for (int r = 0; r < kVT; ++r) {
-                    imp[r] = false;
-                    nd[r] = 0;
-                    if (!valid[r]) continue;
-                    if (is_float) {
-                        const float wf = __int_as_float(we[r]);
-                        if (!(wf >= 0.0f)) {  // negative or NaN
-                            raise_error(ctl, sticky, APSPIE_ERR_INVALID_ARG, kSiteSsspNegWeight);
-                        } else {
-                            nd[r] = __float_as_int(__fadd_rn(__int_as_float(ws.aux[kk[r]]), wf));
-                            imp[r] = nd[r] < cd[r];
-                        }
-                        continue;
-                    }
-                    const long long d = static_cast<long long>(ws.aux[kk[r]]) + we[r];
-                    if (we[r] < 0) {
-                        raise_error(ctl, sticky, APSPIE_ERR_INVALID_ARG, kSiteSsspNegWeight);
-                    } else if (d >= kInf) {
-                        raise_error(ctl, sticky, APSPIE_ERR_INVALID_ARG, kSiteSsspOverflow);
+                for (int r = 0; r < kSsspVT; ++r) {
+                    if (F) {
+                        const float wf32 = __int_as_float(we[r]);
+                        const bool ok = wf32 >= 0.0f;  // neither negative nor NaN
+                        bad |= !ok;
+                        nd[r] = __float_as_int(__fadd_rn(__int_as_float(du[r]), wf32));
+                        got[r] = ok && nd[r] < cd[r];
                     } else {
-                        nd[r] = static_cast<int>(d);
-                        imp[r] = nd[r] < cd[r];
+                        // both below 2^31, so the sum does not wrap; a sum past INT_MAX - 1 is
+                        // never below cd
+                        const unsigned s = static_cast<unsigned>(du[r]) + static_cast<unsigned>(we[r]);
+                        bad |= we[r] < 0;
+                        over |= s >= 0x7fffffffu;
+                        nd[r] = static_cast<int>(s);
+                        got[r] = we[r] >= 0 && s < static_cast<unsigned>(cd[r]);
                     }
                 }
-                bool got[kVT];  // the relaxation lowered v's distance
 #pragma unroll
-                for (int r = 0; r < kVT; ++r) {
-                    if (APSPIE_SSSP_RED) {
-                        if (imp[r]) atomicMin(dist + v[r], nd[r]);
-                        got[r] = imp[r];
-                    } else {
-                        got[r] = imp[r] && nd[r] < atomicMin(dist + v[r], nd[r]);
-                    }
-                }
-                bool near[kVT], far[kVT];
+                for (int r = 0; r < kSsspVT; ++r)
+                    if (got[r]) atomicMin(dist + v[r], nd[r]);
 #pragma unroll
-                for (int r = 0; r < kVT; ++r) {
-                    near[r] = far[r] = false;
-                    if (got[r]) {
+                for (int r = 0; r < kSsspVT; ++r) {
+                    queue[r] = false;
+                    if (got[r] && nd[r] < Tkey) {
                         const unsigned bit = 1u << (v[r] & 31);
-                        const double ndv = is_float ? static_cast<double>(__int_as_float(nd[r]))
-                                                    : static_cast<double>(nd[r]);
-                        if (ndv < T)
-                            near[r] = !(atomicOr(inq + (v[r] >> 5), bit) & bit);
-                        else
-                            far[r] = !(atomicOr(infar + (v[r] >> 5), bit) & bit);
+                        queue[r] = !(atomicOr(inq + (v[r] >> 5), bit) & bit);
                     }
                 }
                 if (banded) {
-                    // every improvement below T (queued now or already) enters the next
-                    // band histogram at its new distance (improvements are a few percent of
-                    // the relaxations, so plain shared-memory atomics rarely collide)
-                    bool rec[kVT];
-                    int dg[kVT];
+                    // improvements below T (queued now or already): a sample enters the next band
+                    // histogram at their new distance; the least distance is exact
 #pragma unroll
-                    for (int r = 0; r < kVT; ++r) {
-                        rec[r] = got[r] &&
-                                 (is_float ? static_cast<double>(__int_as_float(nd[r]))
-                                           : static_cast<double>(nd[r])) < T;
-                        dg[r] = rec[r] ? __ldg(rp + v[r] + 1) - __ldg(rp + v[r]) : 0;
-                    }
-#pragma unroll
-                    for (int r = 0; r < kVT; ++r) {
-                        if (!rec[r]) continue;
-                        atomicAdd(&sh.hist[band_bin(nd[r], base_i, is_float, inv_unit)],
-                                  static_cast<unsigned long long>(dg[r]));
-                        atomicMin(&sh.hmin, nd[r]);
+                    for (int r = 0; r < kSsspVT; ++r) {
+                        if (!(got[r] && nd[r] < Tkey)) continue;
+                        if (nd[r] < *static_cast<volatile int *>(&sh.hmin)) atomicMin(&sh.hmin, nd[r]);
+                        if (sampled(v[r]))
+                            atomicAdd(&sh.hist[band_bin(nd[r], base_i, F, inv_unit)],
+                                      static_cast<unsigned long long>(kSampleOf) *
+                                          static_cast<unsigned>(__ldg(rp + v[r] + 1) - __ldg(rp + v[r])));
                     }
                 }
+                if (staged > 32) send();
 #pragma unroll
-                for (int r = 0; r < kVT; ++r) {
-                    wn.push(near[r], v[r]);
-                    wf.push(far[r], v[r]);
+                for (int r = 0; r < kSsspVT; ++r) {
+                    const unsigned mask = __ballot_sync(0xffffffffu, queue[r]);
+                    if (queue[r]) near[staged + __popc(mask & before)] = v[r];
+                    staged += __popc(mask);
                 }
-            };
-        frontier_expand<kBlock, kSsspVT, false>(
-            nf, E, a.buf.loc_off, a.buf.rs, sm, [&](int jj, int k, SsspSlice &w) { w.aux[k] = __ldcg(snap + jj); },
-            relax, NoPost(), vg);
-        wn.flush();
+                if (piles) {
+#pragma unroll
+                    for (int r = 0; r < kSsspVT; ++r) {
+                        bool far = false;
+                        if (got[r] && nd[r] >= Tkey) {
+                            const unsigned bit = 1u << (v[r] & 31);
+                            far = !(atomicOr(infar + (v[r] >> 5), bit) & bit);
+                        }
+                        wf.push(far, v[r]);
+                    }
+                }
+            });
+        // what is still staged goes out for the whole block at once (4,736 reservations on one
+        // word, one after the other, took most of the 10 us at the end of an iteration)
+        if (lane == 0) sh.sent[wid] = staged;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int all = 0;
+            for (int w = 0; w < kBlock / 32; ++w) {
+                const int c = sh.sent[w];
+                sh.sent[w] = all;
+                all += c;
+            }
+            const int at = all ? atomicAdd(qlen_next, all) : 0;
+            for (int w = 0; w < kBlock / 32; ++w) sh.sent[w] += at;
+        }
+        __syncthreads();
+        for (int i = lane; i < staged; i += 32) qn[sh.sent[wid] + i] = near[i];
         wf.flush();
+        if (bad) raise_error(a.ctl, a.sticky, APSPIE_ERR_INVALID_ARG, kSiteSsspNegWeight);
+        if (over) raise_error(a.ctl, a.sticky, APSPIE_ERR_INVALID_ARG, kSiteSsspOverflow);
         if (banded) {
             __syncthreads();
             const unsigned long long hv = sh.hist[threadIdx.x];
@@ -765,9 +766,10 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
     }
 }
 
-__global__ void __launch_bounds__(kBlock, APSPIE_SSSP_MINB) sssp_kernel(SsspArgs a) {
+template <bool F>
+__global__ void __launch_bounds__(kBlock, 5) sssp_kernel(SsspArgs a) {
     grid_begin(a.ctl);
-    sssp_body(a, hw_grid());
+    sssp_body<F>(a, hw_grid());
 }
 
 // Many sources in one launch: the grid splits into `groups` equal groups of blocks, each
@@ -794,16 +796,15 @@ __device__ __forceinline__ TravBuffers shift_buffers(TravBuffers b, size_t off) 
     b.q3 = sh(b.q3);
     b.rs = sh(b.rs);
     b.loc_off = sh(b.loc_off);
-    b.chunk_sum = sh(b.chunk_sum);
     b.aux = sh(b.aux);
     b.aux2 = sh(b.aux2);
+    b.aux3 = sh(b.aux3);
     b.bits0 = sh(b.bits0);
     b.bits1 = sh(b.bits1);
-    b.bits2 = sh(b.bits2);
     return b;
 }
 
-__global__ void __launch_bounds__(kBlock, APSPIE_SSSP_MINB) sssp_group_kernel(SsspGroupArgs g) {
+__global__ void __launch_bounds__(kBlock, 5) sssp_group_kernel(SsspGroupArgs g) {
     const int bpg = static_cast<int>(gridDim.x) / g.groups;  // the host launches groups * bpg blocks
     const int grp = static_cast<int>(blockIdx.x) / bpg;
     const VGrid vg{static_cast<int>(blockIdx.x) - grp * bpg, bpg};
@@ -821,7 +822,7 @@ __global__ void __launch_bounds__(kBlock, APSPIE_SSSP_MINB) sssp_group_kernel(Ss
             continue;
         }
         a.dist = g.out + static_cast<size_t>(q) * g.m;
-        sssp_body(a, vg);
+        sssp_body<false>(a, vg);
         // every block of the group is done with the control block before it is reset
         if (!grid_barrier(ctl, a.sticky, kSiteSsspGroup, vg)) break;
         if (tid == 0) {
@@ -965,7 +966,7 @@ __device__ __forceinline__ void mis_list_heavy(const MisArgs &a, unsigned long l
 // round counters, the next queue in slot r + 1) are cleared by the round before: their
 // last readers finished a full round earlier, so no block can still be reading them.
 __global__ void __launch_bounds__(kBlock) mis_kernel(MisArgs a) {
-    __shared__ int qbuf[kBlock / 32][3][BfsSmem::QCAP];
+    __shared__ int qbuf[kBlock / 32][3][kQCap];
     __shared__ int s_stop;
     grid_begin(a.ctl);
     const int G = gridDim.x;
@@ -1263,7 +1264,7 @@ void set_bfs_buffers(BfsArgs &a, const TravBuffers &b, int m, int nnz) {
     a.q[1] = EdgeQueue{b.q1, b.q3, b.loc_off, nullptr, nullptr};
     a.vis[0] = b.bits0;
     a.vis[1] = b.bits1;
-    a.shift = edge_unit_shift(nnz, static_cast<long long>(m) + 1);
+    a.shift = edge_unit_shift(nnz, static_cast<long long>(m) + 1, kEqTile);
 }
 
 apspie_status prepare_square(apspie_ctx *ctx, const apspie_csr *A, const char *who) {
@@ -1429,6 +1430,23 @@ apspie_status apspie_sssp_f32(apspie_ctx *ctx, const apspie_csr *A, int32_t sour
 
 namespace apspie {
 namespace {
+// Blocks of a launch: throughput grows with the warps on an SM (553 us with five blocks an SM
+// against 568 us with four and 802 us with two at scale 20), but so do the barriers' times,
+// and an iteration of a smaller graph has no more than a tile for each warp (6.7M entries:
+// 306 us with three, 315 us with four, 333 us with five).
+long long sssp_blocks(const apspie_ctx *ctx, long long nnz) {
+    return static_cast<long long>(ctx->num_sms) * (nnz >= 25000000 ? 5 : nnz >= 12000000 ? 4 : 3);
+}
+
+// Edges per iteration: an eighth of the graph's where an iteration's edges are most of its
+// time (scale 20: 571 us, a fifth 601 us), a fifth of smaller graphs', where its barriers and
+// dependent reads are, so that fewer iterations pay for more relaxations (6.7M entries:
+// 332 -> 314 us, 0.5M entries: 202 -> 190 us).
+long long default_band(long long nnz) {
+    const long long b = nnz >= (1LL << 24) ? nnz / 8 : nnz / 5;
+    return b < (1LL << 16) ? (1LL << 16) : (b > (1LL << 23) ? (1LL << 23) : b);
+}
+
 apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, void *d_dist,
                           apspie_run_stats *stats, bool is_float, int unreached_bits) {
     cudaSetDevice(ctx->device);
@@ -1455,18 +1473,18 @@ apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, 
     if (tp.sssp_band > 0) {
         a.band = tp.sssp_band;
     } else if (tp.sssp_band == 0) {
-        const long long b = A->nnz / 8;
-        a.band = b < (1LL << 18) ? (1LL << 18) : (b > (1LL << 23) ? (1LL << 23) : b);
+        a.band = default_band(A->nnz);
     } else {
         a.band = 0;
     }
-    a.is_float = is_float ? 1 : 0;
     a.unreached_bits = unreached_bits;
     a.buf = carve_trav(base, A->m);
+    a.shift = edge_unit_shift(A->nnz, static_cast<long long>(A->m) + 1, 32 * kSsspVT);
     a.ctl = ctx->d_ctl;
     a.sticky = ctx->d_sticky_err;
     void *args[] = {&a};
-    st = launch_persistent(ctx, reinterpret_cast<const void *>(sssp_kernel), kBlock, args, A->nnz);
+    st = launch_persistent(ctx, is_float ? reinterpret_cast<const void *>(sssp_kernel<true>) : reinterpret_cast<const void *>(sssp_kernel<false>),
+                           kBlock, args, sssp_blocks(ctx, A->nnz) * kWorkPerBlock);
     if (st != APSPIE_OK) return st;
     return finish_call(ctx, stats, "apspie_sssp");
 }
@@ -1516,16 +1534,14 @@ apspie_status sssp_batch_grouped(apspie_ctx *ctx, const apspie_csr *A, const int
         a.band = tp.sssp_band;
     } else if (tp.sssp_band == 0) {
         // the single-query default, scaled to the group's share of the device
-        long long b = A->nnz / 8;
-        b = b < (1LL << 18) ? (1LL << 18) : (b > (1LL << 23) ? (1LL << 23) : b);
-        b = b * bpg / cap;
+        const long long b = default_band(A->nnz) * bpg / cap;
         a.band = b < (1LL << 16) ? (1LL << 16) : b;
     } else {
         a.band = 0;
     }
-    a.is_float = 0;
     a.unreached_bits = -1;
     a.buf = carve_trav(base, m);
+    a.shift = edge_unit_shift(A->nnz, static_cast<long long>(m) + 1, 32 * kSsspVT);
     a.sticky = ctx->d_sticky_err;
     g.srcs = d_sources;
     g.out = d_dists;

@@ -113,7 +113,7 @@ apspie_status apspie_ctx_set_sssp_delta(apspie_ctx *ctx, int32_t delta);
 /* SSSP distance band: each iteration expands only the frontier vertices of lowest
  * distance whose edges add up to about `edges` (the rest wait in the frontier), chosen
  * from a degree-weighted distance histogram gathered on the device. edges == 0 (default):
- * nnz / 8 clamped to [2^18, 2^23]; edges < 0: off (expand the whole frontier). */
+ * nnz / 8 (nnz / 5 below 2^24 entries) clamped to [2^16, 2^23]; edges < 0: off (expand the whole frontier). */
 apspie_status apspie_ctx_set_sssp_band(apspie_ctx *ctx, int64_t edges);
 /* Batched SSSP: <= 0 = the multi-query kernel (default); > 0 = that many query groups,
  * each running the single-source kernel on its share of the sources. */

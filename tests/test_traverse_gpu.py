@@ -448,3 +448,65 @@ def test_bfs_edge_queue_shapes(ctx, shape, symmetric):
                                               err_msg=f"alpha {alpha} beta {beta} source {s}")
     finally:
         ctx.set_bfs_tuning(14.0, 24.0)
+
+
+@pytest.mark.parametrize("kind", ["i32", "f32"])
+@pytest.mark.parametrize("shape", ["star 127", "star 128", "star 129", "star 20000", "path", "dense", "hubs in a row",
+                                   "largest distances", "zero weights"])
+def test_sssp_edge_queue_shapes(ctx, shape, kind):
+    """Rows that fill, just miss and cross the edge queue's units, a row of many units, one
+    entry an iteration, units of more than a tile; with the default band, narrow bands (most
+    entries deferred), no band, and far piles; weights of 0 and distances up to 2^31 - 2."""
+    rng = np.random.default_rng(5)
+    if shape.startswith("star"):
+        k = int(shape.split()[1])
+        m, src, dst = k + 40, np.zeros(k, dtype=np.int64), np.arange(1, k + 1)
+    elif shape in ("path", "largest distances"):
+        m = 150
+        src, dst = np.arange(m - 1), np.arange(1, m)
+    elif shape == "dense":
+        m = 300
+        src, dst = np.nonzero(~np.eye(m, dtype=bool))
+    elif shape == "hubs in a row":
+        m = 6000
+        deg = rng.integers(900, 1100, 200)
+        src = np.concatenate((np.zeros(200, dtype=np.int64), np.repeat(np.arange(1, 201), deg)))
+        dst = np.concatenate((np.arange(1, 201), rng.integers(0, m, deg.sum())))
+    else:
+        m = 2000
+        src, dst = rng.integers(0, m, (2, 16000))
+    g = _csr(m, src[src != dst], dst[src != dst], False)
+    w = rng.integers(1, 256, g.nnz)
+    if shape == "zero weights":
+        w = rng.choice([0, 0, 1, 250], g.nnz)
+    elif shape == "largest distances" and kind == "i32":
+        w = np.full(g.nnz, (2 ** 31 - 2) // g.nnz)
+        w[-1] += (2 ** 31 - 2) - w.sum()
+    val = w.astype(np.int32) if kind == "i32" else (w / np.float32(7)).astype(np.float32)
+    g = ap.HostGraph(m, m, g.row_ptr, g.col_ind, np.ascontiguousarray(val))
+    dg = ap.DeviceGraph(g)
+    import torch
+
+    out = torch.empty(m, dtype=torch.int32 if kind == "i32" else torch.float32, device="cuda")
+    run = ctx.sssp_into if kind == "i32" else ctx.sssp_f32_into
+    if kind == "i32":
+        ref = oracle.sssp(g.row_ptr, g.col_ind, g.val, 0)
+    else:  # the least float32 sum over paths: relaxed to the fixed point, in any order
+        rows = np.repeat(np.arange(m), np.diff(g.row_ptr))
+        ref, old = np.full(m, np.inf, dtype=np.float32), None
+        ref[0] = 0
+        while old is None or not np.array_equal(ref, old):
+            old = ref.copy()
+            np.minimum.at(ref, g.col_ind, old[rows] + g.val)
+        ref[np.isinf(ref)] = -1
+    try:
+        for band, delta in ((0, 0), (1, 0), (500, 0), (-1, 0), (-1, 50), (300, 40)):
+            if delta and shape == "largest distances":
+                continue  # 40 million advances of the far threshold: past the 4 m + 4096 steps a call may take
+            ctx.set_sssp_band(band)
+            ctx.set_sssp_delta(delta)
+            run(dg, 0, out)
+            np.testing.assert_array_equal(out.cpu().numpy(), ref, err_msg=f"band {band} delta {delta}")
+    finally:
+        ctx.set_sssp_band(0)
+        ctx.set_sssp_delta(0)
