@@ -38,8 +38,7 @@ enum : int {
     kSiteSsspBarF1 = 213,
     kSiteSsspGroup = 214,  // and 215
     kSiteSsspBadSource = 216,
-    kSiteMis = 300,
-    kSiteMisRoundCap = 301,
+    kSiteMis = 300,  // and 301
 };
 
 struct TravBuffers {
@@ -848,15 +847,11 @@ __global__ void __launch_bounds__(kBlock, 5) sssp_group_kernel(SsspGroupArgs g) 
 // MIS
 // ================================================================================
 enum : unsigned char { kUndecided = 0, kIn = 1, kOut = 2 };
-#ifndef APSPIE_MIS_THREAD
-#define APSPIE_MIS_THREAD 16
-#endif
-#ifndef APSPIE_MIS_WARP_CHUNKS
-#define APSPIE_MIS_WARP_CHUNKS 8
-#endif
-constexpr int kMisThread = APSPIE_MIS_THREAD;          // neighbours one thread scans (phase S) before handing on
-constexpr int kMisWarpChunks = APSPIE_MIS_WARP_CHUNKS;  // chunks of 32 neighbours a warp scans (phase L)
-constexpr int kMisLightRow = 64;   // joiners with at most this many neighbours push by one thread
+constexpr int kMisThread = 8;           // neighbours a thread scans before handing on to a warp
+constexpr int kMisWarp = 1024;          // neighbours a warp scans before handing on to the block
+constexpr int kMisPart = 16384;         // neighbours a block scans or pushes to in a pass
+constexpr int kMisPush = -2;
+constexpr int kMisLong = 256, kMisHuge = 32;  // room for scans handed on in a pass
 
 struct MisArgs {
     int m, nnz;
@@ -866,16 +861,10 @@ struct MisArgs {
     unsigned char *member;
     int *member_i32;  // when set, the set is written here as int32 1/0 instead
     unsigned char *state;
-    int *pos;          // CSR index of the outranking neighbour that blocks the vertex (row start - 1: none yet)
-    int *queue[2];     // undecided vertices, by round parity
-    int *longq;        // scans that go on past a thread's share (one warp each, phase L)
-    int *longq2;       // scans that go on past a warp's share (one block each, phase L2)
-    int *light;        // vertices that joined with rows of at most kMisLightRow (pushed next round)
-    int *heavy_v;      // vertices that joined with longer rows,
-    int *heavy_base;   // the offset of each one's row in the next round's flat range of pushes,
-    int *heavy_delta;  // and row start - offset (push t of the range is CSR entry t + delta)
-    int *unit_owner;   // the heavy entry holding the first push of each unit of the range
-    int unit_shift;    // units of 1 << unit_shift pushes (one warp each)
+    // each block's undecided vertices (two lists, by pass parity): the vertex, the CSR index its
+    // scan stopped at, and the neighbour there that blocks it (-1: the scan goes on behind it)
+    int *v, *pos, *by;
+    size_t list;  // entries of one list
     TravCtl *ctl;
     int *sticky;
 };
@@ -884,348 +873,374 @@ __device__ __forceinline__ bool outranks(unsigned pu, int u, unsigned pv, int v)
     return pu > pv || (pu == pv && u > v);
 }
 
-// A neighbour's state as a scan reads it: through L1, so the lines of high-degree
-// neighbours (read by many scans at once) are not all fetched from L2. A stale value is
-// safe: states only move from undecided to in or out, so a stale read can only make a scan
-// stop early at a neighbour that is already out, and the next round's blocker check (a
-// coherent read) sees it out and resumes the scan behind it.
-#ifndef APSPIE_MIS_STATE_STRIDE
-#define APSPIE_MIS_STATE_STRIDE 1
-#endif
-constexpr int kMisStateStride = APSPIE_MIS_STATE_STRIDE;  // bytes between consecutive vertices' states
-__device__ __forceinline__ long long sx(int v) { return static_cast<long long>(v) * kMisStateStride; }
-__device__ __forceinline__ unsigned char scan_state(const unsigned char *state, int u) { return state[sx(u)]; }
-
-// One neighbour of a scanning vertex v: does it decide anything (an outranking neighbour
-// that is not out: v's new blocker, or -- if in -- the vertex that knocks v out)?
-__device__ __forceinline__ bool mis_stop(const MisArgs &a, int idx, int v, unsigned pv) {
-    const int u = __ldg(a.col_ind + idx);
-    const unsigned pu = __ldg(a.prio + u);
-    const unsigned char su = scan_state(a.state, u);
-    return u != v && su != kOut && outranks(pu, u, pv, v);
+__device__ __forceinline__ void mis_set(const MisArgs &a, int v, unsigned char s) {
+    asm volatile("st.relaxed.gpu.global.u8 [%0], %1;" ::"l"(a.state + v), "r"(static_cast<unsigned>(s)) : "memory");
 }
 
-// Knock out neighbour u of a vertex that joined. Many joiners share their high-degree
-// neighbours, and stores from many SMs into one line queue up in L2, so (check) a neighbour
-// already seen out (through L1: a stale "undecided" only costs a redundant store) is
-// skipped. In the first push round nothing is out yet.
-__device__ __forceinline__ void mis_knock(const MisArgs &a, int u, bool check) {
-    if (!check || scan_state(a.state, u) != kOut) a.state[sx(u)] = kOut;
+// Does neighbour u, in state su, decide anything for v: is it one that outranks v and is not
+// out? Returns kOut for "nothing to stop at", else its state.
+__device__ __forceinline__ unsigned char mis_look(int u, unsigned pu, unsigned char su, int v, unsigned pv) {
+    return u == v || !outranks(pu, u, pv, v) ? kOut : su;
 }
 
-// v joined with a row [r0, r0 + deg) longer than kMisLightRow: list it for the next
-// round's pushes. One atomic on (entries << 32 | pushes) gives the entry index and the
-// row's offset in the flat range, so offsets ascend with the index; the units starting
-// inside the row record it.
-__device__ __forceinline__ void mis_list_heavy(const MisArgs &a, unsigned long long *heavy, int v, int r0, int deg) {
-    const unsigned long long old = atomicAdd(heavy, (1ull << 32) | static_cast<unsigned>(deg));
-    const int idx = static_cast<int>(old >> 32);
-    const int base = static_cast<int>(old & 0xffffffffull);
-    a.heavy_v[idx] = v;
-    a.heavy_base[idx] = base;
-    a.heavy_delta[idx] = r0 - base;
-    const int sh = a.unit_shift;
-    for (int c = ((base - 1) >> sh) + 1; (c << sh) < base + deg; ++c) a.unit_owner[c] = idx;
+enum : int { kScanBlocked, kScanIn, kScanOut, kScanOn };
+
+// A thread's scan of v from CSR index e to lim: where it stops (pos), at whom (by).
+template <bool FIRST>
+__device__ __forceinline__ int mis_scan_thread(const MisArgs &a, int v, unsigned pv, int e, int lim, int r1, int &pos,
+                                               int &by) {
+    for (; e < lim; e += 4) {
+        int u[4];
+        unsigned pu[4];
+        unsigned char su[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) u[k] = e + k < lim ? __ldg(a.col_ind + e + k) : v;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            pu[k] = __ldg(a.prio + u[k]);
+            if (!FIRST) su[k] = a.state[u[k]];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned char s = mis_look(u[k], pu[k], FIRST ? kUndecided : su[k], v, pv);
+            if (s != kOut) {
+                pos = e + k;
+                by = u[k];
+                return s == kIn ? kScanOut : kScanBlocked;
+            }
+        }
+    }
+    pos = lim - 1;
+    by = -1;
+    return lim >= r1 ? kScanIn : kScanOn;
 }
 
 // Greedy MIS in descending (priority, id) order -- the set spmspvMis converges to
 // (src/spmspvMis.cuh:54-78: candidate if rand > threshold, select if rand > every
 // candidate neighbour's, knock out the neighbours), with ties broken by id instead of
 // left undecided. A vertex joins exactly when every neighbour that outranks it is out;
-// it is out as soon as a neighbour joins.
+// it is out as soon as one of them has joined.
 //
-// Only outranking neighbours can ever decide a vertex (a lower-ranked neighbour cannot
-// join while the vertex is undecided), and a neighbour once seen out or lower-ranked
-// stays so. So each undecided vertex keeps a scan position `pos`: every neighbour before
-// it is settled, and the neighbour at it is its current blocker (undecided, outranking).
-// Each scan stops at the first neighbour that decides anything, so rows are read about
-// once over the whole run and mostly not to their end (about 6.8M of R-MAT scale 20's
-// 31.4M entries). Round r, over the undecided vertices (round 0: all of them, which also
-// sets every state; vertices without neighbours join there) and the vertices that joined
-// in round r - 1:
-//  phase P  (when anything joined) the joiners write out into their neighbours: rows of at
-//           most kMisLightRow one thread each; longer rows, laid end to end in the order
-//           they were listed, in equal units of 1 << unit_shift entries, one warp each.
-//           Only stores (and L1 reads): on the B200 a phase in which many SMs both store
-//           into and read the lines of high-degree vertices' states runs several times
-//           slower, so the pushes are not made by the joining threads during the scans;
-//  phase S  each undecided vertex, by one thread: out -> leaves; its blocker still
-//           undecided (or in: its push comes next round) -> waits; else it scans on, four
-//           neighbours a step, and stops at the first neighbour that outranks it and is not
-//           out (its new blocker); no such neighbour -> it joins and is listed for the next
-//           round's pushes. After kMisThread neighbours without an end the vertex goes to
-//           the long list;
-//  phase L  (only when that list is not empty) one warp per vertex goes on in chunks of
-//           32, for up to kMisWarpChunks chunks; the rest (phase L2) one block each.
-// The pushes of a round are complete before its scans start, so a scan sees every vertex
-// knocked out so far; scans and joins of the same phase race only safely (a vertex joins
-// only if every outranking neighbour was seen out, and out is final). The set is the
-// greedy MIS whatever the timing.
+// Only outranking neighbours decide a vertex, and states never change once decided, so the
+// kernel has no rounds: every block owns every G-th tile of 256 vertices and goes through its
+// undecided ones again and again, on its own, until none is left. A vertex keeps the position
+// of the first outranking neighbour that is not out (everything before it is settled for
+// good): in -> the vertex is out; undecided -> look again in the next pass; out -> scan on
+// behind it. The highest-ranked undecided vertex can always be decided, whichever block owns
+// it, and all blocks are resident, so every block gets to its end; the set does not depend on
+// timing. Scans go on by a warp past kMisThread neighbours and by the block past kMisWarp.
 //
-// The lists a round fills (long lists and joiners in slot r mod 3 of the control block's
-// round counters, the next queue in slot r + 1) are cleared by the round before: their
-// last readers finished a full round earlier, so no block can still be reading them.
-__global__ void __launch_bounds__(kBlock) mis_kernel(MisArgs a) {
-    __shared__ int qbuf[kBlock / 32][3][kQCap];
-    __shared__ int s_stop;
+// A joiner stores "out" into its undecided neighbours, so that a vertex leaves as soon as any
+// outranking neighbour is in, not only the one it waits for: without that, chains of waits
+// thousands of passes long form (3,450 us instead of 283 at R-MAT scale 20). The store is kept
+// from states already seen as out: without the look, every joiner stores into the lines of the
+// same high-degree vertices (3,660 us). The first pass looks at ranks only, when nearly
+// every state is still undecided (260 -> 240 us).
+//
+// Scans and pushes go on by a warp past kMisThread entries and by the block past kMisWarp,
+// kMisPart at a time, so that one long row does not keep the block's other vertices waiting.
+// States are read through L1, which thread 0's acquire drops once a pass: every look in L2
+// had all SMs poll the few lines of the high-degree vertices that most others wait for
+// (240 -> 219 us; 418 -> 362 at 2M vertices). A stale state can only be "undecided" where it
+// is decided by now, and costs a pass.
+//
+// What bounds it: the latency of each pass's chain of gathers (column, priority and state,
+// mostly out of L2 and DRAM) and the number of decisions that follow one another; most of the
+// entries, 7.5M of 31.4M, are looked at in the first two passes. Five blocks an SM (260 us)
+// against four (280) and six (279); tiles of 64, 128 and 512 vertices, steps of 2 and 8
+// entries and warp limits from 128 to 2,048 are all within 10 % or slower. With rounds (the
+// joiners' pushes, then scans, each closed by a grid barrier: 22 barriers at scale 20) 376 us,
+// now 219; 248 -> 125 us at 300,007 vertices, 60 -> 35 at 3,001; a path of 20,000 vertices
+// in rank order, one decision after the other, 78 -> 15 ms.
+//
+// A block that decides nothing waits for others. It gives up (APSPIE_ERR_TIMEOUT) when no
+// block has decided anything for the context's wait limit: blocks count their passes that did
+// in ctl->aux[0].
+__global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
+    __shared__ int s_n[2], s_long, s_huge, s_decided, s_stop, s_end;
+    __shared__ int s_lv[kMisLong], s_lp[kMisLong], s_hv[kMisHuge], s_hp[kMisHuge];
     grid_begin(a.ctl);
-    const int G = gridDim.x;
-    const int gtid = blockIdx.x * kBlock + threadIdx.x;
-    const int gstride = G * kBlock;
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
+    const int G = gridDim.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int m = a.m;
     const int *col = a.col_ind;
-    unsigned char *state = a.state;
-    int *qlen = a.ctl->rcnt;                   // [3] undecided-queue lengths
-    int *l1len = a.ctl->rcnt + 3;              // [3] long list (phase L)
-    int *l2len = a.ctl->rcnt + 6;              // [3] longest list (phase L2)
-    int *nlight = a.ctl->rcnt + 9;             // [3] light joiners
-    unsigned long long *heavy = a.ctl->rcnt64;  // [3] (entries << 32) | pushes of heavy joiners
-    long long pushed = 0, scanned = 0;
-    int r = 0;
-    for (;; ++r) {
-        const int s0 = r % 3, s1 = (r + 1) % 3, s2 = (r + 2) % 3;
-        const int sp = (r + 2) % 3;  // the joiner lists of round r - 1
-        const int nf = r == 0 ? m : ld_volatile_i32(qlen + s0);  // round 0: every vertex
-        const int nl = ld_volatile_i32(nlight + sp);
-        const unsigned long long hh = __ldcg(reinterpret_cast<const unsigned long long *>(heavy + sp));
-        const int nh = static_cast<int>(hh >> 32);
-        const int H = static_cast<int>(hh & 0xffffffffull);
-        const int sh = a.unit_shift;
-        const int nu = H > 0 ? ((H - 1) >> sh) + 1 : 0;
-        if (nf == 0 && nl == 0 && nu == 0) break;
-        if (r > m + 1) {
-            if (gtid == 0) raise_error(a.ctl, a.sticky, APSPIE_ERR_NOT_CONVERGED, kSiteMisRoundCap);
-            break;
-        }
-        const int *qc = a.queue[r & 1];
-        int *qn = a.queue[(r & 1) ^ 1];
+    for (int i = blockIdx.x * kBlock + tid; i < m; i += G * kBlock) a.state[i] = kUndecided;
+    // the part of the lists that holds this block's vertices
+    const int tiles = (m - 1) / kBlock + 1, each = tiles / G, extra = tiles % G, b = blockIdx.x;
+    const size_t part = (static_cast<size_t>(b) * each + min(b, extra)) * kBlock;
+    if (tid == 0) s_n[0] = s_n[1] = s_long = s_huge = s_decided = s_end = 0;
+    if (!grid_barrier(a.ctl, a.sticky, kSiteMis)) return;
 
-        // phase P: the last round's joiners knock out their neighbours -- short rows one
-        // thread each, long rows laid end to end and shared out in equal units, one warp
-        // each. Plain byte stores: every neighbour of a vertex in the set is out.
-        if (nl > 0 || nu > 0) {
-            // skipping known outs pays when many joiners share neighbours; with few of them
-            // the read before each store only lengthens the chain
-            const bool check = r >= 2 && nl + nh >= 4096;
-            // lanes per joiner: 1 when the joiners fill the grid, up to 8 when they are few,
-            // so that a short round's rows are not walked one entry at a time by one thread
-            int lpj = 1;
-            while (lpj < 8 && static_cast<long long>(nl) * lpj * 2 <= gstride) lpj <<= 1;
-            const int sub = gtid & (lpj - 1);
-            for (int i = gtid / lpj; i < nl; i += gstride / lpj) {
-                const int j = __ldcg(a.light + i);
-                const int r0 = __ldg(a.row_ptr + j), r1 = __ldg(a.row_ptr + j + 1);
-                if (sub == 0) pushed += r1 - r0;
-                for (int e = r0 + sub; e < r1; e += 8 * lpj) {
-                    int u[8];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) u[k] = e + k * lpj < r1 ? __ldg(col + e + k * lpj) : j;
-#pragma unroll
-                    for (int k = 0; k < 8; ++k)
-                        if (u[k] != j) mis_knock(a, u[k], check);
-                }
-            }
-            const int gw = gtid >> 5, nw = gstride >> 5;
-            for (int c = gw; c < nu; c += nw) {
-                // a unit spans the end of one row and the start of the next where rows meet in it
-                const int t0 = c << sh, t1 = min(H, t0 + (1 << sh));
-                int i = __ldcg(a.unit_owner + c);
-                int hv = __ldcg(a.heavy_v + i), hd = __ldcg(a.heavy_delta + i);
-                int nb = i + 1 < nh ? __ldcg(a.heavy_base + i + 1) : INT_MAX;
-                if (lane == 0) pushed += t1 - t0;
-                for (int tb = t0; tb < t1; tb += 128) {
-                    int e[4], w[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int t = tb + 32 * q + lane;
-                        while (t < t1 && t >= nb) {
-                            ++i;
-                            hv = __ldcg(a.heavy_v + i);
-                            hd = __ldcg(a.heavy_delta + i);
-                            nb = i + 1 < nh ? __ldcg(a.heavy_base + i + 1) : INT_MAX;
-                        }
-                        e[q] = t < t1 ? t + hd : -1;
-                        w[q] = hv;
-                    }
-                    int u[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) u[q] = e[q] >= 0 ? __ldg(col + e[q]) : -1;
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (u[q] >= 0 && u[q] != w[q]) mis_knock(a, u[q], check);
-                }
-            }
-            if (!grid_barrier(a.ctl, a.sticky, kSiteMis + 2)) return;
-        }
-        // the lists this round fills start empty; their slots were last read a round ago
-        if (gtid == 0) {
-            qlen[s2] = 0;
-            l1len[s1] = 0;
-            l2len[s1] = 0;
-            nlight[s1] = 0;
-            heavy[s1] = 0ull;
-        }
-
-        // phase S: blocker checks, short scans and decisions, one thread per vertex; each
-        // scan step loads four neighbours at once and takes the first that decides anything
-        {
-            WQ wq(qbuf[wid][0], qn, qlen + s1);
-            WQ wj(qbuf[wid][1], a.light, nlight + s0);
-            WQ wl(qbuf[wid][2], a.longq, l1len + s0);
-            for (int base = blockIdx.x * kBlock; base < nf; base += gstride) {
-                const int i = base + threadIdx.x;
-                bool keep = false, light = false, along = false;
-                int v = 0;
-                if (i < nf) {
-                    // round 0 takes every vertex and writes every state: vertices without
-                    // neighbours join at once, the others start undecided with no blocker
-                    v = r == 0 ? i : __ldcg(qc + i);
-                    const int r0 = __ldg(a.row_ptr + v), r1 = __ldg(a.row_ptr + v + 1);
-                    if (r == 0 && r1 == r0) {
-                        state[sx(v)] = kIn;
-                    } else if (r == 0 || __ldcg(state + sx(v)) == kUndecided) {
-                        const int p = r == 0 ? r0 - 1 : __ldcg(a.pos + v);
-                        if (r == 0) state[sx(v)] = kUndecided;
-                        if (p >= r0 && __ldcg(state + sx(__ldg(col + p))) != kOut) {
-                            keep = true;  // its blocker is undecided (or joined: its push comes next)
-                        } else {
-                            const unsigned pv = __ldg(a.prio + v);
-                            const int start = p + 1, lim = min(r1, start + kMisThread);
-                            int stop = -1, e = start;
-                            for (; e < lim && stop < 0; e += 4) {
-                                int u[4];
-                                unsigned pu[4];
-                                unsigned char su[4];
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) u[k] = e + k < lim ? __ldg(col + e + k) : v;
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    pu[k] = __ldg(a.prio + u[k]);
-                                    // in the first round every vertex with neighbours is undecided
-                                    su[k] = r == 0 ? kUndecided : scan_state(state, u[k]);
-                                }
-#pragma unroll
-                                for (int k = 0; k < 4; ++k)
-                                    if (stop < 0 && u[k] != v && su[k] != kOut && outranks(pu[k], u[k], pv, v))
-                                        stop = e + k;
-                            }
-                            scanned += (stop >= 0 ? stop + 1 : lim) - start;
-                            if (stop >= 0) {
-                                keep = true;
-                                a.pos[v] = stop;
-                            } else if (lim >= r1) {
-                                state[sx(v)] = kIn;
-                                light = r1 - r0 <= kMisLightRow;
-                                if (!light) mis_list_heavy(a, heavy + s0, v, r0, r1 - r0);
-                            } else {  // settled up to lim - 1: a warp goes on
-                                a.pos[v] = lim - 1;
-                                along = true;
-                            }
-                        }
-                    }
-                }
-                wq.push(keep, v);
-                wj.push(light, v);
-                wl.push(along, v);
-            }
-            wq.flush();
-            wj.flush();
-            wl.flush();
-        }
-        if (!grid_barrier(a.ctl, a.sticky, kSiteMis + 3)) return;
-
-        // phase L: longer scans, one warp per vertex (up to kMisWarpChunks chunks of 32)
-        const int n1 = ld_volatile_i32(l1len + s0);
-        if (n1 > 0) {
-            WQ wq(qbuf[wid][0], qn, qlen + s1);
-            WQ wj(qbuf[wid][1], a.light, nlight + s0);
-            const int gw = gtid >> 5, nw = gstride >> 5;
-            for (int k = gw; k < n1; k += nw) {
-                const int v = __ldcg(a.longq + k);
-                const int r1 = __ldg(a.row_ptr + v + 1);
-                const int start = __ldcg(a.pos + v) + 1;
-                const unsigned pv = __ldg(a.prio + v);
-                int stop = -1, c = 0;
-                for (; c < kMisWarpChunks && start + 32 * c < r1; ++c) {
-                    const int idx = start + 32 * c + lane;
-                    const unsigned b = __ballot_sync(0xffffffffu, idx < r1 && mis_stop(a, idx, v, pv));
-                    if (b) {
-                        stop = start + 32 * c + __ffs(b) - 1;
-                        break;
-                    }
-                }
-                const bool end = stop < 0 && start + 32 * c >= r1;
-                bool light = false;
-                if (lane == 0) {
-                    scanned += min(r1, stop >= 0 ? stop + 1 : start + 32 * c) - start;
-                    if (stop >= 0) {
-                        a.pos[v] = stop;
-                    } else if (end) {
-                        state[sx(v)] = kIn;
-                        const int r0 = __ldg(a.row_ptr + v);
-                        light = r1 - r0 <= kMisLightRow;
-                        if (!light) mis_list_heavy(a, heavy + s0, v, r0, r1 - r0);
-                    } else {
-                        a.pos[v] = start + 32 * kMisWarpChunks - 1;
-                        a.longq2[atomicAdd(l2len + s0, 1)] = v;
-                    }
-                }
-                wq.push(stop >= 0 && lane == 0, v);
-                wj.push(light, v);
-            }
-            wq.flush();
-            wj.flush();
-            if (!grid_barrier(a.ctl, a.sticky, kSiteMis + 4)) return;
-        }
-
-        // phase L2: the longest scans, one block per vertex
-        const int n2 = n1 > 0 ? ld_volatile_i32(l2len + s0) : 0;
-        if (n2 > 0) {
-            for (int k = blockIdx.x; k < n2; k += G) {
-                const int v = __ldcg(a.longq2 + k);
-                const int r1 = __ldg(a.row_ptr + v + 1);
-                const int start = __ldcg(a.pos + v) + 1;
-                const unsigned pv = __ldg(a.prio + v);
-                if (threadIdx.x == 0) s_stop = kInf;
-                __syncthreads();
-                for (int b0 = start; b0 < r1; b0 += kBlock) {
-                    const int idx = b0 + threadIdx.x;
-                    const bool st = idx < r1 && mis_stop(a, idx, v, pv);
-                    if (st) atomicMin(&s_stop, idx);
-                    if (__syncthreads_or(st)) break;
-                }
-                if (threadIdx.x == 0) {
-                    const int spos = s_stop;
-                    scanned += (spos != kInf ? spos + 1 : r1) - start;
-                    if (spos != kInf) {
-                        a.pos[v] = spos;
-                        qn[atomicAdd(qlen + s1, 1)] = v;
-                    } else {
-                        state[sx(v)] = kIn;
-                        const int r0 = __ldg(a.row_ptr + v);
-                        if (r1 - r0 <= kMisLightRow)
-                            a.light[atomicAdd(nlight + s0, 1)] = v;
-                        else
-                            mis_list_heavy(a, heavy + s0, v, r0, r1 - r0);
-                    }
-                }
-                __syncthreads();
-            }
-            if (!grid_barrier(a.ctl, a.sticky, kSiteMis + 5)) return;
-        }
-    }
-    long long insz = 0;
-    for (int i = gtid; i < m; i += gstride) {
-        const unsigned char s = a.state[sx(i)];
+    long long insz = 0, scanned = 0;
+    auto decide = [&](int v, bool in) {
+        mis_set(a, v, in ? kIn : kOut);
         if (a.member_i32)
-            a.member_i32[i] = (s == kIn) ? 1 : 0;
+            a.member_i32[v] = in ? 1 : 0;
         else
-            a.member[i] = (s == kIn) ? 1 : 0;
-        insz += (s == kIn);
+            a.member[v] = in ? 1 : 0;
+        insz += in;
+        s_decided = 1;
+    };
+    auto keep = [&](int to, int v, int pos, int by) {
+        const size_t at = part + to * a.list + atomicAdd(&s_n[to], 1);
+        a.v[at] = v;
+        a.pos[at] = pos;
+        a.by[at] = by;
+    };
+    // hands v's scan behind pos (kMisPush: the push of a joiner) on to a warp; without room it
+    // goes on in the next pass
+    auto hand_on = [&](int to, int v, int pos, int from) {
+        const int at = atomicAdd(&s_long, 1);
+        if (at < kMisLong) {
+            s_lv[at] = v;
+            s_lp[at] = from;
+            return true;
+        }
+        keep(to, v, pos, -1);
+        return false;
+    };
+    auto outcome = [&](int to, int code, int v, int pos, int by) {
+        if (code == kScanOut) {
+            decide(v, false);
+        } else if (code == kScanBlocked) {
+            keep(to, v, pos, by);
+        } else if (code == kScanOn) {
+            hand_on(to, v, pos, pos);
+        } else {
+            const int r0 = __ldg(a.row_ptr + v), r1 = __ldg(a.row_ptr + v + 1);
+            if (r1 - r0 > kMisThread) {
+                if (hand_on(to, v, r1 - 1, kMisPush)) decide(v, true);
+            } else {
+                decide(v, true);
+                scanned += r1 - r0;
+                for (int e = r0; e < r1; e += 4) {
+                    int u[4];
+                    unsigned char s[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) u[k] = e + k < r1 ? __ldg(col + e + k) : v;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) s[k] = a.state[u[k]];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (u[k] != v && s[k] == kUndecided) mis_set(a, u[k], kOut);
+                }
+            }
+        }
+    };
+    unsigned long long t0 = 0, seen = 0;  // thread 0's: when something was last decided anywhere
+    int pass = 0, idle = 0;
+    for (;; ++pass) {
+        const int cur = pass & 1, nxt = cur ^ 1;
+        if (pass == 0) {
+            for (int t = b; t < tiles; t += G) {
+                const int v = t * kBlock + tid;
+                if (v >= m) continue;
+                const int r0 = __ldg(a.row_ptr + v), r1 = __ldg(a.row_ptr + v + 1);
+                int pos = 0, by = -1;
+                const int code = mis_scan_thread<true>(a, v, __ldg(a.prio + v), r0, min(r1, r0 + kMisThread), r1, pos, by);
+                scanned += pos + 1 - r0;
+                outcome(nxt, code, v, pos, by);
+            }
+        } else {
+            const int n = s_n[cur];
+            for (int i = tid; i < n; i += kBlock) {
+                const size_t at = part + cur * a.list + i;
+                const int v = a.v[at], by = a.by[at];
+                int pos = a.pos[at];
+                if (by == v) {  // a push that goes on
+                    const int h = atomicAdd(&s_huge, 1);
+                    if (h < kMisHuge) {
+                        s_hv[h] = v;
+                        s_hp[h] = pos;
+                    } else {
+                        keep(nxt, v, pos, v);
+                    }
+                    continue;
+                }
+                const int r1 = __ldg(a.row_ptr + v + 1);  // fetched alongside the states
+                const unsigned pv = __ldg(a.prio + v);
+                const unsigned char own = a.state[v];
+                const unsigned char s = by < 0 ? kOut : a.state[by];
+                if (own == kOut) {
+                    decide(v, false);
+                } else if (s == kUndecided) {
+                    keep(nxt, v, pos, by);
+                } else if (s == kIn) {
+                    decide(v, false);
+                } else {
+                    const int e = pos + 1;
+                    int who = -1;
+                    const int code =
+                        mis_scan_thread<false>(a, v, pv, e, min(r1, e + kMisThread), r1, pos, who);
+                    scanned += pos + 1 - e;
+                    outcome(nxt, code, v, pos, who);
+                }
+            }
+        }
+        __syncthreads();
+        // longer scans, a warp each, 128 neighbours a step
+        const int nlong = min(s_long, kMisLong);
+        for (int i = wid; i < nlong; i += kBlock / 32) {
+            const int v = s_lv[i], r1 = __ldg(a.row_ptr + v + 1);
+            if (s_lp[i] == kMisPush) {
+                const int r0 = __ldg(a.row_ptr + v);
+                if (r1 - r0 > kMisWarp) {
+                    if (lane == 0) {
+                        const int at = atomicAdd(&s_huge, 1);
+                        if (at < kMisHuge) {
+                            s_hv[at] = v;
+                            s_hp[at] = -2 - r0;
+                        } else {
+                            keep(nxt, v, -2 - r0, v);
+                        }
+                    }
+                    continue;
+                }
+                for (int e = r0; e < r1; e += 128) {
+                    int u[4];
+                    unsigned char s[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) u[k] = e + 32 * k + lane < r1 ? __ldg(col + e + 32 * k + lane) : v;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) s[k] = a.state[u[k]];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (u[k] != v && s[k] == kUndecided) mis_set(a, u[k], kOut);
+                }
+                if (lane == 0) scanned += r1 - r0;
+                continue;
+            }
+            const int first = s_lp[i] + 1;
+            const unsigned pv = __ldg(a.prio + v);
+            const int lim = min(r1, first + kMisWarp);
+            int code = lim >= r1 ? kScanIn : kScanOn, pos = lim - 1, by = -1;
+            for (int e = first; e < lim && pos >= e; e += 128) {
+                int u[4];
+                unsigned char s[4];
+                unsigned pu[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) u[k] = e + 32 * k + lane < lim ? __ldg(col + e + 32 * k + lane) : v;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    pu[k] = __ldg(a.prio + u[k]);
+                    s[k] = a.state[u[k]];
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) s[k] = mis_look(u[k], pu[k], s[k], v, pv);
+#pragma unroll
+                for (int k = 3; k >= 0; --k) {  // the first stop counts
+                    const unsigned stops = __ballot_sync(0xffffffffu, s[k] != kOut);
+                    if (stops) {
+                        const int l = __ffs(stops) - 1;
+                        pos = e + 32 * k + l;
+                        by = __shfl_sync(0xffffffffu, u[k], l);
+                        code = __shfl_sync(0xffffffffu, static_cast<int>(s[k]), l) == kIn ? kScanOut : kScanBlocked;
+                    }
+                }
+                if (by >= 0) break;
+            }
+            if (lane == 0) {
+                scanned += pos + 1 - first;
+                if (code == kScanIn) {
+                    keep(nxt, v, r1 - 1, -1);  // joins in the next pass, which hands its push on
+                } else if (code != kScanOn) {
+                    outcome(nxt, code, v, pos, by);
+                } else {
+                    const int at = atomicAdd(&s_huge, 1);
+                    if (at < kMisHuge) {
+                        s_hv[at] = v;
+                        s_hp[at] = pos;
+                    } else {
+                        keep(nxt, v, pos, -1);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        // the longest, by the block, 1,024 neighbours a step and kMisPart at a time
+        const int nhuge = min(s_huge, kMisHuge);
+        for (int i = 0; i < nhuge; ++i) {
+            const int v = s_hv[i], r1 = __ldg(a.row_ptr + v + 1), p = s_hp[i];
+            if (p < -1) {  // a push, from CSR index -2 - p on
+                const int first = -2 - p, lim = min(static_cast<long long>(r1), first + static_cast<long long>(kMisPart));
+                for (int e = first + tid; e < lim; e += 4 * kBlock) {
+                    int u[4];
+                    unsigned char s[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) u[k] = e + k * kBlock < lim ? __ldg(col + e + k * kBlock) : v;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) s[k] = a.state[u[k]];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (u[k] != v && s[k] == kUndecided) mis_set(a, u[k], kOut);
+                }
+                if (tid == 0) {
+                    s_decided = 1;
+                    scanned += lim - first;
+                    if (lim < r1) keep(nxt, v, -2 - lim, v);
+                }
+                continue;
+            }
+            const int first = p + 1, lim = min(static_cast<long long>(r1), first + static_cast<long long>(kMisPart));
+            const unsigned pv = __ldg(a.prio + v);
+            if (tid == 0) s_stop = kInf;
+            __syncthreads();
+            for (int e = first; e < lim; e += 4 * kBlock) {
+                int stop = kInf, u[4];
+                unsigned pu[4];
+                unsigned char s[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) u[k] = e + k * kBlock + tid < lim ? __ldg(col + e + k * kBlock + tid) : v;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    pu[k] = __ldg(a.prio + u[k]);
+                    s[k] = a.state[u[k]];
+                }
+#pragma unroll
+                for (int k = 3; k >= 0; --k)
+                    if (mis_look(u[k], pu[k], s[k], v, pv) != kOut) stop = e + k * kBlock + tid;
+                if (stop != kInf) atomicMin(&s_stop, stop);
+                if (__syncthreads_or(stop != kInf)) break;
+            }
+            if (tid == 0) {
+                const int stop = s_stop;
+                s_decided = 1;
+                scanned += (stop != kInf ? stop + 1 : lim) - first;
+                if (stop == kInf)
+                    keep(nxt, v, lim - 1, -1);  // goes on, or joins, in the next pass
+                else
+                    keep(nxt, v, stop, __ldg(col + stop));  // whose state may have changed since
+            }
+            __syncthreads();
+        }
+        if (tid == 0) {
+            // the next pass reads states through L1, which this acquire has dropped
+            ld_acquire_u64(&a.ctl->aux[0]);
+            s_n[cur] = 0;
+            s_long = s_huge = 0;
+            if (s_n[nxt] == 0) s_end = 1;
+            if (s_decided) {
+                s_decided = 0;
+                idle = 0;
+                t0 = 0;
+                if (!s_end) atomicAdd(reinterpret_cast<unsigned long long *>(&a.ctl->aux[0]), 1ull);
+            } else if ((++idle & 63) == 0) {
+                const unsigned long long now = globaltimer_ns();
+                const unsigned long long count = *reinterpret_cast<volatile unsigned long long *>(&a.ctl->aux[0]);
+                const unsigned long long limit = a.ctl->wait_limit_ns ? a.ctl->wait_limit_ns : kBarrierTimeoutNs;
+                if (ld_volatile_i32(&a.ctl->err) != 0) s_end = 1;
+                if (t0 == 0 || count != seen) {
+                    t0 = now;
+                    seen = count;
+                } else if (now - t0 > limit) {
+                    raise_error(a.ctl, a.sticky, APSPIE_ERR_TIMEOUT, kSiteMis + 1);
+                    s_end = 1;
+                }
+            }
+        }
+        __syncthreads();
+        if (s_end) break;
     }
-    long long work = scanned + pushed;
+    long long work = scanned;
     for (int o = 16; o; o >>= 1) {
         insz += __shfl_down_sync(0xffffffffu, insz, o);
         work += __shfl_down_sync(0xffffffffu, work, o);
@@ -1236,10 +1251,10 @@ __global__ void __launch_bounds__(kBlock) mis_kernel(MisArgs a) {
     if (lane == 0 && work)
         atomicAdd(reinterpret_cast<unsigned long long *>(&a.ctl->edges_expanded),
                   static_cast<unsigned long long>(work));
-    if (gtid == 0) {
-        a.ctl->iterations = r;
-        a.ctl->push_iterations = r;
-        a.ctl->edges_component = a.nnz;
+    if (tid == 0) {
+        atomicMax(&a.ctl->iterations, pass + 1);
+        atomicMax(&a.ctl->push_iterations, pass + 1);
+        if (blockIdx.x == 0) a.ctl->edges_component = a.nnz;
     }
 }
 
@@ -1341,11 +1356,10 @@ cudaError_t noalloc_scratch(void **out) {
 
 size_t traversal_scratch_need(int m) { return trav_scratch_bytes(m); }
 
-// what mis_common reserves: the traversal buffers, the state array, the push-unit owners
-// and the list of light joiners
+// what mis_common reserves: the states and the blocks' lists (whole tiles)
 size_t mis_scratch_need(int m) {
-    const size_t mi = static_cast<size_t>(m) + 1;
-    return trav_scratch_bytes(m) + Carver::need({static_cast<size_t>(m) * kMisStateStride, mi * 4, mi * 4});
+    const size_t l = (static_cast<size_t>(m) + kBlock) * 8;
+    return Carver::need({static_cast<size_t>(m), l, l, l});
 }
 
 apspie_status trav_reserve(apspie_ctx *ctx, int m) {
@@ -1586,8 +1600,6 @@ static apspie_status mis_common(apspie_ctx *ctx, const apspie_csr *A, const uint
     if (st != APSPIE_OK) return st;
     if (!d_priority) return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_mis: NULL priority");
     void *base;
-    const size_t tb = trav_scratch_bytes(A->m);
-    const size_t mi = static_cast<size_t>(A->m) + 1;
     st = scratch_reserve(ctx, mis_scratch_need(A->m), &base);
     if (st != APSPIE_OK) return st;
     if ((st = reset_ctl(ctx)) != APSPIE_OK) return st;
@@ -1599,23 +1611,12 @@ static apspie_status mis_common(apspie_ctx *ctx, const apspie_csr *A, const uint
     a.prio = d_priority;
     a.member = d_member;
     a.member_i32 = d_member_i32;
-    const TravBuffers buf = carve_trav(base, A->m);
-    a.pos = buf.aux;
-    a.queue[0] = buf.q0;
-    a.queue[1] = buf.q1;
-    a.longq = buf.q2;
-    a.longq2 = buf.aux2;
-    a.heavy_v = buf.q3;
-    a.heavy_base = buf.rs;
-    a.heavy_delta = buf.loc_off;
-    Carver c(static_cast<char *>(base) + tb);
-    a.state = c.take<unsigned char>(static_cast<size_t>(A->m) * kMisStateStride);
-    a.unit_owner = c.take<int>(mi);
-    a.light = c.take<int>(mi);
-    // push units hold at least 128 entries, and few enough that the units of a round's
-    // pushes (at most nnz entries) fit the m + 1 slots of unit_owner
-    a.unit_shift = 7;
-    while ((static_cast<long long>(A->nnz) >> a.unit_shift) + 1 > static_cast<long long>(mi)) ++a.unit_shift;
+    Carver c(base);
+    a.state = c.take<unsigned char>(static_cast<size_t>(A->m));
+    a.list = static_cast<size_t>(A->m) + kBlock;
+    a.v = c.take<int>(2 * a.list);
+    a.pos = c.take<int>(2 * a.list);
+    a.by = c.take<int>(2 * a.list);
     a.ctl = ctx->d_ctl;
     a.sticky = ctx->d_sticky_err;
     void *args[] = {&a};

@@ -399,6 +399,49 @@ def test_mis_int32_layout(ctx, rmat14):
     np.testing.assert_array_equal(out.cpu().numpy(), oracle.mis_greedy(g.row_ptr, g.col_ind, pr).astype(np.int32))
 
 
+@pytest.mark.parametrize("prio", ["up", "down", "random", "equal"])
+@pytest.mark.parametrize("shape", ["path 700", "star 8", "star 9", "star 1024", "star 1025", "star 40000",
+                                   "hubs 300", "loops", "m 255", "m 256", "m 257", "one vertex", "no edges"])
+@pytest.mark.parametrize("grid", [1, 0])
+def test_mis_scans_and_pushes(ctx, shape, prio, grid):
+    """Scans and pushes that end in a thread, go on in a warp and in the block, and in several passes of
+    the block; more of each in one block than its lists hold (a grid of one block); chains as long as the
+    graph; ties; self-loops; vertices around a whole tile. The set is unique."""
+    import torch
+
+    kind, _, size = shape.partition(" ")
+    rng = np.random.default_rng(5)
+    if kind == "path":
+        m = int(size)
+        src, dst = np.arange(m - 1), np.arange(1, m)
+    elif kind == "star":
+        m = int(size) + 1
+        src, dst = np.zeros(m - 1, np.int64), np.arange(1, m)
+    elif kind == "hubs":
+        k, m = int(size), 3000 + int(size)
+        src, dst = np.repeat(np.arange(k), 3000), np.tile(np.arange(k, m), k)
+    elif kind == "m":
+        m = int(size)
+        src, dst = rng.integers(0, m, 4 * m), rng.integers(0, m, 4 * m)
+    elif kind == "loops":
+        m = 600
+        src = np.concatenate((np.arange(m), rng.integers(0, m, 2 * m)))
+        dst = np.concatenate((np.arange(m), rng.integers(0, m, 2 * m)))
+    else:
+        m = 1 if kind == "one" else 300
+        src = dst = np.zeros(0, np.int64)
+    g = _csr(m, src, dst, True)
+    pr = {"up": np.arange(m), "down": np.arange(m)[::-1], "random": rng.integers(0, 2**32, m),
+          "equal": np.full(m, 7)}[prio].astype(np.uint32)
+    out = torch.empty(m, dtype=torch.int32, device="cuda")
+    ctx.set_max_grid(grid)
+    try:
+        ctx.mis_int32_into(ap.DeviceGraph(g), torch.from_numpy(pr.view(np.int32)).cuda(), out)
+    finally:
+        ctx.set_max_grid(0)
+    np.testing.assert_array_equal(out.cpu().numpy(), oracle.mis_greedy(g.row_ptr, g.col_ind, pr).astype(np.int32))
+
+
 def _csr(m, src, dst, symmetric):
     if symmetric:
         src, dst = np.concatenate((src, dst)), np.concatenate((dst, src))
