@@ -1,5 +1,5 @@
-// The frontier expander shared by the persistent BFS and SSSP kernels (single-source and
-// batched).
+// What the persistent traversal kernels share: the merge-path frontier expander (batched BFS) and the
+// edge queues (BFS, SSSP and batched SSSP).
 //
 // It replaces the reference's per-level library chain (src/mXv.cuh:142-176,
 // src/spmspvBfs.cuh:178-186, src/spmspvMis.cuh:245-263): Scan -> streamCompact ->
@@ -23,35 +23,29 @@
 //           pass (no materialised neighbour list, no sort).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace apspie {
 
-// Per-warp staging slice. EXTRA adds the second payload and the per-entry accumulator
-// (batched BFS and SSSP); BFS and SSSP leave them out to keep shared memory (occupancy) down.
-template <int WT, bool EXTRA>
+// Per-warp staging slice.
+template <int WT>
 struct WarpSlice {
     int off[WT + 1];   // global edge offset of each staged entry
     int rs[WT + 1];    // CSR row start of each staged entry
-    int aux[WT + 1];   // per-entry payload (distance snapshot, vertex id, ...)
-    int aux2[WT + 1];  // second payload (priority, ...)
+    int aux[WT + 1];   // per-entry payloads
+    int aux2[WT + 1];
     int flag[WT + 1];  // per-entry accumulator flushed after the tile
     int seg[WT];       // tile edge slot -> staged entry
 };
-template <int WT>
-struct WarpSlice<WT, false> {
-    int off[WT + 1];
-    int rs[WT + 1];
-    int aux[WT + 1];
-    int seg[WT];
-};
 
-template <int BLOCK, int VT, bool EXTRA = true>
+template <int BLOCK, int VT>
 struct ExpandSmem {
     static constexpr int NWARP = BLOCK / 32;
     static constexpr int WT = 32 * VT;  // items (entries + edges) per warp tile
     static constexpr int BATCH = BLOCK; // warp tiles whose splits are found together
-    using Warp = WarpSlice<WT, EXTRA>;
+    using Warp = WarpSlice<WT>;
     static constexpr int QCAP = 128;  // per-warp queue staging (see WarpQueue)
     int qbuf[NWARP][2][QCAP];
     int base[kMaxGrid + 1];  // exclusive prefix of chunk totals
@@ -61,21 +55,16 @@ struct ExpandSmem {
     Warp w[NWARP];
 };
 
-struct RowIsEntry {
-    __device__ __forceinline__ int operator()(int e) const { return e; }
-};
-
 // Phase A over this block's chunk of queue q[0, nf). hook(i, v, deg) may rewrite the
-// degree (e.g. 0 for an entry that needs no expansion) and do per-entry work; the CSR row
-// of queue entry e is row_of(e) (the entry itself unless the entry packs more).
-template <int BLOCK, class Hook, class RowOf = RowIsEntry>
+// degree (e.g. 0 for an entry that needs no expansion) and do per-entry work.
+template <int BLOCK, class Hook>
 __device__ __forceinline__ void frontier_phase_a(const int *__restrict__ q, int nf,
                                                  const int *__restrict__ row_ptr, int *rs,
                                                  int *loc_off, int *chunk_sum, int *scan_tmp,
-                                                 Hook hook, RowOf row_of = RowOf(), VGrid vg = hw_grid()) {
-    const int G = vg.n;
+                                                 Hook hook) {
+    const int G = gridDim.x;
     const int C = (nf + G - 1) / G;
-    const int c0 = min(vg.id * C, nf);
+    const int c0 = min(static_cast<int>(blockIdx.x) * C, nf);
     const int c1 = min(c0 + C, nf);
     int carry = 0;
     for (int base = c0; base < c1; base += BLOCK) {
@@ -83,9 +72,8 @@ __device__ __forceinline__ void frontier_phase_a(const int *__restrict__ q, int 
         int deg = 0;
         if (i < c1) {
             const int v = __ldcg(q + i);
-            const int row = row_of(v);
-            const int r0 = __ldg(row_ptr + row);
-            deg = __ldg(row_ptr + row + 1) - r0;
+            const int r0 = __ldg(row_ptr + v);
+            deg = __ldg(row_ptr + v + 1) - r0;
             deg = hook(i, v, deg);
             rs[i] = r0;
         }
@@ -94,15 +82,15 @@ __device__ __forceinline__ void frontier_phase_a(const int *__restrict__ q, int 
         if (i < c1) loc_off[i] = carry + ex;
         carry += tot;
     }
-    if (threadIdx.x == 0) chunk_sum[vg.id] = carry;
+    if (threadIdx.x == 0) chunk_sum[blockIdx.x] = carry;
 }
 
 // Loads the chunk totals of phase A into base[] as an exclusive prefix; returns the total
 // number of edges of the frontier.
 template <int BLOCK>
 __device__ __forceinline__ int frontier_chunk_bases(const int *__restrict__ chunk_sum, int *base,
-                                                    int *scan_tmp, VGrid vg = hw_grid()) {
-    const int G = vg.n;
+                                                    int *scan_tmp) {
+    const int G = gridDim.x;
     const int per = (G + BLOCK - 1) / BLOCK;
     const int t0 = threadIdx.x * per;
     int local = 0;
@@ -157,18 +145,18 @@ __device__ __forceinline__ int frontier_merge_path(long long diag, int nf, int E
 // Phase B. load(j, k, ws) stages entry j's payload into the warp slice at k;
 // op(valid, k, idx, ws) handles a lane's VT edges (CSR positions idx[], owning staged
 // entries k[]); post(ne, ws) runs after the tile's edges (per-entry flushes). All three
-// are called by every lane of the warp, so they may use warp collectives. DYN: warps claim
-// the tiles of their block's batch in turn (else tile i goes to warp i % NWARP).
-template <int BLOCK, int VT, bool EXTRA, bool DYN = true, class Load, class Op, class Post>
+// are called by every lane of the warp, so they may use warp collectives. Warps claim
+// the tiles of their block's batch in turn.
+template <int BLOCK, int VT, class Load, class Op, class Post>
 __device__ __forceinline__ void frontier_expand(int nf, int E, const int *__restrict__ loc_off,
                                                 const int *__restrict__ rs,
-                                                ExpandSmem<BLOCK, VT, EXTRA> &sm, Load load, Op op,
-                                                Post post, VGrid vg = hw_grid()) {
-    using S = ExpandSmem<BLOCK, VT, EXTRA>;
+                                                ExpandSmem<BLOCK, VT> &sm, Load load, Op op,
+                                                Post post) {
+    using S = ExpandSmem<BLOCK, VT>;
     constexpr int WT = S::WT;
     constexpr int NWARP = S::NWARP;
     constexpr int BATCH = S::BATCH;
-    const int G = vg.n;
+    const int G = gridDim.x;
     const int C = (nf + G - 1) / G;
     const long long total = static_cast<long long>(nf) + E;
     const long long ntiles = (total + WT - 1) / WT;
@@ -254,19 +242,15 @@ __device__ __forceinline__ void frontier_expand(int nf, int E, const int *__rest
         // cost (atomics, queue flushes) do not leave warps idle at the batch's barrier
         for (long long tile = tb + wid; tile < te;) {
             run_tile(tile, tb);
-            if (DYN) {
-                int nt = 0;
-                if (lane == 0) nt = atomicAdd(&sm.next_tile, 1);
-                tile = tb + __shfl_sync(0xffffffffu, nt, 0);
-            } else {
-                tile += NWARP;
-            }
+            int nt = 0;
+            if (lane == 0) nt = atomicAdd(&sm.next_tile, 1);
+            tile = tb + __shfl_sync(0xffffffffu, nt, 0);
             __syncwarp();
         }
         __syncthreads();
     };
     const long long per = (ntiles + G - 1) / G;
-    const long long t_begin = static_cast<long long>(vg.id) * per;
+    const long long t_begin = static_cast<long long>(blockIdx.x) * per;
     const long long t_end = t_begin + per < ntiles ? t_begin + per : ntiles;
     for (long long tb = t_begin; tb < t_end; tb += BATCH) run_batch(tb, tb + BATCH < t_end ? tb + BATCH : t_end);
 }
@@ -281,7 +265,8 @@ __device__ __forceinline__ void frontier_expand(int nf, int E, const int *__rest
 // on, and the edges, all of them a fixed number of dependent reads.
 //
 // It replaces phase A, its grid barrier and the merge-path searches above where the entries'
-// row lengths are final when they are appended (BFS); rows of length zero are only counted.
+// row lengths are final when they are appended (BFS), and the searches where an iteration takes its
+// entries off another queue first (SSSP, batched SSSP); rows of length zero are only counted.
 struct EdgeQueue {
     int *off;                  // edge offset of each entry
     int *delta;                // row start - off: edge t of the queue is CSR entry t + delta
@@ -416,16 +401,25 @@ __host__ __device__ inline int edge_unit_shift(long long nnz, long long slots, i
     return s;
 }
 
-// op(valid, pay, idx) on every edge of the queue, VT per lane (CSR positions idx[]; with PAY,
-// pay[] is the `payload` of each edge's entry), called by all lanes of the warp. A tile's
+struct NoPayload {};
+__device__ __forceinline__ NoPayload ld_payload(const NoPayload *) { return NoPayload{}; }
+template <class P>
+__device__ __forceinline__ P ld_payload(const P *p) {
+    return __ldcg(p);
+}
+
+// op(valid, pay, idx) on every edge of the queue, VT per lane (CSR positions idx[]; pay[] is the
+// `payload` of each edge's entry, unless NoPayload), called by all lanes of the warp. A tile's
 // entries are read 32 at a time; where each begins goes into a mask of its edges in registers, so
-// an edge finds its entry by counting bits. `slice`: 32 * VT ints of shared memory (twice as
-// many with PAY), private to the warp; units are at least a tile. (Fetching the next tile's entries, columns and weights
+// an edge finds its entry by counting bits. `slice`: shared memory private to the warp, 32 * VT
+// ints and payloads; units are at least a tile. (Fetching the next tile's entries, columns and weights
 // while one is worked on made SSSP slower: 650 us against 619 us at scale 20.)
-template <int VT, bool PAY, class Op>
-__device__ __forceinline__ void edge_expand(const EdgeQueue &q, const int *payload, int nf, int E, int shift,
+template <int VT, class P, class Op>
+__device__ __forceinline__ void edge_expand(const EdgeQueue &q, const P *payload, int nf, int E, int shift,
                                             int *slice, int gwarp, int nwarps, Op op) {
     constexpr int TILE = 32 * VT;
+    constexpr bool PAY = !std::is_same<P, NoPayload>::value;
+    P *pslice = reinterpret_cast<P *>(slice + TILE);
     const int lane = threadIdx.x & 31;
     const unsigned upto = lane == 31 ? 0xffffffffu : (2u << lane) - 1u;
     const int units = E > 0 ? ((E - 1) >> shift) + 1 : 0;
@@ -444,7 +438,7 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const int *paylo
             int n = 0, next = 0x7fffffff;
             if (one) {
                 if (lane == 0) slice[0] = __ldcg(q.delta + k);
-                if (PAY && lane == 1) slice[TILE] = __ldcg(payload + k);
+                if (PAY && lane == 1) pslice[0] = ld_payload(payload + k);
                 begin[0] = 1u;
                 n = 1;
             }
@@ -452,11 +446,11 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const int *paylo
                 const int j = k + n + lane;
                 const int o = j < nf ? __ldcg(q.off + j) : 0x7fffffff;
                 const int d = j < nf ? __ldcg(q.delta + j) : 0;
-                const int p = PAY && j < nf ? __ldcg(payload + j) : 0;
+                const P p = PAY && j < nf ? ld_payload(payload + j) : P{};
                 const bool in = o < t1;
                 const int s = o > t0 ? o - t0 : 0;
                 if (in) slice[n + lane] = d;
-                if (PAY && in) slice[TILE + n + lane] = p;
+                if (PAY && in) pslice[n + lane] = p;
 #pragma unroll
                 for (int r = 0; r < VT; ++r)
                     begin[r] |= __reduce_or_sync(0xffffffffu, in && (s >> 5) == r ? 1u << (s & 31) : 0u);
@@ -469,7 +463,8 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const int *paylo
             }
             __syncwarp();
             bool valid[VT];
-            int pay[VT], idx[VT];
+            P pay[VT];
+            int idx[VT];
             int before = -1;
 #pragma unroll
             for (int r = 0; r < VT; ++r) {
@@ -478,7 +473,7 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const int *paylo
                 before += __popc(begin[r]);
                 valid[r] = t < t1;
                 idx[r] = valid[r] ? t + slice[i] : 0;
-                pay[r] = PAY && valid[r] ? slice[TILE + i] : 0;
+                pay[r] = PAY && valid[r] ? pslice[i] : P{};
             }
             op(valid, pay, idx);
             k += next == t1 ? n : n - 1;  // the entry that holds the next tile's first edge

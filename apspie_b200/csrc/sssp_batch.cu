@@ -9,20 +9,25 @@
 // Labels are vertex-major: the distances of one vertex for the 32 queries of word w sit in
 // one 128-byte line, lab[(v * W + w) * 32 + q % 32]. Frontier entries are (vertex u, query
 // word w) pairs whose "changed" bits (the queries whose distance at u dropped in the
-// previous iteration) are non-zero; an entry's weight is deg(u), so the merge-path
-// expander balances the edges. A warp keeps its tile's edges as 16-byte records in shared
-// memory and walks them four at a time, eight lanes to an edge, four queries to a lane: a lane
-// reads 16 bytes of u's and of v's label line, relaxes nd = dist[q][u] + w(u,v) where q
-// changed at u, and atomicMin's the label; the improved queries replace the changed ones in
-// the record, and at the end of the tile each lane ORs its own edges' into v's next changed
-// word, enqueueing (v, w) on the first bit.
+// previous iteration) are non-zero. An iteration puts them on an edge queue (frontier.cuh)
+// with their changed word, so that the edges are shared out evenly. A warp keeps its tile's
+// edges as 16-byte records in shared memory and walks them four at a time, eight lanes to an
+// edge, four queries to a lane: a lane reads 16 bytes of u's and of v's label line, relaxes
+// nd = dist[q][u] + w(u,v) where q changed at u, and atomicMin's the label; the improved
+// queries go into the record, a byte per lane, and at the end of the tile each lane ORs its
+// own edges' into v's next changed word, enqueueing (v, w) on the first bit.
 //
-// What bounds it: instruction issue (62 % of the slots used with one edge at a time) and the
+// What bounds it: instruction issue (half of the slots; 16 instructions a visit) and the
 // latency of the label reads. 100 queries on R-MAT of 2^19 vertices (345M visits of a row's
 // entry for a word): one edge at a time, a lane per query, 18.9 ms; four edges a step with
-// their fields by shuffles 15.1 ms, target labels through L1 too 14.2 ms, fields as records
-// 12.9 ms (one step in flight instead of two: 14.6 ms; four blocks per SM instead of five:
-// 13.1 ms).
+// their fields as records 12.9 ms (26.6 instructions a visit, half of them in the merge-path
+// searches that shared out the edges); edge queue and improved queries as bytes instead of
+// shuffles 10.3 ms; no branch around the label reads 9.3 ms; five blocks per SM instead of
+// four 8.9 ms. One step in flight instead of two 10.0, four 9.5 ms; tiles of 32, 64 and 96
+// edges 9.8, 8.9 and 9.4 ms. Bands of distances per query, also counted from each query's
+// distance to the highest-degree vertex, and bounds by way of up to 32 such vertices spare
+// relaxations but hardly any visits (5.5 to 18 a row's entry instead of 6.4): a visit serves
+// all 32 queries of a word, and some of them want it in each iteration.
 // Every query reaches the same label-correcting fixed point as apspie_sssp computes alone
 // (exact shortest distances for non-negative integer weights). A last pass transposes the
 // labels into the query-major output out[q * m + v] (0xFFFFFFFF, -1 as int32, unreached).
@@ -36,40 +41,50 @@ namespace apspie {
 namespace {
 
 constexpr int kSbBlock = 256;
-constexpr int kSbVT = 2;
+constexpr int kSbVT = 4;
+constexpr int kSbTile = 32 * kSbVT;
 constexpr int kSbSteps = 2;  // steps of four edges whose label reads a warp issues together
-// every lane's edge is visited exactly once per pass: a second visit would not record the
-// queries it improves
-static_assert(32 % (4 * kSbSteps) == 0, "the steps must divide the warp");
-using SbSmem = ExpandSmem<kSbBlock, kSbVT>;
-using SbWarp = SbSmem::Warp;
-using SbWQ = WarpQueue<SbSmem::QCAP>;
+constexpr int kSbPA = 4;  // entries a thread takes off the queue together
+constexpr int kSbQCap = 128;
+// every edge of a tile is visited exactly once
+static_assert(kSbTile % (4 * kSbSteps) == 0, "the steps must divide the tile");
+using SbWQ = WarpQueue<kSbQCap>;
 
 enum : int { kSiteSb = 500, kSiteSbNeg = 501, kSiteSbOverflow = 502, kSiteSbCap = 503, kSiteSbBadSource = 504 };
 
+// Bit of a query in the words that say which queries changed: its label's place in the 128-byte
+// line is 4 l + c (lane l of the eight at an edge, component c), and the lanes' four bits are
+// stored as bytes and folded, l and l + 4 into the same byte.
+__device__ __forceinline__ int sb_shift(int l) { return ((l & 3) << 3) | ((l >> 2) << 2); }
+__device__ __forceinline__ unsigned sb_bit(int q) { return 1u << (sb_shift((q & 31) >> 2) + (q & 3)); }
+
 struct SbArgs {
-    int m, nnz, nq, W;
+    int m, nnz, nq, W, shift;
     const int *__restrict__ row_ptr;
     const int *__restrict__ col_ind;
     const int *__restrict__ wt;
     const int *__restrict__ srcs;
     unsigned *lab;         // m x W x 32 labels, vertex-major, pre-filled with 0xFFFFFFFF
-    unsigned *chg[2];      // m x W changed-query words (ping-pong)
-    unsigned *cbits;       // per frontier entry: its changed word (copied in phase A)
-    int *q[2];             // frontier entries u * W + w
-    int *rs, *loc_off, *chunk_sum;
+    unsigned *chg;         // m x W changed-query words
+    int *q;                // frontier: u * W + w of the non-zero ones
+    uint2 *ent;            // the edge queue's entries: u * W + w and its changed word
+    int *off, *delta, *owner;
     TravCtl *ctl;
     int *sticky;
 };
 
-struct RowOfPacked {
-    int W;
-    __device__ __forceinline__ int operator()(int e) const { return e / W; }
+struct SbShared {
+    union {
+        int slice[kSbBlock / 32][3 * kSbTile];  // edge_expand's
+        unsigned long long scan[33];            // phase A's
+    };
+    uint4 rec[kSbBlock / 32][kSbTile];
+    int qbuf[kSbBlock / 32][kSbQCap];
+    unsigned long long abase;
 };
 
 __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
-    __shared__ SbSmem sm;
-    __shared__ uint4 s_rec[kSbBlock / 32][32 * kSbVT];
+    __shared__ __align__(16) SbShared sh;
     grid_begin(a.ctl);
     const int G = gridDim.x;
     const int gtid = blockIdx.x * kSbBlock + threadIdx.x;
@@ -79,14 +94,14 @@ __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
     const int wid = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    for (long long i = gtid; i < mw; i += gstride) {
-        a.chg[0][i] = 0u;
-        a.chg[1][i] = 0u;
+    for (long long i = gtid; i < mw; i += gstride) a.chg[i] = 0u;
+    if (gtid == 0) {
+        a.ctl->qlen[0] = a.ctl->qlen[1] = 0;
+        a.ctl->rcnt64[0] = a.ctl->rcnt64[1] = 0ull;
     }
-    if (gtid == 0) a.ctl->qlen[0] = a.ctl->qlen[1] = 0;
     if (!grid_barrier(a.ctl, a.sticky, kSiteSb)) return;
     {
-        SbWQ wq(sm.qbuf[wid][0], a.q[0], &a.ctl->qlen[0]);
+        SbWQ wq(sh.qbuf[wid], a.q, &a.ctl->qlen[0]);
         for (int base = blockIdx.x * kSbBlock; base < a.nq; base += gstride) {
             const int qi = base + threadIdx.x;
             bool fresh = false;
@@ -98,7 +113,7 @@ __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
                 } else {
                     e = v * W + (qi >> 5);
                     a.lab[static_cast<size_t>(e) * 32 + (qi & 31)] = 0u;
-                    fresh = atomicOr(a.chg[0] + e, 1u << (qi & 31)) == 0u;
+                    fresh = atomicOr(a.chg + e, sb_bit(qi)) == 0u;
                 }
             }
             wq.push(fresh, e);
@@ -116,65 +131,103 @@ __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
             if (gtid == 0) raise_error(a.ctl, a.sticky, APSPIE_ERR_NOT_CONVERGED, kSiteSbCap);
             break;
         }
-        ++iters;
-        int *qc = a.q[cur];
-        int *qn = a.q[cur ^ 1];
-        unsigned *cc = a.chg[cur];
-        unsigned *cn = a.chg[cur ^ 1];
-        unsigned *cbits = a.cbits;
-        // phase A: take each entry's changed word (and clear it for reuse), row degrees
-        frontier_phase_a<kSbBlock>(qc, nf, a.row_ptr, a.rs, a.loc_off, a.chunk_sum, sm.scan_tmp,
-                                   [&](int i, int e, int deg) {
-                                       const unsigned b = __ldcg(cc + e);
-                                       cbits[i] = b;
-                                       cc[e] = 0u;
-                                       return b ? deg : 0;
-                                   },
-                                   RowOfPacked{W});
-        if (gtid == 0) a.ctl->qlen[cur ^ 1] = 0;
+        // phase A: take each entry's changed word (and clear it for reuse) and put the entry on
+        // the iteration's edge queue
+        unsigned long long *asize = a.ctl->rcnt64 + (iters & 1);
+        {
+            const int C = (nf + G - 1) / G;
+            const int c0 = min(static_cast<int>(blockIdx.x) * C, nf);
+            const int c1 = min(c0 + C, nf);
+            for (int base = c0; base < c1; base += kSbBlock * kSbPA) {
+                int e[kSbPA], r0[kSbPA], deg[kSbPA];
+                unsigned bits[kSbPA];
+#pragma unroll
+                for (int k = 0; k < kSbPA; ++k) {
+                    const int i = base + k * kSbBlock + threadIdx.x;
+                    e[k] = i < c1 ? __ldcg(a.q + i) : -1;
+                }
+                int sum = 0, cnt = 0;
+#pragma unroll
+                for (int k = 0; k < kSbPA; ++k) {
+                    r0[k] = deg[k] = 0;
+                    bits[k] = 0u;
+                    if (e[k] >= 0) {
+                        const int u = e[k] / W;
+                        bits[k] = __ldcg(a.chg + e[k]);
+                        r0[k] = __ldg(a.row_ptr + u);
+                        deg[k] = __ldg(a.row_ptr + u + 1) - r0[k];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kSbPA; ++k) {
+                    if (e[k] >= 0) a.chg[e[k]] = 0u;
+                    sum += deg[k];
+                    cnt += deg[k] > 0;
+                }
+                const unsigned long long mine = (static_cast<unsigned long long>(cnt) << 32) | static_cast<unsigned>(sum);
+                const unsigned long long incl = block_inclusive_scan_u64<kSbBlock>(mine, sh.scan);
+                if (threadIdx.x == 0 && sh.scan[32]) sh.abase = atomicAdd(asize, sh.scan[32]);
+                __syncthreads();
+                const unsigned long long at = sh.abase + incl - mine;
+                int idx = static_cast<int>(at >> 32), off = static_cast<int>(at & 0xffffffffull);
+#pragma unroll
+                for (int k = 0; k < kSbPA; ++k) {
+                    const bool some = deg[k] > 0;
+                    eq_write(a.off, a.delta, a.owner, a.shift, some, idx, off, r0[k], deg[k]);
+                    if (some) a.ent[idx] = make_uint2(static_cast<unsigned>(e[k]), bits[k]);
+                    idx += some;
+                    off += deg[k];
+                }
+                __syncthreads();  // the scan's words and the base are reused by the next step
+            }
+        }
         if (!grid_barrier(a.ctl, a.sticky, kSiteSb + 1)) return;
-        const int E = frontier_chunk_bases<kSbBlock>(a.chunk_sum, sm.base, sm.scan_tmp);
+        // the queue has been read: phase B fills it again, and counts in the other length
+        const unsigned long long asz = __ldcg(asize);
+        const int ne = static_cast<int>(asz >> 32), E = static_cast<int>(asz & 0xffffffffull);
+        if (gtid == 0) {
+            a.ctl->qlen[cur] = 0;
+            a.ctl->rcnt64[(iters & 1) ^ 1] = 0ull;
+        }
+        ++iters;
         relaxed += E;
-        SbWQ wq(sm.qbuf[wid][0], qn, &a.ctl->qlen[cur ^ 1]);
+        SbWQ wq(sh.qbuf[wid], a.q, &a.ctl->qlen[cur ^ 1]);
         const int *col = a.col_ind;
         const int *wt = a.wt;
         unsigned *lab = a.lab;
+        unsigned *chg = a.chg;
+        uint4 *rec = sh.rec[wid];
         TravCtl *ctl = a.ctl;
         int *sticky = a.sticky;
-        frontier_expand<kSbBlock, kSbVT, true>(
-            nf, E, a.loc_off, a.rs, sm,
-            [&](int j, int k, SbWarp &ws) {
-                const int e = __ldcg(qc + j);
-                ws.aux[k] = e;                  // entry u * W + w
-                ws.flag[k] = e - (e / W) * W;   // query word w
-                ws.aux2[k] = static_cast<int>(__ldcg(cbits + j));
-            },
-            [&](const bool (&valid)[kSbVT], const int (&kk)[kSbVT], const int (&idx)[kSbVT], SbWarp &ws) {
+        EdgeQueue qe{a.off, a.delta, a.owner, nullptr, nullptr};
+        edge_expand<kSbVT>(
+            qe, a.ent, ne, E, a.shift, sh.slice[wid], wid * G + blockIdx.x, G * (kSbBlock / 32),
+            [&](const bool (&valid)[kSbVT], const uint2 (&src)[kSbVT], const int (&idx)[kSbVT]) {
                 // the tile's edges as records: target entry (v, w), weight + 1, source entry and
-                // its changed bits, which the edge's improved queries replace
-                uint4 *rec = s_rec[wid];
+                // its changed queries; the improved queries replace the last two, a byte per lane
                 int ned = 0, tv[kSbVT];
+                int v[kSbVT], we[kSbVT];
 #pragma unroll
                 for (int r = 0; r < kSbVT; ++r) {
-                    uint4 e = make_uint4(0u, 0u, 0u, 0u);
-                    tv[r] = 0;
-                    if (valid[r]) {
-                        const int v = __ldg(col + idx[r]);
-                        const int we = __ldg(wt + idx[r]);
-                        tv[r] = v * W + ws.flag[kk[r]];
-                        e = make_uint4(static_cast<unsigned>(tv[r]), static_cast<unsigned>(we) + 1u,
-                                       static_cast<unsigned>(ws.aux[kk[r]]), static_cast<unsigned>(ws.aux2[kk[r]]));
-                        if (we < 0) {  // reported once here; the edge is then left out
-                            raise_error(ctl, sticky, APSPIE_ERR_INVALID_ARG, kSiteSbNeg);
-                            e.w = 0u;
-                        }
+                    v[r] = valid[r] ? __ldg(col + idx[r]) : 0;
+                    we[r] = valid[r] ? __ldg(wt + idx[r]) : 0;
+                }
+#pragma unroll
+                for (int r = 0; r < kSbVT; ++r) {
+                    const unsigned e = src[r].x;
+                    unsigned bits = src[r].y;
+                    tv[r] = v[r] * W + static_cast<int>(e - (e / static_cast<unsigned>(W)) * static_cast<unsigned>(W));
+                    if (we[r] < 0) {  // reported once here; the edge is then left out
+                        raise_error(ctl, sticky, APSPIE_ERR_INVALID_ARG, kSiteSbNeg);
+                        bits = 0u;
                     }
-                    rec[r * 32 + lane] = e;
+                    rec[r * 32 + lane] =
+                        make_uint4(static_cast<unsigned>(tv[r]), static_cast<unsigned>(we[r]) + 1u, e, bits);
                     ned += __popc(__ballot_sync(0xffffffffu, valid[r]));
                 }
                 __syncwarp();
                 // four edges a step, eight lanes each, four queries (16 bytes of the label line) a lane
-                const int sub4 = 4 * (lane & 7), grp = lane >> 3;
+                const int sub = lane & 7, grp = lane >> 3, sub4 = 4 * sub, shift = sb_shift(sub);
                 bool over = false;
 #pragma unroll 1
                 for (int l0 = 0; l0 < ned; l0 += 4 * kSbSteps) {
@@ -184,67 +237,59 @@ __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
 #pragma unroll
                     for (int t = 0; t < kSbSteps; ++t) {
                         const uint4 e = rec[l0 + 4 * t + grp];
-                        act[t] = (e.w >> sub4) & 15u;
+                        act[t] = (e.w >> shift) & 15u;
                         w1[t] = e.y;
                         lv[t] = lab + static_cast<size_t>(e.x) * 32 + sub4;
-                        if (act[t]) {
-                            // through L1 (a row's edges all read the same source line, and many edges
-                            // the lines of high-degree targets). u's labels: one lowered in this
-                            // iteration has its change bit set for the next, so any value since the
-                            // barrier will do. v's: a stale, larger value only costs an atomic and
-                            // one more expansion of v's query
-                            du[t] = *reinterpret_cast<const uint4 *>(lab + static_cast<size_t>(e.z) * 32 + sub4);
-                            dv[t] = *reinterpret_cast<const uint4 *>(lv[t]);
-                        }
+                        // through L1 (a row's edges all read the same source line, and many edges the
+                        // lines of high-degree targets), by all lanes (of the lanes with no query to
+                        // relax, one in twelve, a branch costs more than the reads). u's labels: one
+                        // lowered in this iteration has its change bit set for the next, so any value
+                        // since the barrier will do. v's: a stale, larger value only costs an atomic
+                        // and one more expansion of v's query
+                        du[t] = *reinterpret_cast<const uint4 *>(lab + static_cast<size_t>(e.z) * 32 + sub4);
+                        dv[t] = *reinterpret_cast<const uint4 *>(lv[t]);
                     }
+                    __syncwarp();  // the records are read: their last halves take the results
                     // an improvement over the label just read is reported without waiting for the
                     // atomic's old value: if another edge lowered the label further meanwhile, v's
                     // query is only re-expanded once more (same values)
 #pragma unroll
                     for (int t = 0; t < kSbSteps; ++t) {
-                        unsigned imp = 0u;
-                        if (act[t]) {
-                            // s = candidate + 1. An active label is finite (< 2^31 - 1) and the weight
-                            // non-negative, so s does not wrap, and s > 2^31 - 1 is an overflow; an
-                            // inactive, unreached label wraps to the weight, below that
-                            unsigned s0 = du[t].x + w1[t], s1 = du[t].y + w1[t];
-                            unsigned s2 = du[t].z + w1[t], s3 = du[t].w + w1[t];
-                            if (static_cast<int>(s0 | s1 | s2 | s3) < 0) {
-                                const unsigned big = (s0 >> 31) | ((s1 >> 31) << 1) | ((s2 >> 31) << 2) | ((s3 >> 31) << 3);
-                                over |= (big & act[t]) != 0u;
-                                act[t] &= ~big;
-                            }
-                            imp = ((s0 <= dv[t].x ? 1u : 0u) | (s1 <= dv[t].y ? 2u : 0u) | (s2 <= dv[t].z ? 4u : 0u) |
-                                   (s3 <= dv[t].w ? 8u : 0u)) &
-                                  act[t];
-                            if (imp) {
-                                if (imp & 1u) atomicMin(lv[t], s0 - 1u);
-                                if (imp & 2u) atomicMin(lv[t] + 1, s1 - 1u);
-                                if (imp & 4u) atomicMin(lv[t] + 2, s2 - 1u);
-                                if (imp & 8u) atomicMin(lv[t] + 3, s3 - 1u);
-                            }
+                        // s = candidate + 1. An active label is finite (< 2^31 - 1) and the weight
+                        // non-negative, so s does not wrap, and s > 2^31 - 1 is an overflow; an
+                        // inactive, unreached label wraps to the weight, below that
+                        const unsigned s0 = du[t].x + w1[t], s1 = du[t].y + w1[t];
+                        const unsigned s2 = du[t].z + w1[t], s3 = du[t].w + w1[t];
+                        if (static_cast<int>(s0 | s1 | s2 | s3) < 0) {
+                            const unsigned big = (s0 >> 31) | ((s1 >> 31) << 1) | ((s2 >> 31) << 2) | ((s3 >> 31) << 3);
+                            over |= (big & act[t]) != 0u;
+                            act[t] &= ~big;
                         }
-                        unsigned m = 0u;
-                        if (__any_sync(0xffffffffu, imp != 0u)) {
-                            m = imp << sub4;
-                            m |= __shfl_xor_sync(0xffffffffu, m, 1);
-                            m |= __shfl_xor_sync(0xffffffffu, m, 2);
-                            m |= __shfl_xor_sync(0xffffffffu, m, 4);
+                        const unsigned imp = ((s0 <= dv[t].x ? 1u : 0u) | (s1 <= dv[t].y ? 2u : 0u) |
+                                              (s2 <= dv[t].z ? 4u : 0u) | (s3 <= dv[t].w ? 8u : 0u)) &
+                                             act[t];
+                        if (imp) {
+                            if (imp & 1u) atomicMin(lv[t], s0 - 1u);
+                            if (imp & 2u) atomicMin(lv[t] + 1, s1 - 1u);
+                            if (imp & 4u) atomicMin(lv[t] + 2, s2 - 1u);
+                            if (imp & 8u) atomicMin(lv[t] + 3, s3 - 1u);
                         }
-                        if (sub4 == 0) rec[l0 + 4 * t + grp].w = m;
+                        reinterpret_cast<unsigned char *>(&rec[l0 + 4 * t + grp].z)[sub] = static_cast<unsigned char>(imp);
                     }
                 }
                 if (over) raise_error(ctl, sticky, APSPIE_ERR_INVALID_ARG, kSiteSbOverflow);
                 __syncwarp();
 #pragma unroll
                 for (int r = 0; r < kSbVT; ++r) {
-                    const unsigned mine = rec[r * 32 + lane].w;  // improved queries of this lane's edge r
+                    // improved queries of this lane's edge r (a slot without an edge was either not
+                    // visited or has none)
+                    const uint4 e = rec[r * 32 + lane];
+                    const unsigned mine = valid[r] ? e.z | (e.w << 4) : 0u;
                     bool fresh = false;
-                    if (mine) fresh = atomicOr(cn + tv[r], mine) == 0u;
+                    if (mine) fresh = atomicOr(chg + tv[r], mine) == 0u;
                     wq.push(fresh, tv[r]);
                 }
-            },
-            [](int, SbWarp &) {});
+            });
         wq.flush();
         if (!grid_barrier(a.ctl, a.sticky, kSiteSb + 2)) return;
         cur ^= 1;
@@ -285,7 +330,7 @@ size_t sssp_batch_scratch_need(int m, int nq) {
     const int W = ((nq < 512 ? nq : 512) + 31) / 32;
     const size_t mw = static_cast<size_t>(m) * (W > 0 ? W : 1);
     const size_t multi =
-        Carver::need({mw * 128, mw * 4, mw * 4, mw * 4, mw * 4, mw * 4, mw * 4, mw * 4, kMaxGrid * 4});
+        Carver::need({mw * 128, mw * 4, mw * 4, mw * 8, mw * 4, mw * 4, mw * 4 + 4});
     // the grouped form (groups > 0): at most 4 groups are costed here
     const size_t grouped = sssp_group_scratch_need(m, std::max(1, std::min(nq, 4)));
     return std::max(multi, grouped);
@@ -322,20 +367,19 @@ extern "C" apspie_status apspie_sssp_batch(apspie_ctx *ctx, const apspie_csr *A,
         const size_t mw = static_cast<size_t>(m) * W;
         void *base;
         st = scratch_reserve(
-            ctx, Carver::need({mw * 128, mw * 4, mw * 4, mw * 4, mw * 4, mw * 4, mw * 4, mw * 4, kMaxGrid * 4}),
+            ctx, Carver::need({mw * 128, mw * 4, mw * 4, mw * 8, mw * 4, mw * 4, mw * 4 + 4}),
             &base);
         if (st != APSPIE_OK) return st;
         Carver c(base);
         SbArgs a;
         a.lab = c.take<unsigned>(mw * 32);
-        a.chg[0] = c.take<unsigned>(mw);
-        a.chg[1] = c.take<unsigned>(mw);
-        a.cbits = c.take<unsigned>(mw);
-        a.q[0] = c.take<int>(mw);
-        a.q[1] = c.take<int>(mw);
-        a.rs = c.take<int>(mw);
-        a.loc_off = c.take<int>(mw);
-        a.chunk_sum = c.take<int>(kMaxGrid);
+        a.chg = c.take<unsigned>(mw);
+        a.q = c.take<int>(mw);
+        a.ent = c.take<uint2>(mw);
+        a.off = c.take<int>(mw);
+        a.delta = c.take<int>(mw);
+        a.owner = c.take<int>(mw + 1);
+        a.shift = edge_unit_shift(static_cast<long long>(A->nnz) * W, static_cast<long long>(mw) + 1, kSbTile);
         a.m = m;
         a.nnz = A->nnz;
         a.nq = nq;

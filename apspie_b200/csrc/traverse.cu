@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_kernel(BfsArgs a) {
             // while few vertices are visited, claiming at once saves a trip to L2 per level; later
             // most neighbours are visited and a look spares the atomic
             const bool look = reached * 16 > m;
-            edge_expand<4, false>(qc, nullptr, nq, E, a.shift, s_slice[wid], gwarp, nwarps,
-                        [&](const bool (&valid)[4], const int (&)[4], const int (&idx)[4]) {
+            edge_expand<4>(qc, static_cast<const NoPayload *>(nullptr), nq, E, a.shift, s_slice[wid], gwarp, nwarps,
+                        [&](const bool (&valid)[4], const NoPayload (&)[4], const int (&idx)[4]) {
                             int v[4];
                             unsigned word[4];
                             bool fresh[4];
@@ -627,7 +627,7 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
         WQ wf(sh.far[wid], fcur, &a.ctl->flen[fc]);
         bool bad = false, over = false;
         EdgeQueue qa{a.buf.rs, a.buf.loc_off, a.buf.aux3, nullptr, nullptr};
-        edge_expand<kSsspVT, true>(
+        edge_expand<kSsspVT>(
             qa, snap, nact, E, a.shift, sh.slice[wid], wid * G + vg.id, G * (kBlock / 32),
             [&](const bool (&valid)[kSsspVT], const int (&du)[kSsspVT], const int (&idx)[kSsspVT]) {
                 int v[kSsspVT], we[kSsspVT], cd[kSsspVT], nd[kSsspVT];

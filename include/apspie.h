@@ -238,7 +238,7 @@ apspie_status apspie_bfs_batch(apspie_ctx *ctx, const apspie_csr *A, const int32
 /* Batched multi-source SSSP over int32 weights in one persistent launch. d_dists is
  * num_sources x m int32, query-major (row q = what apspie_sssp returns for d_sources[q]);
  * -1 unreached. By default a multi-query kernel relaxes all changed queries of a frontier
- * row together, one warp per edge with a lane per query over vertex-major labels
+ * row together, eight lanes per edge with four queries a lane over vertex-major labels
  * (32*W queries per launch with (nnz + m) * W < 2^31, W <= 16; device scratch about
  * 160 * m * W bytes). With apspie_ctx_set_sssp_batch_groups(ctx, g > 0) the launch's blocks
  * split into g query groups instead, each running the single-source kernel on its share. */

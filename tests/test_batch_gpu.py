@@ -258,6 +258,39 @@ def test_sssp_batch_label_arithmetic_limits(ctx, case, nq):
         assert out[0, -1] == 2 ** 31 - 2
 
 
+@pytest.mark.parametrize("nq", [3, 32, 97])
+@pytest.mark.parametrize("shape", ["star 127", "star 128", "star 129", "star 20000", "comb", "ring of hubs"])
+def test_sssp_batch_edge_queue_shapes(ctx, shape, nq):
+    """Rows that fill, just miss and cross the edge queue's units and a warp's tile; a row of many
+    units; tiles of rows of one and two entries; several long rows of one frontier. Every query of
+    a word improves something, so each place in the changed words is used."""
+    import torch
+
+    rng = np.random.default_rng(7)
+    kind, _, size = shape.partition(" ")
+    if kind == "star":
+        m = int(size) + 1
+        src, dst = np.zeros(m - 1, np.int64), np.arange(1, m)
+    elif kind == "comb":
+        m = 4000
+        src, dst = np.arange(m - 1), np.arange(1, m)
+        src, dst = np.concatenate((src, np.arange(0, m - 9, 7))), np.concatenate((dst, np.arange(9, m, 7)[:len(np.arange(0, m - 9, 7))]))
+    else:
+        hubs, spokes = 40, 150
+        m = hubs * (spokes + 1)
+        h = np.arange(hubs)
+        src = np.concatenate((h, np.repeat(h, spokes)))
+        dst = np.concatenate(((h + 1) % hubs, np.arange(hubs, m)))
+    s2, d2 = np.concatenate((src, dst)), np.concatenate((dst, src))
+    key = np.unique(s2 * m + d2)
+    rp = np.concatenate(([0], np.cumsum(np.bincount(key // m, minlength=m)))).astype(np.int32)
+    g = ap.HostGraph(m, m, rp, (key % m).astype(np.int32), rng.integers(0, 256, len(key)).astype(np.int32))
+    sources = rng.integers(0, m, nq).astype(np.int32)
+    out = ctx.sssp_batch(ap.DeviceGraph(g), torch.from_numpy(sources).cuda()).cpu().numpy()
+    for q, s in enumerate(sources):
+        np.testing.assert_array_equal(out[q], oracle.sssp(g.row_ptr, g.col_ind, g.val, int(s)), err_msg=str(q))
+
+
 @pytest.mark.parametrize("nq", [1, 33, 100, 129, 300])
 @pytest.mark.parametrize("m", [4096, 4097, 9001])
 def test_bfs_batch_row_classes_and_long_paths(ctx, nq, m):
