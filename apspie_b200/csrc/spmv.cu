@@ -75,14 +75,37 @@ apspie_status launch_spmv(apspie_ctx *ctx, const apspie_csr *A, const float *x, 
 constexpr int kPrBlock = 256;
 constexpr int kPrItems = 8;
 constexpr int kPrChunk = kPrBlock * kPrItems;
-constexpr int kPrVec = 1024;  // threads a block in the vector kernels: two blocks an SM, one atomic each
+constexpr int kPrVec = 256;  // threads a block in the vector kernels, four blocks an SM
+constexpr int kPrOwn = 2;    // vertices whose data a thread fetches together
 constexpr int kPrBatch = 4;
 
+// Sums over the vertices, each in kPrSlots parts, and the word that every block looks at first, all
+// in cache lines of their own: blocks that start while others still write to the line of their
+// first look wait for it (with everything in one line the gathers of 700,001 vertices and 10.7M
+// entries took 683 us in 16 iterations and the updates 187; 1, 2, 4, 8 and 16 parts: 759, 753, 736, 747 and
+// 768 us together).
+constexpr int kPrSlots = 4;
 struct PrState {
-    double dang[2];  // rank mass of the vertices without out-edges, by iteration parity
-    double diff[2];  // L1 change, by iteration parity
-    int done;        // iterations after which the change was below tol (0: not yet)
+    struct {
+        double dang[2];  // rank mass of the vertices without out-edges, by iteration parity
+        double diff[2];  // L1 change, by iteration parity
+        double pad[12];
+    } part[kPrSlots];
+    int done;  // iterations after which the change was below tol (0: not yet)
     int pad;
+
+    __host__ __device__ double dang(int i) const {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < kPrSlots; ++k) s += part[k].dang[i];
+        return s;
+    }
+    __host__ __device__ double diff(int i) const {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < kPrSlots; ++k) s += part[k].diff[i];
+        return s;
+    }
 };
 
 __device__ __forceinline__ double block_sum(double v, double *tmp) {
@@ -129,7 +152,7 @@ __global__ void __launch_bounds__(kPrVec) pr_init(int n, const int *__restrict__
         if (d == 0) dang += r0;
     }
     dang = block_sum(dang, tmp);
-    if (threadIdx.x == 0 && dang != 0.0) atomicAdd(&st->dang[0], dang);
+    if (threadIdx.x == 0 && dang != 0.0) atomicAdd(&st->part[blockIdx.x % kPrSlots].dang[0], dang);
 }
 
 // VEC: col is 16-byte aligned
@@ -141,19 +164,10 @@ __global__ void __launch_bounds__(kPrBlock) pr_gather(long long nnz, const int *
                                                       const int *err) {
     __shared__ float s_val[kPrBlock / 32];
     __shared__ int s_any[kPrBlock / 32];
-    if (err && ld_volatile_i32(err) != 0) return;
-    if (ld_volatile_i32(&st->done) != 0) return;
-    if (it > 0 && st->diff[(it - 1) & 1] < tol) {  // every block sees the same: the last launch wrote it
-        if (blockIdx.x == 0 && threadIdx.x == 0) st->done = it;
-        return;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // read by the last launch, added to by the next
-        st->dang[(it + 1) & 1] = 0.0;
-        st->diff[it & 1] = 0.0;
-    }
+    // the columns are fetched beside the words that say whether they are to be used (604 -> 580 us
+    // in 16 iterations)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long c0 = static_cast<long long>(blockIdx.x) * kPrChunk;
-    if (c0 >= nnz) return;
     const long long e0 = c0 + tid * kPrItems;
     int u[kPrItems];
     if (VEC && e0 + kPrItems <= nnz) {
@@ -166,6 +180,19 @@ __global__ void __launch_bounds__(kPrBlock) pr_gather(long long nnz, const int *
         for (int j = 0; j < kPrItems; ++j) u[j] = e0 + j < nnz ? __ldg(col + e0 + j) : -1;
     }
     const unsigned m = e0 < nnz ? __ldg(heads + (e0 >> 3)) : 0u;
+    const int bad = err ? ld_volatile_i32(err) : 0;
+    const int done = ld_volatile_i32(&st->done);
+    const double change = it > 0 ? st->diff((it - 1) & 1) : 0.0;  // the last launch wrote it
+    if (bad != 0 || done != 0) return;
+    if (it > 0 && change < tol) {  // every block sees the same
+        if (blockIdx.x == 0 && tid == 0) st->done = it;
+        return;
+    }
+    if (blockIdx.x == 0 && tid < kPrSlots) {  // read by the last launch, added to by the next
+        st->part[tid].dang[(it + 1) & 1] = 0.0;
+        st->part[tid].diff[it & 1] = 0.0;
+    }
+    if (c0 >= nnz) return;
     float v[kPrItems];
 #pragma unroll
     for (int j = 0; j < kPrItems; ++j) v[j] = u[j] >= 0 ? __ldg(x + u[j]) : 0.0f;
@@ -233,38 +260,56 @@ __global__ void __launch_bounds__(kPrBlock) pr_gather(long long nnz, const int *
 }
 
 // r'[v] = (1 - d) / n + d * (sum over in-edges + dangling / n), the L1 change, and the next
-// iteration's x and dangling mass; 14 us for 700,001 vertices before (two kernels, 34 us, and
-// a wait for the host every iteration).
+// iteration's x and dangling mass. 7.0 us for 700,001 vertices (14 MB, 2.1 us at the copy rate:
+// launch, the loads' latency and the blocks' sums); with one vertex at a time and the sums beside
+// the first look's word 11.7 us; one vertex, four blocks of 512 7.9 us.
 __global__ void __launch_bounds__(kPrVec) pr_update(int n, float damping, const int *__restrict__ in_rp,
                                                       const int *__restrict__ out_rp, const float *__restrict__ y,
                                                       const float *__restrict__ carry, float *r, float *x,
                                                       PrState *st, int it, const int *err) {
     __shared__ double tmp[kPrVec / 32];
-    if (err && ld_volatile_i32(err) != 0) return;
-    if (ld_volatile_i32(&st->done) != 0) return;
-    const float base = static_cast<float>((1.0 - damping) / n + damping * st->dang[it & 1] / n);
+    const int bad = err ? ld_volatile_i32(err) : 0;
+    const int done = ld_volatile_i32(&st->done);
+    if (bad != 0 || done != 0) return;
+    const float base = static_cast<float>((1.0 - damping) / n + damping * st->dang(it & 1) / n);
     double diff = 0.0, dang = 0.0;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const int a = __ldg(in_rp + v), b = __ldg(in_rp + v + 1);
-        float s = 0.0f;
-        if (b > a) {
-            s = y[v];
-            const int c1 = (b - 1) / kPrChunk;
-#pragma unroll 4
-            for (int c = a / kPrChunk + 1; c <= c1; ++c) s += __ldg(carry + c);
+    const int stride = gridDim.x * blockDim.x;
+    for (int v0 = blockIdx.x * blockDim.x + threadIdx.x; v0 < n; v0 += kPrOwn * stride) {
+        int a[kPrOwn], b[kPrOwn], d[kPrOwn];
+        float s[kPrOwn], old[kPrOwn];
+#pragma unroll
+        for (int k = 0; k < kPrOwn; ++k) {
+            const int v = v0 + k * stride;
+            const bool in = v < n && v >= v0;
+            a[k] = in ? __ldg(in_rp + v) : 0;
+            b[k] = in ? __ldg(in_rp + v + 1) : 0;
+            d[k] = in ? __ldg(out_rp + v + 1) - __ldg(out_rp + v) : 1;
+            s[k] = in ? y[v] : 0.0f;  // rows without entries have none
+            old[k] = in ? r[v] : 0.0f;
         }
-        const float nr = __fmaf_rn(damping, s, base);
-        diff += fabs(static_cast<double>(nr) - static_cast<double>(r[v]));
-        r[v] = nr;
-        const int d = __ldg(out_rp + v + 1) - __ldg(out_rp + v);
-        x[v] = d > 0 ? nr / static_cast<float>(d) : 0.0f;
-        if (d == 0) dang += nr;
+#pragma unroll
+        for (int k = 0; k < kPrOwn; ++k) {
+            const int v = v0 + k * stride;
+            if (v >= n || v < v0) break;
+            if (b[k] > a[k]) {
+                const int c1 = (b[k] - 1) / kPrChunk;
+#pragma unroll 4
+                for (int c = a[k] / kPrChunk + 1; c <= c1; ++c) s[k] += __ldg(carry + c);
+            } else {
+                s[k] = 0.0f;
+            }
+            const float nr = __fmaf_rn(damping, s[k], base);
+            diff += fabs(static_cast<double>(nr) - static_cast<double>(old[k]));
+            r[v] = nr;
+            x[v] = d[k] > 0 ? nr / static_cast<float>(d[k]) : 0.0f;
+            if (d[k] == 0) dang += nr;
+        }
     }
     diff = block_sum(diff, tmp);
     dang = block_sum(dang, tmp);
     if (threadIdx.x == 0) {
-        if (diff != 0.0) atomicAdd(&st->diff[it & 1], diff);
-        if (dang != 0.0) atomicAdd(&st->dang[(it + 1) & 1], dang);
+        if (diff != 0.0) atomicAdd(&st->part[blockIdx.x % kPrSlots].diff[it & 1], diff);
+        if (dang != 0.0) atomicAdd(&st->part[blockIdx.x % kPrSlots].dang[(it + 1) & 1], dang);
     }
 }
 
@@ -325,7 +370,7 @@ apspie_status apspie_pagerank(apspie_ctx *ctx, const apspie_csr *A, float dampin
     st = sym ? expand_entry_rows(ctx, A, reinterpret_cast<unsigned *>(mat_base))
              : transpose_pattern(ctx, A, mat_base, &in);
     if (st != APSPIE_OK) return st;
-    const int vblocks = std::max(1, std::min((n + kPrVec - 1) / kPrVec, ctx->num_sms * 2));
+    const int vblocks = std::max(1, std::min((n + kPrVec - 1) / kPrVec, ctx->num_sms * 4));
     const int gblocks = static_cast<int>((nnz + kPrChunk - 1) / kPrChunk);
     if (nnz > 0)
         pr_heads<<<static_cast<int>(std::min<long long>((nnz / 8 + 256) / 256, ctx->num_sms * 8LL)), 256, 0,
@@ -353,7 +398,7 @@ apspie_status apspie_pagerank(apspie_ctx *ctx, const apspie_csr *A, float dampin
             it = h.done;
             break;
         }
-        if (it >= max_iter || h.diff[(it - 1) & 1] < tol) break;
+        if (it >= max_iter || h.diff((it - 1) & 1) < tol) break;
     }
     if (iterations) *iterations = it;
     return APSPIE_OK;
