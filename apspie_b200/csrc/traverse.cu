@@ -957,7 +957,7 @@ __device__ __forceinline__ int mis_scan_thread(const MisArgs &a, int v, unsigned
 // block has decided anything for the context's wait limit: blocks count their passes that did
 // in ctl->aux[0].
 __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
-    __shared__ int s_n[2], s_long, s_huge, s_decided, s_stop, s_end;
+    __shared__ int s_n[2], s_long, s_huge[2], s_decided, s_stop, s_end;
     __shared__ int s_lv[kMisLong], s_lp[kMisLong], s_hv[kMisHuge], s_hp[kMisHuge];
     grid_begin(a.ctl);
     const int G = gridDim.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -967,7 +967,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
     // the part of the lists that holds this block's vertices
     const int tiles = (m - 1) / kBlock + 1, each = tiles / G, extra = tiles % G, b = blockIdx.x;
     const size_t part = (static_cast<size_t>(b) * each + min(b, extra)) * kBlock;
-    if (tid == 0) s_n[0] = s_n[1] = s_long = s_huge = s_decided = s_end = 0;
+    if (tid == 0) s_n[0] = s_n[1] = s_long = s_huge[0] = s_huge[1] = s_decided = s_end = 0;
     if (!grid_barrier(a.ctl, a.sticky, kSiteMis)) return;
 
     long long insz = 0, scanned = 0;
@@ -1047,7 +1047,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
                 const int v = a.v[at], by = a.by[at];
                 int pos = a.pos[at];
                 if (by == v) {  // a push that goes on
-                    const int h = atomicAdd(&s_huge, 1);
+                    const int h = atomicAdd(&s_huge[cur], 1);
                     if (h < kMisHuge) {
                         s_hv[h] = v;
                         s_hp[h] = pos;
@@ -1085,7 +1085,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
                 const int r0 = __ldg(a.row_ptr + v);
                 if (r1 - r0 > kMisWarp) {
                     if (lane == 0) {
-                        const int at = atomicAdd(&s_huge, 1);
+                        const int at = atomicAdd(&s_huge[cur], 1);
                         if (at < kMisHuge) {
                             s_hv[at] = v;
                             s_hp[at] = -2 - r0;
@@ -1145,7 +1145,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
                 } else if (code != kScanOn) {
                     outcome(nxt, code, v, pos, by);
                 } else {
-                    const int at = atomicAdd(&s_huge, 1);
+                    const int at = atomicAdd(&s_huge[cur], 1);
                     if (at < kMisHuge) {
                         s_hv[at] = v;
                         s_hp[at] = pos;
@@ -1157,7 +1157,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
         }
         __syncthreads();
         // the longest, by the block, 1,024 neighbours a step and kMisPart at a time
-        const int nhuge = min(s_huge, kMisHuge);
+        const int nhuge = min(s_huge[cur], kMisHuge);
         for (int i = 0; i < nhuge; ++i) {
             const int v = s_hv[i], r1 = __ldg(a.row_ptr + v + 1), p = s_hp[i];
             if (p < -1) {  // a push, from CSR index -2 - p on
@@ -1216,7 +1216,8 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
             // the next pass reads states through L1, which this acquire has dropped
             ld_acquire_u64(&a.ctl->aux[0]);
             s_n[cur] = 0;
-            s_long = s_huge = 0;
+            s_long = 0;
+            s_huge[nxt] = 0;  // (a warp may still be about to read this pass's)
             if (s_n[nxt] == 0) s_end = 1;
             if (s_decided) {
                 s_decided = 0;
