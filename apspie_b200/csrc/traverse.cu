@@ -1357,6 +1357,14 @@ cudaError_t noalloc_scratch(void **out) {
 
 size_t traversal_scratch_need(int m) { return trav_scratch_bytes(m); }
 
+// Blocks of a BFS launch, one to three an SM: more shorten a level's expansion, fewer its barrier
+// and its queue (a block's reservations are made one after the other). R-MAT, one / two / three:
+// 1.7M entries 32.5 / 34.0 / 37.2 us; 4.3M 37.2 / 36.9 / 41.1; 7.6M 44.7 / 41.4 / 43.6; 11.7M
+// 52.2 / 45.8 / 45.8; 31.4M 86 / 64 / 60.
+long long bfs_blocks(int num_sms, long long nnz) {
+    return static_cast<long long>(num_sms) * (nnz >= 10000000 ? 3 : nnz >= 3000000 ? 2 : 1);
+}
+
 // what mis_common reserves: the states and the blocks' lists (whole tiles)
 size_t mis_scratch_need(int m) {
     const size_t l = (static_cast<size_t>(m) + kBlock) * 8;
@@ -1411,7 +1419,8 @@ apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, i
     a.beta = tp.bfs_beta;
     a.allow_pull = (A->flags & APSPIE_CSR_SYMMETRIC) ? 1 : 0;
     void *args[] = {&a};
-    st = launch_persistent(ctx, reinterpret_cast<const void *>(bfs_kernel), kBfsBlock, args, A->nnz);
+    st = launch_persistent(ctx, reinterpret_cast<const void *>(bfs_kernel), kBfsBlock, args,
+                           bfs_blocks(ctx->num_sms, A->nnz) * kWorkPerBlock);
     if (st != APSPIE_OK) return st;
     return finish_call(ctx, stats, "apspie_bfs");
 }
@@ -1448,9 +1457,11 @@ namespace {
 // Blocks of a launch: throughput grows with the warps on an SM (553 us with five blocks an SM
 // against 568 us with four and 802 us with two at scale 20), but so do the barriers' times,
 // and an iteration of a smaller graph has no more than a tile for each warp (6.7M entries:
-// 306 us with three, 315 us with four, 333 us with five).
+// 306 us with three, 315 us with four, 333 us with five; 3.1M: 247 us with three, 239 with two;
+// 0.43M: 190 with three, 177 with one; 0.04M: 168 and 160).
 long long sssp_blocks(const apspie_ctx *ctx, long long nnz) {
-    return static_cast<long long>(ctx->num_sms) * (nnz >= 25000000 ? 5 : nnz >= 12000000 ? 4 : 3);
+    return static_cast<long long>(ctx->num_sms) *
+           (nnz >= 25000000 ? 5 : nnz >= 12000000 ? 4 : nnz >= 5000000 ? 3 : nnz >= 1200000 ? 2 : 1);
 }
 
 // Edges per iteration: an eighth of the graph's where an iteration's edges are most of its
@@ -1670,8 +1681,7 @@ apspie_status apspie_bfs_noalloc(const apspie_csr *A, int32_t source, int32_t de
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_kernel, kBfsBlock, 0) != cudaSuccess ||
         per_sm < 1)
         return APSPIE_ERR_CUDA;
-    long long grid = (static_cast<long long>(A->nnz) + kWorkPerBlock - 1) / kWorkPerBlock;
-    if (grid < sms) grid = sms;
+    long long grid = bfs_blocks(sms, A->nnz);
     if (grid > static_cast<long long>(per_sm) * sms) grid = static_cast<long long>(per_sm) * sms;
     if (grid > kMaxGrid) grid = kMaxGrid;
     void *args[] = {&a};
