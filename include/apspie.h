@@ -78,7 +78,7 @@ typedef struct apspie_csr_owned {
 /* Per-call statistics (filled only when a non-NULL pointer is passed; that call then
  * synchronises the stream). */
 typedef struct apspie_run_stats {
-    int32_t iterations;        /* BFS levels / SSSP iterations / MIS rounds executed */
+    int32_t iterations;        /* BFS levels / SSSP iterations / MIS passes (of the block with most) */
     int32_t push_iterations;   /* iterations expanded top-down (push) */
     int32_t pull_iterations;   /* iterations expanded bottom-up (pull) */
     int32_t reserved;
@@ -153,7 +153,7 @@ int64_t apspie_ctx_scratch_bytes(const apspie_ctx *ctx);
  * knobs of its kind (unless apspie_ctx_set_autotune(ctx, 0)). No reference counterpart:
  * the reference's thresholds are compile-time constants. */
 typedef struct apspie_tune_params {
-    float bfs_alpha;          /* BFS push -> pull when frontier edges > unvisited edges / alpha */
+    float bfs_alpha;          /* BFS push -> pull when frontier edges > max(unvisited edges, nnz / 8) / alpha */
     float bfs_beta;           /* BFS pull -> push when frontier < m / beta */
     float batch_push_frac;    /* batched BFS: push while frontier edges < frac * nnz */
     int32_t sssp_delta;       /* SSSP far-pile step (<= 0: none with the band, else device-chosen) */
