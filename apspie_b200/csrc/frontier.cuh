@@ -412,18 +412,27 @@ __device__ __forceinline__ P ld_payload(const P *p) {
 // `payload` of each edge's entry, unless NoPayload), called by all lanes of the warp. A tile's
 // entries are read 32 at a time; where each begins goes into a mask of its edges in registers, so
 // an edge finds its entry by counting bits. `slice`: shared memory private to the warp, 32 * VT
-// ints and payloads; units are at least a tile. (Fetching the next tile's entries, columns and weights
+// ints and payloads; units are at least a tile. A block has every nblocks-th unit and its warps take
+// them in turn (`claim`: in shared memory, zero at first): units differ in their rows and in what
+// they improve, and with a fixed share per warp the blocks waited for their slowest warps (SSSP
+// scale 20 558 -> 534 us, batched SSSP 8.75 -> 8.03 ms, BFS 60.1 -> 58.9 us). (Fetching the next tile's entries, columns and weights
 // while one is worked on made SSSP slower: 650 us against 619 us at scale 20.)
 template <int VT, class P, class Op>
 __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const P *payload, int nf, int E, int shift,
-                                            int *slice, int gwarp, int nwarps, Op op) {
+                                            int *slice, int *claim, int block, int nblocks, Op op) {
     constexpr int TILE = 32 * VT;
     constexpr bool PAY = !std::is_same<P, NoPayload>::value;
     P *pslice = reinterpret_cast<P *>(slice + TILE);
     const int lane = threadIdx.x & 31;
     const unsigned upto = lane == 31 ? 0xffffffffu : (2u << lane) - 1u;
     const int units = E > 0 ? ((E - 1) >> shift) + 1 : 0;
-    for (int u = gwarp; u < units; u += nwarps) {
+    auto take = [&]() {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(claim, 1);
+        const long long u = block + static_cast<long long>(__shfl_sync(0xffffffffu, i, 0)) * nblocks;
+        return static_cast<int>(u < units ? u : units);
+    };
+    for (int u = take(); u < units; u = take()) {
         int k = __ldcg(q.owner + u);
         // the next unit's owner, read beside it: when it is the same entry, the unit lies inside
         // that entry's row

@@ -23,7 +23,7 @@
 // their fields as records 12.9 ms (26.6 instructions a visit, half of them in the merge-path
 // searches that shared out the edges); edge queue and improved queries as bytes instead of
 // shuffles 10.3 ms; no branch around the label reads 9.3 ms; five blocks per SM instead of
-// four 8.9 ms. One step in flight instead of two 10.0, four 9.5 ms; tiles of 32, 64 and 96
+// four 8.9 ms; warps taking their block's units in turn 8.0 ms. With a fixed share: one step in flight instead of two 10.0, four 9.5 ms; tiles of 32, 64 and 96
 // edges 9.8, 8.9 and 9.4 ms. Bands of distances per query, also counted from each query's
 // distance to the highest-degree vertex, and bounds by way of up to 32 such vertices spare
 // relaxations but hardly any visits (5.5 to 18 a row's entry instead of 6.4): a visit serves
@@ -81,6 +81,7 @@ struct SbShared {
     uint4 rec[kSbBlock / 32][kSbTile];
     int qbuf[kSbBlock / 32][kSbQCap];
     unsigned long long abase;
+    int claim[2];  // units taken, by iteration parity
 };
 
 __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
     const int lane = threadIdx.x & 31;
 
     for (long long i = gtid; i < mw; i += gstride) a.chg[i] = 0u;
+    if (threadIdx.x < 2) sh.claim[threadIdx.x] = 0;
     if (gtid == 0) {
         a.ctl->qlen[0] = a.ctl->qlen[1] = 0;
         a.ctl->rcnt64[0] = a.ctl->rcnt64[1] = 0ull;
@@ -191,6 +193,7 @@ __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
         }
         ++iters;
         relaxed += E;
+        if (threadIdx.x == 0) sh.claim[(iters & 1) ^ 1] = 0;
         SbWQ wq(sh.qbuf[wid], a.q, &a.ctl->qlen[cur ^ 1]);
         const int *col = a.col_ind;
         const int *wt = a.wt;
@@ -201,7 +204,7 @@ __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
         int *sticky = a.sticky;
         EdgeQueue qe{a.off, a.delta, a.owner, nullptr, nullptr};
         edge_expand<kSbVT>(
-            qe, a.ent, ne, E, a.shift, sh.slice[wid], wid * G + blockIdx.x, G * (kSbBlock / 32),
+            qe, a.ent, ne, E, a.shift, sh.slice[wid], &sh.claim[iters & 1], blockIdx.x, G,
             [&](const bool (&valid)[kSbVT], const uint2 (&src)[kSbVT], const int (&idx)[kSbVT]) {
                 // the tile's edges as records: target entry (v, w), weight + 1, source entry and
                 // its changed queries; the improved queries replace the last two, a byte per lane

@@ -125,8 +125,9 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_kernel(BfsArgs a) {
     __shared__ int s_buf[kBfsBlock / 32][kEqCap];
     __shared__ int s_slice[kBfsBlock / 32][kEqTile];
     __shared__ EqBlock<kBfsBlock> s_blk;
+    __shared__ int s_claim[2];  // units taken, by level parity
     grid_begin(a.ctl);
-    if (threadIdx.x == 0) s_blk.empty = 0;
+    if (threadIdx.x == 0) s_blk.empty = s_claim[0] = s_claim[1] = 0;
     const int gtid = blockIdx.x * kBfsBlock + threadIdx.x;
     const int gstride = gridDim.x * kBfsBlock;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -176,6 +177,7 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_kernel(BfsArgs a) {
             pull = false;
         }
         ++levels;
+        if (threadIdx.x == 0) s_claim[(L & 1) ^ 1] = 0;
         if (gtid == 0) {
             size[s2] = 0ull;
             empty[s2] = 0;
@@ -205,7 +207,8 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_kernel(BfsArgs a) {
             // while few vertices are visited, claiming at once saves a trip to L2 per level; later
             // most neighbours are visited and a look spares the atomic
             const bool look = reached * 16 > m;
-            edge_expand<4>(qc, static_cast<const NoPayload *>(nullptr), nq, E, a.shift, s_slice[wid], gwarp, nwarps,
+            edge_expand<4>(qc, static_cast<const NoPayload *>(nullptr), nq, E, a.shift, s_slice[wid],
+                           &s_claim[L & 1], blockIdx.x, gridDim.x,
                         [&](const bool (&valid)[4], const NoPayload (&)[4], const int (&idx)[4]) {
                             int v[4];
                             unsigned word[4];
@@ -343,6 +346,7 @@ struct SsspShared {
     int hmin;                             // least distance this block queued
     int dbase;                            // where this block's deferred entries go
     unsigned long long abase;             // and its expanded entries and their edges
+    int claim[2];                         // units taken, by iteration parity
     int sent[kBlock / 32];                // per warp: vertices it queues at the end, then where
 };
 
@@ -419,7 +423,10 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
         a.ctl->rcnt64[0] = a.ctl->rcnt64[1] = 0ull;
     }
     sh.hist[threadIdx.x] = 0ull;
-    if (threadIdx.x == 0) sh.hmin = INF;
+    if (threadIdx.x == 0) {
+        sh.hmin = INF;
+        sh.claim[0] = sh.claim[1] = 0;
+    }
     if (!grid_barrier(a.ctl, a.sticky, kSiteSssp, vg)) return;
 
     const bool banded = a.band > 0;
@@ -606,6 +613,7 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
         const int nact = static_cast<int>(asz >> 32), E = static_cast<int>(asz & 0xffffffffull);
         expanded += E;
         ++iters;
+        if (threadIdx.x == 0) sh.claim[(iters & 1) ^ 1] = 0;
         const int *col = a.col_ind;
         const int *wt = a.w;
         const int *rp = a.row_ptr;
@@ -628,7 +636,7 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
         bool bad = false, over = false;
         EdgeQueue qa{a.buf.rs, a.buf.loc_off, a.buf.aux3, nullptr, nullptr};
         edge_expand<kSsspVT>(
-            qa, snap, nact, E, a.shift, sh.slice[wid], wid * G + vg.id, G * (kBlock / 32),
+            qa, snap, nact, E, a.shift, sh.slice[wid], &sh.claim[iters & 1], vg.id, G,
             [&](const bool (&valid)[kSsspVT], const int (&du)[kSsspVT], const int (&idx)[kSsspVT]) {
                 int v[kSsspVT], we[kSsspVT], cd[kSsspVT], nd[kSsspVT];
                 bool got[kSsspVT], queue[kSsspVT];
