@@ -452,6 +452,7 @@ template <int W, bool SERVE>
 __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_kernel(MsArgs a) {
     __shared__ MsSmem sm;
     __shared__ unsigned s_qmask[W];   // query slots in flight this level
+    __shared__ int s_claim[2];        // pull tiles taken by the block's warps, by level parity
     __shared__ unsigned s_alive[W];   // bits this block found in the next frontier (engine)
     __shared__ int *s_row[SERVE ? 32 * W : 1];  // engine: each slot's output row this level
     __shared__ int s_base[SERVE ? 32 * W : 1];  // engine: each slot's start level
@@ -498,6 +499,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
         *qlen_ptr(a.ctl, 2) = 0;
         *tqlen = 0;
     }
+    if (threadIdx.x < 2) s_claim[threadIdx.x] = 0;
     if (threadIdx.x < W) {
         s_qmask[threadIdx.x] = query_mask(a.nq, threadIdx.x);
         s_alive[threadIdx.x] = 0u;
@@ -597,6 +599,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
         if (!SERVE && nA == 0) break;
         if (!SERVE && a.depth_cap > 0 && L + 1 >= a.depth_cap) break;
         ++levels;
+        if (threadIdx.x == 0) s_claim[(L & 1) ^ 1] = 0;
         if (!SERVE && L + 2 - plane_base >= 1 << kPlanes) {  // the planes are full: their depths go out
             write_depths<W, true>(a, mw, plane_base, !written);
             written = true;
@@ -712,8 +715,17 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
             static_assert(sizeof(MsWarp) >= 32 * (W + 1) * 4 + 32 * 4, "a warp's results fit its slice");
             unsigned *s_got = reinterpret_cast<unsigned *>(&sm.w[wid]);
             int *s_list = reinterpret_cast<int *>(s_got + 32 * (W + 1));
-            for (int base = blockIdx.x * kMsBlock; base < m; base += gstride) {
-                const int v = base + threadIdx.x;
+            // the block's warps take its vertices in turn, 32 at a time (with a fixed share per
+            // warp 1,386 us instead of 1,322 for 32 sources on 4.2M vertices, 1,082 instead of
+            // 1,029 for 64 on 2.1M)
+            for (;;) {
+                int t = 0;
+                if (lane == 0) t = atomicAdd(&s_claim[L & 1], 1);
+                t = __shfl_sync(FULL, t, 0);
+                const long long tile = blockIdx.x + static_cast<long long>(t / (kMsBlock / 32)) * gridDim.x;
+                const long long v0 = tile * kMsBlock;
+                if (v0 >= m) break;
+                const int v = static_cast<int>(v0) + t % (kMsBlock / 32) * 32 + lane;
                 int r0 = 0, r1 = 0;
                 bool todo = false, grouped = false;
                 unsigned got[W];
