@@ -46,7 +46,7 @@ struct TcInfo {
     unsigned long long count;
     int overflow;
     int not_lower;  // an entry with column >= row
-    int dup;        // two equal entries next to each other in a row
+    int unsorted;   // a row whose entries don't ascend strictly (it may hold an entry twice)
     int ticket;     // owners handed out
     int owners[2];  // owners with many partners, with few
 };
@@ -155,11 +155,11 @@ __global__ void __launch_bounds__(kTcColumnsBlock) tc_columns(unsigned nnz, int 
         s_cnt[k] = 0;
     }
     __syncthreads();
-    bool bad = false, dup = false;
+    bool bad = false, unsorted = false;
     for (unsigned e = blockIdx.x * kTcColumnsBlock + threadIdx.x; e < nnz; e += gridDim.x * kTcColumnsBlock) {
         const int i = static_cast<int>(__ldg(row + e)), j = __ldg(ci + e);
         bad |= j >= i || j < 0;
-        dup |= e > 0 && __ldg(ci + e - 1) == j && static_cast<int>(__ldg(row + e - 1)) == i;
+        unsorted |= e > 0 && __ldg(ci + e - 1) >= j && static_cast<int>(__ldg(row + e - 1)) == i;
         if (j < 0 || j >= m) continue;
         const int k = j & (kTcSlots - 1);
         int of = s_col[k];
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kTcColumnsBlock) tc_columns(unsigned nnz, int 
             atomicAdd(deg + j, 1);
     }
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&info->not_lower, 1);
-    if (__any_sync(0xffffffffu, dup) && (threadIdx.x & 31) == 0) atomicOr(&info->dup, 1);
+    if (__any_sync(0xffffffffu, unsorted) && (threadIdx.x & 31) == 0) atomicOr(&info->unsorted, 1);
     __syncthreads();
     for (int k = threadIdx.x; k < kTcSlots; k += kTcColumnsBlock)
         if (s_cnt[k]) atomicAdd(deg + s_col[k], s_cnt[k]);
@@ -436,9 +436,10 @@ __global__ void __launch_bounds__(kTcBlock) tc_block(const int *__restrict__ row
 // Measured at scale 18: counting 2.74 ms with hash sets; 0.55 ms with bitmaps (and 0.14 ms for the
 // partner lists), at 64 % of the issue slots and 72 % of the L1/shared-memory pipe.
 //
-// Needs: L strict lower triangular without equal neighbours in a row (both found out on the
-// way: a row's list then is a set, so that either side may be the bitmap), and the bitmap to
-// fit an SM's shared memory. Everything else is counted by the hash path above.
+// Needs: L strict lower triangular with strictly ascending rows (both found out on the way: a
+// row's list then is a set, so that either side may be the bitmap; in rows out of order an entry
+// may be repeated anywhere), and the bitmap to fit an SM's shared memory. Everything else is
+// counted by the hash path above.
 constexpr int kTcBitmapVertices = 1600 * 1024;  // 200 KB of bits
 constexpr int kTcManyPartners = 256;            // owners with at least this many start first
 
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(1024) tc_bits(int m, const int *__restrict__ l
                                                 const int *__restrict__ plist, TcInfo *info) {
     extern __shared__ unsigned bits[];
     __shared__ int s_next;
-    if (info->not_lower || info->dup) return;
+    if (info->not_lower || info->unsorted) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nthreads = blockDim.x, nwarps = nthreads >> 5;
     const int nmany = info->owners[0], nall = nmany + info->owners[1];
@@ -627,7 +628,7 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
         (e = cudaMemcpyAsync(&h, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
         return cuda_error(ctx, e, "tc result");
-    if (h.not_lower || h.dup) return APSPIE_OK;
+    if (h.not_lower || h.unsorted) return APSPIE_OK;
     if (h.overflow) return set_error(ctx, APSPIE_ERR_HASH_OVERFLOW, "apspie_tc: mask set overflow");
     *count = static_cast<int64_t>(h.count);
     *counted = true;

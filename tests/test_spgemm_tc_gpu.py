@@ -275,3 +275,26 @@ def test_tc_of_what_is_no_set_of_lower_entries(ctx, what):
         assert got == int(((D @ D) * (D > 0)).sum())
     else:
         assert got == int(((d @ d) * d).sum())
+
+
+@pytest.mark.parametrize("m,p", [(60, 0.5), (400, 0.1)])
+def test_tc_of_rows_out_of_order(ctx, m, p):
+    """Rows whose entries don't ascend: as many triangles as in order without repeated entries;
+    with entries repeated at the end of their row (never beside each other), the wedges of the
+    oriented edges whose end is in the first vertex's set, each as often as its edges are given."""
+    rng = np.random.default_rng(m)
+    rows, cols = np.nonzero(np.tril(rng.random((m, m)) < p, -1))
+    for repeats in (0, rows.size // 3):
+        largest = np.append(rows[1:] != rows[:-1], True)
+        again = rng.choice(np.nonzero(~largest)[0], repeats, replace=False)
+        r, c = np.concatenate((rows, rows[again])), np.concatenate((cols, cols[again]))
+        order = np.lexsort((c if repeats else -c, np.arange(r.size) >= rows.size, r))
+        r, c = r[order], c[order]
+        assert not np.any((r[1:] == r[:-1]) & (c[1:] == c[:-1]))
+        deg = np.bincount(r, minlength=m) + np.bincount(c, minlength=m)
+        fwd = (deg[r] < deg[c]) | ((deg[r] == deg[c]) & (r < c))
+        D = np.zeros((m, m), dtype=np.int64)
+        np.add.at(D, (np.where(fwd, r, c), np.where(fwd, c, r)), 1)
+        rp = np.concatenate(([0], np.cumsum(np.bincount(r, minlength=m)))).astype(np.int32)
+        got = ctx.tc(ap.DeviceGraph(ap.HostGraph(m, m, rp, c.astype(np.int32))))
+        assert got == int(((D @ D) * (D > 0)).sum()), repeats
