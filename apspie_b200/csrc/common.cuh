@@ -55,6 +55,15 @@ constexpr size_t kCtlHostBytes = offsetof(TravCtl, sbase);
 
 // Upper bound on a persistent grid (chunk sums are staged in shared memory).
 constexpr int kMaxGrid = 1024;
+
+// A position in a CSR's entries that a loop steps past the end: nnz may be 2^31 - 1, where an
+// int would turn negative.
+using Pos = unsigned;
+// Entries up to which a kernel may step past the end in an int (by a block's step at most); it is
+// faster in places, and what is beyond takes the path that does not.
+constexpr int kMaxStepped = 0x7fffffff - (1 << 16);
+// The end of the next `step` entries from `from` on, none past `end`.
+__host__ __device__ inline int step_end(int from, int step, int end) { return end - from > step ? from + step : end; }
 // A grid barrier gives up after this long (ns) and raises APSPIE_ERR_TIMEOUT, unless the
 // context sets another bound (apspie_ctx_set_wait_limit).
 constexpr unsigned long long kBarrierTimeoutNs = 4000000000ull;

@@ -439,8 +439,8 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const P *payload
         const bool one = u + 1 < units && __ldcg(q.owner + u + 1) == k;
         const long long uend = (static_cast<long long>(u) + 1) << shift;
         const int end = uend < E ? static_cast<int>(uend) : E;
-        for (int t0 = u << shift; t0 < end; t0 += TILE) {
-            const int t1 = min(t0 + TILE, end);
+        for (int t0 = u << shift, t1; t0 < end; t0 = t1) {
+            t1 = step_end(t0, TILE, end);
             unsigned begin[VT];
 #pragma unroll
             for (int r = 0; r < VT; ++r) begin[r] = 0u;
@@ -477,11 +477,11 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const P *payload
             int before = -1;
 #pragma unroll
             for (int r = 0; r < VT; ++r) {
-                const int t = t0 + r * 32 + lane;
+                const int x = r * 32 + lane;  // behind t0
                 const int i = before + __popc(begin[r] & upto);
                 before += __popc(begin[r]);
-                valid[r] = t < t1;
-                idx[r] = valid[r] ? t + slice[i] : 0;
+                valid[r] = x < t1 - t0;
+                idx[r] = valid[r] ? t0 + x + slice[i] : 0;
                 pay[r] = PAY && valid[r] ? pslice[i] : P{};
             }
             op(valid, pay, idx);

@@ -339,7 +339,7 @@ __device__ __forceinline__ void load_words(unsigned (&x)[VW], const unsigned *p)
 // Lane `sub` of the group holds words [VW * (sub % LQ), ...) of need and, at the end, of got.
 // The frontier words are read through L1: nobody writes them during the level.
 template <int W, int P>
-__device__ __forceinline__ void pull_row(const int *__restrict__ col, const unsigned *frc, int r0, int r1, int sub,
+__device__ __forceinline__ void pull_row(const int *__restrict__ col, const unsigned *frc, Pos r0, Pos r1, int sub,
                                          const unsigned (&need)[PullShape<W>::VW],
                                          unsigned (&got)[PullShape<W>::VW]) {
     constexpr int LQ = PullShape<W>::LQ, VW = PullShape<W>::VW, NB = P / LQ, U = 4;
@@ -348,7 +348,7 @@ __device__ __forceinline__ void pull_row(const int *__restrict__ col, const unsi
 #pragma unroll
     for (int k = 0; k < VW; ++k) got[k] = 0u;
     bool more = r0 < r1;
-    for (int e = r0 + slot; __any_sync(0xffffffffu, more); e += U * NB) {
+    for (Pos e = r0 + slot; __any_sync(0xffffffffu, more); e += U * NB) {
         int u[U];
         unsigned f[U][VW];
 #pragma unroll
@@ -753,7 +753,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
                     if (W <= 4 && d > 0 && d <= kLaneDeg) {
                         int u[kLaneDeg];
 #pragma unroll
-                        for (int k = 0; k < kLaneDeg; ++k) u[k] = __ldg(a.col_ind + min(r0 + k, r1 - 1));
+                        for (int k = 0; k < kLaneDeg; ++k) u[k] = __ldg(a.col_ind + r0 + min(k, d - 1));
 #pragma unroll
                         for (int k = 0; k < kLaneDeg; ++k) {
                             unsigned f[VW];
@@ -866,7 +866,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
                     some |= nd[k] != 0u;
                 }
                 if (!__any_sync(FULL, some)) continue;
-                const int r0 = __ldg(a.row_ptr + v) + pc.y, r1 = min(r0 + kPiece, __ldg(a.row_ptr + v + 1));
+                const int r0 = __ldg(a.row_ptr + v) + pc.y, r1 = step_end(r0, kPiece, __ldg(a.row_ptr + v + 1));
                 pull_row<W, 32>(a.col_ind, frc, r0, r1, lane, nd, g);
                 bool fresh = false;
 #pragma unroll

@@ -42,6 +42,9 @@ constexpr int kBinDense = 5;   // 5-7: dense accumulator tier, by size class (se
 // The dense tier serves every row past the shared-table tier when C has at most this many
 // columns: an accumulator and a bit per column fit in an SM's shared memory (200 KB).
 constexpr int kDenseCols = 48 * 1024;
+bool takes_dense(const apspie_csr *A, const apspie_csr *B) {
+    return B->n <= kDenseCols && A->nnz <= kMaxStepped && B->nnz <= kMaxStepped;
+}
 constexpr int kDenseBlock = 1024;
 constexpr int kBlockTS = 2048;
 constexpr int kSgBlock = 256;
@@ -791,7 +794,7 @@ apspie_status sg_plan(apspie_ctx *ctx, const apspie_csr *A, const apspie_csr *B,
     cudaError_t e = cudaMemsetAsync(p.info, 0, sizeof(SgInfo), ctx->stream);
     if (e != cudaSuccess) return cuda_error(ctx, e, "spgemm info reset");
     Mat a{A->row_ptr, A->col_ind, A->val}, b{B->row_ptr, B->col_ind, B->val};
-    p.dense = B->n <= kDenseCols;
+    p.dense = takes_dense(A, B);
     if (m > 0) {
         const int blocks = std::min<long long>((static_cast<long long>(m) * 8 + 255) / 256, ctx->num_sms * 16LL);
         const apspie_tune_params tp = effective_params(ctx, APSPIE_TUNE_SPGEMM, A);
@@ -959,7 +962,7 @@ bool sg_cache_load(apspie_ctx *ctx, const apspie_csr *A, const apspie_csr *B, Sg
     for (int b = 0; b < kBins; ++b) p.h.bin_count[b] = static_cast<int>(c.host[b]);
     p.h.global_slots = c.host[8];
     p.row_bin = reinterpret_cast<unsigned char *>(c.host[9]);
-    p.dense = B->n <= kDenseCols;
+    p.dense = takes_dense(A, B);
     return true;
 }
 

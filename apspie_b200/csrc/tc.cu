@@ -744,7 +744,7 @@ apspie_status apspie_tc(apspie_ctx *ctx, const apspie_csr *L, int64_t *count) {
     if (st != APSPIE_OK) return st;
     if (L->m != L->n) return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_tc: L must be square");
     if (ctx->validate && (st = validate_csr(ctx, L, true)) != APSPIE_OK) return st;
-    if (L->m > 0 && L->nnz > 0 && L->m <= kTcBitmapVertices) {
+    if (L->m > 0 && L->nnz > 0 && L->m <= kTcBitmapVertices && L->nnz <= kMaxStepped) {
         bool counted = false;
         st = tc_by_bitmaps(ctx, L, count, &counted);
         if (st != APSPIE_OK || counted) return st;

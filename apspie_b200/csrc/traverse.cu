@@ -895,7 +895,7 @@ enum : int { kScanBlocked, kScanIn, kScanOut, kScanOn };
 
 // A thread's scan of v from CSR index e to lim: where it stops (pos), at whom (by).
 template <bool FIRST>
-__device__ __forceinline__ int mis_scan_thread(const MisArgs &a, int v, unsigned pv, int e, int lim, int r1, int &pos,
+__device__ __forceinline__ int mis_scan_thread(const MisArgs &a, int v, unsigned pv, Pos e, Pos lim, int r1, int &pos,
                                                int &by) {
     for (; e < lim; e += 4) {
         int u[4];
@@ -912,15 +912,15 @@ __device__ __forceinline__ int mis_scan_thread(const MisArgs &a, int v, unsigned
         for (int k = 0; k < 4; ++k) {
             const unsigned char s = mis_look(u[k], pu[k], FIRST ? kUndecided : su[k], v, pv);
             if (s != kOut) {
-                pos = e + k;
+                pos = static_cast<int>(e) + k;
                 by = u[k];
                 return s == kIn ? kScanOut : kScanBlocked;
             }
         }
     }
-    pos = lim - 1;
+    pos = static_cast<int>(lim) - 1;
     by = -1;
-    return lim >= r1 ? kScanIn : kScanOn;
+    return lim >= static_cast<Pos>(r1) ? kScanIn : kScanOn;
 }
 
 // Greedy MIS in descending (priority, id) order -- the set spmspvMis converges to
@@ -1014,13 +1014,13 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
         } else if (code == kScanOn) {
             hand_on(to, v, pos, pos);
         } else {
-            const int r0 = __ldg(a.row_ptr + v), r1 = __ldg(a.row_ptr + v + 1);
+            const Pos r0 = __ldg(a.row_ptr + v), r1 = __ldg(a.row_ptr + v + 1);
             if (r1 - r0 > kMisThread) {
-                if (hand_on(to, v, r1 - 1, kMisPush)) decide(v, true);
+                if (hand_on(to, v, static_cast<int>(r1) - 1, kMisPush)) decide(v, true);
             } else {
                 decide(v, true);
                 scanned += r1 - r0;
-                for (int e = r0; e < r1; e += 4) {
+                for (Pos e = r0; e < r1; e += 4) {
                     int u[4];
                     unsigned char s[4];
 #pragma unroll
@@ -1044,7 +1044,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
                 if (v >= m) continue;
                 const int r0 = __ldg(a.row_ptr + v), r1 = __ldg(a.row_ptr + v + 1);
                 int pos = 0, by = -1;
-                const int code = mis_scan_thread<true>(a, v, __ldg(a.prio + v), r0, min(r1, r0 + kMisThread), r1, pos, by);
+                const int code = mis_scan_thread<true>(a, v, __ldg(a.prio + v), r0, step_end(r0, kMisThread, r1), r1, pos, by);
                 scanned += pos + 1 - r0;
                 outcome(nxt, code, v, pos, by);
             }
@@ -1078,7 +1078,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
                     const int e = pos + 1;
                     int who = -1;
                     const int code =
-                        mis_scan_thread<false>(a, v, pv, e, min(r1, e + kMisThread), r1, pos, who);
+                        mis_scan_thread<false>(a, v, pv, e, step_end(e, kMisThread, r1), r1, pos, who);
                     scanned += pos + 1 - e;
                     outcome(nxt, code, v, pos, who);
                 }
@@ -1088,22 +1088,23 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
         // longer scans, a warp each, 128 neighbours a step
         const int nlong = min(s_long, kMisLong);
         for (int i = wid; i < nlong; i += kBlock / 32) {
-            const int v = s_lv[i], r1 = __ldg(a.row_ptr + v + 1);
+            const int v = s_lv[i];
+            const Pos r1 = __ldg(a.row_ptr + v + 1);
             if (s_lp[i] == kMisPush) {
-                const int r0 = __ldg(a.row_ptr + v);
+                const Pos r0 = __ldg(a.row_ptr + v);
                 if (r1 - r0 > kMisWarp) {
                     if (lane == 0) {
                         const int at = atomicAdd(&s_huge[cur], 1);
                         if (at < kMisHuge) {
                             s_hv[at] = v;
-                            s_hp[at] = -2 - r0;
+                            s_hp[at] = -2 - static_cast<int>(r0);
                         } else {
-                            keep(nxt, v, -2 - r0, v);
+                            keep(nxt, v, -2 - static_cast<int>(r0), v);
                         }
                     }
                     continue;
                 }
-                for (int e = r0; e < r1; e += 128) {
+                for (Pos e = r0; e < r1; e += 128) {
                     int u[4];
                     unsigned char s[4];
 #pragma unroll
@@ -1119,9 +1120,9 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
             }
             const int first = s_lp[i] + 1;
             const unsigned pv = __ldg(a.prio + v);
-            const int lim = min(r1, first + kMisWarp);
-            int code = lim >= r1 ? kScanIn : kScanOn, pos = lim - 1, by = -1;
-            for (int e = first; e < lim && pos >= e; e += 128) {
+            const Pos lim = step_end(first, kMisWarp, r1);
+            int code = lim >= r1 ? kScanIn : kScanOn, pos = static_cast<int>(lim) - 1, by = -1;
+            for (Pos e = first; e < lim; e += 128) {
                 int u[4];
                 unsigned char s[4];
                 unsigned pu[4];
@@ -1139,7 +1140,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
                     const unsigned stops = __ballot_sync(0xffffffffu, s[k] != kOut);
                     if (stops) {
                         const int l = __ffs(stops) - 1;
-                        pos = e + 32 * k + l;
+                        pos = static_cast<int>(e) + 32 * k + l;
                         by = __shfl_sync(0xffffffffu, u[k], l);
                         code = __shfl_sync(0xffffffffu, static_cast<int>(s[k]), l) == kIn ? kScanOut : kScanBlocked;
                     }
@@ -1149,7 +1150,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
             if (lane == 0) {
                 scanned += pos + 1 - first;
                 if (code == kScanIn) {
-                    keep(nxt, v, r1 - 1, -1);  // joins in the next pass, which hands its push on
+                    keep(nxt, v, static_cast<int>(r1) - 1, -1);  // joins in the next pass, which hands its push on
                 } else if (code != kScanOn) {
                     outcome(nxt, code, v, pos, by);
                 } else {
@@ -1169,12 +1170,12 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
         for (int i = 0; i < nhuge; ++i) {
             const int v = s_hv[i], r1 = __ldg(a.row_ptr + v + 1), p = s_hp[i];
             if (p < -1) {  // a push, from CSR index -2 - p on
-                const int first = -2 - p, lim = min(static_cast<long long>(r1), first + static_cast<long long>(kMisPart));
-                for (int e = first + tid; e < lim; e += 4 * kBlock) {
+                const int first = -2 - p, lim = step_end(first, kMisPart, r1);
+                for (Pos e = first + tid; e < static_cast<Pos>(lim); e += 4 * kBlock) {
                     int u[4];
                     unsigned char s[4];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) u[k] = e + k * kBlock < lim ? __ldg(col + e + k * kBlock) : v;
+                    for (int k = 0; k < 4; ++k) u[k] = e + k * kBlock < static_cast<Pos>(lim) ? __ldg(col + e + k * kBlock) : v;
 #pragma unroll
                     for (int k = 0; k < 4; ++k) s[k] = a.state[u[k]];
 #pragma unroll
@@ -1188,16 +1189,16 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
                 }
                 continue;
             }
-            const int first = p + 1, lim = min(static_cast<long long>(r1), first + static_cast<long long>(kMisPart));
+            const int first = p + 1, lim = step_end(first, kMisPart, r1);
             const unsigned pv = __ldg(a.prio + v);
             if (tid == 0) s_stop = kInf;
             __syncthreads();
-            for (int e = first; e < lim; e += 4 * kBlock) {
+            for (Pos e = first; e < static_cast<Pos>(lim); e += 4 * kBlock) {
                 int stop = kInf, u[4];
                 unsigned pu[4];
                 unsigned char s[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) u[k] = e + k * kBlock + tid < lim ? __ldg(col + e + k * kBlock + tid) : v;
+                for (int k = 0; k < 4; ++k) u[k] = e + k * kBlock + tid < static_cast<Pos>(lim) ? __ldg(col + e + k * kBlock + tid) : v;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     pu[k] = __ldg(a.prio + u[k]);
@@ -1205,7 +1206,7 @@ __global__ void __launch_bounds__(kBlock, 5) mis_kernel(MisArgs a) {
                 }
 #pragma unroll
                 for (int k = 3; k >= 0; --k)
-                    if (mis_look(u[k], pu[k], s[k], v, pv) != kOut) stop = e + k * kBlock + tid;
+                    if (mis_look(u[k], pu[k], s[k], v, pv) != kOut) stop = static_cast<int>(e) + k * kBlock + tid;
                 if (stop != kInf) atomicMin(&s_stop, stop);
                 if (__syncthreads_or(stop != kInf)) break;
             }
@@ -1365,6 +1366,9 @@ cudaError_t noalloc_scratch(void **out) {
 
 size_t traversal_scratch_need(int m) { return trav_scratch_bytes(m); }
 
+// Pull levels need a symmetric pattern, and step past a row's end in an int.
+int bfs_may_pull(const apspie_csr *A) { return (A->flags & APSPIE_CSR_SYMMETRIC) && A->nnz <= kMaxStepped; }
+
 // Blocks of a BFS launch, one to three an SM: more shorten a level's expansion, fewer its barrier
 // and its queue (a block's reservations are made one after the other). R-MAT, one / two / three:
 // 1.7M entries 32.5 / 34.0 / 37.2 us; 4.3M 37.2 / 36.9 / 41.1; 7.6M 44.7 / 41.4 / 43.6; 11.7M
@@ -1425,7 +1429,7 @@ apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, i
     const apspie_tune_params tp = effective_params(ctx, APSPIE_TUNE_BFS, A);
     a.alpha = tp.bfs_alpha;
     a.beta = tp.bfs_beta;
-    a.allow_pull = (A->flags & APSPIE_CSR_SYMMETRIC) ? 1 : 0;
+    a.allow_pull = bfs_may_pull(A);
     void *args[] = {&a};
     st = launch_persistent(ctx, reinterpret_cast<const void *>(bfs_kernel), kBfsBlock, args,
                            bfs_blocks(ctx->num_sms, A->nnz) * kWorkPerBlock);
@@ -1683,7 +1687,7 @@ apspie_status apspie_bfs_noalloc(const apspie_csr *A, int32_t source, int32_t de
     a.sticky = sticky;
     a.alpha = 14.0f;
     a.beta = 24.0f;
-    a.allow_pull = (A->flags & APSPIE_CSR_SYMMETRIC) ? 1 : 0;
+    a.allow_pull = bfs_may_pull(A);
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_kernel, kBfsBlock, 0) != cudaSuccess ||
