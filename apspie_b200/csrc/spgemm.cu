@@ -860,7 +860,10 @@ apspie_status sg_run(apspie_ctx *ctx, const apspie_csr *A, const apspie_csr *B, 
         const void *fn = reinterpret_cast<const void *>(sg_dense<NUMERIC, V>);
         const size_t smem = dense_smem<NUMERIC, V>(B->n);
         int per_sm = 0;
-        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        // the limit belongs to the kernel on the device, not to this call: always the most it can
+        // ask for, so that contexts of other threads that launch it with another size agree on it
+        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(dense_smem<NUMERIC, V>(kDenseCols)));
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kDenseBlock, smem);
         if (e == cudaSuccess) e = cudaMemsetAsync(&p.info->ticket, 0, sizeof(int), ctx->stream);

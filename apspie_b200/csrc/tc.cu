@@ -619,7 +619,8 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
     const size_t smem = (static_cast<size_t>(m) + 31) / 32 * 4;
     const int threads = smem <= 36 * 1024 ? 256 : smem <= 72 * 1024 ? 512 : 1024;
     int per_sm = 0;
-    e = cudaFuncSetAttribute(tc_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    // the limit belongs to the kernel on the device: the same from every thread's calls
+    e = cudaFuncSetAttribute(tc_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcBitmapVertices / 8);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_bits, threads, smem);
     if (e != cudaSuccess) return cuda_error(ctx, e, "tc launch");
     tc_bits<<<std::max(per_sm, 1) * ctx->num_sms, threads, smem, ctx->stream>>>(m, list, rp, ci, prp, plist, info);

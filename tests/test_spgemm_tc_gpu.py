@@ -298,3 +298,57 @@ def test_tc_of_rows_out_of_order(ctx, m, p):
         rp = np.concatenate(([0], np.cumsum(np.bincount(r, minlength=m)))).astype(np.int32)
         got = ctx.tc(ap.DeviceGraph(ap.HostGraph(m, m, rp, c.astype(np.int32))))
         assert got == int(((D @ D) * (D > 0)).sum()), repeats
+
+
+def test_sizes_of_threads_do_not_meet(ctx):
+    """Contexts are independent: threads with contexts of their own and small or large operands,
+    whose kernels take shared memory by the operands' size (five seconds of calls, since a call
+    has to fall between two steps of another)."""
+    import threading
+    import time
+
+    import torch
+
+    n = 60
+    rng = np.random.default_rng(5)
+    d = (rng.random((n, n)) < 0.6).astype(np.int32)
+    low = np.tril(d, -1)
+
+    def operand(a, m, val):
+        rp = np.full(m + 1, np.count_nonzero(a), dtype=np.int32)
+        rp[: n + 1] = np.concatenate(([0], np.cumsum(a.sum(1))))
+        ci = np.nonzero(a)[1].astype(np.int32)
+        return ap.HostGraph(m, m, rp, ci, np.ones(ci.size, dtype=np.int32) if val else None)
+
+    want, triangles = d @ d, int(((low @ low) * low).sum())
+    errors = []
+
+    def work(kind, m):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream), ap.Context(0, stream) as c:
+                g = ap.DeviceGraph(operand(d if kind == "spgemm" else low, m, kind == "spgemm"))
+                stream.synchronize()
+                end, k = time.monotonic() + 5.0, 0
+                while time.monotonic() < end and not errors:
+                    if kind == "tc":
+                        assert c.tc(g) == triangles
+                        continue
+                    rp, ci, v = c.spgemm_two_step(g, g)
+                    if k % 64 == 0:
+                        rows = np.repeat(np.arange(m), np.diff(rp.cpu().numpy()))
+                        got = np.zeros((n, n), dtype=np.int64)
+                        got[rows, ci.cpu().numpy()] = v.cpu().numpy()
+                        np.testing.assert_array_equal(got, want)
+                    k += 1
+        except BaseException as e:  # noqa: BLE001
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=a)
+               for a in (("tc", 100), ("tc", 600000), ("spgemm", 100), ("spgemm", 49000))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
