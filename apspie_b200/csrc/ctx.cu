@@ -9,8 +9,8 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <unordered_map>
 
+#include "block_cache.cuh"
 #include "common.cuh"
 
 namespace apspie {
@@ -50,132 +50,34 @@ unsigned long long current_ctx_id() {
     return id;
 }
 
-// ---- memory of library-owned matrices ------------------------------------------------
-// A call that returns a matrix used to spend more time in cudaMalloc and cudaFree than on the
-// device (building R-MAT scale 20, 256 MB of output: 1.7 ms + 1.2 ms beside 1.65 ms of
-// kernels): the driver maps and unmaps the memory each time. Blocks that are freed are kept
-// instead, up to kOwnedCacheBytes in all, and handed out again for requests of about their
-// size. owned_free waits for the device as cudaFree does, so a kept block has no work
-// pending on any stream, whichever thread or stream gets it next. Blocks belong to the CUDA
-// context they were made in and are only reused there; they go back to the driver when
-// something larger needs the room in the cache, when an allocation fails, and with the last
-// apspie_ctx.
+// Memory of library-owned matrices (block_cache.cuh): at most 1 GiB is kept in a CUDA context.
 namespace {
-constexpr size_t kOwnedCacheBytes = size_t(1) << 30;
-
-struct OwnedBlock {
-    void *p;
-    size_t bytes;
-    unsigned long long ctx_id;
+struct CudaBlocks {
+    using Error = cudaError_t;
+    static constexpr Error kOk = cudaSuccess, kOutOfMemory = cudaErrorMemoryAllocation;
+    static unsigned long long context() { return current_ctx_id(); }
+    static Error alloc(void **p, size_t bytes) {
+        const Error e = cudaMalloc(p, bytes);
+        if (e == kOutOfMemory) (void)cudaGetLastError();
+        return e;
+    }
+    static void free(void *p) {
+        (void)cudaFree(p);
+        (void)cudaGetLastError();
+    }
+    static Error wait() { return cudaDeviceSynchronize(); }
 };
 
-struct OwnedCache {
-    std::mutex mu;
-    std::unordered_map<void *, OwnedBlock> live;  // handed out
-    std::vector<OwnedBlock> kept;                 // oldest first
-    size_t kept_bytes = 0;
-    int contexts = 0;  // apspie_ctx alive
-};
-
-OwnedCache &owned_cache() {
-    static OwnedCache *c = new OwnedCache();  // never destroyed: matrices may outlive static destructors
+BlockCache<CudaBlocks> &blocks() {
+    static auto *c = new BlockCache<CudaBlocks>(size_t(1) << 30);  // never destroyed: matrices may outlive statics
     return *c;
 }
 
-// Gives the oldest blocks back until at most `most` bytes are kept (mu held).
-void owned_trim(OwnedCache &c, size_t most) {
-    size_t n = 0;
-    while (n < c.kept.size() && c.kept_bytes > most) {
-        (void)cudaFree(c.kept[n].p);
-        (void)cudaGetLastError();  // a block of a context that is gone is gone with it
-        c.kept_bytes -= c.kept[n].bytes;
-        ++n;
-    }
-    c.kept.erase(c.kept.begin(), c.kept.begin() + static_cast<std::ptrdiff_t>(n));
-}
-
-void owned_contexts(int change) {
-    OwnedCache &c = owned_cache();
-    std::lock_guard<std::mutex> lock(c.mu);
-    c.contexts += change;
-    if (c.contexts <= 0) owned_trim(c, 0);
-}
-
-// cudaMalloc, trying again without the kept blocks when memory is short.
-cudaError_t malloc_or_trim(void **p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaErrorMemoryAllocation) return e;
-    (void)cudaGetLastError();
-    OwnedCache &c = owned_cache();
-    {
-        std::lock_guard<std::mutex> lock(c.mu);
-        if (c.kept.empty()) return e;
-        owned_trim(c, 0);
-    }
-    return cudaMalloc(p, bytes);
-}
+cudaError_t malloc_or_trim(void **p, size_t bytes) { return blocks().alloc(p, bytes); }
 }  // namespace
 
-cudaError_t owned_alloc(void **p, size_t bytes) {
-    // whole granules, so that matrices of nearly the same size share blocks
-    const size_t granule = bytes >= (size_t(1) << 20) ? size_t(1) << 20 : 4096;
-    bytes = (bytes + granule - 1) / granule * granule;
-    OwnedCache &c = owned_cache();
-    const unsigned long long id = current_ctx_id();
-    if (id != 0) {
-        std::lock_guard<std::mutex> lock(c.mu);
-        size_t best = c.kept.size();
-        for (size_t i = 0; i < c.kept.size(); ++i)
-            if (c.kept[i].ctx_id == id && c.kept[i].bytes >= bytes && c.kept[i].bytes <= bytes + bytes / 4 &&
-                (best == c.kept.size() || c.kept[i].bytes < c.kept[best].bytes))
-                best = i;
-        if (best < c.kept.size()) {
-            const OwnedBlock b = c.kept[best];
-            c.kept.erase(c.kept.begin() + static_cast<std::ptrdiff_t>(best));
-            c.kept_bytes -= b.bytes;
-            c.live[b.p] = b;
-            *p = b.p;
-            return cudaSuccess;
-        }
-    }
-    cudaError_t e = malloc_or_trim(p, bytes);
-    if (e != cudaSuccess) return e;
-    const unsigned long long made_in = id != 0 ? id : current_ctx_id();
-    if (made_in != 0) {
-        std::lock_guard<std::mutex> lock(c.mu);
-        c.live[*p] = OwnedBlock{*p, bytes, made_in};
-    }
-    return cudaSuccess;
-}
-
-void owned_free(void *p) {
-    if (!p) return;
-    OwnedCache &c = owned_cache();
-    const unsigned long long id = current_ctx_id();
-    OwnedBlock b{p, 0, 0};
-    {
-        std::lock_guard<std::mutex> lock(c.mu);
-        auto it = c.live.find(p);
-        if (it != c.live.end()) {
-            b = it->second;
-            c.live.erase(it);
-        }
-    }
-    // another context's block, one too large to keep, or one that must not be kept because the
-    // device reported an error: as cudaFree does it
-    if (b.ctx_id == 0 || b.ctx_id != id || b.bytes > kOwnedCacheBytes / 2 || cudaDeviceSynchronize() != cudaSuccess) {
-        (void)cudaFree(p);
-        return;
-    }
-    std::lock_guard<std::mutex> lock(c.mu);
-    if (c.contexts <= 0) {
-        (void)cudaFree(p);
-        return;
-    }
-    owned_trim(c, kOwnedCacheBytes - b.bytes);
-    c.kept.push_back(b);
-    c.kept_bytes += b.bytes;
-}
+cudaError_t owned_alloc(void **p, size_t bytes) { return blocks().take(p, bytes); }
+void owned_free(void *p) { blocks().give(p); }
 
 apspie_status scratch_reserve(apspie_ctx *ctx, size_t bytes, void **out) {
     ++ctx->scratch_epoch;
@@ -403,8 +305,7 @@ apspie_status apspie_ctx_create(int device, void *cuda_stream, apspie_ctx **out)
         return APSPIE_ERR_OOM;
     }
     *out = ctx;
-    owned_contexts(1);
-    ctx->counted = true;
+    if ((ctx->cuda_ctx_id = current_ctx_id()) != 0) blocks().enter(ctx->cuda_ctx_id);
     return APSPIE_OK;
 }
 
@@ -419,7 +320,7 @@ void apspie_ctx_destroy(apspie_ctx *ctx) {
     if (ctx->h_ctl) cudaFreeHost(ctx->h_ctl);
     if (ctx->h_word) cudaFreeHost(ctx->h_word);
     if (ctx->h_limit) cudaFreeHost(ctx->h_limit);
-    if (ctx->counted) owned_contexts(-1);
+    if (ctx->cuda_ctx_id != 0) blocks().leave(ctx->cuda_ctx_id, current_ctx_id() == ctx->cuda_ctx_id);
     delete ctx;
 }
 
