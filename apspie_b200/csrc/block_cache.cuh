@@ -97,6 +97,12 @@ class BlockCache {
             if (it != live_.end()) {
                 b = it->second;
                 live_.erase(it);
+            } else {
+                // a matrix freed twice (through a copy of its struct): the block is not the
+                // caller's any more, and freeing it would leave it among the kept ones
+                for (const auto &l : of_)
+                    for (const Block &k : l.second.kept)
+                        if (k.p == p) return;
             }
         }
         // another context's block, one too large to keep, or one that must not be kept because

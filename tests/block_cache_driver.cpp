@@ -130,13 +130,34 @@ void devices() {
     Fake::now = 1;
     c.leave(1, true);
 }
+
+// A second free of a matrix does nothing, as long as its memory has not been handed out again.
+void twice() {
+    Cache c(64 * MB);
+    c.enter(1);
+    void *a, *b, *d;
+    c.take(&a, 20 * MB);
+    c.give(a);
+    c.give(a);
+    check(held_by(1) == 20 * MB, "the kept block stays kept");
+    c.take(&b, 20 * MB);
+    c.take(&d, 20 * MB);
+    check(b == a && d != b && held_by(1) == 40 * MB, "the block is handed out once");
+    c.give(b);
+    Fake::now = 11;
+    c.give(b);  // with another device current
+    Fake::now = 1;
+    c.give(d);
+    c.leave(1, true);
+    check(held_by(1) == 0, "everything is given back");
+}
 }  // namespace
 
 int main(int argc, char **argv) {
     const struct {
         const char *name;
         void (*f)();
-    } all[] = {{"reuse", reuse}, {"reset", reset}, {"devices", devices}};
+    } all[] = {{"reuse", reuse}, {"reset", reset}, {"devices", devices}, {"twice", twice}};
     for (auto &s : all)
         if (argc > 1 && !std::strcmp(argv[1], s.name)) {
             s.f();

@@ -1,5 +1,5 @@
 """The cache of matrix memory (csrc/block_cache.cuh) on a stand-in for CUDA, without a GPU:
-contexts that are reset, several devices, memory that runs short."""
+contexts that are reset, several devices, memory that runs short, matrices freed twice."""
 import os
 import subprocess
 
@@ -17,7 +17,7 @@ def driver(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["reuse", "reset", "devices"])
+@pytest.mark.parametrize("what", ["reuse", "reset", "devices", "twice"])
 def test_block_cache(driver, what):
     res = subprocess.run([driver, what], capture_output=True, text=True, timeout=60)
     assert res.returncode == 0, res.stdout[-2000:]
