@@ -11,6 +11,10 @@
 // last apspie_ctx of that CUDA context. The blocks of a CUDA context that was reset went with it,
 // and their addresses may be someone else's by now: they are forgotten, not freed.
 //
+// Freeing a matrix waits for nothing (cudaFree does, and so may not be called in a stream capture
+// of the default mode); the device is waited for when a block is handed out again, if it has not
+// been since the block was freed. The calls that ask for one wait for their own stream anyway.
+//
 // Gpu is CUDA (ctx.cu), or what a test puts in its place: Error with Gpu::kOk and
 // Gpu::kOutOfMemory, the id of the current CUDA context (0: none or unknown), alloc, free, wait.
 #pragma once
@@ -60,6 +64,9 @@ class BlockCache {
         const std::size_t granule = bytes >= (std::size_t(1) << 20) ? std::size_t(1) << 20 : 4096;
         bytes = (bytes + granule - 1) / granule * granule;
         const unsigned long long id = Gpu::context();
+        Block got{nullptr, 0, 0};
+        bool idle = false;
+        unsigned long long until = 0;
         {
             std::lock_guard<std::mutex> lock(mu_);
             auto it = of_.find(id);
@@ -71,14 +78,27 @@ class BlockCache {
                         (best == l.kept.size() || l.kept[i].bytes < l.kept[best].bytes))
                         best = i;
                 if (best < l.kept.size()) {
-                    const Block b = l.kept[best];
+                    got = l.kept[best];
                     l.kept.erase(l.kept.begin() + static_cast<std::ptrdiff_t>(best));
-                    l.bytes -= b.bytes;
-                    live_[b.p] = Live{b.bytes, id};
-                    *p = b.p;
-                    return Gpu::kOk;
+                    l.bytes -= got.bytes;
+                    idle = got.freed <= l.idle;
+                    until = frees_;
                 }
             }
+        }
+        if (got.p) {
+            // what was in flight when the block was freed may still use it, on any stream
+            const Error e = idle ? Gpu::kOk : Gpu::wait();
+            if (e != Gpu::kOk) {
+                Gpu::free(got.p);
+                return e;
+            }
+            std::lock_guard<std::mutex> lock(mu_);
+            auto it = of_.find(id);
+            if (it != of_.end() && it->second.idle < until) it->second.idle = until;
+            live_[got.p] = Live{got.bytes, id};
+            *p = got.p;
+            return Gpu::kOk;
         }
         const Error e = alloc(p, bytes);
         if (e == Gpu::kOk && id != 0) {
@@ -105,10 +125,8 @@ class BlockCache {
                         if (k.p == p) return;
             }
         }
-        // another context's block, one too large to keep, or one that must not be kept because
-        // the device reported an error: as cudaFree does it. The wait is cudaFree's too: a kept
-        // block has no work pending on any stream, whichever thread or stream gets it next
-        if (b.id == 0 || b.id != id || b.bytes > most_ / 2 || Gpu::wait() != Gpu::kOk) {
+        // another context's block, or one too large to keep
+        if (b.id == 0 || b.id != id || b.bytes > most_ / 2) {
             Gpu::free(p);
             return;
         }
@@ -119,7 +137,7 @@ class BlockCache {
             return;
         }
         trim(it->second, most_ - b.bytes);
-        it->second.kept.push_back(Block{p, b.bytes});
+        it->second.kept.push_back(Block{p, b.bytes, ++frees_});
         it->second.bytes += b.bytes;
     }
 
@@ -127,6 +145,7 @@ class BlockCache {
     struct Block {
         void *p;
         std::size_t bytes;
+        unsigned long long freed;  // number of the free that kept it
     };
     struct Live {
         std::size_t bytes;
@@ -136,6 +155,7 @@ class BlockCache {
         std::vector<Block> kept;  // oldest first
         std::size_t bytes = 0;
         int contexts = 0;  // apspie_ctx alive
+        unsigned long long idle = 0;  // the device has been waited for since this free
     };
 
     // Gives the oldest blocks of the current CUDA context's list back until at most `most` bytes
@@ -153,6 +173,7 @@ class BlockCache {
     std::mutex mu_;
     std::unordered_map<void *, Live> live_;  // handed out
     std::unordered_map<unsigned long long, List> of_;
+    unsigned long long frees_ = 0;
 };
 
 }  // namespace apspie

@@ -23,7 +23,7 @@ struct Fake {
     static unsigned long long now;                       // the current CUDA context
     static std::map<unsigned long long, std::map<std::size_t, std::size_t>> held;  // context -> address -> bytes
     static std::size_t room;                             // bytes a context can hold
-    static int waits;
+    static int waits, wait_error;
 
     static unsigned long long context() { return now; }
     static Error alloc(void **p, std::size_t bytes) {
@@ -45,12 +45,12 @@ struct Fake {
         for (auto &c : held) n += c.second.erase(reinterpret_cast<std::size_t>(p));
         check(n == 1, "freed what nobody holds");
     }
-    static Error wait() { return ++waits, kOk; }
+    static Error wait() { return ++waits, wait_error; }
 };
 unsigned long long Fake::now = 1;
 std::map<unsigned long long, std::map<std::size_t, std::size_t>> Fake::held;
 std::size_t Fake::room = std::size_t(64) << 30;
-int Fake::waits = 0;
+int Fake::waits = 0, Fake::wait_error = 0;
 
 std::size_t held_by(unsigned long long id) {
     std::size_t n = 0;
@@ -151,13 +151,40 @@ void twice() {
     c.leave(1, true);
     check(held_by(1) == 0, "everything is given back");
 }
+
+// Freeing waits for nothing; a block is handed out when the device has been waited for since.
+void waits() {
+    Cache c(64 * MB);
+    c.enter(1);
+    void *a, *b, *d;
+    c.take(&a, 10 * MB);
+    c.take(&b, 20 * MB);
+    Fake::waits = 0;
+    c.give(a);
+    c.give(b);
+    check(Fake::waits == 0, "a free does not wait");
+    c.take(&d, 20 * MB);
+    check(d == b && Fake::waits == 1, "a reuse waits");
+    c.take(&b, 10 * MB);
+    check(b == a && Fake::waits == 1, "once for all blocks freed before");
+    c.give(d);
+    c.take(&a, 20 * MB);
+    check(a == d && Fake::waits == 2, "and again for one freed since");
+    c.give(a);
+    Fake::wait_error = 1;
+    c.take(&d, 20 * MB);
+    check(held_by(1) == 10 * MB, "a block is not reused when the device reports an error");
+    Fake::wait_error = 0;
+    c.give(b);
+    c.leave(1, true);
+}
 }  // namespace
 
 int main(int argc, char **argv) {
     const struct {
         const char *name;
         void (*f)();
-    } all[] = {{"reuse", reuse}, {"reset", reset}, {"devices", devices}, {"twice", twice}};
+    } all[] = {{"reuse", reuse}, {"reset", reset}, {"devices", devices}, {"twice", twice}, {"waits", waits}};
     for (auto &s : all)
         if (argc > 1 && !std::strcmp(argv[1], s.name)) {
             s.f();

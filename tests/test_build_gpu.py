@@ -222,3 +222,24 @@ def test_memory_kept_from_freed_matrices_is_bounded(ctx):
     torch.cuda.synchronize()
     # at most 1 GiB of blocks, the context's scratch, and what the driver rounds up
     assert before - torch.cuda.mem_get_info()[0] <= (1 << 30) + scratch + (64 << 20)
+
+
+def test_matrix_freed_during_a_stream_capture(ctx):
+    """Freeing a matrix leaves a capture under way alone, and its memory is reused afterwards."""
+    import torch
+
+    src = torch.arange(300000, dtype=torch.int32, device="cuda") % 3000
+    A = ctx.build_csr(3000, src, src.flip(0).contiguous())
+    x = torch.arange(1000, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        y = x + 1
+        A.free()
+        z = y * 2
+    graph.replay()
+    assert torch.equal(z, (x + 1) * 2)
+    B = ctx.build_csr(3000, src, src.flip(0).contiguous())
+    rp, ci, _ = B.to_numpy()
+    assert rp[-1] == 300000 and np.array_equal(np.sort(ci), np.sort(src.cpu().numpy()))
+    B.free()
