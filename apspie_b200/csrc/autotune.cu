@@ -135,7 +135,7 @@ struct TuneBuffers {
     template <typename T>
     T *get(size_t n) {
         void *p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
+        if (device_alloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
             (void)cudaGetLastError();
             return nullptr;
         }

@@ -7,8 +7,9 @@
 // size.
 //
 // A block is reused and given back in the CUDA context it was made in and nowhere else: when
-// something larger needs the room among the kept blocks, when an allocation fails, and with the
-// last apspie_ctx of that CUDA context. The blocks of a CUDA context that was reset went with it,
+// something larger needs the room among the kept blocks, when an allocation of the library fails
+// (all of them are made by alloc or take), when the caller asks for it (apspie_ctx_trim), and with
+// the last apspie_ctx of that CUDA context. The blocks of a CUDA context that was reset went with it,
 // and their addresses may be someone else's by now: they are forgotten, not freed.
 //
 // Freeing a matrix waits for nothing (cudaFree does, and so may not be called in a stream capture
@@ -139,6 +140,13 @@ class BlockCache {
         trim(it->second, most_ - b.bytes);
         it->second.kept.push_back(Block{p, b.bytes, ++frees_});
         it->second.bytes += b.bytes;
+    }
+
+    // Gives every kept block of the current CUDA context back.
+    void trim() {
+        std::lock_guard<std::mutex> lock(mu_);
+        auto it = of_.find(Gpu::context());
+        if (it != of_.end()) trim(it->second, 0);
     }
 
   private:

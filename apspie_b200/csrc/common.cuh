@@ -209,8 +209,10 @@ apspie_status transpose_pattern(apspie_ctx *ctx, const apspie_csr *A, void *scra
 // row_of[e] = the row of A's entry e.
 apspie_status expand_entry_rows(apspie_ctx *ctx, const apspie_csr *A, unsigned *row_of);
 
-// Device memory of library-owned matrices (ctx.cu): cudaMalloc behind a small cache of blocks
-// that owned_free gave back.
+// Device memory (ctx.cu). device_alloc: cudaMalloc, again without the kept blocks of freed matrices
+// when memory is short; every allocation of the library is made by it (and freed by cudaFree).
+// owned_alloc, owned_free: library-owned matrices, whose freed blocks are kept (block_cache.cuh).
+cudaError_t device_alloc(void **p, size_t bytes);
 cudaError_t owned_alloc(void **p, size_t bytes);
 void owned_free(void *p);
 // The process-unique id of the CUDA context current on this thread, 0 when there is none or

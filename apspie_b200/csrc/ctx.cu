@@ -72,10 +72,9 @@ BlockCache<CudaBlocks> &blocks() {
     static auto *c = new BlockCache<CudaBlocks>(size_t(1) << 30);  // never destroyed: matrices may outlive statics
     return *c;
 }
-
-cudaError_t malloc_or_trim(void **p, size_t bytes) { return blocks().alloc(p, bytes); }
 }  // namespace
 
+cudaError_t device_alloc(void **p, size_t bytes) { return blocks().alloc(p, bytes); }
 cudaError_t owned_alloc(void **p, size_t bytes) { return blocks().take(p, bytes); }
 void owned_free(void *p) { blocks().give(p); }
 
@@ -92,7 +91,7 @@ apspie_status scratch_reserve(apspie_ctx *ctx, size_t bytes, void **out) {
     ctx->scratch = nullptr;
     ctx->scratch_bytes = 0;
     size_t want = bytes + bytes / 8;  // headroom so slightly larger graphs reuse it
-    e = malloc_or_trim(&ctx->scratch, want);
+    e = device_alloc(&ctx->scratch, want);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         e = cudaMalloc(&ctx->scratch, bytes);
@@ -115,7 +114,7 @@ apspie_status scratch2_reserve(apspie_ctx *ctx, size_t bytes, void **out) {
     if (ctx->scratch2) cudaFree(ctx->scratch2);
     ctx->scratch2 = nullptr;
     ctx->scratch2_bytes = 0;
-    e = malloc_or_trim(&ctx->scratch2, bytes);
+    e = device_alloc(&ctx->scratch2, bytes);
     if (e != cudaSuccess) return cuda_error(ctx, e, "scratch2_reserve cudaMalloc");
     ctx->scratch2_bytes = bytes;
     *out = ctx->scratch2;
@@ -292,8 +291,8 @@ apspie_status apspie_ctx_create(int device, void *cuda_stream, apspie_ctx **out)
     ctx->device = device;
     ctx->stream = static_cast<cudaStream_t>(cuda_stream);
     cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
-    bool ok = cudaMalloc(&ctx->d_ctl, sizeof(TravCtl)) == cudaSuccess &&
-              cudaMalloc(&ctx->d_sticky_err, sizeof(int)) == cudaSuccess &&
+    bool ok = device_alloc(reinterpret_cast<void **>(&ctx->d_ctl), sizeof(TravCtl)) == cudaSuccess &&
+              device_alloc(reinterpret_cast<void **>(&ctx->d_sticky_err), sizeof(int)) == cudaSuccess &&
               cudaMallocHost(&ctx->h_ctl, sizeof(TravCtl)) == cudaSuccess &&
               cudaMallocHost(&ctx->h_word, 64) == cudaSuccess &&
               cudaMallocHost(&ctx->h_limit, 64) == cudaSuccess &&
@@ -432,6 +431,12 @@ apspie_status apspie_ctx_timeline(const apspie_ctx *ctx, int32_t *sites, int64_t
     }
     *count = n;
     return APSPIE_OK;
+}
+
+void apspie_ctx_trim(apspie_ctx *ctx) {
+    if (!ctx) return;
+    cudaSetDevice(ctx->device);
+    blocks().trim();
 }
 
 int64_t apspie_ctx_scratch_bytes(const apspie_ctx *ctx) {

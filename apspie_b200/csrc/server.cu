@@ -285,7 +285,7 @@ void launch_batch(apspie_server *s, Slot &sl) {
             if (sl.stage) cudaFree(sl.stage);
             sl.stage = nullptr;
             sl.stage_cap = 0;
-            if (cudaMalloc(&sl.stage, rows) != cudaSuccess) {
+            if (device_alloc(reinterpret_cast<void **>(&sl.stage), rows) != cudaSuccess) {
                 (void)cudaGetLastError();
                 st = APSPIE_ERR_OOM;
             } else {
@@ -297,7 +297,7 @@ void launch_batch(apspie_server *s, Slot &sl) {
             if (sl.d_src) cudaFree(sl.d_src);
             sl.d_src = nullptr;
             sl.src_cap = 0;
-            if (cudaMalloc(&sl.d_src, std::max(n, 512) * sizeof(int32_t)) != cudaSuccess) {
+            if (device_alloc(reinterpret_cast<void **>(&sl.d_src), std::max(n, 512) * sizeof(int32_t)) != cudaSuccess) {
                 (void)cudaGetLastError();
                 st = APSPIE_ERR_OOM;
             } else {
@@ -690,9 +690,9 @@ apspie_status apspie_server_add_graph(apspie_server *s, const apspie_host_csr *g
     G.bytes = rp + ci + (w ? ci : 0) + static_cast<size_t>(g->m) * 4;
     if (s->graph_bytes + G.bytes > static_cast<size_t>(s->budget)) return APSPIE_ERR_OOM;
     if (bfs_engine_create(&G.eng) != APSPIE_OK) return APSPIE_ERR_OOM;
-    bool ok = cudaMalloc(&G.row_ptr, rp) == cudaSuccess && cudaMalloc(&G.col_ind, std::max<size_t>(ci, 4)) == cudaSuccess &&
-              cudaMalloc(&G.prio, static_cast<size_t>(g->m) * 4) == cudaSuccess &&
-              (!w || cudaMalloc(&G.weights, std::max<size_t>(ci, 4)) == cudaSuccess);
+    auto get = [](auto **p, size_t bytes) { return device_alloc(reinterpret_cast<void **>(p), bytes) == cudaSuccess; };
+    const bool ok = get(&G.row_ptr, rp) && get(&G.col_ind, std::max<size_t>(ci, 4)) &&
+                    get(&G.prio, static_cast<size_t>(g->m) * 4) && (!w || get(&G.weights, std::max<size_t>(ci, 4)));
     if (!ok) {
         (void)cudaGetLastError();
         cudaFree(G.row_ptr);

@@ -315,6 +315,10 @@ class Context:
                                                 ctypes.byref(n)), "timeline")
         return list(zip(sites[:n.value].tolist(), ns[:n.value].tolist()))
 
+    def trim(self) -> None:
+        """Gives the memory kept from freed matrices on this device back to CUDA."""
+        L.lib().apspie_ctx_trim(self.handle)
+
     def scratch_bytes(self) -> int:
         return int(L.lib().apspie_ctx_scratch_bytes(self.handle))
 

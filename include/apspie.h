@@ -142,6 +142,9 @@ apspie_status apspie_grid_barrier_check(apspie_ctx *ctx, int32_t rounds, int32_t
  * kernel started (globaltimer). Site 0 is the kernel start. */
 apspie_status apspie_ctx_timeline(const apspie_ctx *ctx, int32_t *sites, int64_t *ns, int32_t cap,
                                   int32_t *count);
+/* Gives the memory of freed matrices that is kept on the context's device (apspie_csr_free)
+ * back to CUDA. */
+void apspie_ctx_trim(apspie_ctx *ctx);
 /* Bytes of device scratch the context currently holds. */
 int64_t apspie_ctx_scratch_bytes(const apspie_ctx *ctx);
 
@@ -328,6 +331,11 @@ apspie_status apspie_spgemm_symbolic(apspie_ctx *ctx, const apspie_csr *A, const
                                      int32_t *d_row_ptr_c, int64_t *nnz_c);
 apspie_status apspie_spgemm_numeric(apspie_ctx *ctx, const apspie_csr *A, const apspie_csr *B,
                                     const int32_t *d_row_ptr_c, int32_t *d_col_c, void *d_val_c);
+/* Releases a matrix. Its memory stays with the library for later matrices, up to 1 GiB on each
+ * device: it goes back to CUDA when an allocation of the library fails, with
+ * apspie_ctx_trim and with the device's last context. A call that returns a matrix may wait
+ * for the device before it reuses such memory. Releasing a copy of a released struct does
+ * nothing while its memory is unused. */
 void apspie_csr_free(apspie_csr_owned *C);
 
 /* ---- graph construction on the device ---------------------------------------------- */

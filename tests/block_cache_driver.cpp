@@ -178,13 +178,38 @@ void waits() {
     c.give(b);
     c.leave(1, true);
 }
+
+// The kept blocks make room for any allocation, and go when they are asked to, in their context.
+void room() {
+    Cache c(64 * MB);
+    c.enter(1);
+    c.enter(11);
+    void *a, *b;
+    Fake::room = 100 * MB;
+    c.take(&a, 30 * MB);
+    c.give(a);
+    Fake::now = 11;
+    check(c.alloc(&b, 101 * MB) == Fake::kOutOfMemory && held_by(1) == 30 * MB, "another device's blocks are no room");
+    c.trim();
+    check(held_by(1) == 30 * MB, "nor are they given back from there");
+    Fake::now = 1;
+    check(c.alloc(&b, 90 * MB) == Fake::kOk && held_by(1) == 90 * MB, "the kept block makes room");
+    Fake::free(b);
+    c.take(&a, 30 * MB);
+    c.give(a);
+    c.trim();
+    check(held_by(1) == 0, "the kept blocks are given back");
+    c.leave(1, true);
+    Fake::now = 11;
+    c.leave(11, true);
+}
 }  // namespace
 
 int main(int argc, char **argv) {
     const struct {
         const char *name;
         void (*f)();
-    } all[] = {{"reuse", reuse}, {"reset", reset}, {"devices", devices}, {"twice", twice}, {"waits", waits}};
+    } all[] = {{"reuse", reuse}, {"reset", reset}, {"devices", devices}, {"twice", twice}, {"waits", waits}, {"room", room}};
     for (auto &s : all)
         if (argc > 1 && !std::strcmp(argv[1], s.name)) {
             s.f();

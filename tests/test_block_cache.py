@@ -17,7 +17,7 @@ def driver(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["reuse", "reset", "devices", "twice", "waits"])
+@pytest.mark.parametrize("what", ["reuse", "reset", "devices", "twice", "waits", "room"])
 def test_block_cache(driver, what):
     res = subprocess.run([driver, what], capture_output=True, text=True, timeout=60)
     assert res.returncode == 0, res.stdout[-2000:]

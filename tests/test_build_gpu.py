@@ -243,3 +243,34 @@ def test_matrix_freed_during_a_stream_capture(ctx):
     rp, ci, _ = B.to_numpy()
     assert rp[-1] == 300000 and np.array_equal(np.sort(ci), np.sort(src.cpu().numpy()))
     B.free()
+
+
+def test_kept_memory_makes_room(ctx):
+    """What is kept of freed matrices is given to the library's other allocations when memory
+    is short, and back to CUDA on demand."""
+    import torch
+
+    one = torch.zeros(1, dtype=torch.int32, device="cuda")
+    g = ap.gen_rmat(16, 8, 1, 3, weights=False)
+    dg = ap.DeviceGraph(g)
+    nq = 1024  # the tuner's output: 268 MB
+    with ap.Context(0) as c:
+        c.autotune(ap.TUNE_BFS_BATCH, dg, sources=[1] * 32, reps=1)  # scratch
+        c.bfs_batch(dg, torch.ones(512, dtype=torch.int32, device="cuda"))
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        kept = [c.build_csr(100_000_000, one, one) for _ in range(2)]  # 400 MB each, and scratch
+        for k in kept:
+            k.free()
+        free = torch.cuda.mem_get_info()[0]
+        rest = torch.empty(free - (160 << 20), dtype=torch.uint8, device="cuda")
+        assert torch.cuda.mem_get_info()[0] < 200 << 20
+        best, _ = c.autotune(ap.TUNE_BFS_BATCH, dg, sources=[1] * nq, reps=1)
+        assert best["batch_push_frac"] > 0
+        kept = c.build_csr(100_000_000, one, one)
+        kept.free()
+        low = torch.cuda.mem_get_info()[0]
+        c.trim()
+        assert torch.cuda.mem_get_info()[0] >= low + (380 << 20)
+        del rest
+    torch.cuda.empty_cache()
