@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256) coo_keys(long long ne, int m, const int *
 // Drops sentinels (keys >= `sentinel`, which sort last) and, with dedup, all but the first of
 // equal keys, in one pass: tiles are taken in order, a look-back gives each tile's place.
 // start[r] becomes the first kept pair whose upper field is >= r, for r up to the last kept
-// pair's field, and the kept keys' digits are counted for the sort by the lower field
+// pair's field (start null: not), and the kept keys' digits are counted for the sort by the lower field
 // (pl2.passes = 0: not). One read and one write of the pairs where flags, scan and compaction
 // took three.
 //
@@ -151,7 +151,8 @@ __global__ void __launch_bounds__(256) compact_pairs(long long n, const unsigned
                 vout[at[i]] = val[i];
                 const int r = static_cast<int>(key[i] >> B);
                 const int rp = w0 + 32 * (i0 + i) > 0 ? static_cast<int>(prev[i] >> B) : -1;
-                for (int x = rp + 1; x <= r; ++x) start[x] = at[i];
+                if (start)
+                    for (int x = rp + 1; x <= r; ++x) start[x] = at[i];
                 rs_count(h, key[i], pl2);
             }
         }
@@ -181,6 +182,31 @@ __global__ void fill_tail(long long n, const K *__restrict__ keys, int shift, K 
     const int last = n > 0 ? static_cast<int>((keys[n - 1] >> shift) & fmask) : -1;
     for (int x = last + 1 + blockIdx.x * blockDim.x + threadIdx.x; x <= m; x += gridDim.x * blockDim.x)
         start[x] = static_cast<int>(n);
+}
+
+// The same for every r up to m when there are fewer keys than rows, and most rows are gaps that
+// one thread would fill: a block takes 1,024 rows, finds the keys that lie in them and looks each
+// row up among those. (64 entries in 2^25 rows: the transpose took 91 ms by the two above and a
+// scan of all rows for the entries', 21 ms before that; now 0.27 ms.)
+template <class K>
+__global__ void __launch_bounds__(256) search_starts(long long n, const K *__restrict__ keys, int shift, K fmask, int m,
+                                                     int *start, const int *err) {
+    if (ld_volatile_i32(err) != 0) return;
+    auto bound = [&](long long lo, long long hi, long long r) {  // first of [lo, hi) with a field >= r
+        while (lo < hi) {
+            const long long mid = (lo + hi) >> 1;
+            if (static_cast<long long>((__ldg(keys + mid) >> shift) & fmask) < r)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        return lo;
+    };
+    for (long long r0 = blockIdx.x * 1024ll; r0 <= m; r0 += gridDim.x * 1024ll) {
+        const long long lo = bound(0, n, r0), hi = bound(lo, n, r0 + 1024);
+        for (long long r = r0 + threadIdx.x; r < r0 + 1024 && r <= m; r += 256)
+            start[r] = static_cast<int>(bound(lo, hi, r));
+    }
 }
 
 __global__ void plain_fill(long long n, const unsigned long long *__restrict__ keys, const unsigned *__restrict__ vals,
@@ -227,7 +253,10 @@ __global__ void sym_row_ptr(int m, const int *__restrict__ up, const int *__rest
 // The row of every entry: row_of[e], or (KEYS) keys[e] = column << 32 | row. A block takes
 // kExpandTile entries whatever rows they belong to (a warp per row left a row of 50,000
 // entries to one warp): it finds the row of its first entry by a 32-way search, marks where
-// rows begin and spreads the marks by a running maximum.
+// rows begin and spreads the marks by a running maximum. A block whose entries lie so far apart
+// that it has not gone past their rows after kExpandSteps steps of 256 rows looks each entry's
+// row up instead: going on would walk through millions of empty rows alone.
+constexpr int kExpandSteps = 64;
 constexpr int kExpandItems = 16;
 constexpr int kExpandTile = 256 * kExpandItems;
 template <bool KEYS>
@@ -253,15 +282,48 @@ __global__ void __launch_bounds__(256) expand_rows(int m, long long nnz, const i
         hi = nh < hi ? static_cast<int>(nh) : hi;
     }
     __syncthreads();
-    for (int r0 = lo; r0 < m; r0 += 256) {
-        const int r = r0 + tid;
+    bool far = false;  // the same for all threads
+    int steps = 0;
+    for (long long r0 = lo; r0 < m; r0 += 256) {
+        if (steps++ == kExpandSteps) {
+            far = true;
+            break;
+        }
+        const long long r = r0 + tid;
         int b = 0, e = 0;
         if (r < m) {
             b = __ldg(rp + r);
             e = __ldg(rp + r + 1);
-            if (e > b && b < t1) s_row[at(static_cast<int>((b > t0 ? b : t0) - t0))] = r;
+            if (e > b && b < t1) s_row[at(static_cast<int>((b > t0 ? b : t0) - t0))] = static_cast<int>(r);
         }
         if (__syncthreads_or(r < m && e >= t1)) break;
+    }
+    if (far) {
+        for (int i0 = 0; i0 < kExpandItems; i0 += 4) {
+            long long e[4];
+            int row[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                e[k] = t0 + (i0 + k) * 256 + tid;
+                row[k] = lo;
+            }
+            for (long long s = 1ll << 30; s > 0; s >>= 1) {  // the last row that begins at or before e
+                if (lo + s >= m) continue;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (row[k] + s < m && __ldg(rp + row[k] + s) <= e[k]) row[k] += static_cast<int>(s);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (e[k] >= t1) continue;
+                if (KEYS)
+                    keys[e[k]] = (static_cast<unsigned long long>(static_cast<unsigned>(__ldg(ci + e[k]))) << 32) |
+                                 static_cast<unsigned>(row[k]);
+                else
+                    row_of[e[k]] = static_cast<unsigned>(row[k]);
+            }
+        }
+        return;
     }
     int run = -1;
 #pragma unroll
@@ -315,6 +377,18 @@ int grid_for(const apspie_ctx *ctx, long long n) {
     return static_cast<int>(std::max<long long>(1, std::min<long long>((n + 255) / 256, ctx->num_sms * 16LL)));
 }
 
+// Row starts out of n sorted keys.
+template <class K>
+void launch_starts(apspie_ctx *ctx, long long n, const K *keys, int shift, K fmask, int m, int *start, const int *err) {
+    const int g = grid_for(ctx, std::max<long long>(n, m + 1ll));
+    if (n < m) {
+        search_starts<K><<<g, 256, 0, ctx->stream>>>(n, keys, shift, fmask, m, start, err);
+        return;
+    }
+    run_starts<K><<<g, 256, 0, ctx->stream>>>(n, keys, shift, fmask, start, err);
+    fill_tail<K><<<g, 256, 0, ctx->stream>>>(n, keys, shift, fmask, m, start, err);
+}
+
 apspie_status alloc_owned(apspie_ctx *ctx, int m, int n, long long nnz, int val_type, apspie_csr_owned *out) {
     std::memset(out, 0, sizeof(*out));
     cudaError_t e = owned_alloc(reinterpret_cast<void **>(&out->row_ptr), (static_cast<size_t>(m) + 1) * 4);
@@ -339,7 +413,7 @@ apspie_status alloc_owned(apspie_ctx *ctx, int m, int n, long long nnz, int val_
 static apspie_status sort_pattern(apspie_ctx *ctx, const apspie_csr *A, SortBufs<unsigned> &s, unsigned *row_of,
                                   int *out_rp, int *out_col, const unsigned **keys) {
     const long long nnz = A->nnz;
-    const int n = A->n, g = grid_for(ctx, nnz);
+    const int n = A->n;
     const RsPlan pl = rs_plan(0, bit_length(n));
     s.v[last_pair(pl.passes)] = reinterpret_cast<unsigned *>(out_col);
     cudaError_t e = launch_expand_rows<false>(ctx, A, row_of, nullptr);
@@ -348,8 +422,7 @@ static apspie_status sort_pattern(apspie_ctx *ctx, const apspie_csr *A, SortBufs
     apspie_status st =
         radix_sort(ctx, s, pl, reinterpret_cast<const unsigned *>(A->col_ind), row_of, nnz, 0, &which);
     if (st != APSPIE_OK) return st;
-    if (nnz > 0) run_starts<unsigned><<<g, 256, 0, ctx->stream>>>(nnz, s.k[which], 0, ~0u, out_rp, s.err);
-    fill_tail<unsigned><<<grid_for(ctx, n + 1LL), 256, 0, ctx->stream>>>(nnz, s.k[which], 0, ~0u, n, out_rp, s.err);
+    launch_starts<unsigned>(ctx, nnz, s.k[which], 0, ~0u, n, out_rp, s.err);
     *keys = s.k[which];
     e = cudaGetLastError();
     return e == cudaSuccess ? APSPIE_OK : cuda_error(ctx, e, "transpose");
@@ -432,7 +505,7 @@ apspie_status apspie_csr_build(apspie_ctx *ctx, int32_t m, int64_t nedges, const
     if (n > 0)
         compact_pairs<<<static_cast<int>(std::min<long long>((n + kCompactTile - 1) / kCompactTile, ctx->num_sms * 4LL)),
                         256, 0, ctx->stream>>>(n, s.k[which], s.v[which], sentinel, dedup ? 1 : 0, B, pl2,
-                                               s.hist_of(1), s.k[o], s.v[o], up, s.status, s.ticket + kRsOwn, flag + 1,
+                                               s.hist_of(1), s.k[o], s.v[o], n < m ? nullptr : up, s.status, s.ticket + kRsOwn, flag + 1,
                                                s.err);
     int h_flag[2] = {0, 0}, sort_err = 0;
     if ((e = cudaGetLastError()) != cudaSuccess ||
@@ -449,7 +522,10 @@ apspie_status apspie_csr_build(apspie_ctx *ctx, int32_t m, int64_t nedges, const
     const int gp = grid_for(ctx, np);
     const int gm = grid_for(ctx, m + 1LL);
     const unsigned long long fmask = (1ull << B) - 1ull;
-    fill_tail<unsigned long long><<<gm, 256, 0, ctx->stream>>>(np, s.k[o], B, fmask, m, up, s.err);
+    if (n < m)
+        search_starts<unsigned long long><<<gm, 256, 0, ctx->stream>>>(np, s.k[o], B, fmask, m, up, s.err);
+    else
+        fill_tail<unsigned long long><<<gm, 256, 0, ctx->stream>>>(np, s.k[o], B, fmask, m, up, s.err);
     if (!sym) {
         e = cudaMemcpyAsync(out->row_ptr, up, mi * 4, cudaMemcpyDeviceToDevice, ctx->stream);
         if (np > 0) plain_fill<<<gp, 256, 0, ctx->stream>>>(np, s.k[o], s.v[o], fmask, out->col_ind, oval);
@@ -466,9 +542,7 @@ apspie_status apspie_csr_build(apspie_ctx *ctx, int32_t m, int64_t nedges, const
             apspie_csr_free(out);
             return st;
         }
-        if (np > 0)
-            run_starts<unsigned long long><<<gp, 256, 0, ctx->stream>>>(np, t.k[hw], 0, fmask, low, s.err);
-        fill_tail<unsigned long long><<<gm, 256, 0, ctx->stream>>>(np, t.k[hw], 0, fmask, m, low, s.err);
+        launch_starts<unsigned long long>(ctx, np, t.k[hw], 0, fmask, m, low, s.err);
         sym_row_ptr<<<gm, 256, 0, ctx->stream>>>(m, up, low, out->row_ptr);
         if (np > 0)
             sym_fill<<<gp, 256, 0, ctx->stream>>>(np, s.k[o], s.v[o], t.k[hw], t.v[hw], B, up, low, out->col_ind, oval,
@@ -507,8 +581,6 @@ apspie_status apspie_csr_transpose(apspie_ctx *ctx, const apspie_csr *A, apspie_
     if (st != APSPIE_OK) return st;
     if ((st = alloc_owned(ctx, n, A->m, nnz, A->val ? A->val_type : APSPIE_VAL_NONE, out)) != APSPIE_OK) return st;
     Carver c(base);
-    const int g = grid_for(ctx, nnz);
-    const int gn = grid_for(ctx, n + 1LL);
     const int *err = nullptr;
     cudaError_t e = cudaSuccess;
     int which = 0;
@@ -522,13 +594,8 @@ apspie_status apspie_csr_transpose(apspie_ctx *ctx, const apspie_csr *A, apspie_
         if (e == cudaSuccess)
             st = radix_sort(ctx, s, pl, s.k[1], static_cast<const unsigned *>(A->val), nnz, 0, &which);
         if (e == cudaSuccess && st == APSPIE_OK) {
-            if (nnz > 0) {
-                run_starts<unsigned long long><<<g, 256, 0, ctx->stream>>>(nnz, s.k[which], 32, ~0ull, out->row_ptr,
-                                                                           err);
-                low_half<<<g, 256, 0, ctx->stream>>>(nnz, s.k[which], out->col_ind);
-            }
-            fill_tail<unsigned long long><<<gn, 256, 0, ctx->stream>>>(nnz, s.k[which], 32, ~0ull, n, out->row_ptr,
-                                                                       err);
+            launch_starts<unsigned long long>(ctx, nnz, s.k[which], 32, ~0ull, n, out->row_ptr, err);
+            if (nnz > 0) low_half<<<grid_for(ctx, nnz), 256, 0, ctx->stream>>>(nnz, s.k[which], out->col_ind);
         }
     } else {
         SortBufs<unsigned> s = carve_sort<unsigned>(c, nnz);

@@ -274,3 +274,71 @@ def test_kept_memory_makes_room(ctx):
         assert torch.cuda.mem_get_info()[0] >= low + (380 << 20)
         del rest
     torch.cuda.empty_cache()
+
+
+def _few_entries(m, n):
+    """n entries between vertices spread over all of 0 .. m - 1, the first and the last among them."""
+    rng = np.random.default_rng(n)
+    u, v = rng.integers(0, m, (2, n))
+    u[0], v[0] = m - 1, 0
+    return u.astype(np.int32), v.astype(np.int32)
+
+
+@pytest.mark.parametrize("m,n", [(20000, 3), (17000, 4096), (3_000_000, 70), (3_000_000, 9000), (3_000_000, 2_999_999),
+                                 (200_000, 200_000)])
+@pytest.mark.parametrize("flags", [0, DROP])
+def test_build_and_transpose_of_mostly_empty_rows(ctx, m, n, flags):
+    """Fewer entries than rows, and entries of a block in rows far apart."""
+    import torch
+
+    u, v = _few_entries(m, n)
+    if n > 5000:  # a part in neighbouring rows, a part in rows far apart
+        u[: n // 2] = 77 + np.arange(n // 2) % 4000
+    val = np.arange(n, dtype=np.int32)
+    d = [torch.from_numpy(x).cuda() for x in (u, v, val)]
+    A = ctx.build_csr(m, *d, flags)
+    rp, ci, va = A.to_numpy()
+    if flags:
+        for x, y in zip((rp, ci, va), _ref_build(m, u, v, val, flags)):
+            np.testing.assert_array_equal(x, y)
+    else:
+        order = np.lexsort((np.arange(n), v, u))
+        np.testing.assert_array_equal(rp, np.concatenate(([0], np.cumsum(np.bincount(u, minlength=m)))))
+        np.testing.assert_array_equal(ci, v[order])
+        np.testing.assert_array_equal(va, val[order])
+    rows = np.repeat(np.arange(m), np.diff(rp))
+    back = np.argsort(ci, kind="stable")
+    want = np.concatenate(([0], np.cumsum(np.bincount(ci, minlength=m))))
+    host = ap.HostGraph(m, m, rp, ci, None)
+    for T, vals in ((ctx.transpose(A), True), (ctx.transpose(ap.DeviceGraph(host)), False)):
+        trp, tci, tva = T.to_numpy()
+        np.testing.assert_array_equal(trp, want)
+        np.testing.assert_array_equal(tci, rows[back])
+        if vals:
+            np.testing.assert_array_equal(tva, va[back])
+        T.free()
+    A.free()
+
+
+def test_few_entries_in_many_rows_take_little_time(ctx):
+    """The empty rows are filled by all of the device: 64 entries in 2^25 rows."""
+    import time
+
+    import torch
+
+    m = 1 << 25
+    u, v = _few_entries(m, 64)
+    d = [torch.from_numpy(x).cuda() for x in (u, v, np.arange(64, dtype=np.int32))]
+    seconds = []
+    for _ in range(4):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        A = ctx.build_csr(m, *d, 0)
+        T = ctx.transpose(A)
+        torch.cuda.synchronize()
+        seconds.append(time.perf_counter() - t0)
+        T.free()
+        A.free()
+    # writing the two 134 MB arrays of row starts takes 0.05 ms; a thread or a block that fills or
+    # walks the rows alone 10 ms and more
+    assert min(seconds) < 8e-3, seconds
