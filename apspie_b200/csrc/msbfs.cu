@@ -13,7 +13,8 @@
 //       by its length (long rows in pieces), ORing the neighbours' frontier words restricted
 //       to its still-unvisited queries, and stopping as soon as every such query is covered.
 // Depths are kept as bit planes beside the visited bits and written to the query-major output
-// out[q * m + v] at the end, every entry once.
+// out[q * m + v] at the end, every entry once; past the planes' 14 levels they are written and
+// later depths stored as they are found.
 // The per-query answers are exactly those of independent BFS runs.
 //
 // Measured (32 queries at scale 22 / 100 at scale 20 / 512 at scale 18): a lane per row of up
@@ -120,8 +121,8 @@ struct MsArgs {
     int *const *rows;     // else: query q's depths go to rows[q][0..m)
     unsigned *vis;        // m x W
     unsigned *fr[2];      // m x W each
-    // Batch: depths as bit planes, bit k of (depth + 1 - base) of every (vertex, query) in
-    // planes + k * m * W, laid out as vis; 0: not found since base (see write_depths)
+    // Batch: depths as bit planes, bit k of depth + 1 of every (vertex, query) in
+    // planes + k * m * W, laid out as vis; 0: not found (see write_depths)
     unsigned *planes;
     unsigned *touched;    // m bits
     int *q[3];            // active lists (rotating)
@@ -278,16 +279,22 @@ __device__ __forceinline__ int *depth_row(const MsArgs &a, int q) {
     return a.rows ? a.rows[q] : a.out + static_cast<long long>(q) * a.m;
 }
 
-// Engine: writes depth L + 1 of vertex v for query slot q, relative to the level the query
+// Stores depth L + 1 of vertex v for query q. Engine: relative to the level the query slot's query
 // started at, into the row its request gave (both are copied into shared memory at the start
 // of every level: s_row, s_base).
-__device__ __forceinline__ void put_depth(int q, int v, int L, int *const *s_row, const int *s_base) {
-    s_row[q][v] = L + 1 - s_base[q];
+template <bool SERVE>
+__device__ __forceinline__ void put_depth(const MsArgs &a, int q, int v, int L, int *const *s_row, const int *s_base) {
+    if (SERVE)
+        s_row[q][v] = L + 1 - s_base[q];
+    else
+        depth_row(a, q)[v] = L + 1;
 }
 
-// Batch: the depths of the queries `bits` of word x (= v * W + w) are `code` - 1 above the
-// planes' base. ATOMIC: other warps may be setting bits of the same word.
+// Batch: the depths of the queries `bits` of word x (= v * W + w) are `code` - 1. ATOMIC: other
+// warps may be setting bits of the same word.
 constexpr int kPlanes = 4;
+constexpr int kPlaneLevels = (1 << kPlanes) - 2;  // levels whose depths have codes
+
 template <bool ATOMIC>
 __device__ __forceinline__ void set_planes(const MsArgs &a, long long mw, long long x, unsigned bits, int code) {
 #pragma unroll
@@ -381,15 +388,16 @@ __device__ __forceinline__ unsigned spread_nibbles(unsigned x) {
     return (x | (x << 3)) & 0x11111111u;
 }
 
-// Turns the planes into depths, a warp per 128 vertices: query-major rows written once, 512
-// bytes at a time (four consecutive vertices a lane) where rows begin at multiples of 16
+// Turns the planes into depths (-1: no code), a warp per 128 vertices: query-major rows written
+// once, 512 bytes at a time (four consecutive vertices a lane) where rows begin at multiples of 16
 // bytes, else 128 at a time (vertices 32 apart). Depths that were stored
 // as they were found (each a 4-byte write into another row, or a part of one by a warp, over
-// rows that a memset had filled before) made three quarters of the traffic of a batch. With
-// `all`, entries without a code get -1; without, they are left alone (they were written
-// before). CLEAR: the planes start over.
-template <int W, bool CLEAR>
-__device__ void write_depths(const MsArgs &a, long long mw, int base, bool all) {
+// rows that a memset had filled before) made three quarters of the traffic of a batch. A search
+// deeper than the planes' codes writes the rows when they are full and stores what it finds after
+// that at once: the few vertices of a level of such a graph cost less than another sweep over
+// all planes and rows (512 sources on a grid of 1,024 x 1,024: 677 ms with a sweep each 15 levels).
+template <int W>
+__device__ void write_depths(const MsArgs &a, long long mw) {
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * kMsBlock + threadIdx.x) >> 5, nwarps = gridDim.x * kMsBlock / 32;
     const bool quads = (a.m & 3) == 0 && (a.rows || (reinterpret_cast<uintptr_t>(a.out) & 15u) == 0);
@@ -410,11 +418,6 @@ __device__ void write_depths(const MsArgs &a, long long mw, int base, bool all) 
 #pragma unroll
                     for (int i = 0; i < 4; ++i) p[k][i] = i < nv ? at[i * step * W] : 0u;
                 }
-                if (CLEAR) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (i < nv) at[i * step * W] = 0u;
-                }
             }
             const int nq = min(32, a.nq - w * 32);
             for (int q0 = 0; q0 < nq; q0 += 8) {
@@ -432,15 +435,15 @@ __device__ void write_depths(const MsArgs &a, long long mw, int base, bool all) 
                     for (int i = 0; i < 4; ++i) {
                         const int code = codes[i] & 15u;
                         codes[i] >>= 4;
-                        d[i] = code ? base + code - 1 : -1;
+                        d[i] = code - 1;
                     }
                     int *out = depth_row(a, w * 32 + q0 + q) + v;
-                    if (all && quads && nv == 4 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+                    if (quads && nv == 4 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
                         __stcs(reinterpret_cast<int4 *>(out), make_int4(d[0], d[1], d[2], d[3]));
                     } else {
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
-                            if (i < nv && (all || d[i] >= 0)) __stcs(out + i * step, d[i]);
+                            if (i < nv) __stcs(out + i * step, d[i]);
                     }
                 }
             }
@@ -544,8 +547,6 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
     const double mean_deg = m ? static_cast<double>(a.nnz) / m : 0.0;
     int prev_n = 0;  // length of the level L-1 list (all blocks read it at that level)
     int levels = 0, npush = 0, npull = 0;
-    int plane_base = 0;    // batch: a code is depth + 1 - plane_base
-    bool written = false;  // batch: every entry of the output has been written
     for (int L = 0;; ++L) {
         const int cur = L % 3, nxt = (L + 1) % 3, prv = (L + 2) % 3;
         if (SERVE) {
@@ -600,12 +601,9 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
         if (!SERVE && a.depth_cap > 0 && L + 1 >= a.depth_cap) break;
         ++levels;
         if (threadIdx.x == 0) s_claim[(L & 1) ^ 1] = 0;
-        if (!SERVE && L + 2 - plane_base >= 1 << kPlanes) {  // the planes are full: their depths go out
-            write_depths<W, true>(a, mw, plane_base, !written);
-            written = true;
-            plane_base = L + 1;
-        }
-        const int code = L + 2 - plane_base;  // of depth L + 1
+        if (!SERVE && L == kPlaneLevels) write_depths<W>(a, mw);  // the planes are full
+        const bool direct = SERVE || L >= kPlaneLevels;           // depths are stored as they are found
+        const int code = L + 2;                                   // of depth L + 1
         const unsigned *frc = a.fr[L & 1];
         unsigned *frn = a.fr[(L + 1) & 1];
         // zero the level L-1 frontier words (buffer frn) and reset the next list
@@ -692,10 +690,10 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
                         if (nb) {
                             vv[w] |= nb;
                             any = true;
-                            if (SERVE) {
-                                atomicOr(&s_alive[w], nb);
+                            if (SERVE) atomicOr(&s_alive[w], nb);
+                            if (direct) {
                                 for (unsigned b = nb; b; b &= b - 1)
-                                    put_depth(w * 32 + __ffs(b) - 1, v, L, s_row, s_base);
+                                    put_depth<SERVE>(a, w * 32 + __ffs(b) - 1, v, L, s_row, s_base);
                             } else {
                                 set_planes<false>(a, mw, static_cast<long long>(v) * W + w, nb, code);
                             }
@@ -796,19 +794,19 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
                         any = true;
                         frw[static_cast<long long>(v) * W + w] = got[w];
                         a.vis[static_cast<long long>(v) * W + w] |= got[w];
-                        if (!SERVE) set_planes<false>(a, mw, static_cast<long long>(v) * W + w, got[w], code);
+                        if (!direct) set_planes<false>(a, mw, static_cast<long long>(v) * W + w, got[w], code);
                     }
                 }
-                // engine: depths at once, one coalesced store per query that any lane found
-                if (SERVE) {
+                // depths at once, one coalesced store per query that any lane found
+                if (direct) {
 #pragma unroll
                     for (int w = 0; w < W; ++w) {
                         const unsigned found = __reduce_or_sync(FULL, got[w]);
                         for (unsigned anyb = found; anyb; anyb &= anyb - 1) {
                             const int bit = __ffs(anyb) - 1;
-                            if ((got[w] >> bit) & 1u) put_depth(w * 32 + bit, v, L, s_row, s_base);
+                            if ((got[w] >> bit) & 1u) put_depth<SERVE>(a, w * 32 + bit, v, L, s_row, s_base);
                         }
-                        if (lane == 0 && found) atomicOr(&s_alive[w], found);
+                        if (SERVE && lane == 0 && found) atomicOr(&s_alive[w], found);
                     }
                 }
                 aw.push(any, v);
@@ -834,9 +832,9 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
                     const unsigned got = __shfl_sync(FULL, g[w % VW], w / VW);
                     if (got == 0u) continue;
                     any = true;
-                    if (SERVE) {
-                        if ((got >> lane) & 1u) put_depth(w * 32 + lane, v, L, s_row, s_base);
-                        if (lane == 0) atomicOr(&s_alive[w], got);
+                    if (SERVE && lane == 0) atomicOr(&s_alive[w], got);
+                    if (direct) {
+                        if ((got >> lane) & 1u) put_depth<SERVE>(a, w * 32 + lane, v, L, s_row, s_base);
                     } else if (lane == 0) {
                         set_planes<false>(a, mw, static_cast<long long>(v) * W + w, got, code);
                     }
@@ -882,9 +880,9 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
                 for (int w = 0; w < W; ++w) {
                     const unsigned got = __shfl_sync(FULL, g[w % VW], w / VW);
                     if (got == 0u) continue;
-                    if (SERVE) {
-                        if ((got >> lane) & 1u) put_depth(w * 32 + lane, v, L, s_row, s_base);
-                        if (lane == 0) atomicOr(&s_alive[w], got);
+                    if (SERVE && lane == 0) atomicOr(&s_alive[w], got);
+                    if (direct) {
+                        if ((got >> lane) & 1u) put_depth<SERVE>(a, w * 32 + lane, v, L, s_row, s_base);
                     } else if (lane == 0) {
                         set_planes<true>(a, mw, static_cast<long long>(v) * W + w, got, code);
                     }
@@ -909,7 +907,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
         if (!grid_barrier(a.ctl, a.sticky, kSiteMs + 5)) return;
         prev_n = nA;
     }
-    if (!SERVE) write_depths<W, false>(a, mw, plane_base, !written);
+    if (!SERVE && levels <= kPlaneLevels) write_depths<W>(a, mw);
     if (gtid == 0) {
         a.ctl->iterations = levels;
         a.ctl->push_iterations = npush;

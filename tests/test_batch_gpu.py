@@ -328,3 +328,51 @@ def test_bfs_batch_row_classes_and_long_paths(ctx, nq, m):
         ctx.set_batch_push_frac(0.05)
     cap = ctx.bfs_batch(dg, torch.from_numpy(sources[:1]).cuda(), depth_cap=18).cpu().numpy()[0]
     np.testing.assert_array_equal(cap, ctx.bfs(dg, int(sources[0]), depth_cap=18).cpu().numpy())
+
+
+def _grid(n):
+    """An n x n grid (its hop counts reach 2 n - 2)."""
+    i = np.arange(n * n)
+    u = np.concatenate((i[i % n < n - 1], i[:-n]))
+    v = np.concatenate((i[i % n < n - 1] + 1, i[n:]))
+    rows, cols = np.concatenate((u, v)), np.concatenate((v, u))
+    order = np.lexsort((cols, rows))
+    rp = np.concatenate(([0], np.cumsum(np.bincount(rows, minlength=n * n)))).astype(np.int32)
+    return ap.HostGraph(n * n, n * n, rp, cols[order].astype(np.int32), None, True)
+
+
+@pytest.mark.parametrize("n,nq", [(8, 3), (9, 33), (33, 70), (60, 300), (61, 512)])
+def test_bfs_batch_deeper_than_the_planes(ctx, n, nq):
+    """More levels than the depth planes have codes: rows written once when they are full, later
+    depths as they are found; with a cap at, before and after that level."""
+    import torch
+
+    g = ap.DeviceGraph(_grid(n))
+    rng = np.random.default_rng(n)
+    src = rng.integers(0, n * n, nq).astype(np.int32)
+    y, x = np.divmod(np.arange(n * n), n)
+    want = np.abs(y[None, :] - y[src][:, None]) + np.abs(x[None, :] - x[src][:, None])
+    d_src = torch.from_numpy(src).cuda()
+    for cap in (0, 13, 14, 15, 16, 17):
+        got = ctx.bfs_batch(g, d_src, depth_cap=cap).cpu().numpy()
+        np.testing.assert_array_equal(got, want if cap == 0 else np.where(want < cap, want, -1))
+
+
+def test_bfs_batch_on_a_deep_graph_takes_little_time(ctx):
+    """512 sources on a grid of 510 levels: a level costs what its frontier does."""
+    import time
+
+    import torch
+
+    g = ap.DeviceGraph(_grid(256))
+    src = torch.arange(512, dtype=torch.int32, device="cuda") * 127
+    out = torch.empty((512, g.m), dtype=torch.int32, device="cuda")
+    seconds = []
+    for _ in range(4):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        ctx.bfs_batch_into(g, src, out)
+        torch.cuda.synchronize()
+        seconds.append(time.perf_counter() - t0)
+    # 15 ms, where a sweep over all planes and rows every 15 levels made it 31
+    assert min(seconds) < 24e-3, seconds
