@@ -925,6 +925,19 @@ const void *msbfs_serve_fn() {
     return reinterpret_cast<const void *>(msbfs_kernel<W, true>);
 }
 
+// Blocks of a batch, one to five an SM: more shorten a level's work, fewer its three barriers. By
+// the words that a visit of every entry reads; us with one / two / three / four an SM:
+// 0.04M (2 queries on R-MAT) 91 / 97 / 107 / 119, 0.3M (32 on a grid, 510 levels) 5,836 / 5,918 /
+// 6,596 / 7,426, 0.4M 118 / 130 / 138 / 149; 1.2M 121 / 120 / 125 / 140, 4.2M (512 on that grid)
+// 18,148 / 14,600 / 15,215, 7.3M 294 / 289 / 309 / 338; 15M 403 / 352 / 344 / 352; 24M 971 / 693 /
+// 586 / 560. Five fit for up to 64 queries: 1,400 instead of 1,457 at 2^27, 482 instead of 473 at
+// 2^25.
+long long msbfs_blocks(const apspie_ctx *ctx, long long nnz, int W) {
+    const long long w = nnz * W;
+    if (nnz >= (1 << 26)) return kMaxGrid;
+    return static_cast<long long>(ctx->num_sms) * (w >= 20000000 ? 4 : w >= 10000000 ? 3 : w >= 1000000 ? 2 : 1);
+}
+
 size_t batch_need(int m, int Wp) {  // without the depth planes of the batch
     const size_t mi = static_cast<size_t>(m) + 1;
     const size_t mw = static_cast<size_t>(m) * Wp;
@@ -1023,10 +1036,7 @@ apspie_status bfs_batch_impl(apspie_ctx *ctx, const apspie_csr *A, const int32_t
         const void *fn = Wp == 1 ? msbfs_fn<1>() : Wp == 2 ? msbfs_fn<2>() : Wp == 4 ? msbfs_fn<4>()
                          : Wp == 8 ? msbfs_fn<8>() : msbfs_fn<16>();
         void *args[] = {&a};
-        // up to 64 queries five blocks fit on an SM: worth their dearer barriers on large graphs
-        // only (32 queries at scale 22: 1,400 us against 1,457 us, at scale 20: 482 against 473)
-        const long long blocks = A->nnz >= (1 << 26) ? kMaxGrid : 4LL * ctx->num_sms;
-        st = launch_persistent(ctx, fn, kMsBlock, args, blocks * kWorkPerBlock);
+        st = launch_persistent(ctx, fn, kMsBlock, args, msbfs_blocks(ctx, A->nnz, Wp) * kWorkPerBlock);
         if (st != APSPIE_OK) return st;
         if (stats) {
             apspie_run_stats part;
