@@ -13,7 +13,8 @@
 // under L, 0.66G under D, largest row 8,083 -> 411).
 //
 // On up to 1.6M vertices the count is then taken edge by edge, each as the intersection of
-// its endpoints' rows of D, the longer one a bitmap in shared memory (see tc_bits). Larger
+// its endpoints' rows of D, the longer one a bitmap in shared memory (see tc_bits; rows that are
+// both short a warp's, see tc_small). Larger
 // graphs, and inputs that the bitmaps cannot count, take masks in hash sets: each row i of D
 // is loaded into a hash set (its mask); every wedge (k in D(i,:), j in D(k,:)) probes the set, and hits are
 // counted in int64. Rows with masks of at most 256 entries are cut into warp tasks of at
@@ -48,7 +49,8 @@ struct TcInfo {
     int not_lower;  // an entry with column >= row
     int unsorted;   // a row whose entries don't ascend strictly (it may hold an entry twice)
     int ticket;     // owners handed out
-    int owners[2];  // owners with many partners, with few
+    int beyond;     // entries of D far back in their lists (tc_even_limit)
+    int owners[3];  // owners with many partners, with few, vertices with short lists (tc_owners)
 };
 
 __device__ __forceinline__ unsigned tc_hash(int key, int log2ts) {
@@ -187,24 +189,57 @@ __device__ __forceinline__ void tc_edge(const int *deg, int i, int j, int &a, in
     b = fwd ? j : i;
 }
 
+// Edges between vertices with short lists are counted by a warp for each vertex (tc_small), the
+// others from the bitmap of the longer list by a block (tc_bits): its round of setting, testing
+// and clearing takes 0.4 to 1.8 us, whatever it tests, and the larger the bitmap the fewer blocks
+// there are. "Short" is up to 64 entries in graphs of about even degrees (up to 32 edges a vertex,
+// and less than 1 in 32 of D's entries past three times the mean list: grids, uniform graphs);
+// else it grows with the vertices, and the blocks count everything up to 131,072, and up to 8,192
+// in any graph (what a launch takes is more than what it spares). Whole counts in
+// us, with hash sets / all by blocks / so: a 1,024 x 1,024 grid 1,440 / 13,340 / 604, uniform 2^19
+// (10M edges) 1,226 / 3,380 / 1,082, 2^16 (0.5M) 192 / 227 / 142, 2^16 (2M) 367 / 379 / 350; R-MAT of
+// 1.5M (ef 4) 3,270 / 3,560 / 1,526, 2^19 (ef 20) 12,960 / 2,640 / 2,354, 2^18 (ef 16) 3,620 / 866 /
+// 850; of 2^16 (ef 6) 339 / 173 / 173 (181 with lists up to 16, 222 with 64).
+constexpr int kTcSmallList = 64, kTcNoSmall = 8192;
+inline int tc_even_limit(int m, unsigned nnz) {  // past which D's entries are counted
+    return m <= kTcNoSmall ? 0x7fffffff : 3 * static_cast<int>(nnz / m + 1);
+}
+__device__ __forceinline__ int tc_small_list(int m, unsigned nnz, const TcInfo *info) {
+    if (m <= kTcNoSmall) return 0;
+    if (nnz / m < 32 && static_cast<unsigned>(info->beyond) <= nnz / 32) return kTcSmallList;
+    return m <= 131072 ? 0 : min(kTcSmallList, m >> 13);
+}
+
 // place[e] = the edge's place in its tail's list; len[a] the list's length
 __global__ void tc_out_places(unsigned nnz, const unsigned *__restrict__ row, const int *__restrict__ ci,
-                              const int *__restrict__ deg, int *len, int *place, const TcInfo *info) {
+                              const int *__restrict__ deg, int *len, int *place, int even_limit, TcInfo *info) {
+    __shared__ int s_beyond;
     if (info->not_lower) return;
+    if (threadIdx.x == 0) s_beyond = 0;
+    __syncthreads();
+    int beyond = 0;
     for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
         int a, b;
         tc_edge(deg, static_cast<int>(__ldg(row + e)), __ldg(ci + e), a, b);
-        place[e] = atomicAdd(len + a, 1);
+        const int at = atomicAdd(len + a, 1);
+        place[e] = at;
+        beyond += at >= even_limit;
     }
+    if (even_limit == 0x7fffffff) return;
+    beyond = __reduce_add_sync(0xffffffffu, beyond);
+    if ((threadIdx.x & 31) == 0 && beyond) atomicAdd(&s_beyond, beyond);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_beyond) atomicAdd(&info->beyond, s_beyond);
 }
 
 // Writes D (unless D is L as it is: dci null) and, for the bitmap path (partners not null),
 // hands out the edge's place in its owner's list of partners; -1 where the shorter list is
-// empty.
+// empty or both are short (tc_small).
 __global__ void tc_owner_places(unsigned nnz, const unsigned *__restrict__ row, const int *__restrict__ ci,
                                 const int *__restrict__ deg, const int *__restrict__ drp, int *dci, int *place,
-                                int *partners, const TcInfo *info) {
+                                int *partners, int m, const TcInfo *info) {
     if (info->not_lower) return;
+    const int small_list = partners ? tc_small_list(m, nnz, info) : 0;
     for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
         int a, b;
         tc_edge(deg, static_cast<int>(__ldg(row + e)), __ldg(ci + e), a, b);
@@ -212,9 +247,14 @@ __global__ void tc_owner_places(unsigned nnz, const unsigned *__restrict__ row, 
         const int lb = __ldg(drp + b + 1) - __ldg(drp + b);
         if (dci) dci[a0 + place[e]] = b;
         if (!partners) continue;
-        const int owner = lb <= 0 ? -1 : la >= lb ? a : b;  // la > 0: it holds this edge
+        // la > 0: it holds this edge
+        const int owner = lb <= 0 || max(la, lb) <= small_list ? -1 : la >= lb ? a : b;
         // consecutive entries often have one owner: one atomic for the lanes that share it
         const unsigned active = __activemask();
+        if (!__any_sync(active, owner >= 0)) {
+            place[e] = -1;
+            continue;
+        }
         const unsigned peers = __match_any_sync(active, owner);
         const int first = __ffs(peers) - 1, lane = threadIdx.x & 31;
         int base = 0;
@@ -433,8 +473,9 @@ __global__ void __launch_bounds__(kTcBlock) tc_block(const int *__restrict__ row
 // R-MAT scale 18, 321M tests instead of the 660M wedges of sum((D*D) .* D), and a test is one
 // shared-memory word instead of a probe chain in a hash set.
 //
-// Measured at scale 18: counting 2.74 ms with hash sets; 0.55 ms with bitmaps (and 0.14 ms for the
-// partner lists), at 64 % of the issue slots and 72 % of the L1/shared-memory pipe.
+// Measured at scale 18: counting 2.74 ms with hash sets; 0.51 ms with bitmaps and tc_small (and
+// 0.13 ms for the partner lists), tc_bits at 64 % of the issue slots and 72 % of the L1/shared-memory
+// pipe.
 //
 // Needs: L strict lower triangular with strictly ascending rows (both found out on the way: a
 // row's list then is a set, so that either side may be the bitmap; in rows out of order an entry
@@ -442,12 +483,11 @@ __global__ void __launch_bounds__(kTcBlock) tc_block(const int *__restrict__ row
 // counted by the hash path above.
 constexpr int kTcBitmapVertices = 1600 * 1024;  // 200 KB of bits
 constexpr int kTcManyPartners = 256;            // owners with at least this many start first
-
-__global__ void tc_partner_lists(unsigned nnz, const unsigned *__restrict__ row, const int *__restrict__ ci,
+__global__ void tc_partner_lists(int m, unsigned nnz, const unsigned *__restrict__ row, const int *__restrict__ ci,
                                  const int *__restrict__ deg, const int *__restrict__ drp,
                                  const int *__restrict__ place, const int *__restrict__ prp, int *plist,
                                  const TcInfo *info) {
-    if (info->not_lower) return;
+    if (info->not_lower || __ldg(prp + m) == 0) return;
     for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
         const int at = place[e];
         if (at < 0) continue;
@@ -459,21 +499,26 @@ __global__ void tc_partner_lists(unsigned nnz, const unsigned *__restrict__ row,
     }
 }
 
-// Owners with many partners from the front of `list`, the others from its back.
-__global__ void tc_owners(int m, const int *__restrict__ prp, int *list, TcInfo *info) {
+// Owners with many partners from the front of `list`, the others from its back; in `small` the
+// vertices whose lists are short (and long enough for a triangle).
+__global__ void tc_owners(int m, unsigned nnz, const int *__restrict__ drp, const int *__restrict__ prp, int *list,
+                          int *small, TcInfo *info) {
     if (info->not_lower) return;
+    const int small_list = tc_small_list(m, nnz, info);
     const int lane = threadIdx.x & 31;
     for (int v0 = blockIdx.x * blockDim.x; v0 < m; v0 += gridDim.x * blockDim.x) {
         const int v = v0 + threadIdx.x;
         const int n = v < m ? __ldg(prp + v + 1) - __ldg(prp + v) : 0;
+        const int len = v < m && small_list > 0 ? __ldg(drp + v + 1) - __ldg(drp + v) : 0;
+        const int kind = n >= kTcManyPartners ? 0 : n > 0 ? 1 : len >= 2 && len <= small_list ? 2 : -1;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const bool in = k == 0 ? n >= kTcManyPartners : n > 0 && n < kTcManyPartners;
+        for (int k = 0; k < 3; ++k) {
+            const bool in = k == kind;
             const unsigned mask = __ballot_sync(0xffffffffu, in);
             int base = 0;
             if (lane == 0 && mask) base = atomicAdd(&info->owners[k], __popc(mask));
             base = __shfl_sync(0xffffffffu, base, 0) + __popc(mask & ((1u << lane) - 1u));
-            if (in) list[k == 0 ? base : m - 1 - base] = v;
+            if (in) (k == 2 ? small : list)[k == 1 ? m - 1 - base : base] = v;
         }
     }
 }
@@ -490,6 +535,7 @@ __global__ void __launch_bounds__(1024) tc_bits(int m, const int *__restrict__ l
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nthreads = blockDim.x, nwarps = nthreads >> 5;
     const int nmany = info->owners[0], nall = nmany + info->owners[1];
+    if (nall == 0) return;
     for (int w = tid; w < (m + 31) >> 5; w += nthreads) bits[w] = 0u;
     unsigned long long hits = 0;
     for (;;) {
@@ -530,6 +576,85 @@ __global__ void __launch_bounds__(1024) tc_bits(int m, const int *__restrict__ l
         }
         __syncthreads();
         for (int e = r0 + tid; e < r1; e += nthreads) bits[__ldg(dci + e) >> 5] = 0u;
+    }
+    for (int o = 16; o; o >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, o);
+    if (lane == 0 && hits) atomicAdd(&info->count, hits);
+}
+
+// Vertices with short lists, a warp each: the list goes into a hash set in shared memory, and the
+// short ones among the lists of its entries, one after the other, are looked up in it, 128
+// entries at a time. What bounds it: the chain of reads (vertex, its list, an entry's list)
+// with 64 warps on an SM.
+struct TcSmallSmem {
+    int keys[4 * kTcSmallList];
+    int rs[kTcSmallList];        // of each list looked up: where it begins, minus
+    int soff[kTcSmallList + 1];  // the entries before it
+};
+__global__ void __launch_bounds__(kTcBlock) tc_small(int m, unsigned nnz, const int *__restrict__ small,
+                                                     const int *__restrict__ drp, const int *__restrict__ dci,
+                                                     TcInfo *info) {
+    __shared__ TcSmallSmem smem[kTcBlock / 32];
+    const int small_list = tc_small_list(m, nnz, info);
+    if (small_list == 0 || info->not_lower || info->unsorted) return;
+    TcSmallSmem &sm = smem[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const unsigned upto = lane == 31 ? 0xffffffffu : (2u << lane) - 1u;
+    const int n = info->owners[2];
+    const int nwarps = (gridDim.x * kTcBlock) >> 5;
+    unsigned long long hits = 0;
+    for (long long w = (blockIdx.x * kTcBlock + threadIdx.x) >> 5; w < n; w += nwarps) {
+        const int v = __ldg(small + w);
+        const int r0 = __ldg(drp + v), d = __ldg(drp + v + 1) - r0;
+        // a power of two of slots, at least four times the list's
+        const int log2ts = max(5, 32 - __clz(4 * d - 1)), ts = 1 << log2ts;
+        for (int s = lane; s < ts; s += 32) sm.keys[s] = kEmpty;
+        __syncwarp();
+        int nv = 0, all = 0;
+        for (int t0 = 0; t0 < d; t0 += 32) {
+            int b0 = 0, len = 0;
+            if (t0 + lane < d) {
+                const int k = __ldg(dci + r0 + t0 + lane);
+                b0 = __ldg(drp + k);
+                len = __ldg(drp + k + 1) - b0;
+                set_insert(sm.keys, ts, log2ts, k, info);
+                if (len > small_list) len = 0;  // the blocks count it
+            }
+            const unsigned some = __ballot_sync(0xffffffffu, len > 0);
+            int incl = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            if (len > 0) {
+                const int at = nv + __popc(some & ((1u << lane) - 1u));
+                sm.soff[at] = all + incl - len;
+                sm.rs[at] = b0 - (all + incl - len);
+            }
+            nv += __popc(some);
+            all += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        __syncwarp();
+        int o0 = 0;  // the list of the chunk's first entry
+        unsigned found = 0u;
+        for (int base = 0; base < all; base += 128) {
+            int j[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const int cb = base + 32 * h;
+                const int nb = o0 + 1 + lane;
+                const int st = nb < nv ? sm.soff[nb] - cb : 32;
+                const unsigned starts = __reduce_or_sync(0xffffffffu, st >= 0 && st < 32 ? 1u << st : 0u);
+                const int q = cb + lane;
+                j[h] = q < all ? __ldg(dci + sm.rs[o0 + __popc(starts & upto)] + q) : -1;
+                o0 += __popc(starts);
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+                if (j[h] >= 0) found += set_find<false>(sm.keys, ts, log2ts, j[h]) ? 1u : 0u;
+        }
+        hits += found;
+        __syncwarp();
     }
     for (int o = 16; o; o >>= 1) hits += __shfl_down_sync(0xffffffffu, hits, o);
     if (lane == 0 && hits) atomicAdd(&info->count, hits);
@@ -582,10 +707,10 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
     if (st != APSPIE_OK) return st;
     Carver c(base);
     TcInfo *info = c.take<TcInfo>(1);
-    int *deg = c.take<int>(mi);
     int *len = c.take<int>(mi);
-    int *drp = c.take<int>(mi);
     int *partners = c.take<int>(mi);
+    int *deg = c.take<int>(mi);
+    int *drp = c.take<int>(mi);
     int *prp = c.take<int>(mi);
     int *list = c.take<int>(mi);
     unsigned *row = c.take<unsigned>(nz);
@@ -593,9 +718,8 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
     int *dci = c.take<int>(nz);
     int *plist = c.take<int>(nz);
     void *stmp = c.take<char>(scan_scratch_bytes(m) + 64);
-    cudaError_t e = cudaMemsetAsync(info, 0, sizeof(TcInfo), ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(len, 0, mi * 4, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(partners, 0, mi * 4, ctx->stream);
+    const size_t zeroed = static_cast<size_t>(reinterpret_cast<char *>(partners + mi) - reinterpret_cast<char *>(info));
+    cudaError_t e = cudaMemsetAsync(info, 0, zeroed, ctx->stream);  // info, len, partners
     if (e != cudaSuccess) return cuda_error(ctx, e, "tc reset");
     const bool orient = effective_params(ctx, APSPIE_TUNE_TC, L).tc_orient != 0;
     const int eb = entry_blocks(ctx, nnz), vb = std::min((m + 255) / 256, ctx->num_sms * 8);
@@ -605,16 +729,19 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
     const int *rp = L->row_ptr, *ci = L->col_ind, *degree = nullptr;
     if (orient) {
         degree = deg;
-        tc_out_places<<<eb, 256, 0, ctx->stream>>>(nnz, row, L->col_ind, degree, len, place, info);
+        tc_out_places<<<eb, 256, 0, ctx->stream>>>(nnz, row, L->col_ind, degree, len, place, tc_even_limit(m, nnz), info);
         if ((st = device_exclusive_scan(ctx, len, m, drp, stmp, &info->overflow)) != APSPIE_OK) return st;
         rp = drp;
         ci = dci;
     }
     tc_owner_places<<<eb, 256, 0, ctx->stream>>>(nnz, row, L->col_ind, degree, rp, orient ? dci : nullptr, place,
-                                                 partners, info);
+                                                 partners, m, info);
     if ((st = device_exclusive_scan(ctx, partners, m, prp, stmp, &info->overflow)) != APSPIE_OK) return st;
-    tc_partner_lists<<<eb, 256, 0, ctx->stream>>>(nnz, row, L->col_ind, degree, rp, place, prp, plist, info);
-    tc_owners<<<vb, 256, 0, ctx->stream>>>(m, prp, list, info);
+    tc_partner_lists<<<eb, 256, 0, ctx->stream>>>(m, nnz, row, L->col_ind, degree, rp, place, prp, plist, info);
+    int *small = partners;  // prp has taken its place
+    tc_owners<<<vb, 256, 0, ctx->stream>>>(m, nnz, rp, prp, list, small, info);
+    if (m > kTcNoSmall)
+        tc_small<<<ctx->num_sms * 8, kTcBlock, 0, ctx->stream>>>(m, nnz, small, rp, ci, info);
     // threads enough to fill an SM beside the bitmaps that fit on it
     const size_t smem = (static_cast<size_t>(m) + 31) / 32 * 4;
     const int threads = smem <= 36 * 1024 ? 256 : smem <= 72 * 1024 ? 512 : 1024;
@@ -674,9 +801,9 @@ apspie_status tc_by_hash_sets(apspie_ctx *ctx, const apspie_csr *L, int64_t *cou
         if ((st = expand_entry_rows(ctx, L, row)) != APSPIE_OK) return st;
         tc_row_lengths<<<std::min((m + 255) / 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, rp, deg);
         tc_columns<<<std::min(eb, ctx->num_sms * 4), kTcColumnsBlock, 0, ctx->stream>>>(nnz, m, row, ci, deg, info);
-        tc_out_places<<<eb, 256, 0, ctx->stream>>>(nnz, row, ci, deg, len, place, info);
+        tc_out_places<<<eb, 256, 0, ctx->stream>>>(nnz, row, ci, deg, len, place, tc_even_limit(m, nnz), info);
         if ((st = device_exclusive_scan(ctx, len, m, drp, stmp, &info->overflow)) != APSPIE_OK) return st;
-        tc_owner_places<<<eb, 256, 0, ctx->stream>>>(nnz, row, ci, deg, drp, dci, place, nullptr, info);
+        tc_owner_places<<<eb, 256, 0, ctx->stream>>>(nnz, row, ci, deg, drp, dci, place, nullptr, m, info);
         rp = drp;
         ci = dci;
     }

@@ -352,3 +352,51 @@ def test_sizes_of_threads_do_not_meet(ctx):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("uneven", [False, True])
+@pytest.mark.parametrize("m", [8192, 8193, 131072, 140000, 600000])
+def test_tc_lists_of_every_size(ctx, m, uneven):
+    """Lists around the limits of what a warp counts (17 entries, or 64), beside many vertices of
+    degree one and two: of about even degrees, and with a vertex that meets half of them."""
+    rng = np.random.default_rng(m)
+    at = m // 3
+    edges = [np.stack((np.arange(1, at), np.arange(at - 1)))]  # a path
+    if uneven:
+        edges.append(np.stack((np.arange(2, at), np.zeros(at - 2, dtype=np.int64))))
+        i, j = np.tril_indices(200, -1)
+        edges.append(np.stack((i, j)))
+    for c in (3, 8, 9, 10, 17, 18, 19, 33, 34, 64, 65, 66, 67):  # cliques: lists up to c - 1
+        i, j = np.tril_indices(c, -1)
+        edges.append(np.stack((i + at, j + at)))
+        at += c
+    for hubs, leaves in ((2, 31), (2, 32), (2, 33), (5, 40), (9, 33), (20, 300)):  # hubs joined, all to every leaf
+        i, j = np.tril_indices(hubs, -1)
+        edges.append(np.stack((i + at, j + at)))
+        a, b = np.meshgrid(np.arange(hubs), np.arange(leaves))
+        edges.append(np.stack((b.ravel() + at + hubs, a.ravel() + at)))
+        at += hubs + leaves
+    e = np.concatenate(edges, axis=1)
+    e = rng.permutation(m)[e]  # ids in no order
+    key = np.unique(np.maximum(*e).astype(np.int64) * m + np.minimum(*e))
+    rp = np.concatenate(([0], np.cumsum(np.bincount(key // m, minlength=m)))).astype(np.int32)
+    ci = (key % m).astype(np.int32)
+    assert ctx.tc(ap.DeviceGraph(ap.HostGraph(m, m, rp, ci))) == oracle.tc(rp, ci)
+
+
+def test_tc_of_low_degrees_takes_little_time(ctx):
+    """A grid of a million vertices: two entries a row, no triangles."""
+    import time
+
+    n = 1024
+    i = np.arange(n * n)
+    key = np.sort(np.concatenate((i[i % n > 0] * (n * n + 1) - 1, i[n:] * (n * n + 1) - n)))
+    rp = np.concatenate(([0], np.cumsum(np.bincount(key // (n * n), minlength=n * n)))).astype(np.int32)
+    g = ap.DeviceGraph(ap.HostGraph(n * n, n * n, rp, (key % (n * n)).astype(np.int32)))
+    seconds = []
+    for _ in range(4):
+        t0 = time.perf_counter()
+        assert ctx.tc(g) == 0
+        seconds.append(time.perf_counter() - t0)
+    # 0.7 ms, where a block's round for each vertex made it 13
+    assert min(seconds) < 4e-3, seconds
