@@ -239,6 +239,7 @@ __global__ void tc_owner_places(unsigned nnz, const unsigned *__restrict__ row, 
                                 const int *__restrict__ deg, const int *__restrict__ drp, int *dci, int *place,
                                 int *partners, int m, const TcInfo *info) {
     if (info->not_lower) return;
+    if (info->unsorted) partners = nullptr;  // the hash sets count it
     const int small_list = partners ? tc_small_list(m, nnz, info) : 0;
     for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
         int a, b;
@@ -487,7 +488,7 @@ __global__ void tc_partner_lists(int m, unsigned nnz, const unsigned *__restrict
                                  const int *__restrict__ deg, const int *__restrict__ drp,
                                  const int *__restrict__ place, const int *__restrict__ prp, int *plist,
                                  const TcInfo *info) {
-    if (info->not_lower || __ldg(prp + m) == 0) return;
+    if (info->not_lower || info->unsorted || __ldg(prp + m) == 0) return;
     for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
         const int at = place[e];
         if (at < 0) continue;
@@ -503,7 +504,7 @@ __global__ void tc_partner_lists(int m, unsigned nnz, const unsigned *__restrict
 // vertices whose lists are short (and long enough for a triangle).
 __global__ void tc_owners(int m, unsigned nnz, const int *__restrict__ drp, const int *__restrict__ prp, int *list,
                           int *small, TcInfo *info) {
-    if (info->not_lower) return;
+    if (info->not_lower || info->unsorted) return;
     const int small_list = tc_small_list(m, nnz, info);
     const int lane = threadIdx.x & 31;
     for (int v0 = blockIdx.x * blockDim.x; v0 < m; v0 += gridDim.x * blockDim.x) {
@@ -694,15 +695,95 @@ int entry_blocks(const apspie_ctx *ctx, unsigned nnz) {
     return static_cast<int>(std::min<long long>((static_cast<long long>(nnz) + 255) / 256, ctx->num_sms * 16LL));
 }
 
-// The bitmap path; *counted stays false when L turns out not to fit it.
-apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count, bool *counted) {
+// What counting by hash sets takes beside D, and a scan's scratch.
+struct TcHashBufs {
+    int *bin_rows;
+    long long *tbl_off;
+    unsigned char *row_bin;
+    int *ntask, *task_ptr;
+    static size_t need(int m) {
+        const size_t mi = static_cast<size_t>(m) + 1;
+        return Carver::need({kTcBins * mi * 4, mi * 8, mi, mi * 4, mi * 4});
+    }
+    static TcHashBufs carve(Carver &c, int m) {
+        const size_t mi = static_cast<size_t>(m) + 1;
+        TcHashBufs b;
+        b.bin_rows = c.take<int>(kTcBins * mi);
+        b.tbl_off = c.take<long long>(mi);
+        b.row_bin = c.take<unsigned char>(mi);
+        b.ntask = c.take<int>(mi);
+        b.task_ptr = c.take<int>(mi);
+        return b;
+    }
+};
+
+// sum((D*D) .* D) of D = (rp, ci) by hash sets; *info is cleared. With `check`, an L that is not
+// strictly lower (info->not_lower, set when D was made from it) is counted as given instead.
+apspie_status tc_count_by_hash(apspie_ctx *ctx, const apspie_csr *L, const int *rp, const int *ci, bool check,
+                               const TcHashBufs &b, void *stmp, TcInfo *info, int64_t *count) {
+    apspie_status st;
+    cudaError_t e = cudaSuccess;
+    const int m = L->m;
+    const int task_work = effective_params(ctx, APSPIE_TUNE_TC, L).tc_task_work;
+    const int rblocks = std::max(1, std::min<int>((m * 8LL + 255) / 256, ctx->num_sms * 16));
+    const int lblocks = std::max(1, std::min<int>((m + 255LL) / 256, ctx->num_sms * 8));
+    TcInfo h;
+    int ntasks = 0;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        if (m > 0) {
+            tc_rowinfo<<<rblocks, 256, 0, ctx->stream>>>(m, rp, ci, task_work, b.row_bin, b.ntask, b.tbl_off, info);
+            tc_binlists<<<lblocks, 256, 0, ctx->stream>>>(m, b.row_bin, b.bin_rows, info);
+            if ((st = device_exclusive_scan(ctx, b.ntask, m, b.task_ptr, stmp, &info->overflow)) != APSPIE_OK) return st;
+            if ((e = cudaMemcpyAsync(&ntasks, b.task_ptr + m, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream)) !=
+                cudaSuccess)
+                return cuda_error(ctx, e, "tc plan");
+        }
+        if ((e = cudaMemcpyAsync(&h, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
+            return cuda_error(ctx, e, "tc plan");
+        if (!h.not_lower || attempt == 1 || !check) break;
+        // not a strict lower triangle: count sum((L*L) .* L) on L as given
+        rp = L->row_ptr;
+        ci = L->col_ind;
+        if ((e = cudaMemsetAsync(info, 0, sizeof(TcInfo), ctx->stream)) != cudaSuccess)
+            return cuda_error(ctx, e, "tc reset");
+    }
+    int *gkeys = nullptr;
+    if (h.global_slots > 0) {
+        void *tb;
+        if ((st = scratch2_reserve(ctx, static_cast<size_t>(h.global_slots) * 4 + 256, &tb)) != APSPIE_OK)
+            return st;
+        gkeys = static_cast<int *>(tb);
+    }
+    const int cap = ctx->num_sms * 8;
+    if (ntasks > 0)
+        tc_warp<<<std::min((ntasks + 7) / 8, cap), kTcBlock, 0, ctx->stream>>>(b.task_ptr, m, ntasks, task_work, rp, ci,
+                                                                                 info);
+    if (h.bin_count[2] > 0)
+        tc_block<false><<<std::min(h.bin_count[2], cap), kTcBlock, 0, ctx->stream>>>(
+            b.bin_rows + 2 * static_cast<size_t>(m), h.bin_count[2], rp, ci, b.tbl_off, gkeys, info);
+    if (h.bin_count[3] > 0)
+        tc_block<true><<<std::min(h.bin_count[3], cap), kTcBlock, 0, ctx->stream>>>(
+            b.bin_rows + 3 * static_cast<size_t>(m), h.bin_count[3], rp, ci, b.tbl_off, gkeys, info);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(ctx, e, "tc launch");
+    if ((e = cudaMemcpyAsync(&h, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
+        return cuda_error(ctx, e, "tc result");
+    if (h.overflow) return set_error(ctx, APSPIE_ERR_HASH_OVERFLOW, "apspie_tc: mask set overflow");
+    *count = static_cast<int64_t>(h.count);
+    return APSPIE_OK;
+}
+
+// By bitmaps; an L that turns out not to fit them is counted by hash sets, on the D that was made.
+apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count) {
     const int m = L->m;
     const unsigned nnz = static_cast<unsigned>(L->nnz);
     const size_t mi = static_cast<size_t>(m) + 1, nz = static_cast<size_t>(nnz);
     void *base;
     apspie_status st = scratch_reserve(ctx,
                                        Carver::need({sizeof(TcInfo), mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4,
-                                                     nz * 4, nz * 4, nz * 4, nz * 4, scan_scratch_bytes(m) + 64}),
+                                                     nz * 4, nz * 4, nz * 4, nz * 4, scan_scratch_bytes(m) + 64,
+                                                     TcHashBufs::need(m)}),
                                        &base);
     if (st != APSPIE_OK) return st;
     Carver c(base);
@@ -718,6 +799,7 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
     int *dci = c.take<int>(nz);
     int *plist = c.take<int>(nz);
     void *stmp = c.take<char>(scan_scratch_bytes(m) + 64);
+    const TcHashBufs hash = TcHashBufs::carve(c, m);
     const size_t zeroed = static_cast<size_t>(reinterpret_cast<char *>(partners + mi) - reinterpret_cast<char *>(info));
     cudaError_t e = cudaMemsetAsync(info, 0, zeroed, ctx->stream);  // info, len, partners
     if (e != cudaSuccess) return cuda_error(ctx, e, "tc reset");
@@ -756,14 +838,20 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
         (e = cudaMemcpyAsync(&h, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
         return cuda_error(ctx, e, "tc result");
-    if (h.not_lower || h.unsorted) return APSPIE_OK;
     if (h.overflow) return set_error(ctx, APSPIE_ERR_HASH_OVERFLOW, "apspie_tc: mask set overflow");
-    *count = static_cast<int64_t>(h.count);
-    *counted = true;
-    return APSPIE_OK;
+    if (!h.not_lower && !h.unsorted) {
+        *count = static_cast<int64_t>(h.count);
+        return APSPIE_OK;
+    }
+    if (h.not_lower) {
+        rp = L->row_ptr;
+        ci = L->col_ind;
+    }
+    if ((e = cudaMemsetAsync(info, 0, sizeof(TcInfo), ctx->stream)) != cudaSuccess) return cuda_error(ctx, e, "tc reset");
+    return tc_count_by_hash(ctx, L, rp, ci, false, hash, stmp, info, count);
 }
 
-// The hash path: any L, any size.
+// By hash sets: any L, any size.
 apspie_status tc_by_hash_sets(apspie_ctx *ctx, const apspie_csr *L, int64_t *count) {
     apspie_status st;
     const int m = L->m;
@@ -771,30 +859,26 @@ apspie_status tc_by_hash_sets(apspie_ctx *ctx, const apspie_csr *L, int64_t *cou
     const size_t nz = static_cast<size_t>(L->nnz > 0 ? L->nnz : 1);
     void *base;
     st = scratch_reserve(ctx,
-                         Carver::need({kTcBins * mi * 4, mi * 8, sizeof(TcInfo), mi, mi * 4, mi * 4, mi * 4,
-                                       nz * 4, scan_scratch_bytes(m) + 64, mi * 4, mi * 4, nz * 4, nz * 4}),
+                         Carver::need({TcHashBufs::need(m), sizeof(TcInfo), mi * 4, mi * 4, mi * 4, nz * 4,
+                                       scan_scratch_bytes(m) + 64, nz * 4, nz * 4}),
                          &base);
     if (st != APSPIE_OK) return st;
     Carver c(base);
-    int *bin_rows = c.take<int>(kTcBins * mi);
-    long long *tbl_off = c.take<long long>(mi);
+    const TcHashBufs hash = TcHashBufs::carve(c, m);
     TcInfo *info = c.take<TcInfo>(1);
-    unsigned char *row_bin = c.take<unsigned char>(mi);
     int *deg = c.take<int>(mi);
     int *len = c.take<int>(mi);
     int *drp = c.take<int>(mi);
     int *dci = c.take<int>(nz);
     void *stmp = c.take<char>(scan_scratch_bytes(m) + 64);
-    int *ntask = c.take<int>(mi);
-    int *task_ptr = c.take<int>(mi);
     unsigned *row = c.take<unsigned>(nz);
     int *place = c.take<int>(nz);
     cudaError_t e = cudaMemsetAsync(info, 0, sizeof(TcInfo), ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(len, 0, mi * 4, ctx->stream);
     if (e != cudaSuccess) return cuda_error(ctx, e, "tc reset");
     const int *rp = L->row_ptr, *ci = L->col_ind;
-    const apspie_tune_params tp = effective_params(ctx, APSPIE_TUNE_TC, L);
-    if (m > 0 && L->nnz > 0 && tp.tc_orient) {
+    const bool orient = effective_params(ctx, APSPIE_TUNE_TC, L).tc_orient != 0;
+    if (m > 0 && L->nnz > 0 && orient) {
         // D: L's edges oriented from lower to higher (degree, id) rank
         const unsigned nnz = static_cast<unsigned>(L->nnz);
         const int eb = entry_blocks(ctx, nnz);
@@ -807,56 +891,8 @@ apspie_status tc_by_hash_sets(apspie_ctx *ctx, const apspie_csr *L, int64_t *cou
         rp = drp;
         ci = dci;
     }
-    const int rblocks = std::max(1, std::min<int>((m * 8LL + 255) / 256, ctx->num_sms * 16));
-    const int lblocks = std::max(1, std::min<int>((m + 255LL) / 256, ctx->num_sms * 8));
-    TcInfo h;
-    int ntasks = 0;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-        if (m > 0) {
-            tc_rowinfo<<<rblocks, 256, 0, ctx->stream>>>(m, rp, ci, tp.tc_task_work, row_bin, ntask, tbl_off,
-                                                         info);
-            tc_binlists<<<lblocks, 256, 0, ctx->stream>>>(m, row_bin, bin_rows, info);
-            if ((st = device_exclusive_scan(ctx, ntask, m, task_ptr, stmp, &info->overflow)) != APSPIE_OK) return st;
-            if ((e = cudaMemcpyAsync(&ntasks, task_ptr + m, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream)) !=
-                cudaSuccess)
-                return cuda_error(ctx, e, "tc plan");
-        }
-        if ((e = cudaMemcpyAsync(&h, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
-            return cuda_error(ctx, e, "tc plan");
-        if (!h.not_lower || attempt == 1 || !tp.tc_orient) break;
-        // not a strict lower triangle: count sum((L*L) .* L) on L as given
-        rp = L->row_ptr;
-        ci = L->col_ind;
-        if ((e = cudaMemsetAsync(info, 0, sizeof(TcInfo), ctx->stream)) != cudaSuccess)
-            return cuda_error(ctx, e, "tc reset");
-    }
-    int *gkeys = nullptr;
-    if (h.global_slots > 0) {
-        void *tb;
-        if ((st = scratch2_reserve(ctx, static_cast<size_t>(h.global_slots) * 4 + 256, &tb)) != APSPIE_OK)
-            return st;
-        gkeys = static_cast<int *>(tb);
-    }
-    const int cap = ctx->num_sms * 8;
-    if (ntasks > 0)
-        tc_warp<<<std::min((ntasks + 7) / 8, cap), kTcBlock, 0, ctx->stream>>>(task_ptr, m, ntasks,
-                                                                                 tp.tc_task_work, rp, ci, info);
-    if (h.bin_count[2] > 0)
-        tc_block<false><<<std::min(h.bin_count[2], cap), kTcBlock, 0, ctx->stream>>>(
-            bin_rows + 2 * static_cast<size_t>(m), h.bin_count[2], rp, ci, tbl_off, gkeys, info);
-    if (h.bin_count[3] > 0)
-        tc_block<true><<<std::min(h.bin_count[3], cap), kTcBlock, 0, ctx->stream>>>(
-            bin_rows + 3 * static_cast<size_t>(m), h.bin_count[3], rp, ci, tbl_off, gkeys, info);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(ctx, e, "tc launch");
-    if ((e = cudaMemcpyAsync(&h, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
-        return cuda_error(ctx, e, "tc result");
-    if (h.overflow) return set_error(ctx, APSPIE_ERR_HASH_OVERFLOW, "apspie_tc: mask set overflow");
-    *count = static_cast<int64_t>(h.count);
-    return APSPIE_OK;
+    return tc_count_by_hash(ctx, L, rp, ci, orient, hash, stmp, info, count);
 }
-
 
 }  // namespace
 }  // namespace apspie
@@ -872,11 +908,8 @@ apspie_status apspie_tc(apspie_ctx *ctx, const apspie_csr *L, int64_t *count) {
     if (st != APSPIE_OK) return st;
     if (L->m != L->n) return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_tc: L must be square");
     if (ctx->validate && (st = validate_csr(ctx, L, true)) != APSPIE_OK) return st;
-    if (L->m > 0 && L->nnz > 0 && L->m <= kTcBitmapVertices && L->nnz <= kMaxStepped) {
-        bool counted = false;
-        st = tc_by_bitmaps(ctx, L, count, &counted);
-        if (st != APSPIE_OK || counted) return st;
-    }
+    if (L->m > 0 && L->nnz > 0 && L->m <= kTcBitmapVertices && L->nnz <= kMaxStepped)
+        return tc_by_bitmaps(ctx, L, count);
     return tc_by_hash_sets(ctx, L, count);
 }
 
