@@ -250,7 +250,8 @@ __global__ void sym_row_ptr(int m, const int *__restrict__ up, const int *__rest
         row_ptr[r] = up[r] + low[r];
 }
 
-// The row of every entry: row_of[e], or (KEYS) keys[e] = column << 32 | row. A block takes
+// The row of every entry from `first` on: row_of[e - first], or (KEYS) keys[e - first] = column << 32 |
+// row, for entries before `nnz`. A block takes
 // kExpandTile entries whatever rows they belong to (a warp per row left a row of 50,000
 // entries to one warp): it finds the row of its first entry by a 32-way search, marks where
 // rows begin and spreads the marks by a running maximum. A block whose entries lie so far apart
@@ -260,15 +261,17 @@ constexpr int kExpandSteps = 64;
 constexpr int kExpandItems = 16;
 constexpr int kExpandTile = 256 * kExpandItems;
 template <bool KEYS>
-__global__ void __launch_bounds__(256) expand_rows(int m, long long nnz, const int *__restrict__ rp,
+__global__ void __launch_bounds__(256) expand_rows(int m, long long first, long long nnz, const int *__restrict__ rp,
                                                    const int *__restrict__ ci, unsigned *row_of,
                                                    unsigned long long *keys) {
     __shared__ int s_row[kExpandTile + kExpandTile / 32];  // padded: threads walk 16 entries each
     __shared__ int s_max[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto at = [](int i) { return i + (i >> 5); };
-    const long long t0 = static_cast<long long>(blockIdx.x) * kExpandTile;
+    const long long t0 = first + static_cast<long long>(blockIdx.x) * kExpandTile;
     const long long t1 = t0 + kExpandTile < nnz ? t0 + kExpandTile : nnz;
+    row_of -= first;
+    keys -= first;
     for (int i = tid; i < kExpandTile; i += 256) s_row[at(i)] = -1;
     // last row that begins at or before t0: rp[lo] <= t0 < rp[hi]
     int lo = 0, hi = m;
@@ -356,10 +359,11 @@ __global__ void __launch_bounds__(256) expand_rows(int m, long long nnz, const i
 }
 
 template <bool KEYS>
-cudaError_t launch_expand_rows(apspie_ctx *ctx, const apspie_csr *A, unsigned *row_of, unsigned long long *keys) {
-    if (A->nnz > 0)
-        expand_rows<KEYS><<<(A->nnz + kExpandTile - 1) / kExpandTile, 256, 0, ctx->stream>>>(
-            A->m, A->nnz, A->row_ptr, A->col_ind, row_of, keys);
+cudaError_t launch_expand_rows(apspie_ctx *ctx, const apspie_csr *A, long long first, long long n, unsigned *row_of,
+                               unsigned long long *keys) {
+    if (n > 0)
+        expand_rows<KEYS><<<static_cast<int>((n + kExpandTile - 1) / kExpandTile), 256, 0, ctx->stream>>>(
+            A->m, first, first + n, A->row_ptr, A->col_ind, row_of, keys);
     return cudaGetLastError();
 }
 
@@ -416,7 +420,7 @@ static apspie_status sort_pattern(apspie_ctx *ctx, const apspie_csr *A, SortBufs
     const int n = A->n;
     const RsPlan pl = rs_plan(0, bit_length(n));
     s.v[last_pair(pl.passes)] = reinterpret_cast<unsigned *>(out_col);
-    cudaError_t e = launch_expand_rows<false>(ctx, A, row_of, nullptr);
+    cudaError_t e = launch_expand_rows<false>(ctx, A, 0, nnz, row_of, nullptr);
     if (e != cudaSuccess) return cuda_error(ctx, e, "transpose rows");
     int which = 0;
     apspie_status st =
@@ -445,8 +449,8 @@ apspie_status transpose_pattern(apspie_ctx *ctx, const apspie_csr *A, void *scra
     return st;
 }
 
-apspie_status expand_entry_rows(apspie_ctx *ctx, const apspie_csr *A, unsigned *row_of) {
-    cudaError_t e = launch_expand_rows<false>(ctx, A, row_of, nullptr);
+apspie_status expand_entry_rows(apspie_ctx *ctx, const apspie_csr *A, long long first, long long n, unsigned *row_of) {
+    cudaError_t e = launch_expand_rows<false>(ctx, A, first, n, row_of, nullptr);
     return e == cudaSuccess ? APSPIE_OK : cuda_error(ctx, e, "entry rows");
 }
 
@@ -590,7 +594,7 @@ apspie_status apspie_csr_transpose(apspie_ctx *ctx, const apspie_csr *A, apspie_
         s.v[last_pair(pl.passes)] = static_cast<unsigned *>(out->val);
         err = s.err;
         // the keys are made in the pair that the first pass does not write
-        e = launch_expand_rows<true>(ctx, A, nullptr, s.k[1]);
+        e = launch_expand_rows<true>(ctx, A, 0, nnz, nullptr, s.k[1]);
         if (e == cudaSuccess)
             st = radix_sort(ctx, s, pl, s.k[1], static_cast<const unsigned *>(A->val), nnz, 0, &which);
         if (e == cudaSuccess && st == APSPIE_OK) {

@@ -206,8 +206,8 @@ struct PatternCoo {
 // A's transposed pattern, in scratch of transpose_pattern_need(n, nnz) bytes (build.cu).
 size_t transpose_pattern_need(int n, long long nnz);
 apspie_status transpose_pattern(apspie_ctx *ctx, const apspie_csr *A, void *scratch, PatternCoo *out);
-// row_of[e] = the row of A's entry e.
-apspie_status expand_entry_rows(apspie_ctx *ctx, const apspie_csr *A, unsigned *row_of);
+// row_of[k] = the row of A's entry first + k, for n entries.
+apspie_status expand_entry_rows(apspie_ctx *ctx, const apspie_csr *A, long long first, long long n, unsigned *row_of);
 
 // Device memory (ctx.cu). device_alloc: cudaMalloc, again without the kept blocks of freed matrices
 // when memory is short; every allocation of the library is made by it (and freed by cudaFree).

@@ -367,7 +367,7 @@ apspie_status apspie_pagerank(apspie_ctx *ctx, const apspie_csr *A, float dampin
     cudaError_t e = cudaMemsetAsync(state, 0, sizeof(PrState), ctx->stream);
     if (e != cudaSuccess) return cuda_error(ctx, e, "apspie_pagerank reset");
     PatternCoo in{A->row_ptr, reinterpret_cast<const unsigned *>(mat_base), A->col_ind, nullptr};
-    st = sym ? expand_entry_rows(ctx, A, reinterpret_cast<unsigned *>(mat_base))
+    st = sym ? expand_entry_rows(ctx, A, 0, nnz, reinterpret_cast<unsigned *>(mat_base))
              : transpose_pattern(ctx, A, mat_base, &in);
     if (st != APSPIE_OK) return st;
     const int vblocks = std::max(1, std::min((n + kPrVec - 1) / kPrVec, ctx->num_sms * 4));

@@ -232,7 +232,29 @@ __global__ void tc_out_places(unsigned nnz, const unsigned *__restrict__ row, co
     if (threadIdx.x == 0 && s_beyond) atomicAdd(&info->beyond, s_beyond);
 }
 
-// Writes D (unless D is L as it is: dci null) and, for the bitmap path (partners not null),
+// The same in two passes, for the hash path: the lists' lengths, then D, its places handed out by
+// a second count in `cursor`. Nothing is kept per edge between the two.
+__global__ void tc_out_lengths(unsigned nnz, const unsigned *__restrict__ row, const int *__restrict__ ci,
+                               const int *__restrict__ deg, int *len, const TcInfo *info) {
+    if (info->not_lower) return;
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
+        int a, b;
+        tc_edge(deg, static_cast<int>(__ldg(row + e)), __ldg(ci + e), a, b);
+        atomicAdd(len + a, 1);
+    }
+}
+__global__ void tc_out_lists(unsigned nnz, const unsigned *__restrict__ row, const int *__restrict__ ci,
+                             const int *__restrict__ deg, const int *__restrict__ drp, int *cursor, int *dci,
+                             const TcInfo *info) {
+    if (info->not_lower) return;
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
+        int a, b;
+        tc_edge(deg, static_cast<int>(__ldg(row + e)), __ldg(ci + e), a, b);
+        dci[__ldg(drp + a) + atomicAdd(cursor + a, 1)] = b;
+    }
+}
+
+// Writes D (unless D is L as it is: dci null) and
 // hands out the edge's place in its owner's list of partners; -1 where the shorter list is
 // empty or both are short (tc_small).
 __global__ void tc_owner_places(unsigned nnz, const unsigned *__restrict__ row, const int *__restrict__ ci,
@@ -240,7 +262,7 @@ __global__ void tc_owner_places(unsigned nnz, const unsigned *__restrict__ row, 
                                 int *partners, int m, const TcInfo *info) {
     if (info->not_lower) return;
     if (info->unsorted) partners = nullptr;  // the hash sets count it
-    const int small_list = partners ? tc_small_list(m, nnz, info) : 0;
+    const int small_list = tc_small_list(m, nnz, info);
     for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
         int a, b;
         tc_edge(deg, static_cast<int>(__ldg(row + e)), __ldg(ci + e), a, b);
@@ -774,6 +796,62 @@ apspie_status tc_count_by_hash(apspie_ctx *ctx, const apspie_csr *L, const int *
     return APSPIE_OK;
 }
 
+// By hash sets: any L, any size. Beside D it keeps nothing per entry but the rows of a part of
+// them at a time.
+constexpr long long kTcPart = 1 << 24;
+apspie_status tc_by_hash_sets(apspie_ctx *ctx, const apspie_csr *L, int64_t *count) {
+    apspie_status st;
+    const int m = L->m;
+    const size_t mi = static_cast<size_t>(m) + 1;
+    const size_t nz = static_cast<size_t>(L->nnz > 0 ? L->nnz : 1);
+    const size_t part = std::min(nz, static_cast<size_t>(kTcPart));
+    void *base;
+    st = scratch_reserve(ctx,
+                         Carver::need({TcHashBufs::need(m), sizeof(TcInfo), mi * 4, mi * 4, mi * 4, nz * 4,
+                                       scan_scratch_bytes(m) + 64, part * 4}),
+                         &base);
+    if (st != APSPIE_OK) return st;
+    Carver c(base);
+    const TcHashBufs hash = TcHashBufs::carve(c, m);
+    TcInfo *info = c.take<TcInfo>(1);
+    int *deg = c.take<int>(mi);
+    int *len = c.take<int>(mi);
+    int *drp = c.take<int>(mi);
+    int *dci = c.take<int>(nz);
+    void *stmp = c.take<char>(scan_scratch_bytes(m) + 64);
+    unsigned *row = c.take<unsigned>(part);
+    cudaError_t e = cudaMemsetAsync(info, 0, sizeof(TcInfo), ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(len, 0, mi * 4, ctx->stream);
+    if (e != cudaSuccess) return cuda_error(ctx, e, "tc reset");
+    const int *rp = L->row_ptr, *ci = L->col_ind;
+    const bool orient = effective_params(ctx, APSPIE_TUNE_TC, L).tc_orient != 0;
+    if (m > 0 && L->nnz > 0 && orient) {
+        // D: L's edges oriented from lower to higher (degree, id) rank
+        tc_row_lengths<<<std::min((m + 255) / 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, rp, deg);
+        for (int pass = 0; pass < 3; ++pass) {
+            for (long long first = 0; first < L->nnz; first += kTcPart) {
+                const unsigned n = static_cast<unsigned>(std::min<long long>(kTcPart, L->nnz - first));
+                const int eb = entry_blocks(ctx, n);
+                if ((pass == 0 || L->nnz > kTcPart) && (st = expand_entry_rows(ctx, L, first, n, row)) != APSPIE_OK)
+                    return st;
+                if (pass == 0)
+                    tc_columns<<<std::min(eb, ctx->num_sms * 4), kTcColumnsBlock, 0, ctx->stream>>>(n, m, row, ci + first,
+                                                                                                   deg, info);
+                else if (pass == 1)
+                    tc_out_lengths<<<eb, 256, 0, ctx->stream>>>(n, row, ci + first, deg, len, info);
+                else
+                    tc_out_lists<<<eb, 256, 0, ctx->stream>>>(n, row, ci + first, deg, drp, len, dci, info);
+            }
+            if (pass != 1) continue;
+            if ((st = device_exclusive_scan(ctx, len, m, drp, stmp, &info->overflow)) != APSPIE_OK) return st;
+            if ((e = cudaMemsetAsync(len, 0, mi * 4, ctx->stream)) != cudaSuccess) return cuda_error(ctx, e, "tc reset");
+        }
+        rp = drp;
+        ci = dci;
+    }
+    return tc_count_by_hash(ctx, L, rp, ci, orient, hash, stmp, info, count);
+}
+
 // By bitmaps; an L that turns out not to fit them is counted by hash sets, on the D that was made.
 apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count) {
     const int m = L->m;
@@ -785,6 +863,7 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
                                                      nz * 4, nz * 4, nz * 4, nz * 4, scan_scratch_bytes(m) + 64,
                                                      TcHashBufs::need(m)}),
                                        &base);
+    if (st == APSPIE_ERR_OOM) return tc_by_hash_sets(ctx, L, count);  // a quarter of that an entry
     if (st != APSPIE_OK) return st;
     Carver c(base);
     TcInfo *info = c.take<TcInfo>(1);
@@ -805,7 +884,7 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
     if (e != cudaSuccess) return cuda_error(ctx, e, "tc reset");
     const bool orient = effective_params(ctx, APSPIE_TUNE_TC, L).tc_orient != 0;
     const int eb = entry_blocks(ctx, nnz), vb = std::min((m + 255) / 256, ctx->num_sms * 8);
-    if ((st = expand_entry_rows(ctx, L, row)) != APSPIE_OK) return st;
+    if ((st = expand_entry_rows(ctx, L, 0, nnz, row)) != APSPIE_OK) return st;
     tc_row_lengths<<<vb, 256, 0, ctx->stream>>>(m, L->row_ptr, deg);
     tc_columns<<<std::min(eb, ctx->num_sms * 4), kTcColumnsBlock, 0, ctx->stream>>>(nnz, m, row, L->col_ind, deg, info);
     const int *rp = L->row_ptr, *ci = L->col_ind, *degree = nullptr;
@@ -849,49 +928,6 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
     }
     if ((e = cudaMemsetAsync(info, 0, sizeof(TcInfo), ctx->stream)) != cudaSuccess) return cuda_error(ctx, e, "tc reset");
     return tc_count_by_hash(ctx, L, rp, ci, false, hash, stmp, info, count);
-}
-
-// By hash sets: any L, any size.
-apspie_status tc_by_hash_sets(apspie_ctx *ctx, const apspie_csr *L, int64_t *count) {
-    apspie_status st;
-    const int m = L->m;
-    const size_t mi = static_cast<size_t>(m) + 1;
-    const size_t nz = static_cast<size_t>(L->nnz > 0 ? L->nnz : 1);
-    void *base;
-    st = scratch_reserve(ctx,
-                         Carver::need({TcHashBufs::need(m), sizeof(TcInfo), mi * 4, mi * 4, mi * 4, nz * 4,
-                                       scan_scratch_bytes(m) + 64, nz * 4, nz * 4}),
-                         &base);
-    if (st != APSPIE_OK) return st;
-    Carver c(base);
-    const TcHashBufs hash = TcHashBufs::carve(c, m);
-    TcInfo *info = c.take<TcInfo>(1);
-    int *deg = c.take<int>(mi);
-    int *len = c.take<int>(mi);
-    int *drp = c.take<int>(mi);
-    int *dci = c.take<int>(nz);
-    void *stmp = c.take<char>(scan_scratch_bytes(m) + 64);
-    unsigned *row = c.take<unsigned>(nz);
-    int *place = c.take<int>(nz);
-    cudaError_t e = cudaMemsetAsync(info, 0, sizeof(TcInfo), ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(len, 0, mi * 4, ctx->stream);
-    if (e != cudaSuccess) return cuda_error(ctx, e, "tc reset");
-    const int *rp = L->row_ptr, *ci = L->col_ind;
-    const bool orient = effective_params(ctx, APSPIE_TUNE_TC, L).tc_orient != 0;
-    if (m > 0 && L->nnz > 0 && orient) {
-        // D: L's edges oriented from lower to higher (degree, id) rank
-        const unsigned nnz = static_cast<unsigned>(L->nnz);
-        const int eb = entry_blocks(ctx, nnz);
-        if ((st = expand_entry_rows(ctx, L, row)) != APSPIE_OK) return st;
-        tc_row_lengths<<<std::min((m + 255) / 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m, rp, deg);
-        tc_columns<<<std::min(eb, ctx->num_sms * 4), kTcColumnsBlock, 0, ctx->stream>>>(nnz, m, row, ci, deg, info);
-        tc_out_places<<<eb, 256, 0, ctx->stream>>>(nnz, row, ci, deg, len, place, tc_even_limit(m, nnz), info);
-        if ((st = device_exclusive_scan(ctx, len, m, drp, stmp, &info->overflow)) != APSPIE_OK) return st;
-        tc_owner_places<<<eb, 256, 0, ctx->stream>>>(nnz, row, ci, deg, drp, dci, place, nullptr, m, info);
-        rp = drp;
-        ci = dci;
-    }
-    return tc_count_by_hash(ctx, L, rp, ci, orient, hash, stmp, info, count);
 }
 
 }  // namespace

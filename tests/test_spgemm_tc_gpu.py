@@ -400,3 +400,44 @@ def test_tc_of_low_degrees_takes_little_time(ctx):
         seconds.append(time.perf_counter() - t0)
     # 0.7 ms, where a block's round for each vertex made it 13
     assert min(seconds) < 4e-3, seconds
+
+
+def _joined_halves(rows, cols):
+    """`rows` vertices that meet all of the first `cols`, of which the first two meet: rows triangles."""
+    m = rows + cols
+    deg = np.zeros(m, dtype=np.int64)
+    deg[1] = 1
+    deg[cols:] = cols
+    rp = np.concatenate(([0], np.cumsum(deg))).astype(np.int32)
+    ci = np.concatenate(([0], np.tile(np.arange(cols), rows))).astype(np.int32)
+    return ap.HostGraph(m, m, rp, ci)
+
+
+def test_tc_when_memory_is_short(ctx):
+    """Where the bitmap path's scratch (16 bytes an entry) does not fit, the hash path's (4) does."""
+    import torch
+
+    g = ap.DeviceGraph(_joined_halves(8000, 2000))
+    with ap.Context(0) as c:
+        ctx.trim()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        rest = torch.empty(free - (200 << 20), dtype=torch.uint8, device="cuda")
+        assert torch.cuda.mem_get_info()[0] < 230 << 20
+        assert c.tc(g) == 8000
+        assert c.scratch_bytes() < 200 << 20
+        del rest
+    torch.cuda.empty_cache()
+    assert ctx.tc(g) == 8000
+
+
+@pytest.mark.parametrize("rows,cols", [(2100, 4000), (9000, 1865)])
+def test_tc_hash_path_in_parts(ctx, rows, cols):
+    """More vertices than the bitmaps take, and more entries than a part of the hash path (2^24):
+    the orientation is made part by part."""
+    g = _joined_halves(rows, cols)
+    m = 1_700_000
+    rp = np.concatenate((g.row_ptr, np.full(m - g.m, g.row_ptr[-1], dtype=np.int32)))
+    assert (g.nnz > 1 << 24) == (rows == 9000)
+    assert ctx.tc(ap.DeviceGraph(ap.HostGraph(m, m, rp, g.col_ind))) == rows
