@@ -339,8 +339,14 @@ apspie_status apspie_autotune(apspie_ctx *ctx, int32_t kind, const apspie_csr *A
         break;
     }
     case APSPIE_TUNE_TC: {
+        // only what is counted by hash sets has tasks: a size chosen among equal times is none
+        int64_t first = 0;
+        const apspie_status st = apspie_tc(ctx, A, &first);
+        if (st != APSPIE_OK) return st;
+        std::vector<int> sizes{saved.tc_task_work};
+        if (!ctx->tc_by_bitmaps) sizes = {1024, 2048, 4096, 8192, 16384};
         for (int o : {1, 0})
-            for (int tw : {1024, 2048, 4096, 8192, 16384})
+            for (int tw : sizes)
                 with([&](apspie_tune_params &p) {
                     p.tc_orient = o;
                     p.tc_task_work = tw;

@@ -123,6 +123,7 @@ struct apspie_ctx {
     unsigned long long wait_limit_ns = 0;  // grid-barrier wait bound (0: kBarrierTimeoutNs)
     unsigned long long *h_limit = nullptr;  // pinned copy of it, the source of the per-call upload
     std::vector<apspie_tune_entry> tune_table;
+    bool tc_by_bitmaps = false;  // how the last triangle count was made
     unsigned long long cuda_ctx_id = 0;  // the CUDA context it was made in (0: unknown)
 };
 

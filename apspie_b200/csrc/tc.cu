@@ -919,6 +919,7 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
         return cuda_error(ctx, e, "tc result");
     if (h.overflow) return set_error(ctx, APSPIE_ERR_HASH_OVERFLOW, "apspie_tc: mask set overflow");
     if (!h.not_lower && !h.unsorted) {
+        ctx->tc_by_bitmaps = true;
         *count = static_cast<int64_t>(h.count);
         return APSPIE_OK;
     }
@@ -944,6 +945,7 @@ apspie_status apspie_tc(apspie_ctx *ctx, const apspie_csr *L, int64_t *count) {
     if (st != APSPIE_OK) return st;
     if (L->m != L->n) return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_tc: L must be square");
     if (ctx->validate && (st = validate_csr(ctx, L, true)) != APSPIE_OK) return st;
+    ctx->tc_by_bitmaps = false;
     if (L->m > 0 && L->nnz > 0 && L->m <= kTcBitmapVertices && L->nnz <= kMaxStepped)
         return tc_by_bitmaps(ctx, L, count);
     return tc_by_hash_sets(ctx, L, count);

@@ -189,7 +189,8 @@ apspie_status apspie_ctx_set_autotune(apspie_ctx *ctx, int32_t use);
  * BFS/SSSP: A and host `sources[0]`; BFS_BATCH: A and `nsources` host sources; SPGEMM:
  * A and B; TC: A = strict lower triangle. Output buffers are allocated for the duration
  * of the call. Candidates: BFS alpha x beta; SSSP band sizes; batched BFS push fraction;
- * SpGEMM register-tier limit x shared-table limit; TC task size x orientation. */
+ * SpGEMM register-tier limit x shared-table limit; TC orientation, and task size where hash
+ * sets count (else the context's is kept). */
 apspie_status apspie_autotune(apspie_ctx *ctx, int32_t kind, const apspie_csr *A, const apspie_csr *B,
                               const int32_t *sources, int32_t nsources, int32_t reps,
                               apspie_tune_params *best, double *best_ms);

@@ -146,3 +146,19 @@ def test_set_params_rejects_out_of_range(ctx):
         with pytest.raises(ap.ApspieError):
             ctx.set_params(**knobs)
     assert ctx.get_params()["spgemm_reg_max"] == 128
+
+
+def test_autotune_tc_keeps_the_task_size_that_bitmaps_do_not_use():
+    """Task sizes are tried where the hash sets count: among equal times none is chosen."""
+    with ap.Context(0) as c:
+        c.set_params(tc_task_work=333)
+        for scale in (8, 9, 10):
+            Ld = c.strict_lower(ap.DeviceGraph(ap.gen_rmat(scale, 16, 1, 3, weights=False)))
+            best, _ = c.autotune(ap.TUNE_TC, Ld, reps=1)
+            assert best["tc_task_work"] == 333
+            assert c.tune_lookup(ap.TUNE_TC, Ld)[0]["tc_task_work"] == 333
+            Ld.free()
+        # a whole symmetric pattern is the hash sets': one of the sizes
+        full = ap.DeviceGraph(ap.gen_rmat(10, 16, 1, 3, weights=False))
+        best, _ = c.autotune(ap.TUNE_TC, full, reps=1)
+        assert best["tc_task_work"] in (1024, 2048, 4096, 8192, 16384)
