@@ -46,26 +46,24 @@ struct TravBuffers {
     unsigned *bits0, *bits1;
 };
 
-size_t trav_scratch_bytes(int m) {
+// Int arrays of m + 1 that a call uses of these (a new context's first call is mostly their
+// allocation): BFS, SSSP, SSSP with far piles.
+constexpr int kBfsLists = 6, kSsspLists = 7, kSsspPileLists = 9;
+
+size_t trav_scratch_bytes(int m, int lists) {
     const size_t words = (static_cast<size_t>(m) + 31) / 32;
-    const size_t mi = static_cast<size_t>(m) + 1;
-    return Carver::need({mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, mi * 4, words * 4, words * 4});
+    size_t n = Carver::need({words * 4, words * 4});
+    for (int k = 0; k < lists; ++k) n += Carver::need({(static_cast<size_t>(m) + 1) * 4});
+    return n;
 }
 
-TravBuffers carve_trav(void *base, int m) {
+TravBuffers carve_trav(void *base, int m, int lists) {
     const size_t words = (static_cast<size_t>(m) + 31) / 32;
-    const size_t mi = static_cast<size_t>(m) + 1;
     Carver c(base);
-    TravBuffers b;
-    b.q0 = c.take<int>(mi);
-    b.q1 = c.take<int>(mi);
-    b.q2 = c.take<int>(mi);
-    b.q3 = c.take<int>(mi);
-    b.rs = c.take<int>(mi);
-    b.loc_off = c.take<int>(mi);
-    b.aux = c.take<int>(mi);
-    b.aux2 = c.take<int>(mi);
-    b.aux3 = c.take<int>(mi);
+    TravBuffers b{};
+    int **const bfs[] = {&b.q0, &b.q1, &b.q2, &b.q3, &b.rs, &b.loc_off};
+    int **const sssp[] = {&b.q0, &b.q1, &b.rs, &b.loc_off, &b.aux, &b.aux2, &b.aux3, &b.q2, &b.q3};
+    for (int k = 0; k < lists; ++k) *(lists == kBfsLists ? bfs : sssp)[k] = c.take<int>(static_cast<size_t>(m) + 1);
     b.bits0 = c.take<unsigned>(words);
     b.bits1 = c.take<unsigned>(words);
     return b;
@@ -304,7 +302,7 @@ struct SsspArgs {
     const int *__restrict__ w;
     int *dist;
     // bits0 = queued in the near frontier, bits1 = held in the far pile;
-    // q0/q1 near queues (vertices), q2/q3 far piles; rs, loc_off, aux3 = the edge queue of the
+    // q0/q1 near queues (vertices), q2/q3 far piles (if any); rs, loc_off, aux3 = the edge queue of the
     // entries expanded this iteration (off, delta, owner), aux = their distances;
     // aux2 = distance each vertex was last expanded with
     TravBuffers buf;
@@ -1364,7 +1362,7 @@ cudaError_t noalloc_scratch(void **out) {
 
 }  // namespace
 
-size_t traversal_scratch_need(int m) { return trav_scratch_bytes(m); }
+size_t traversal_scratch_need(int m) { return trav_scratch_bytes(m, kSsspLists); }
 
 // Pull levels need a symmetric pattern, and step past a row's end in an int.
 int bfs_may_pull(const apspie_csr *A) { return (A->flags & APSPIE_CSR_SYMMETRIC) && A->nnz <= kMaxStepped; }
@@ -1385,7 +1383,7 @@ size_t mis_scratch_need(int m) {
 
 apspie_status trav_reserve(apspie_ctx *ctx, int m) {
     void *base;
-    return scratch_reserve(ctx, std::max(trav_scratch_bytes(m) + static_cast<size_t>(m) * 5 + 512, mis_scratch_need(m)),
+    return scratch_reserve(ctx, std::max(trav_scratch_bytes(m, kSsspPileLists) + static_cast<size_t>(m) * 5 + 512, mis_scratch_need(m)),
                            &base);
 }
 
@@ -1412,7 +1410,7 @@ apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, i
         return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_bfs: source out of range");
     if (!d_depth) return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_bfs: NULL output");
     void *base;
-    st = scratch_reserve(ctx, trav_scratch_bytes(A->m), &base);
+    st = scratch_reserve(ctx, trav_scratch_bytes(A->m, kBfsLists), &base);
     if (st != APSPIE_OK) return st;
     if ((st = reset_ctl(ctx)) != APSPIE_OK) return st;
     BfsArgs a;
@@ -1423,7 +1421,7 @@ apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, i
     a.row_ptr = A->row_ptr;
     a.col_ind = A->col_ind;
     a.depth = d_depth;
-    set_bfs_buffers(a, carve_trav(base, A->m), A->m, A->nnz);
+    set_bfs_buffers(a, carve_trav(base, A->m, kBfsLists), A->m, A->nnz);
     a.ctl = ctx->d_ctl;
     a.sticky = ctx->d_sticky_err;
     const apspie_tune_params tp = effective_params(ctx, APSPIE_TUNE_BFS, A);
@@ -1485,6 +1483,9 @@ long long default_band(long long nnz) {
     return b < (1LL << 16) ? (1LL << 16) : (b > (1LL << 23) ? (1LL << 23) : b);
 }
 
+// A far pile is kept with a step, or without a band (as the kernel decides).
+int sssp_lists(const SsspArgs &a) { return a.delta_hint > 0 || a.band <= 0 ? kSsspPileLists : kSsspLists; }
+
 apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, void *d_dist,
                           apspie_run_stats *stats, bool is_float, int unreached_bits) {
     cudaSetDevice(ctx->device);
@@ -1494,10 +1495,6 @@ apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, 
     if (source < 0 || source >= A->m)
         return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_sssp: source out of range");
     if (!d_dist) return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_sssp: NULL output");
-    void *base;
-    st = scratch_reserve(ctx, trav_scratch_bytes(A->m), &base);
-    if (st != APSPIE_OK) return st;
-    if ((st = reset_ctl(ctx)) != APSPIE_OK) return st;
     SsspArgs a;
     a.m = A->m;
     a.nnz = A->nnz;
@@ -1515,8 +1512,13 @@ apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, 
     } else {
         a.band = 0;
     }
+    void *base;
+    const int lists = sssp_lists(a);
+    st = scratch_reserve(ctx, trav_scratch_bytes(A->m, lists), &base);
+    if (st != APSPIE_OK) return st;
+    if ((st = reset_ctl(ctx)) != APSPIE_OK) return st;
     a.unreached_bits = unreached_bits;
-    a.buf = carve_trav(base, A->m);
+    a.buf = carve_trav(base, A->m, lists);
     a.shift = edge_unit_shift(A->nnz, static_cast<long long>(A->m) + 1, 32 * kSsspVT);
     a.ctl = ctx->d_ctl;
     a.sticky = ctx->d_sticky_err;
@@ -1529,7 +1531,7 @@ apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, 
 }  // namespace
 
 size_t sssp_group_scratch_need(int m, int groups) {
-    const size_t per = (trav_scratch_bytes(m) + 255) / 256 * 256;
+    const size_t per = (trav_scratch_bytes(m, kSsspPileLists) + 255) / 256 * 256;
     return per * static_cast<size_t>(groups) + static_cast<size_t>(groups) * ((sizeof(TravCtl) + 255) / 256 * 256);
 }
 
@@ -1554,7 +1556,7 @@ apspie_status sssp_batch_grouped(apspie_ctx *ctx, const apspie_csr *A, const int
     apspie_status st = scratch_reserve(ctx, sssp_group_scratch_need(m, groups), &base);
     if (st != APSPIE_OK) return st;
     if ((st = reset_ctl(ctx)) != APSPIE_OK) return st;
-    const size_t per = (trav_scratch_bytes(m) + 255) / 256 * 256;
+    const size_t per = (trav_scratch_bytes(m, kSsspPileLists) + 255) / 256 * 256;
     TravCtl *ctls = reinterpret_cast<TravCtl *>(static_cast<char *>(base) + per * groups);
     if ((e = cudaMemsetAsync(ctls, 0, groups * ((sizeof(TravCtl) + 255) / 256 * 256), ctx->stream)) != cudaSuccess)
         return cuda_error(ctx, e, "apspie_sssp_batch reset");
@@ -1578,7 +1580,7 @@ apspie_status sssp_batch_grouped(apspie_ctx *ctx, const apspie_csr *A, const int
         a.band = 0;
     }
     a.unreached_bits = -1;
-    a.buf = carve_trav(base, m);
+    a.buf = carve_trav(base, m, kSsspPileLists);
     a.shift = edge_unit_shift(A->nnz, static_cast<long long>(m) + 1, 32 * kSsspVT);
     a.sticky = ctx->d_sticky_err;
     g.srcs = d_sources;

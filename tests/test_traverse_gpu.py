@@ -553,3 +553,25 @@ def test_sssp_edge_queue_shapes(ctx, shape, kind):
     finally:
         ctx.set_sssp_band(0)
         ctx.set_sssp_delta(0)
+
+
+def test_a_first_call_reserves_what_it_uses(ctx):
+    """A new context's scratch: int arrays of m + 1 entries and two bitmaps, an eighth more as
+    headroom. Six arrays for a BFS, seven for an SSSP, nine with far piles."""
+    import torch
+
+    m = 1 << 18
+    rp = np.zeros(m + 1, dtype=np.int32)
+    rp[1:] = 1
+    g = ap.DeviceGraph(ap.HostGraph(m, m, rp, np.array([1], dtype=np.int32), np.array([3], dtype=np.int32)))
+
+    def bound(lists):
+        return (lists * 4 * (m + 1 + 64) + 2 * (m // 8 + 256)) * 9 // 8 + 4096
+
+    for lists, call in ((6, lambda c: c.bfs(g, 0)), (7, lambda c: c.sssp(g, 0)),
+                        (9, lambda c: (c.set_sssp_delta(5), c.sssp(g, 0))[1]),
+                        (9, lambda c: (c.set_sssp_band(-1), c.sssp(g, 0))[1])):
+        with ap.Context(0) as c:
+            out = call(c).cpu().numpy()
+            assert bound(lists - 1) < c.scratch_bytes() <= bound(lists), lists
+            assert out[0] == 0 and out[1] in (1, 3) and (out[2:] == -1).all()
