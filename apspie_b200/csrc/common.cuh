@@ -87,6 +87,10 @@ struct apspie_tune_entry {
     double ms;
 };
 
+namespace apspie {
+constexpr size_t kPinnedBytes = 64;
+}
+
 struct apspie_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -104,7 +108,7 @@ struct apspie_ctx {
     apspie::TravCtl *d_ctl = nullptr;
     apspie::TravCtl *h_ctl = nullptr;
     int *d_sticky_err = nullptr;  // errors of asynchronous calls, read by synchronize
-    int *h_word = nullptr;        // pinned scratch word for small device->host reads
+    int *h_word = nullptr;        // kPinnedBytes of pinned memory for small device->host reads
     int validate = 0;
     float bfs_alpha = 14.0f;
     float bfs_beta = 24.0f;

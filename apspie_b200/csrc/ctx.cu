@@ -294,7 +294,7 @@ apspie_status apspie_ctx_create(int device, void *cuda_stream, apspie_ctx **out)
     bool ok = device_alloc(reinterpret_cast<void **>(&ctx->d_ctl), sizeof(TravCtl)) == cudaSuccess &&
               device_alloc(reinterpret_cast<void **>(&ctx->d_sticky_err), sizeof(int)) == cudaSuccess &&
               cudaMallocHost(&ctx->h_ctl, sizeof(TravCtl)) == cudaSuccess &&
-              cudaMallocHost(&ctx->h_word, 64) == cudaSuccess &&
+              cudaMallocHost(&ctx->h_word, kPinnedBytes) == cudaSuccess &&
               cudaMallocHost(&ctx->h_limit, 64) == cudaSuccess &&
               cudaMemset(ctx->d_sticky_err, 0, sizeof(int)) == cudaSuccess &&
               cudaMemset(ctx->d_ctl, 0, sizeof(TravCtl)) == cudaSuccess;

@@ -805,9 +805,12 @@ apspie_status sg_plan(apspie_ctx *ctx, const apspie_csr *A, const apspie_csr *B,
         sg_binlists<<<lblocks, 256, 0, ctx->stream>>>(m, p.row_bin, p.bin_rows, p.info);
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(ctx, e, "spgemm rowinfo");
     }
-    e = cudaMemcpyAsync(&p.h, p.info, sizeof(SgInfo), cudaMemcpyDeviceToHost, ctx->stream);
+    // into pinned memory (a copy to pageable memory is waited for by itself)
+    static_assert(sizeof(SgInfo) <= kPinnedBytes, "room");
+    e = cudaMemcpyAsync(ctx->h_word, p.info, sizeof(SgInfo), cudaMemcpyDeviceToHost, ctx->stream);
     if (e != cudaSuccess) return cuda_error(ctx, e, "spgemm info copy");
     if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return cuda_error(ctx, e, "spgemm sync");
+    std::memcpy(&p.h, ctx->h_word, sizeof(SgInfo));
     // global-tier hash tables live in the context's secondary arena
     const size_t gslots = static_cast<size_t>(p.h.global_slots);
     p.gkeys = nullptr;
@@ -899,14 +902,14 @@ apspie_status sg_symbolic(apspie_ctx *ctx, const apspie_csr *A, const apspie_csr
         st = sg_run<false, int>(ctx, A, B, p, nullptr, nullptr, nullptr);
     if (st != APSPIE_OK) return st;
     if ((st = device_exclusive_scan(ctx, p.cnt, m, crp, p.scan_tmp, &p.info->overflow)) != APSPIE_OK) return st;
-    int tail[2] = {0, 0};
-    cudaError_t e = cudaMemcpyAsync(&tail[0], crp + m, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    cudaError_t e = cudaMemcpyAsync(ctx->h_word, crp + m, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&p.h.overflow, &p.info->overflow, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+        e = cudaMemcpyAsync(ctx->h_word + 1, &p.info->overflow, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_error(ctx, e, "spgemm symbolic sync");
+    p.h.overflow = ctx->h_word[1];
     if (p.h.overflow) return set_error(ctx, APSPIE_ERR_HASH_OVERFLOW, "spgemm: hash table or nnz(C) overflow");
-    *nnz = tail[0];
+    *nnz = ctx->h_word[0];
     return APSPIE_OK;
 }
 
