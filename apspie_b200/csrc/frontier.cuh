@@ -415,9 +415,11 @@ __device__ __forceinline__ P ld_payload(const P *p) {
 // ints and payloads; units are at least a tile. A block has every nblocks-th unit and its warps take
 // them in turn (`claim`: in shared memory, zero at first): units differ in their rows and in what
 // they improve, and with a fixed share per warp the blocks waited for their slowest warps (SSSP
-// scale 20 558 -> 534 us, batched SSSP 8.75 -> 8.03 ms, BFS 60.1 -> 58.9 us). (Fetching the next tile's entries, columns and weights
+// scale 20 558 -> 534 us, batched SSSP 8.75 -> 8.03 ms, BFS 60.1 -> 58.9 us). WIDE: E may be more
+// than kMaxStepped (a plain step is up to 1 % faster in BFS and SSSP, the other one 4 % in batched
+// SSSP). (Fetching the next tile's entries, columns and weights
 // while one is worked on made SSSP slower: 650 us against 619 us at scale 20.)
-template <int VT, class P, class Op>
+template <int VT, bool WIDE, class P, class Op>
 __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const P *payload, int nf, int E, int shift,
                                             int *slice, int *claim, int block, int nblocks, Op op) {
     constexpr int TILE = 32 * VT;
@@ -439,8 +441,8 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const P *payload
         const bool one = u + 1 < units && __ldcg(q.owner + u + 1) == k;
         const long long uend = (static_cast<long long>(u) + 1) << shift;
         const int end = uend < E ? static_cast<int>(uend) : E;
-        for (int t0 = u << shift, t1; t0 < end; t0 = t1) {
-            t1 = step_end(t0, TILE, end);
+        for (int t0 = u << shift, t1; t0 < end; t0 = WIDE ? t1 : t0 + TILE) {
+            t1 = WIDE ? step_end(t0, TILE, end) : min(t0 + TILE, end);
             unsigned begin[VT];
 #pragma unroll
             for (int r = 0; r < VT; ++r) begin[r] = 0u;
@@ -480,8 +482,8 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const P *payload
                 const int x = r * 32 + lane;  // behind t0
                 const int i = before + __popc(begin[r] & upto);
                 before += __popc(begin[r]);
-                valid[r] = x < t1 - t0;
-                idx[r] = valid[r] ? t0 + x + slice[i] : 0;
+                valid[r] = WIDE ? x < t1 - t0 : t < t1;
+                idx[r] = valid[r] ? t + slice[i] : 0;
                 pay[r] = PAY && valid[r] ? pslice[i] : P{};
             }
             op(valid, pay, idx);

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kSbBlock, 5) sssp_batch_kernel(SbArgs a) {
         TravCtl *ctl = a.ctl;
         int *sticky = a.sticky;
         EdgeQueue qe{a.off, a.delta, a.owner, nullptr, nullptr};
-        edge_expand<kSbVT>(
+        edge_expand<kSbVT, true>(
             qe, a.ent, ne, E, a.shift, sh.slice[wid], &sh.claim[iters & 1], blockIdx.x, G,
             [&](const bool (&valid)[kSbVT], const uint2 (&src)[kSbVT], const int (&idx)[kSbVT]) {
                 // the tile's edges as records: target entry (v, w), weight + 1, source entry and

@@ -119,6 +119,7 @@ struct BfsArgs {
 // lengths, two barriers a level and frontier bitmaps: 43.9 / 113 us; now 31 / 63 us. Blocks
 // of 256 threads, three an SM: four an SM 36 / 65 us, 512 threads 38 / 65 us, 128 threads
 // 34 / 68 us (fewer blocks make the barrier cheaper, more warps the pull levels).
+template <bool WIDE>
 __global__ void __launch_bounds__(kBfsBlock, 3) bfs_kernel(BfsArgs a) {
     __shared__ int s_buf[kBfsBlock / 32][kEqCap];
     __shared__ int s_slice[kBfsBlock / 32][kEqTile];
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_kernel(BfsArgs a) {
             // while few vertices are visited, claiming at once saves a trip to L2 per level; later
             // most neighbours are visited and a look spares the atomic
             const bool look = reached * 16 > m;
-            edge_expand<4>(qc, static_cast<const NoPayload *>(nullptr), nq, E, a.shift, s_slice[wid],
+            edge_expand<4, WIDE>(qc, static_cast<const NoPayload *>(nullptr), nq, E, a.shift, s_slice[wid],
                            &s_claim[L & 1], blockIdx.x, gridDim.x,
                         [&](const bool (&valid)[4], const NoPayload (&)[4], const int (&idx)[4]) {
                             int v[4];
@@ -373,7 +374,7 @@ struct SsspShared {
 // between batches, and every entry read in full each iteration, 709 us; edge queues 619 us;
 // reading only the distance of deferred entries and queueing per block 571 us; five blocks
 // per SM 553 us. Two, six or eight edges per lane instead of four: 596 / 623 / 580 us.
-template <bool F>
+template <bool F, bool WIDE>
 __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
     static_assert(kBlock == kBandBins, "one histogram bin per thread");
     __shared__ SsspShared sh;
@@ -633,7 +634,7 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
         WQ wf(sh.far[wid], fcur, &a.ctl->flen[fc]);
         bool bad = false, over = false;
         EdgeQueue qa{a.buf.rs, a.buf.loc_off, a.buf.aux3, nullptr, nullptr};
-        edge_expand<kSsspVT>(
+        edge_expand<kSsspVT, WIDE>(
             qa, snap, nact, E, a.shift, sh.slice[wid], &sh.claim[iters & 1], vg.id, G,
             [&](const bool (&valid)[kSsspVT], const int (&du)[kSsspVT], const int (&idx)[kSsspVT]) {
                 int v[kSsspVT], we[kSsspVT], cd[kSsspVT], nd[kSsspVT];
@@ -771,10 +772,10 @@ __device__ __forceinline__ void sssp_body(SsspArgs a, VGrid vg) {
     }
 }
 
-template <bool F>
+template <bool F, bool WIDE>
 __global__ void __launch_bounds__(kBlock, 5) sssp_kernel(SsspArgs a) {
     grid_begin(a.ctl);
-    sssp_body<F>(a, hw_grid());
+    sssp_body<F, WIDE>(a, hw_grid());
 }
 
 // Many sources in one launch: the grid splits into `groups` equal groups of blocks, each
@@ -827,7 +828,7 @@ __global__ void __launch_bounds__(kBlock, 5) sssp_group_kernel(SsspGroupArgs g) 
             continue;
         }
         a.dist = g.out + static_cast<size_t>(q) * g.m;
-        sssp_body<false>(a, vg);
+        sssp_body<false, true>(a, vg);
         // every block of the group is done with the control block before it is reset
         if (!grid_barrier(ctl, a.sticky, kSiteSsspGroup, vg)) break;
         if (tid == 0) {
@@ -1366,6 +1367,10 @@ size_t traversal_scratch_need(int m) { return trav_scratch_bytes(m, kSsspLists);
 
 // Pull levels need a symmetric pattern, and step past a row's end in an int.
 int bfs_may_pull(const apspie_csr *A) { return (A->flags & APSPIE_CSR_SYMMETRIC) && A->nnz <= kMaxStepped; }
+const void *bfs_fn(const apspie_csr *A) {
+    return A->nnz <= kMaxStepped ? reinterpret_cast<const void *>(bfs_kernel<false>)
+                                 : reinterpret_cast<const void *>(bfs_kernel<true>);
+}
 
 // Blocks of a BFS launch, one to three an SM: more shorten a level's expansion, fewer its barrier
 // and its queue (a block's reservations are made one after the other). R-MAT, one / two / three:
@@ -1429,7 +1434,7 @@ apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, i
     a.beta = tp.bfs_beta;
     a.allow_pull = bfs_may_pull(A);
     void *args[] = {&a};
-    st = launch_persistent(ctx, reinterpret_cast<const void *>(bfs_kernel), kBfsBlock, args,
+    st = launch_persistent(ctx, bfs_fn(A), kBfsBlock, args,
                            bfs_blocks(ctx->num_sms, A->nnz) * kWorkPerBlock);
     if (st != APSPIE_OK) return st;
     return finish_call(ctx, stats, "apspie_bfs");
@@ -1523,8 +1528,12 @@ apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, 
     a.ctl = ctx->d_ctl;
     a.sticky = ctx->d_sticky_err;
     void *args[] = {&a};
-    st = launch_persistent(ctx, is_float ? reinterpret_cast<const void *>(sssp_kernel<true>) : reinterpret_cast<const void *>(sssp_kernel<false>),
-                           kBlock, args, sssp_blocks(ctx, A->nnz) * kWorkPerBlock);
+    const bool wide = A->nnz > kMaxStepped;
+    const void *fn = is_float ? wide ? reinterpret_cast<const void *>(sssp_kernel<true, true>)
+                                     : reinterpret_cast<const void *>(sssp_kernel<true, false>)
+                     : wide   ? reinterpret_cast<const void *>(sssp_kernel<false, true>)
+                              : reinterpret_cast<const void *>(sssp_kernel<false, false>);
+    st = launch_persistent(ctx, fn, kBlock, args, sssp_blocks(ctx, A->nnz) * kWorkPerBlock);
     if (st != APSPIE_OK) return st;
     return finish_call(ctx, stats, "apspie_sssp");
 }
@@ -1692,14 +1701,14 @@ apspie_status apspie_bfs_noalloc(const apspie_csr *A, int32_t source, int32_t de
     a.allow_pull = bfs_may_pull(A);
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_kernel, kBfsBlock, 0) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_fn(A), kBfsBlock, 0) != cudaSuccess ||
         per_sm < 1)
         return APSPIE_ERR_CUDA;
     long long grid = bfs_blocks(sms, A->nnz);
     if (grid > static_cast<long long>(per_sm) * sms) grid = static_cast<long long>(per_sm) * sms;
     if (grid > kMaxGrid) grid = kMaxGrid;
     void *args[] = {&a};
-    if (cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(bfs_kernel), dim3(static_cast<int>(grid)),
+    if (cudaLaunchCooperativeKernel(bfs_fn(A), dim3(static_cast<int>(grid)),
                                     dim3(kBfsBlock), args, 0, stream) != cudaSuccess) {
         (void)cudaGetLastError();
         return APSPIE_ERR_CUDA;
