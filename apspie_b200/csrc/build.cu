@@ -384,13 +384,13 @@ int grid_for(const apspie_ctx *ctx, long long n) {
 // Row starts out of n sorted keys.
 template <class K>
 void launch_starts(apspie_ctx *ctx, long long n, const K *keys, int shift, K fmask, int m, int *start, const int *err) {
-    const int g = grid_for(ctx, std::max<long long>(n, m + 1ll));
+    const int gm = grid_for(ctx, m + 1ll);
     if (n < m) {
-        search_starts<K><<<g, 256, 0, ctx->stream>>>(n, keys, shift, fmask, m, start, err);
+        search_starts<K><<<gm, 256, 0, ctx->stream>>>(n, keys, shift, fmask, m, start, err);
         return;
     }
-    run_starts<K><<<g, 256, 0, ctx->stream>>>(n, keys, shift, fmask, start, err);
-    fill_tail<K><<<g, 256, 0, ctx->stream>>>(n, keys, shift, fmask, m, start, err);
+    if (n > 0) run_starts<K><<<grid_for(ctx, n), 256, 0, ctx->stream>>>(n, keys, shift, fmask, start, err);
+    fill_tail<K><<<gm, 256, 0, ctx->stream>>>(n, keys, shift, fmask, m, start, err);
 }
 
 apspie_status alloc_owned(apspie_ctx *ctx, int m, int n, long long nnz, int val_type, apspie_csr_owned *out) {

@@ -717,6 +717,15 @@ int entry_blocks(const apspie_ctx *ctx, unsigned nnz) {
     return static_cast<int>(std::min<long long>((static_cast<long long>(nnz) + 255) / 256, ctx->num_sms * 16LL));
 }
 
+// *info by way of pinned memory (a copy to pageable memory is waited for by itself).
+cudaError_t read_info(apspie_ctx *ctx, const TcInfo *info, TcInfo &h) {
+    static_assert(sizeof(TcInfo) <= kPinnedBytes, "room");
+    cudaError_t e = cudaMemcpyAsync(ctx->h_word, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) std::memcpy(&h, ctx->h_word, sizeof(TcInfo));
+    return e;
+}
+
 // What counting by hash sets takes beside D, and a scan's scratch.
 struct TcHashBufs {
     int *bin_rows;
@@ -760,8 +769,7 @@ apspie_status tc_count_by_hash(apspie_ctx *ctx, const apspie_csr *L, const int *
                 cudaSuccess)
                 return cuda_error(ctx, e, "tc plan");
         }
-        if ((e = cudaMemcpyAsync(&h, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
+        if ((e = read_info(ctx, info, h)) != cudaSuccess)
             return cuda_error(ctx, e, "tc plan");
         if (!h.not_lower || attempt == 1 || !check) break;
         // not a strict lower triangle: count sum((L*L) .* L) on L as given
@@ -788,8 +796,7 @@ apspie_status tc_count_by_hash(apspie_ctx *ctx, const apspie_csr *L, const int *
         tc_block<true><<<std::min(h.bin_count[3], cap), kTcBlock, 0, ctx->stream>>>(
             b.bin_rows + 3 * static_cast<size_t>(m), h.bin_count[3], rp, ci, b.tbl_off, gkeys, info);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(ctx, e, "tc launch");
-    if ((e = cudaMemcpyAsync(&h, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
+    if ((e = read_info(ctx, info, h)) != cudaSuccess)
         return cuda_error(ctx, e, "tc result");
     if (h.overflow) return set_error(ctx, APSPIE_ERR_HASH_OVERFLOW, "apspie_tc: mask set overflow");
     *count = static_cast<int64_t>(h.count);
@@ -914,8 +921,7 @@ apspie_status tc_by_bitmaps(apspie_ctx *ctx, const apspie_csr *L, int64_t *count
     tc_bits<<<std::max(per_sm, 1) * ctx->num_sms, threads, smem, ctx->stream>>>(m, list, rp, ci, prp, plist, info);
     TcInfo h;
     if ((e = cudaGetLastError()) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&h, info, sizeof(TcInfo), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
+        (e = read_info(ctx, info, h)) != cudaSuccess)
         return cuda_error(ctx, e, "tc result");
     if (h.overflow) return set_error(ctx, APSPIE_ERR_HASH_OVERFLOW, "apspie_tc: mask set overflow");
     if (!h.not_lower && !h.unsorted) {
