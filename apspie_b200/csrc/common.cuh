@@ -437,19 +437,6 @@ __device__ __forceinline__ unsigned long long block_inclusive_scan_u64(unsigned 
     return tmp[wid] + incl;
 }
 
-// Warp-aggregated append of `v` to queue `q` for lanes with pred set. All 32 lanes of
-// the warp must call it.
-__device__ __forceinline__ void warp_append(bool pred, int v, int *q, int *qlen) {
-    unsigned mask = __ballot_sync(0xffffffffu, pred);
-    if (mask == 0) return;
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(mask) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(qlen, __popc(mask));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (pred) q[base + __popc(mask & ((1u << lane) - 1u))] = v;
-}
-
 // Per-warp staging buffer for queue appends: entries collect in shared memory and one
 // atomicAdd on the queue length reserves room for up to QCAP of them at a time, instead
 // of one contended global atomic per warp step. `count` is warp-uniform (a register of

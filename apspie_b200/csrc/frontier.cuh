@@ -34,13 +34,12 @@ template <int WT>
 struct WarpSlice {
     int off[WT + 1];   // global edge offset of each staged entry
     int rs[WT + 1];    // CSR row start of each staged entry
-    int aux[WT + 1];   // per-entry payloads
-    int aux2[WT + 1];
-    int flag[WT + 1];  // per-entry accumulator flushed after the tile
+    int aux[WT + 1];   // per-entry payload
     int seg[WT];       // tile edge slot -> staged entry
 };
 
-template <int BLOCK, int VT>
+// ROOM: ints that the kernel uses a warp's slice for otherwise, outside the expansion.
+template <int BLOCK, int VT, int ROOM = 1>
 struct ExpandSmem {
     static constexpr int NWARP = BLOCK / 32;
     static constexpr int WT = 32 * VT;  // items (entries + edges) per warp tile
@@ -52,7 +51,10 @@ struct ExpandSmem {
     int tsplit[BATCH + 1];   // merge-path split of each warp tile of the current batch
     int next_tile;           // tiles of the batch handed out so far (warps take them in turn)
     int scan_tmp[33];
-    Warp w[NWARP];
+    union Slice {
+        Warp w;
+        int room[ROOM];
+    } w[NWARP];
 };
 
 // Phase A over this block's chunk of queue q[0, nf). hook(i, v, deg) may rewrite the
@@ -144,15 +146,13 @@ __device__ __forceinline__ int frontier_merge_path(long long diag, int nf, int E
 
 // Phase B. load(j, k, ws) stages entry j's payload into the warp slice at k;
 // op(valid, k, idx, ws) handles a lane's VT edges (CSR positions idx[], owning staged
-// entries k[]); post(ne, ws) runs after the tile's edges (per-entry flushes). All three
-// are called by every lane of the warp, so they may use warp collectives. Warps claim
-// the tiles of their block's batch in turn.
-template <int BLOCK, int VT, class Load, class Op, class Post>
+// entries k[]). Both are called by every lane of the warp, so they may use warp collectives.
+// Warps claim the tiles of their block's batch in turn.
+template <int BLOCK, int VT, int ROOM, class Load, class Op>
 __device__ __forceinline__ void frontier_expand(int nf, int E, const int *__restrict__ loc_off,
                                                 const int *__restrict__ rs,
-                                                ExpandSmem<BLOCK, VT> &sm, Load load, Op op,
-                                                Post post) {
-    using S = ExpandSmem<BLOCK, VT>;
+                                                ExpandSmem<BLOCK, VT, ROOM> &sm, Load load, Op op) {
+    using S = ExpandSmem<BLOCK, VT, ROOM>;
     constexpr int WT = S::WT;
     constexpr int NWARP = S::NWARP;
     constexpr int BATCH = S::BATCH;
@@ -162,7 +162,7 @@ __device__ __forceinline__ void frontier_expand(int nf, int E, const int *__rest
     const long long ntiles = (total + WT - 1) / WT;
     const int lane = threadIdx.x & 31;
     const int wid = threadIdx.x >> 5;
-    typename S::Warp &ws = sm.w[wid];
+    typename S::Warp &ws = sm.w[wid].w;
     // one warp tile: stage its entries, label its edge slots, run the operation
     auto run_tile = [&](long long tile, long long tb) {
         const long long d0 = tile * WT;
@@ -227,7 +227,6 @@ __device__ __forceinline__ void frontier_expand(int nf, int E, const int *__rest
         }
         op(valid, kk, idx, ws);
         __syncwarp();
-        post(ne, ws);
     };
     // the tiles [tb, te) of one batch: split points found together, then the warps
     auto run_batch = [&](long long tb, long long te) {
@@ -479,7 +478,7 @@ __device__ __forceinline__ void edge_expand(const EdgeQueue &q, const P *payload
             int before = -1;
 #pragma unroll
             for (int r = 0; r < VT; ++r) {
-                const int x = r * 32 + lane;  // behind t0
+                const int x = r * 32 + lane, t = static_cast<int>(static_cast<Pos>(t0) + x);  // past 2^31: not valid
                 const int i = before + __popc(begin[r] & upto);
                 before += __popc(begin[r]);
                 valid[r] = WIDE ? x < t1 - t0 : t < t1;

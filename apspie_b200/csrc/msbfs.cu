@@ -38,9 +38,12 @@ namespace {
 
 constexpr int kMsBlock = 256;
 constexpr int kMsVT = 4;
-using MsSmem = ExpandSmem<kMsBlock, kMsVT>;
-using MsWarp = MsSmem::Warp;
-using MsWQ = WarpQueue<MsSmem::QCAP>;
+// A warp's slice of the expander holds, in pull levels, the W words of 32 rows scanned by groups
+// (padded by one) and the list of those rows.
+template <int W>
+using MsSmem = ExpandSmem<kMsBlock, kMsVT, 32 * (W + 1) + 32>;
+using MsWarp = MsSmem<1>::Warp;
+using MsWQ = WarpQueue<MsSmem<1>::QCAP>;
 
 enum : int { kSiteMs = 400, kSiteMsBadSource = 450 };
 // Pull: rows of at most kLaneDeg neighbours are scanned by a lane (up to 128 queries), of at
@@ -453,7 +456,7 @@ __device__ void write_depths(const MsArgs &a, long long mw) {
 
 template <int W, bool SERVE>
 __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_kernel(MsArgs a) {
-    __shared__ MsSmem sm;
+    __shared__ MsSmem<W> sm;
     __shared__ unsigned s_qmask[W];   // query slots in flight this level
     __shared__ int s_claim[2];        // pull tiles taken by the block's warps, by level parity
     __shared__ unsigned s_alive[W];   // bits this block found in the next frontier (engine)
@@ -638,7 +641,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
             const int *qc = a.q[cur];
             unsigned *vis = a.vis;
             unsigned *touched = a.touched;
-            frontier_expand<kMsBlock, kMsVT>(
+            frontier_expand(
                 nA, E, a.loc_off, a.rs, sm, [&](int j, int k, MsWarp &ws) { ws.aux[k] = __ldcg(qc + j); },
                 [&](const bool (&valid)[kMsVT], const int (&kk)[kMsVT], const int (&idx)[kMsVT], MsWarp &ws) {
                     int v[kMsVT];
@@ -667,8 +670,7 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
                         }
                         tw.push(add, v[r]);
                     }
-                },
-                [](int, MsWarp &) {});
+                });
             tw.flush();
             if (!grid_barrier(a.ctl, a.sticky, kSiteMs + 4)) return;
             // finalize the touched vertices
@@ -709,10 +711,8 @@ __global__ void __launch_bounds__(kMsBlock, W >= 16 ? 3 : W <= 2 ? 5 : 4) msbfs_
             constexpr int LQ = PullShape<W>::LQ, VW = PullShape<W>::VW;
             constexpr unsigned FULL = 0xffffffffu;
             unsigned *frw = a.fr[(L + 1) & 1];
-            // the expander's slice of this warp holds the results of rows scanned by groups
-            static_assert(sizeof(MsWarp) >= 32 * (W + 1) * 4 + 32 * 4, "a warp's results fit its slice");
-            unsigned *s_got = reinterpret_cast<unsigned *>(&sm.w[wid]);
-            int *s_list = reinterpret_cast<int *>(s_got + 32 * (W + 1));
+            unsigned *s_got = reinterpret_cast<unsigned *>(sm.w[wid].room);
+            int *s_list = sm.w[wid].room + 32 * (W + 1);
             // the block's warps take its vertices in turn, 32 at a time (with a fixed share per
             // warp 1,386 us instead of 1,322 for 32 sources on 4.2M vertices, 1,082 instead of
             // 1,029 for 64 on 2.1M)
