@@ -3,7 +3,8 @@
 // (spmspv.cu). One read of the keys counts every pass's digits; a pass then reads and
 // writes each pair once: its tiles are taken in order from a ticket, each ranks its keys in
 // input order with warp match masks, publishes its digit counts, adds up the counts of the
-// tiles before it (decoupled look-back), reorders the tile by digit in shared memory and
+// tiles before it (decoupled look-back: Merrill and Garland, "Single-pass Parallel Prefix Scan
+// with Decoupled Look-back", 2016), reorders the tile by digit in shared memory and
 // writes every digit's run with consecutive threads.
 //
 // Measured over 16.8M pairs of 12 bytes (0.40 GB, 61 us at the copy rate): 138 us a pass;

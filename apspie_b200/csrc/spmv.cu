@@ -67,8 +67,9 @@ apspie_status launch_spmv(apspie_ctx *ctx, const apspie_csr *A, const float *x, 
 // pr_gather cuts the entries, not the rows, into equal chunks: a thread takes 8 consecutive
 // entries (two 128-bit loads), sums the pieces of rows in them, and a segmented scan joins
 // pieces across threads. A chunk writes the sums of the rows that begin in it; what it holds
-// of a row that began earlier goes to carry[], which pr_update adds in chunk order, so
-// repeated calls give the same bits. Bound: 4 bytes an entry from HBM plus one gather from
+// of a row that began earlier goes to carry[], which pr_update adds in chunk order: a row's sum has
+// the same bits in repeated calls (the dangling mass and the change are added up by atomics, so the
+// ranks' last bits may differ). Bound: 4 bytes an entry from HBM plus one gather from
 // L2. Measured, R-MAT of 700,001 vertices and 10.7M entries, per iteration: 16 lanes per
 // row 228 us (the row of 55,000 entries is the last to finish) + 34 us for the two vector
 // kernels, whose warps all added doubles to one word; now see pr_update.

@@ -116,7 +116,7 @@ struct BfsArgs {
 // What bounds it: at scale 14 the chain of dependent L2 reads in a level (queue, entry,
 // column, visited word, claim, row length, reservation) and its barrier; at scale 20 the pull
 // levels' gathers. Kernel time at scale 14 / 20 with a phase that scanned the frontier's row
-// lengths, two barriers a level and frontier bitmaps: 43.9 / 113 us; now 31 / 63 us. Blocks
+// lengths, two barriers a level and frontier bitmaps: 43.9 / 113 us; now 30 / 59 us. Blocks
 // of 256 threads, three an SM: four an SM 36 / 65 us, 512 threads 38 / 65 us, 128 threads
 // 34 / 68 us (fewer blocks make the barrier cheaper, more warps the pull levels).
 template <bool WIDE>

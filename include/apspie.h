@@ -162,10 +162,11 @@ typedef struct apspie_tune_params {
     int32_t sssp_delta;       /* SSSP far-pile step (<= 0: none with the band, else device-chosen) */
     int64_t sssp_band;        /* SSSP edges per iteration (0 auto, < 0 whole frontier) */
     int32_t spgemm_reg_max;   /* SpGEMM rows with at most this many products (0, 32, 64 or 128)
-                                 are sorted by one warp in registers */
+                                 are sorted by 8 or 16 lanes in registers */
     int32_t spgemm_block_max; /* larger rows up to this many products (<= 1024) use a block's
-                                 shared-memory hash table; longer rows a global table */
-    int32_t tc_task_work;     /* triangle counting: wedges per warp task (>= 256) */
+                                 shared-memory hash table; longer rows a dense accumulator in
+                                 shared memory (C of at most 49,152 columns) or a global table */
+    int32_t tc_task_work;     /* triangle counting by hash sets: wedges per warp task (>= 256) */
     int32_t tc_orient;        /* triangle counting: 1 = re-orient L by degree first */
     int32_t reserved[4];
 } apspie_tune_params;
@@ -380,9 +381,11 @@ apspie_status apspie_pagerank(apspie_ctx *ctx, const apspie_csr *A, float dampin
                               float *d_rank, int32_t *iterations);
 
 /* Triangle count = sum((L*L) .* L) for L the strict lower triangle (column < row) of a
- * symmetric graph, rows sorted; masked hash SpGEMM, L*L never materialised; int64 result
- * (synchronises). Replaces the flow of test/tc/main.cu:243-249 (spgemm<T> tc.cuh:63 ->
- * ewiseMultTc tc.cuh:169 -> mgpu::Reduce). */
+ * symmetric graph, rows sorted; L*L never materialised; int64 result (synchronises). Up to
+ * 1,638,400 vertices the rows' bitmaps and small hash sets are intersected; larger graphs, and
+ * rows that do not ascend strictly or reach the diagonal, are counted as a masked hash SpGEMM.
+ * Replaces the flow of test/tc/main.cu:243-249 (spgemm<T> tc.cuh:63 -> ewiseMultTc tc.cuh:169 ->
+ * mgpu::Reduce). */
 apspie_status apspie_tc(apspie_ctx *ctx, const apspie_csr *L, int64_t *count);
 /* Strict lower triangle of a square CSR on the device (buildLower, test/tc/main.cu:39-55,
  * in CSR); library-allocated, release with apspie_csr_free. Values are dropped. */
