@@ -171,7 +171,7 @@ apspie_status launch_persistent(apspie_ctx *ctx, const void *func, int block, vo
 apspie_status finish_call(apspie_ctx *ctx, apspie_run_stats *stats, const char *who);
 
 // Scratch bytes the entry points reserve in a context's arena (for admission control).
-size_t traversal_scratch_need(int m);        // apspie_bfs / apspie_sssp
+size_t traversal_scratch_need(int m, long long nnz);  // apspie_bfs / apspie_sssp
 size_t mis_scratch_need(int m);              // apspie_mis
 size_t bfs_batch_scratch_need(int m, int nq);  // apspie_bfs_batch (nq <= 512 per launch)
 // apspie_bfs_batch into per-query rows h_rows[q] (host array of device pointers) when
@@ -194,9 +194,9 @@ unsigned long long bfs_engine_waiting(const BfsEngine *e);
 void bfs_engine_set_accept(BfsEngine *e, int on);
 std::vector<unsigned long long> bfs_engine_take_back(BfsEngine *e);  // untaken ring entries (launch ended)
 apspie_status bfs_engine_launch(apspie_ctx *ctx, const apspie_csr *A, int W, BfsEngine *e);
-size_t sssp_batch_scratch_need(int m, int nq);  // apspie_sssp_batch (nq <= 512 per launch)
+size_t sssp_batch_scratch_need(int m, long long nnz, int nq);  // apspie_sssp_batch (nq <= 512 per launch)
 // apspie_sssp_batch in query groups (each group of blocks runs single-source SSSPs)
-size_t sssp_group_scratch_need(int m, int groups);
+size_t sssp_group_scratch_need(int m, long long nnz, int groups);
 int sssp_group_count(const apspie_ctx *ctx, int nq);
 apspie_status sssp_batch_grouped(apspie_ctx *ctx, const apspie_csr *A, const int32_t *d_sources, int32_t nq,
                                  int32_t *d_dists, apspie_run_stats *stats);

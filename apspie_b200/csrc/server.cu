@@ -197,9 +197,9 @@ MinBatch min_batch(const apspie_server *s, const apspie_csr &g) {
 // Scratch a launch reserves in the slot's arena (a BFS batch runs on the engine).
 size_t arena_need(const apspie_csr &g, int kind, int n, MinBatch mb) {
     if (kind == APSPIE_QUERY_MIS) return mis_scratch_need(g.m);
-    if (!batched(kind, n, mb)) return traversal_scratch_need(g.m);
+    if (!batched(kind, n, mb)) return traversal_scratch_need(g.m, g.nnz);
     return kind == APSPIE_QUERY_BFS ? bfs_engine_scratch_need(g.m, bfs_engine_words(n))
-                                    : sssp_batch_scratch_need(g.m, n);
+                                    : sssp_batch_scratch_need(g.m, g.nnz, n);
 }
 
 // Batched SSSP launches stage their n rows before copying them out (the BFS engine writes
@@ -756,14 +756,19 @@ apspie_status apspie_server_start(apspie_server *s) {
     // device synchronisation) while requests wait; else the single-query need, and
     // launches then grow it only as far as the budget lets them
     int32_t mmax = 0;
-    for (auto &g : s->graphs) mmax = std::max(mmax, g.view.m);
-    size_t full = traversal_scratch_need(mmax), single = traversal_scratch_need(mmax);
+    size_t full = traversal_scratch_need(0, 0);
+    for (auto &g : s->graphs) {
+        mmax = std::max(mmax, g.view.m);
+        full = std::max(full, traversal_scratch_need(g.view.m, g.view.nnz));
+    }
+    size_t single = full;
     if (mmax > 0) {
         full = std::max(full, mis_scratch_need(mmax));
         single = std::max(single, mis_scratch_need(mmax));
         full = std::max(full, bfs_engine_scratch_need(mmax, bfs_engine_words(s->max_batch)));
         const int fold = std::min(s->sssp_fold, s->max_batch);
-        if (fold > 1) full = std::max(full, sssp_batch_scratch_need(mmax, fold));
+        for (auto &g : s->graphs)
+            if (fold > 1) full = std::max(full, sssp_batch_scratch_need(g.view.m, g.view.nnz, fold));
     }
     if (s->graph_bytes + (single + single / 8) * s->slots.size() > static_cast<size_t>(s->budget))
         return APSPIE_ERR_OOM;

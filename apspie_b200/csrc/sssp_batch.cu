@@ -329,13 +329,19 @@ __global__ void __launch_bounds__(256) sb_unpack(const unsigned *__restrict__ la
 
 }  // namespace
 
-size_t sssp_batch_scratch_need(int m, int nq) {
+// Scratch of a launch on mw (vertex, query word) pairs and so many entries of their rows.
+static size_t multi_need(size_t mw, long long edges) {
+    return Carver::need({mw * 128, mw * 4, mw * 4, mw * 8, mw * 4, mw * 4,
+                         static_cast<size_t>(edge_owner_slots(static_cast<long long>(mw) + 1, edges)) * 4});
+}
+
+size_t sssp_batch_scratch_need(int m, long long nnz, int nq) {
     const int W = ((nq < 512 ? nq : 512) + 31) / 32;
     const size_t mw = static_cast<size_t>(m) * (W > 0 ? W : 1);
     const size_t multi =
-        Carver::need({mw * 128, mw * 4, mw * 4, mw * 8, mw * 4, mw * 4, mw * 4 + 4});
+        multi_need(mw, nnz * (W > 0 ? W : 1));
     // the grouped form (groups > 0): at most 4 groups are costed here
-    const size_t grouped = sssp_group_scratch_need(m, std::max(1, std::min(nq, 4)));
+    const size_t grouped = sssp_group_scratch_need(m, nnz, std::max(1, std::min(nq, 4)));
     return std::max(multi, grouped);
 }
 
@@ -370,7 +376,7 @@ extern "C" apspie_status apspie_sssp_batch(apspie_ctx *ctx, const apspie_csr *A,
         const size_t mw = static_cast<size_t>(m) * W;
         void *base;
         st = scratch_reserve(
-            ctx, Carver::need({mw * 128, mw * 4, mw * 4, mw * 8, mw * 4, mw * 4, mw * 4 + 4}),
+            ctx, multi_need(mw, static_cast<long long>(A->nnz) * W),
             &base);
         if (st != APSPIE_OK) return st;
         Carver c(base);
@@ -381,8 +387,9 @@ extern "C" apspie_status apspie_sssp_batch(apspie_ctx *ctx, const apspie_csr *A,
         a.ent = c.take<uint2>(mw);
         a.off = c.take<int>(mw);
         a.delta = c.take<int>(mw);
-        a.owner = c.take<int>(mw + 1);
-        a.shift = edge_unit_shift(static_cast<long long>(A->nnz) * W, static_cast<long long>(mw) + 1, kSbTile);
+        const long long slots = edge_owner_slots(static_cast<long long>(mw) + 1, static_cast<long long>(A->nnz) * W);
+        a.owner = c.take<int>(static_cast<size_t>(slots));
+        a.shift = edge_unit_shift(static_cast<long long>(A->nnz) * W, slots, kSbTile);
         a.m = m;
         a.nnz = A->nnz;
         a.nq = nq;

@@ -46,24 +46,34 @@ struct TravBuffers {
     unsigned *bits0, *bits1;
 };
 
-// Int arrays of m + 1 that a call uses of these (a new context's first call is mostly their
-// allocation): BFS, SSSP, SSSP with far piles.
-constexpr int kBfsLists = 6, kSsspLists = 7, kSsspPileLists = 9;
+// What a call uses of these (a new context's first call is mostly their allocation): int arrays
+// of m + 1, the last of them (two of BFS's, one of SSSP's) with room for the owners of an edge
+// queue's units.
+struct TravLists {
+    int arrays, owners;
+};
+constexpr TravLists kBfsLists{4, 2}, kSsspLists{6, 1}, kSsspPileLists{8, 1};
 
-size_t trav_scratch_bytes(int m, int lists) {
-    const size_t words = (static_cast<size_t>(m) + 31) / 32;
-    size_t n = Carver::need({words * 4, words * 4});
-    for (int k = 0; k < lists; ++k) n += Carver::need({(static_cast<size_t>(m) + 1) * 4});
-    return n;
+size_t trav_scratch_bytes(int m, long long nnz, TravLists lists) {
+    const size_t words = (static_cast<size_t>(m) + 31) / 32, mi = static_cast<size_t>(m) + 1;
+    return Carver::need({words * 4, words * 4}) + lists.arrays * Carver::need({mi * 4}) +
+           lists.owners * Carver::need({static_cast<size_t>(edge_owner_slots(m + 1ll, nnz)) * 4});
 }
 
-TravBuffers carve_trav(void *base, int m, int lists) {
-    const size_t words = (static_cast<size_t>(m) + 31) / 32;
+TravBuffers carve_trav(void *base, int m, long long nnz, TravLists lists) {
+    const size_t words = (static_cast<size_t>(m) + 31) / 32, mi = static_cast<size_t>(m) + 1;
+    const size_t slots = static_cast<size_t>(edge_owner_slots(m + 1ll, nnz));
     Carver c(base);
     TravBuffers b{};
-    int **const bfs[] = {&b.q0, &b.q1, &b.q2, &b.q3, &b.rs, &b.loc_off};
-    int **const sssp[] = {&b.q0, &b.q1, &b.rs, &b.loc_off, &b.aux, &b.aux2, &b.aux3, &b.q2, &b.q3};
-    for (int k = 0; k < lists; ++k) *(lists == kBfsLists ? bfs : sssp)[k] = c.take<int>(static_cast<size_t>(m) + 1);
+    if (lists.owners == kBfsLists.owners) {
+        for (int **p : {&b.q0, &b.q1, &b.q2, &b.q3}) *p = c.take<int>(mi);
+        for (int **p : {&b.rs, &b.loc_off}) *p = c.take<int>(slots);
+    } else {
+        for (int **p : {&b.q0, &b.q1, &b.rs, &b.loc_off, &b.aux, &b.aux2}) *p = c.take<int>(mi);
+        b.aux3 = c.take<int>(slots);
+        if (lists.arrays == kSsspPileLists.arrays)
+            for (int **p : {&b.q2, &b.q3}) *p = c.take<int>(mi);
+    }
     b.bits0 = c.take<unsigned>(words);
     b.bits1 = c.take<unsigned>(words);
     return b;
@@ -71,7 +81,7 @@ TravBuffers carve_trav(void *base, int m, int lists) {
 
 // BFS's view of the buffers: edge queues in q0-q3, rs and loc_off, visited bitmaps in bits0-1.
 struct BfsArgs;
-void set_bfs_buffers(BfsArgs &a, const TravBuffers &b, int m, int nnz);
+void set_bfs_buffers(BfsArgs &a, const TravBuffers &b, int nnz, long long slots);
 
 // ================================================================================
 // BFS
@@ -1283,12 +1293,12 @@ __global__ void spmspv_bool_kernel(int m, const int *__restrict__ row_ptr,
     }
 }
 
-void set_bfs_buffers(BfsArgs &a, const TravBuffers &b, int m, int nnz) {
+void set_bfs_buffers(BfsArgs &a, const TravBuffers &b, int nnz, long long slots) {
     a.q[0] = EdgeQueue{b.q0, b.q2, b.rs, nullptr, nullptr};
     a.q[1] = EdgeQueue{b.q1, b.q3, b.loc_off, nullptr, nullptr};
     a.vis[0] = b.bits0;
     a.vis[1] = b.bits1;
-    a.shift = edge_unit_shift(nnz, static_cast<long long>(m) + 1, kEqTile);
+    a.shift = edge_unit_shift(nnz, slots, kEqTile);
 }
 
 apspie_status prepare_square(apspie_ctx *ctx, const apspie_csr *A, const char *who) {
@@ -1363,7 +1373,7 @@ cudaError_t noalloc_scratch(void **out) {
 
 }  // namespace
 
-size_t traversal_scratch_need(int m) { return trav_scratch_bytes(m, kSsspLists); }
+size_t traversal_scratch_need(int m, long long nnz) { return trav_scratch_bytes(m, nnz, kSsspLists); }
 
 // Pull levels need a symmetric pattern, and step past a row's end in an int.
 int bfs_may_pull(const apspie_csr *A) { return (A->flags & APSPIE_CSR_SYMMETRIC) && A->nnz <= kMaxStepped; }
@@ -1386,9 +1396,9 @@ size_t mis_scratch_need(int m) {
     return Carver::need({static_cast<size_t>(m), l, l, l});
 }
 
-apspie_status trav_reserve(apspie_ctx *ctx, int m) {
+apspie_status trav_reserve(apspie_ctx *ctx, int m, long long nnz) {
     void *base;
-    return scratch_reserve(ctx, std::max(trav_scratch_bytes(m, kSsspPileLists) + static_cast<size_t>(m) * 5 + 512, mis_scratch_need(m)),
+    return scratch_reserve(ctx, std::max(trav_scratch_bytes(m, nnz, kSsspPileLists) + static_cast<size_t>(m) * 5 + 512, mis_scratch_need(m)),
                            &base);
 }
 
@@ -1399,10 +1409,9 @@ using namespace apspie;
 extern "C" {
 
 apspie_status apspie_ctx_reserve(apspie_ctx *ctx, int32_t m, int64_t nnz) {
-    (void)nnz;
     if (!ctx || m < 0) return APSPIE_ERR_INVALID_ARG;
     cudaSetDevice(ctx->device);
-    return trav_reserve(ctx, m);
+    return trav_reserve(ctx, m, std::max<long long>(0, nnz));
 }
 
 apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, int32_t depth_cap,
@@ -1415,7 +1424,7 @@ apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, i
         return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_bfs: source out of range");
     if (!d_depth) return set_error(ctx, APSPIE_ERR_INVALID_ARG, "apspie_bfs: NULL output");
     void *base;
-    st = scratch_reserve(ctx, trav_scratch_bytes(A->m, kBfsLists), &base);
+    st = scratch_reserve(ctx, trav_scratch_bytes(A->m, A->nnz, kBfsLists), &base);
     if (st != APSPIE_OK) return st;
     if ((st = reset_ctl(ctx)) != APSPIE_OK) return st;
     BfsArgs a;
@@ -1426,7 +1435,7 @@ apspie_status apspie_bfs(apspie_ctx *ctx, const apspie_csr *A, int32_t source, i
     a.row_ptr = A->row_ptr;
     a.col_ind = A->col_ind;
     a.depth = d_depth;
-    set_bfs_buffers(a, carve_trav(base, A->m, kBfsLists), A->m, A->nnz);
+    set_bfs_buffers(a, carve_trav(base, A->m, A->nnz, kBfsLists), A->nnz, edge_owner_slots(A->m + 1ll, A->nnz));
     a.ctl = ctx->d_ctl;
     a.sticky = ctx->d_sticky_err;
     const apspie_tune_params tp = effective_params(ctx, APSPIE_TUNE_BFS, A);
@@ -1489,7 +1498,7 @@ long long default_band(long long nnz) {
 }
 
 // A far pile is kept with a step, or without a band (as the kernel decides).
-int sssp_lists(const SsspArgs &a) { return a.delta_hint > 0 || a.band <= 0 ? kSsspPileLists : kSsspLists; }
+TravLists sssp_lists(const SsspArgs &a) { return a.delta_hint > 0 || a.band <= 0 ? kSsspPileLists : kSsspLists; }
 
 apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, void *d_dist,
                           apspie_run_stats *stats, bool is_float, int unreached_bits) {
@@ -1518,13 +1527,13 @@ apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, 
         a.band = 0;
     }
     void *base;
-    const int lists = sssp_lists(a);
-    st = scratch_reserve(ctx, trav_scratch_bytes(A->m, lists), &base);
+    const TravLists lists = sssp_lists(a);
+    st = scratch_reserve(ctx, trav_scratch_bytes(A->m, A->nnz, lists), &base);
     if (st != APSPIE_OK) return st;
     if ((st = reset_ctl(ctx)) != APSPIE_OK) return st;
     a.unreached_bits = unreached_bits;
-    a.buf = carve_trav(base, A->m, lists);
-    a.shift = edge_unit_shift(A->nnz, static_cast<long long>(A->m) + 1, 32 * kSsspVT);
+    a.buf = carve_trav(base, A->m, A->nnz, lists);
+    a.shift = edge_unit_shift(A->nnz, edge_owner_slots(A->m + 1ll, A->nnz), 32 * kSsspVT);
     a.ctl = ctx->d_ctl;
     a.sticky = ctx->d_sticky_err;
     void *args[] = {&a};
@@ -1539,8 +1548,8 @@ apspie_status sssp_common(apspie_ctx *ctx, const apspie_csr *A, int32_t source, 
 }
 }  // namespace
 
-size_t sssp_group_scratch_need(int m, int groups) {
-    const size_t per = (trav_scratch_bytes(m, kSsspPileLists) + 255) / 256 * 256;
+size_t sssp_group_scratch_need(int m, long long nnz, int groups) {
+    const size_t per = (trav_scratch_bytes(m, nnz, kSsspPileLists) + 255) / 256 * 256;
     return per * static_cast<size_t>(groups) + static_cast<size_t>(groups) * ((sizeof(TravCtl) + 255) / 256 * 256);
 }
 
@@ -1562,10 +1571,10 @@ apspie_status sssp_batch_grouped(apspie_ctx *ctx, const apspie_csr *A, const int
     const int groups = std::min(sssp_group_count(ctx, nq), cap);
     const int bpg = std::min(cap / groups, kMaxGrid);
     void *base;
-    apspie_status st = scratch_reserve(ctx, sssp_group_scratch_need(m, groups), &base);
+    apspie_status st = scratch_reserve(ctx, sssp_group_scratch_need(m, A->nnz, groups), &base);
     if (st != APSPIE_OK) return st;
     if ((st = reset_ctl(ctx)) != APSPIE_OK) return st;
-    const size_t per = (trav_scratch_bytes(m, kSsspPileLists) + 255) / 256 * 256;
+    const size_t per = (trav_scratch_bytes(m, A->nnz, kSsspPileLists) + 255) / 256 * 256;
     TravCtl *ctls = reinterpret_cast<TravCtl *>(static_cast<char *>(base) + per * groups);
     if ((e = cudaMemsetAsync(ctls, 0, groups * ((sizeof(TravCtl) + 255) / 256 * 256), ctx->stream)) != cudaSuccess)
         return cuda_error(ctx, e, "apspie_sssp_batch reset");
@@ -1589,8 +1598,8 @@ apspie_status sssp_batch_grouped(apspie_ctx *ctx, const apspie_csr *A, const int
         a.band = 0;
     }
     a.unreached_bits = -1;
-    a.buf = carve_trav(base, m, kSsspPileLists);
-    a.shift = edge_unit_shift(A->nnz, static_cast<long long>(m) + 1, 32 * kSsspVT);
+    a.buf = carve_trav(base, m, A->nnz, kSsspPileLists);
+    a.shift = edge_unit_shift(A->nnz, edge_owner_slots(m + 1ll, A->nnz), 32 * kSsspVT);
     a.sticky = ctx->d_sticky_err;
     g.srcs = d_sources;
     g.out = d_dists;
@@ -1685,7 +1694,7 @@ apspie_status apspie_bfs_noalloc(const apspie_csr *A, int32_t source, int32_t de
     }
     b.bits0 = reinterpret_cast<unsigned *>(p);
     b.bits1 = reinterpret_cast<unsigned *>(p + kNaWordsBytes);
-    set_bfs_buffers(a, b, A->m, A->nnz);
+    set_bfs_buffers(a, b, A->nnz, static_cast<long long>(kNaMaxV) + 1);
     if (cudaMemsetAsync(ctl, 0, kNaCtlBytes, stream) != cudaSuccess) return APSPIE_ERR_CUDA;
     a.m = A->m;
     a.nnz = A->nnz;
