@@ -399,6 +399,32 @@ def test_mis_int32_layout(ctx, rmat14):
     np.testing.assert_array_equal(out.cpu().numpy(), oracle.mis_greedy(g.row_ptr, g.col_ind, pr).astype(np.int32))
 
 
+@pytest.mark.parametrize("prio", ["up", "down", "random"])
+@pytest.mark.parametrize("shape", ["complete 2", "complete 33", "complete 140", "complete 1030", "complete 2100",
+                                   "even 4735", "even 4737", "even 23679", "even 47361", "even 94721"])
+def test_mis_dense_graphs_and_small_tiles(ctx, shape, prio):
+    """Vertices that a push puts out while a warp or the block still scans their rows (complete graphs: a
+    warp's step and more, more than a warp takes), and vertices around the sizes at which tiles shrink."""
+    import torch
+
+    kind, _, size = shape.partition(" ")
+    m = int(size)
+    if kind == "complete":
+        src, dst = np.repeat(np.arange(m), m), np.tile(np.arange(m), m)
+    else:
+        rng = np.random.default_rng(6)
+        src, dst = rng.integers(0, m, 5 * m), rng.integers(0, m, 5 * m)
+    edges = np.unique(np.concatenate((src * m + dst, dst * m + src))[np.concatenate((src, src)) != np.concatenate((dst, dst))])
+    rp = np.concatenate(([0], np.cumsum(np.bincount(edges // m, minlength=m)))).astype(np.int32)
+    ci = (edges % m).astype(np.int32)
+    pr = {"up": np.arange(m), "down": np.arange(m)[::-1], "random": ap.mt19937_u32(7, m)}[prio].astype(np.uint32)
+    dg = ap.DeviceGraph(ap.HostGraph(m, m, rp, ci, None, True))
+    ref = oracle.mis_greedy(rp, ci, pr)
+    dpr = torch.from_numpy(pr.view(np.int32)).cuda()
+    for _ in range(3):
+        np.testing.assert_array_equal(ctx.mis(dg, dpr).cpu().numpy(), ref)
+
+
 @pytest.mark.parametrize("prio", ["up", "down", "random", "equal"])
 @pytest.mark.parametrize("shape", ["path 700", "star 8", "star 9", "star 1024", "star 1025", "star 40000",
                                    "hubs 300", "loops", "m 255", "m 256", "m 257", "one vertex", "no edges"])
