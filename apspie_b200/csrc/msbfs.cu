@@ -399,17 +399,24 @@ __device__ __forceinline__ unsigned spread_nibbles(unsigned x) {
 // deeper than the planes' codes writes the rows when they are full and stores what it finds after
 // that at once: the few vertices of a level of such a graph cost less than another sweep over
 // all planes and rows (512 sources on a grid of 1,024 x 1,024: 677 ms with a sweep each 15 levels).
+// Words apart: 300 sources on 100,000 vertices in cliques of 100, whose 782 parts of 128 vertices left
+// most warps idle, 345 us, now 210; on 8 hubs and 100,000 leaves 458 and 292.
 template <int W>
 __device__ void write_depths(const MsArgs &a, long long mw) {
     const int lane = threadIdx.x & 31;
     const int warp = (blockIdx.x * kMsBlock + threadIdx.x) >> 5, nwarps = gridDim.x * kMsBlock / 32;
     const bool quads = (a.m & 3) == 0 && (a.rows || (reinterpret_cast<uintptr_t>(a.out) & 15u) == 0);
     const int step = quads ? 1 : 32;  // between a lane's vertices
-    for (int v0 = warp * 128; v0 < a.m; v0 += nwarps * 128) {
+    // where there are fewer such than warps, a warp takes a part of their words
+    const int chunks = (a.m - 1) / 128 + 1;
+    int parts = 1;
+    while (parts < W && static_cast<long long>(chunks) * parts < nwarps) parts *= 2;
+    for (long long x = warp; x < static_cast<long long>(chunks) * parts; x += nwarps) {
+        const int v0 = static_cast<int>(x / parts) * 128, w0 = static_cast<int>(x % parts) * (W / parts);
         const int v = v0 + (quads ? 4 * lane : lane);
         const int nv = v < a.m ? min(4, (a.m - 1 - v) / step + 1) : 0;
 #pragma unroll 1
-        for (int w = 0; w < W; ++w) {
+        for (int w = w0; w < w0 + W / parts; ++w) {
             unsigned p[kPlanes][4];
 #pragma unroll
             for (int k = 0; k < kPlanes; ++k) {
@@ -926,16 +933,18 @@ const void *msbfs_serve_fn() {
 }
 
 // Blocks of a batch, one to five an SM: more shorten a level's work, fewer its three barriers. By
-// the words that a visit of every entry reads; us with one / two / three / four an SM:
-// 0.04M (2 queries on R-MAT) 91 / 97 / 107 / 119, 0.3M (32 on a grid, 510 levels) 5,836 / 5,918 /
-// 6,596 / 7,426, 0.4M 118 / 130 / 138 / 149; 1.2M 121 / 120 / 125 / 140, 4.2M (512 on that grid)
-// 18,148 / 14,600 / 15,215, 7.3M 294 / 289 / 309 / 338; 15M 403 / 352 / 344 / 352; 24M 971 / 693 /
-// 586 / 560. Five fit for up to 64 queries: 1,400 instead of 1,457 at 2^27, 482 instead of 473 at
-// 2^25.
-long long msbfs_blocks(const apspie_ctx *ctx, long long nnz, int W) {
-    const long long w = nnz * W;
+// the words that a visit of every entry reads and, eight for each vertex, those of the first and
+// last sweeps; us with one / two / three / four an SM: 0.8M (32 queries on a grid, 510 levels) 5,836 /
+// 5,918 / 6,596 / 7,426, 1.1M (4 on one of 90,000) 9,076 / 9,606 / 10,262 / 11,409; 2.3M (4 on R-MAT of
+// 100,003) 192 / 185 / 176 / 202, 10M (4 on a tree of 2^20) 906 / 769 / 774 / 826, 12.6M (512 on a grid
+// of 65,536) 18,148 / 14,600 / 15,215; 16M (4 on 2^20 uniform) 753 / 505 / 446 / 432; 21M (64 on the
+// tree) 1,738 / 1,239 / 1,126 / 1,106, 32M (4 on R-MAT of 2^20) 1,135 / 777 / 639 / 635, 33M (64 on
+// uniform) 1,444 / 918 / 772 / 698. Five fit for up to 64 queries: 1,400 instead of 1,457 at 2^27, 482
+// instead of 473 at 2^25.
+long long msbfs_blocks(const apspie_ctx *ctx, long long m, long long nnz, int W) {
+    const long long w = (nnz + 8 * m) * W;
     if (nnz >= (1 << 26)) return kMaxGrid;
-    return static_cast<long long>(ctx->num_sms) * (w >= 20000000 ? 4 : w >= 10000000 ? 3 : w >= 1000000 ? 2 : 1);
+    return static_cast<long long>(ctx->num_sms) * (w >= 20000000 ? 4 : w >= 14000000 ? 3 : w >= 1500000 ? 2 : 1);
 }
 
 size_t batch_need(int m, int Wp) {  // without the depth planes of the batch
@@ -1036,7 +1045,7 @@ apspie_status bfs_batch_impl(apspie_ctx *ctx, const apspie_csr *A, const int32_t
         const void *fn = Wp == 1 ? msbfs_fn<1>() : Wp == 2 ? msbfs_fn<2>() : Wp == 4 ? msbfs_fn<4>()
                          : Wp == 8 ? msbfs_fn<8>() : msbfs_fn<16>();
         void *args[] = {&a};
-        st = launch_persistent(ctx, fn, kMsBlock, args, msbfs_blocks(ctx, A->nnz, Wp) * kWorkPerBlock);
+        st = launch_persistent(ctx, fn, kMsBlock, args, msbfs_blocks(ctx, A->m, A->nnz, Wp) * kWorkPerBlock);
         if (st != APSPIE_OK) return st;
         if (stats) {
             apspie_run_stats part;
