@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kTcBlock) tc_block(const int *__restrict__ row
 // shared-memory word instead of a probe chain in a hash set.
 //
 // Measured at scale 18: counting 2.74 ms with hash sets; 0.51 ms with bitmaps and tc_small (and
-// 0.13 ms for the partner lists), tc_bits at 64 % of the issue slots and 72 % of the L1/shared-memory
+// 0.13 ms for the partner lists), tc_bits at 71 % of the issue slots and 83 % of the L1/shared-memory
 // pipe.
 //
 // Needs: L strict lower triangular with strictly ascending rows (both found out on the way: a
